@@ -41,8 +41,9 @@ enum limn_b200_status {
 enum limn_b200_path {
   LIMN_B200_PATH_GENERAL = 0,  /* SIMT kernels: any float dtype, any hd/hd_v */
   LIMN_B200_PATH_TCGEN05 = 1,  /* TMA + tcgen05 kernels: f16/bf16, hd and hd_v multiples of 8 up to 128 (run as 64 or 128), any t_q/t_k, with or without key mask */
-  LIMN_B200_PATH_DECODE = 2    /* forward only: f16/bf16, hd == hd_v in {64, 128}, t_q <= 4 without a causal mask (the step of a
-                                  kv cache): one CTA streams a problem's keys and values once, bound by HBM, no tensor cores */
+  LIMN_B200_PATH_DECODE = 2    /* forward only, no causal mask (the step of a kv cache), hd and hd_v multiples of 8 up to 128,
+                                  dense or strided rows on 16-byte boundaries: t_q <= 4 in f16/bf16, t_q < 16 in float32. One CTA
+                                  or cluster streams a problem's keys and values once, bound by HBM, no tensor cores */
 };
 
 /* "sdpa": replaces emit_sdpa (limn/cuda_emit.py:921-965); oracle limn/sdpa.py:91-137.

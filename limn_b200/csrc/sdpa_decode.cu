@@ -1,14 +1,16 @@
-// "sdpa" forward for decode shapes: a handful of query rows (t_q <= 4) against a long run of keys, f16/bf16 with
-// hd == hd_v in {64, 128}, no causal mask (causal needs t_q == t_k), with or without a key mask. This is the step of a
-// kv cache: one new token reads every slot filled so far (the reference tests the shape at
+// "sdpa" forward for decode shapes: a handful of query rows against a long run of keys, no causal mask (causal needs
+// t_q == t_k), with or without a key mask, hd and hd_v multiples of 8 up to 128: t_q <= 4 in f16/bf16 (more rows go to
+// the tensor cores), t_q < 16 in float32 (in chunks of 4 rows, K and V of the later chunks from L2). This is the step of
+// a kv cache: one new token reads every slot filled so far (the reference tests the shape at
 // tests/test_attention.py:385-396 and serves it with the same one-thread-per-query-row kernel as everything else,
 // limn/cuda_emit.py:921-965, which leaves all but t_q threads of a block idle).
 //
 // The work is reading K and V once; the arithmetic is a few flops per byte, so tensor cores have nothing to add and
 // the 128-row MMA tile of the prefill kernel would spend 127 of its 128 rows on nothing. Here one CTA of 16 warps
-// owns one (batch, head) problem. D / 8 lanes share a key (each holds 8 of its elements as one 16-byte load), so a
-// warp instruction fetches 2 or 4 consecutive keys, 512 contiguous bytes; every group of lanes walks its own
-// subsequence of the keys, four at a time with all eight loads (K and V) issued before the first is used, and keeps an
+// owns one (batch, head) problem. D / 8 lanes share a key (each holds 8 of its elements, one 16-byte load in 16-bit
+// storage and two in float32), so a warp reads 2, 4 or 8 consecutive keys at a time; every group of lanes walks its own
+// subsequence of the keys, four at a time (two in float32: the same bytes in flight, and the same registers, which is
+// what keeps two CTAs on an SM) with all loads of K and V issued before the first is used, and keeps an
 // online softmax of its own per query row: a running maximum, a denominator and 8 accumulator elements per lane. The
 // groups of a warp are merged with shuffles, the 16 warps through shared memory, always in the same order, so two runs
 // give the same bits. A batch too small to fill the GPU with one CTA per problem gets a thread-block cluster of up
@@ -27,20 +29,29 @@ namespace {
 
 constexpr int kWarps = 16;
 constexpr int kThreads = kWarps * 32;
-constexpr int kUnroll = 4;  // keys a group of lanes has in flight
-constexpr int kMaxRows = 4;
+constexpr int kMaxRows = 4;          // query rows a CTA carries
+constexpr int kMaxRowsF32 = 15;      // float32 problems up to here come in chunks of kMaxRows
+enum Kind { kF16, kBF16, kF32 };     // storage of Q, K, V, the mask and O
+template <Kind kKind>
+struct Storage {
+  static constexpr int kBytes = kKind == kF32 ? 4 : 2;
+  static constexpr int kUnroll = kKind == kF32 ? 2 : 4;  // keys a group of lanes has in flight
+  static constexpr int kLoads = kKind == kF32 ? 2 : 1;   // 16-byte loads that hold a lane's 8 elements
+};
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct DecodeParams {
   const void* q;
   const void* k;
   const void* v;
-  const unsigned short* mask;  // (bh, t_k) flags in the storage dtype, 0 hides a key; null without a mask
+  const void* mask;  // (bh, t_k) flags in the storage dtype, 0 hides a key; null without a mask
   void* out;
   float* lse;
   int heads;  // problem p is (batch p / heads, head p % heads)
   Strides q_strides, k_strides, v_strides, o_strides;  // in elements
   int t_q, t_k;
+  int pieces, pieces_v;  // groups of 8 columns a row of Q and K, and of V and O, really has (<= D / 8)
+  int chunks;            // CTAs (or clusters) that share a problem's query rows: ceil(t_q / R)
   float scale;
   int split;  // CTAs per problem (the cluster size): 1, 2, 4 or 8
 };
@@ -62,18 +73,39 @@ __device__ __forceinline__ float peer_shared(const float* mine, unsigned rank) {
   return v;
 }
 
-template <bool kFp16>
-__device__ __forceinline__ void widen8(const uint4& raw, float (&f)[8]) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+template <Kind kKind>
+struct Raw8 {  // a lane's 8 elements as loaded
+  uint4 part[Storage<kKind>::kLoads];
+};
+template <Kind kKind>
+__device__ __forceinline__ Raw8<kKind> load8(const unsigned char* at) {
+  Raw8<kKind> raw;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (kFp16) {
-      const float2 pair = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-      f[2 * i] = pair.x, f[2 * i + 1] = pair.y;
-    } else {
-      f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  for (int i = 0; i < Storage<kKind>::kLoads; ++i) raw.part[i] = reinterpret_cast<const uint4*>(at)[i];
+  return raw;
+}
+template <Kind kKind>
+__device__ __forceinline__ void widen8(const Raw8<kKind>& raw, float (&f)[8]) {
+#pragma unroll
+  for (int p = 0; p < Storage<kKind>::kLoads; ++p) {
+    const uint32_t w[4] = {raw.part[p].x, raw.part[p].y, raw.part[p].z, raw.part[p].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (kKind == kF32) {
+        f[4 * p + i] = __uint_as_float(w[i]);
+      } else if (kKind == kF16) {
+        const float2 pair = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[2 * i] = pair.x, f[2 * i + 1] = pair.y;
+      } else {
+        f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      }
     }
   }
+}
+template <Kind kKind>
+__device__ __forceinline__ bool key_visible(const void* flags, int key) {
+  if (kKind == kF32) return (static_cast<const uint32_t*>(flags)[key] & 0x7fffffffu) != 0;
+  return (static_cast<const unsigned short*>(flags)[key] & 0x7fffu) != 0;
 }
 
 // Fold the running softmax (m_b, l_b, acc_b) into (m_a, l_a, acc_a). Scores are in raw units; sl2 = scale * log2 e.
@@ -90,10 +122,11 @@ __device__ __forceinline__ void merge(float& m_a, float& l_a, float (&acc_a)[8],
 
 // Two CTAs per SM where the registers allow it (one or two query rows), so that every problem of a batch of a few
 // hundred is resident at once and the problems share HBM instead of queueing for SMs.
-template <int D, bool kFp16, bool kMask, int R>
+template <int D, Kind kKind, bool kMask, int R>
 __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(const DecodeParams prm) {
-  constexpr int kLanesPerKey = D / 8;           // 16 or 8
-  constexpr int kGroups = 32 / kLanesPerKey;    // keys per warp instruction: 2 or 4
+  constexpr int kLanesPerKey = D / 8;           // 16, 8 or 4
+  constexpr int kGroups = 32 / kLanesPerKey;    // keys a warp reads side by side: 2, 4 or 8
+  constexpr int kBytes = Storage<kKind>::kBytes, kUnroll = Storage<kKind>::kUnroll;
   __shared__ float part_m[kWarps][R], part_l[kWarps][R];
   __shared__ float part_acc[kWarps][R][D];
   __shared__ float cta_m[R], cta_l[R], cta_o[R][D];  // this CTA's share of the problem, for the cluster's CTA 0
@@ -102,22 +135,32 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   const int group = lane / kLanesPerKey, gl = lane % kLanesPerKey;
   const int split = prm.split;
   const unsigned rank = split > 1 ? cluster_rank() : 0u;
-  const int problem = blockIdx.x / split;
+  const int unit = blockIdx.x / split;  // chunks of a problem are neighbours: they read its keys out of L2 together
+  const int problem = unit / prm.chunks;
+  const int row0 = (unit - problem * prm.chunks) * R;
   const int batch = problem / prm.heads, head = problem - batch * prm.heads;
   const float sl2 = prm.scale * kLog2e;
 
-  const unsigned char* q_base = static_cast<const unsigned char*>(prm.q) + (batch * prm.q_strides.batch + head * prm.q_strides.head) * 2;
-  const unsigned char* k_base = static_cast<const unsigned char*>(prm.k) + (batch * prm.k_strides.batch + head * prm.k_strides.head) * 2;
-  const unsigned char* v_base = static_cast<const unsigned char*>(prm.v) + (batch * prm.v_strides.batch + head * prm.v_strides.head) * 2;
-  const long long k_row = prm.k_strides.row * 2, v_row = prm.v_strides.row * 2;  // bytes between keys
-  const unsigned short* flags = kMask ? prm.mask + static_cast<long long>(problem) * prm.t_k : nullptr;
+  const unsigned char* q_base = static_cast<const unsigned char*>(prm.q) + (batch * prm.q_strides.batch + head * prm.q_strides.head) * kBytes;
+  const unsigned char* k_base = static_cast<const unsigned char*>(prm.k) + (batch * prm.k_strides.batch + head * prm.k_strides.head) * kBytes;
+  const unsigned char* v_base = static_cast<const unsigned char*>(prm.v) + (batch * prm.v_strides.batch + head * prm.v_strides.head) * kBytes;
+  const long long k_row = prm.k_strides.row * kBytes, v_row = prm.v_strides.row * kBytes;  // bytes between keys
+  const void* flags = kMask ? static_cast<const unsigned char*>(prm.mask) + static_cast<long long>(problem) * prm.t_k * kBytes : nullptr;
+  // Lanes beyond a row's columns (a head narrower than D) read the row's first piece again: their q is zero, and what
+  // they gather of V is never stored.
+  const bool real = gl < prm.pieces;
+  const int k_at = (real ? gl : 0) * 8 * kBytes, v_at = (gl < prm.pieces_v ? gl : 0) * 8 * kBytes;
 
   // this lane's 8 elements of every query row
   float q[R][8];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(q_base + (static_cast<long long>(r) * prm.q_strides.row + gl * 8) * 2);
-    widen8<kFp16>(raw, q[r]);
+    const long long row = min(row0 + r, prm.t_q - 1);  // a last chunk's missing rows repeat the last one and are not stored
+    widen8<kKind>(load8<kKind>(q_base + row * prm.q_strides.row * kBytes + k_at), q[r]);
+    if (!real) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q[r][i] = 0.f;
+    }
   }
 
   float m[R], l[R], acc[R][8];
@@ -131,26 +174,26 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   // keys are dealt out so that the groups of a warp, and the warps of the CTA, read consecutive keys together
   constexpr int kPerPass = kWarps * kUnroll * kGroups;
   for (int first = rank * kPerPass; first < prm.t_k; first += split * kPerPass) {
-    uint4 k_raw[kUnroll], v_raw[kUnroll];
+    Raw8<kKind> k_raw[kUnroll], v_raw[kUnroll];
     int key[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       key[u] = first + (u * kWarps + warp) * kGroups + group;
       const int at = min(key[u], prm.t_k - 1);  // past the end: read the last key again, its score is discarded below
-      k_raw[u] = *reinterpret_cast<const uint4*>(k_base + at * k_row + gl * 16);
+      k_raw[u] = load8<kKind>(k_base + at * k_row + k_at);
     }
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const int at = min(key[u], prm.t_k - 1);
-      v_raw[u] = *reinterpret_cast<const uint4*>(v_base + at * v_row + gl * 16);
+      v_raw[u] = load8<kKind>(v_base + at * v_row + v_at);
     }
     float s[R][kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       float kf[8];
-      widen8<kFp16>(k_raw[u], kf);
+      widen8<kKind>(k_raw[u], kf);
       bool visible = key[u] < prm.t_k;
-      if (kMask && visible) visible = (flags[key[u]] & 0x7fffu) != 0;
+      if (kMask && visible) visible = key_visible<kKind>(flags, key[u]);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         float dot = 0.f;
@@ -182,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         float vf[8];
-        widen8<kFp16>(v_raw[u], vf);
+        widen8<kKind>(v_raw[u], vf);
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(p[u], vf[i], acc[r][i]);
       }
@@ -251,59 +294,84 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
         o = o * fa + o_c * fc;
         m_tot = m_new;
       }
+      const int row = row0 + r;
+      if (row >= prm.t_q) continue;
       const float value = o / l_tot;  // 0 / 0 = NaN for a row with no visible key, as the oracle gives
       unsigned char* dst = static_cast<unsigned char*>(prm.out) +
-                           (batch * prm.o_strides.batch + head * prm.o_strides.head + static_cast<long long>(r) * prm.o_strides.row + d) * 2;
-      if (kFp16) *reinterpret_cast<__half*>(dst) = __float2half_rn(value);
-      else *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(value);
-      if (d == 0) prm.lse[static_cast<long long>(problem) * prm.t_q + r] = m_tot * prm.scale + logf(l_tot);
+                           (batch * prm.o_strides.batch + head * prm.o_strides.head + static_cast<long long>(row) * prm.o_strides.row + d) * kBytes;
+      if (d < prm.pieces_v * 8) {
+        if (kKind == kF32) *reinterpret_cast<float*>(dst) = value;
+        else if (kKind == kF16) *reinterpret_cast<__half*>(dst) = __float2half_rn(value);
+        else *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(value);
+      }
+      if (d == 0) prm.lse[static_cast<long long>(problem) * prm.t_q + row] = m_tot * prm.scale + logf(l_tot);
     }
   }
   if (split > 1) cluster_sync();  // no CTA leaves while CTA 0 may still be reading its shared memory
 }
 
-template <int D, bool kFp16, bool kMask, int R>
-int launch_one(const Problem& p, const DecodeParams& prm) {
+template <int D, Kind kKind, bool kMask, int R>
+int launch_one(const Problem& p, DecodeParams& prm) {
+  prm.chunks = (p.t_q + R - 1) / R;
+  // One CTA per problem fills the GPU from a few hundred problems on (two CTAs fit an SM). Below that, 2, 4 or 8
+  // CTAs share a problem, as long as each still has a full pass of keys (16 warps x the keys a warp has in flight).
+  int sms = 0;
+  if (int rc = sm_count(&sms)) return rc;
+  constexpr int per_pass = kWarps * Storage<kKind>::kUnroll * (32 / (D / 8));
+  const long long units = p.bh * prm.chunks;
+  int split = 1;
+  while (split < 8 && units * split * 2 <= 2LL * sms && (p.t_k + per_pass - 1) / per_pass >= split * 2) split *= 2;
+  prm.split = split;
+  if (units * split > 0x7fffffffLL) return fail(LIMN_B200_UNSUPPORTED, "sdpa: %lld problems need more blocks than one grid holds", p.bh);
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(static_cast<unsigned>(p.bh * prm.split));
+  config.gridDim = dim3(static_cast<unsigned>(units * split));
   config.blockDim = dim3(kThreads);
   config.stream = p.stream;
   cudaLaunchAttribute attribute[1];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = static_cast<unsigned>(prm.split);
+  attribute[0].val.clusterDim.x = static_cast<unsigned>(split);
   attribute[0].val.clusterDim.y = 1;
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  LIMN_CUDA(cudaLaunchKernelEx(&config, sdpa_decode_kernel<D, kFp16, kMask, R>, prm), "launching the sdpa decode kernel");
+  const DecodeParams& as_launched = prm;
+  LIMN_CUDA(cudaLaunchKernelEx(&config, sdpa_decode_kernel<D, kKind, kMask, R>, as_launched), "launching the sdpa decode kernel");
   note_launches(1);
   return LIMN_B200_OK;
 }
 
-template <int D, bool kFp16, bool kMask>
-int launch_rows(const Problem& p, const DecodeParams& prm) {
+template <int D, Kind kKind, bool kMask>
+int launch_rows(const Problem& p, DecodeParams& prm) {
   switch (p.t_q) {
-    case 1: return launch_one<D, kFp16, kMask, 1>(p, prm);
-    case 2: return launch_one<D, kFp16, kMask, 2>(p, prm);
-    case 3: return launch_one<D, kFp16, kMask, 3>(p, prm);
-    default: return launch_one<D, kFp16, kMask, 4>(p, prm);
+    case 1: return launch_one<D, kKind, kMask, 1>(p, prm);
+    case 2: return launch_one<D, kKind, kMask, 2>(p, prm);
+    case 3: return launch_one<D, kKind, kMask, 3>(p, prm);
+    default: return launch_one<D, kKind, kMask, 4>(p, prm);
   }
 }
 
+template <int D, Kind kKind>
+int launch_kind(const Problem& p, DecodeParams& prm) {
+  return p.mask ? launch_rows<D, kKind, true>(p, prm) : launch_rows<D, kKind, false>(p, prm);
+}
+
 template <int D>
-int launch_d(const Problem& p, const DecodeParams& prm) {
-  const bool fp16 = p.dtype == LIMN_B200_F16;
-  if (p.mask) return fp16 ? launch_rows<D, true, true>(p, prm) : launch_rows<D, false, true>(p, prm);
-  return fp16 ? launch_rows<D, true, false>(p, prm) : launch_rows<D, false, false>(p, prm);
+int launch_d(const Problem& p, DecodeParams& prm) {
+  switch (p.dtype) {
+    case LIMN_B200_F16: return launch_kind<D, kF16>(p, prm);
+    case LIMN_B200_BF16: return launch_kind<D, kBF16>(p, prm);
+    default: return launch_kind<D, kF32>(p, prm);
+  }
 }
 
 }  // namespace
 
 bool decode_serves(Op op, const Problem& p) {
-  if (op != Op::Fwd) return false;
-  if (p.dtype != LIMN_B200_BF16 && p.dtype != LIMN_B200_F16) return false;
-  if (p.hd != p.hd_v || (p.hd != 64 && p.hd != 128)) return false;
-  if (p.t_q > kMaxRows || p.causal) return false;  // (causal needs t_q == t_k: a prefill shape, however short)
+  if (op != Op::Fwd || p.causal) return false;  // (causal needs t_q == t_k: a prefill shape, however short)
+  if (p.dtype == LIMN_B200_F64) return false;
+  if (p.hd > 128 || p.hd % 8 != 0 || p.hd_v > 128 || p.hd_v % 8 != 0) return false;
+  if (p.t_q > (p.dtype == LIMN_B200_F32 ? kMaxRowsF32 : kMaxRows)) return false;
+  if (p.dtype == LIMN_B200_F32 && (p.strided || p.layout != LIMN_B200_BHTD)) return false;  // dense only in float32
   if (!(p.scale > 0.0) || p.bh > 0x7fffffffLL) return false;
   // 16-byte loads: aligned bases (a null pointer is refused before this is asked in earnest)
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v);
@@ -313,29 +381,24 @@ bool decode_serves(Op op, const Problem& p) {
 int decode_launch(const Problem& p) {
   DecodeParams prm;
   prm.q = p.q, prm.k = p.k, prm.v = p.v;
-  prm.mask = static_cast<const unsigned short*>(p.mask);
+  prm.mask = p.mask;
   prm.out = p.out, prm.lse = static_cast<float*>(p.lse_out);
   prm.heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh);
   prm.q_strides = operand_strides(p, kOpQ, prm.heads, p.t_q, p.hd);
   prm.k_strides = operand_strides(p, kOpK, prm.heads, p.t_k, p.hd);
-  prm.v_strides = operand_strides(p, kOpV, prm.heads, p.t_k, p.hd);
-  prm.o_strides = operand_strides(p, kOpOut, prm.heads, p.t_q, p.hd);
+  prm.v_strides = operand_strides(p, kOpV, prm.heads, p.t_k, p.hd_v);
+  prm.o_strides = operand_strides(p, kOpOut, prm.heads, p.t_q, p.hd_v);
   {
     const long long all = prm.q_strides.batch | prm.q_strides.head | prm.q_strides.row | prm.k_strides.batch | prm.k_strides.head |
                           prm.k_strides.row | prm.v_strides.batch | prm.v_strides.head | prm.v_strides.row;
     if (all & 7) return fail(LIMN_B200_BAD_ARGUMENT, "sdpa: operand strides must be multiples of 8 elements");
   }
   prm.t_q = p.t_q, prm.t_k = p.t_k;
+  prm.pieces = p.hd / 8, prm.pieces_v = p.hd_v / 8;
   prm.scale = static_cast<float>(p.scale);
-  // One CTA per problem fills the GPU from a few hundred problems on (two CTAs fit an SM). Below that, 2, 4 or 8
-  // CTAs share a problem, as long as each still has a full pass of keys (16 warps x 4 in flight x keys per warp load).
-  int sms = 0;
-  if (int rc = sm_count(&sms)) return rc;
-  const int per_pass = kWarps * kUnroll * (32 / (p.hd / 8));
-  int split = 1;
-  while (split < 8 && p.bh * split * 2 <= 2LL * sms && (p.t_k + per_pass - 1) / per_pass >= split * 2) split *= 2;
-  prm.split = split;
-  return p.hd == 128 ? launch_d<128>(p, prm) : launch_d<64>(p, prm);
+  const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
+  if (widest <= 32) return launch_d<32>(p, prm);
+  return widest <= 64 ? launch_d<64>(p, prm) : launch_d<128>(p, prm);
 }
 
 }  // namespace limn_b200

@@ -429,6 +429,45 @@ def test_decode_shapes_on_the_streaming_kernel(case):
         np.testing.assert_array_equal(np.ascontiguousarray(a).view(np.uint8), np.ascontiguousarray(b).view(np.uint8))
 
 
+NARROW_OR_FLOAT32_DECODE_CASES = [
+    # id, dtype, bh, t_q, t_k, hd, hd_v, key mask kind
+    ("f32 d64 one row ragged 1999, padded cache", np.float32, 8, 1, 1999, 64, 64, "pad"),
+    ("f32 d128 four rows, one key", np.float32, 3, 4, 1, 128, 128, None),
+    ("f32 d32 one row, 400 problems (one CTA each)", np.float32, 400, 1, 129, 32, 32, None),
+    ("f32 hd 24 hd_v 104, five rows (a second chunk of one)", np.float32, 5, 5, 300, 24, 104, "holes"),
+    ("f32 d8 fifteen rows (four chunks)", np.float32, 70, 15, 70, 8, 8, None),
+    ("bf16 hd 96 hd_v 40 two rows", BF16, 6, 2, 515, 96, 40, "holes"),
+    ("f16 d16 three rows, 257 keys", np.float16, 9, 3, 257, 16, 16, None),
+]
+
+
+@pytest.mark.parametrize("case", NARROW_OR_FLOAT32_DECODE_CASES, ids=[c[0] for c in NARROW_OR_FLOAT32_DECODE_CASES])
+def test_decode_shapes_in_float32_and_at_every_width(case, dev):
+    """The streaming kernel with float32 storage (t_q < 16, in chunks of four rows) and with heads narrower than the
+    lanes that share a key: edges of chunks, of the key walk and of the cluster split, against the oracle, twice for
+    the bits."""
+    import limn_standin as host
+    from limn_b200._lib import PATH_DECODE, lib
+
+    _, dtype, bh, t_q, t_k, hd, hd_v, kind = case
+    name = "bfloat16" if dtype == BF16 else np.dtype(dtype).name
+    code = {"float32": 0, "float16": 1, "bfloat16": 2}[name]
+    assert lib().limn_b200_sdpa_path(code, bh, t_q, t_k, hd, hd_v, 0, int(kind is not None), hd**-0.5) == PATH_DECODE
+    q, k, v, _ = _random_case(700 + t_k, dtype, (bh, t_q, hd), (bh, t_k, hd), (bh, t_k, hd_v))
+    mask = None
+    if kind == "pad":
+        mask = np.broadcast_to(np.arange(t_k) < t_k * 3 // 4, (bh, t_k)).astype(dtype)
+    elif kind == "holes":
+        mask = (np.random.default_rng(t_k).random((bh, t_k)) > 0.4).astype(dtype)
+        mask[-1] = 0  # the last problem sees no key at all: NaN rows, L = -inf
+    runs = [host.Attention(dev, q, k, v, key_mask=mask).forward() for _ in range(2)]
+    want_out, want_lse = oracle.sdpa_forward(q, k, v, mask, causal=False, scale=hd**-0.5)
+    close(runs[0][0], want_out, FWD_TOL[name], "O")
+    close(runs[0][1], want_lse, LSE_TOL, "L")
+    for a, b in zip(*runs, strict=True):
+        np.testing.assert_array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
 def test_two_runs_give_the_same_bits(dev):
     import limn_standin as host
 
