@@ -229,9 +229,10 @@ int dispatch_op(Op op, const char* name, const Problem& p) {
     return tcgen05_launch(op, p);
   }
   if (op == Op::BwdQ && p.fuse_delta) {
-    // the general kernels read delta: fill it first, as the unfused sequence would
+    // the float32 and the general kernels read delta: fill it first, as the unfused sequence would
     if (int rc = general_delta(p.out, p.dout, const_cast<void*>(p.delta), p.dtype, p.bh * p.t_q, p.hd_v, p.stream)) return rc;
   }
+  if (f32_split_serves(op, p)) return f32_split_launch(op, p);
   return general_launch(op, p);
 }
 

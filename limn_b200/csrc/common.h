@@ -119,10 +119,13 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
 
 // Kernel families. Each returns a status code and enqueues on p.stream.
 int general_launch(Op op, const Problem& p);
-// The tiled members of the general family (float32/float16/bfloat16, head dims up to 256, sides of 16 rows and
-// more); general_launch hands them what they serve and keeps the rest for the one-row-per-warp kernels.
+// The CUDA-core tiled members of the general family (float32/float16/bfloat16, head dims up to 256, sides of 16 rows
+// and more); general_launch hands them what they serve and keeps the rest for the one-row-per-warp kernels.
 bool general_tiled_serves(Op op, const Problem& p);
 int general_tiled_launch(Op op, const Problem& p);
+// float32 with head dims up to 128 on the tensor cores, each operand split into three bfloat16 pieces.
+bool f32_split_serves(Op op, const Problem& p);
+int f32_split_launch(Op op, const Problem& p);
 int general_delta(const void* out, const void* dout, void* delta, int dtype, long long rows, int hd_v,
                   cudaStream_t stream);
 int general_delta_bthd(const void* out, const void* dout, void* delta, int dtype, int batch, int heads, int t, int hd_v,

@@ -1,0 +1,864 @@
+// float32 attention on the tensor cores: head dims up to 128, optional key mask, rectangular t_q x t_k.
+//
+// float32 has to keep its own width (the reference checks it at 1e-5: tests/test_attention.py:250-255), and the tensor
+// cores multiply 8-bit significands in bfloat16. Three of those hold a float32: x = h + m + l, each the bfloat16
+// nearest to what the ones before left, 8 + 8 + 8 bits and two signs. A product of two float32 matrices is then the
+// sum of six bfloat16 products, h h + (h m + m h) + (m m + h l + l h); what is left out (m l, l m, l l) is 2^-26 of it,
+// less than float32's own rounding. The accumulator adds in float32 but truncates, so the six are issued smallest
+// first, and no total stays in tensor memory for longer than one tile: every tile's product starts from zero and is
+// added to the row's total in registers, rounded to nearest, as the CUDA-core kernels in sdpa_general_tiled.cu do.
+//
+// What bounds it: six bfloat16 products at 4096 multiply-adds a clock and SM are 683 float32 multiply-adds a clock,
+// against 128 on the CUDA cores. Measured on B200 (forward / dQ / dK and dV, us, causal; the CUDA-core kernels in
+// brackets): 256 x 256 keys x 64: 42 / 72 / 96 (121 / 166 / 219); 6 x 8192 x 32: 379 / 651 / 901 (1333 / 1777 / 2402);
+// 64 x 1024 x 128: 189 / 267 / 341 (813 / 1117 / 1714). Against float64 every result is as close as before or closer
+// (8192 keys x 32: O 1.6e-7 for 5.8e-7, dK 4.3e-7 for 2.2e-6 in the 2-norm). A block owns 128 rows (query rows in the forward and the dQ pass, key rows in the
+// dK/dV pass), one row to each tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
+// with ordinary loads (the split has to pass through registers anyway), split and left in shared memory in the
+// 128-byte-swizzled layout; probabilities and dS are split in registers and go to tensor memory as the A operand.
+//
+// A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
+// number (inf - inf in the split, inf * 0 between pieces). The split notices (its remainder is NaN), and a block that
+// met one computes its rows again, one row per warp, in plain float32.
+#include <cmath>
+#include <cstdint>
+
+#include "common.h"
+#include "sm100_ptx.cuh"
+
+namespace limn_b200 {
+namespace {
+
+using namespace ptx;
+
+constexpr int kRows = 128;    // rows a block owns
+constexpr int kStream = 64;   // rows of a streamed tile
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kPieceCols = kStream / 2;  // tensor-memory columns of one 16-bit piece of a (kRows x kStream) matrix
+
+struct Params {
+  const float *q, *k, *v, *mask, *dout, *lse_in, *delta;
+  float *out, *lse_out, *dq, *dk, *dv;
+  unsigned* status;
+  long long bh;
+  int slots, group;  // row tiles per problem; problems scheduled side by side
+  int t_q, t_k, hd, hd_v, causal;
+  float scale, c_hi, c_lo;  // c_hi + c_lo = scale * log2(e), c_lo > 0
+  bool wide_qk, wide_v, wide_out;  // 16-byte accesses are safe for (q, k), for (v, dO) and for the results
+};
+
+// ---- x = h + m + l for two floats at a time; `check` becomes NaN when one of them is not finite ----
+__device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, uint64_t& check) {
+  const uint64_t minus = f2_pack(-1.f, -1.f);
+  float a, b;
+  f2_unpack(x, a, b);
+  h = pack_bf16(a, b);
+  x = f2_fma(f2_pack_bits(h << 16, h & 0xffff0000u), minus, x);  // exact
+  f2_unpack(x, a, b);
+  m = pack_bf16(a, b);
+  x = f2_fma(f2_pack_bits(m << 16, m & 0xffff0000u), minus, x);  // exact
+  f2_unpack(x, a, b);
+  l = pack_bf16(a, b);
+  check = f2_fma(x, 0ull, check);
+}
+__device__ __forceinline__ bool is_bad(uint64_t check) {
+  float a, b;
+  f2_unpack(check, a, b);
+  return !(a == 0.f && b == 0.f);
+}
+
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[N]) {
+  if constexpr (N == 32) tmem_ld32(addr, r);
+  else if constexpr (N == 16) tmem_ld16(addr, r);
+  else tmem_ld8(addr, r);
+}
+template <int N>
+__device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&r)[N]) {
+  if constexpr (N == 16) tmem_st16(addr, r);
+  else tmem_st8(addr, r);
+}
+
+// Eight consecutive floats of row `row`, zero beyond the matrix.
+__device__ __forceinline__ void load8(float (&x)[8], const float* src, int row, int rows, int col, int width, bool wide) {
+  const float* at = src + static_cast<long long>(row) * width + col;
+  if (wide) {  // the width is a multiple of 4 and the base 16-byte aligned
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 a = row < rows && col < width ? *reinterpret_cast<const float4*>(at) : none;
+    const float4 b = row < rows && col + 4 < width ? reinterpret_cast<const float4*>(at)[1] : none;
+    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = row < rows && col + i < width ? at[i] : 0.f;
+  }
+}
+
+// Rows [first, first + R) of a (rows, width) matrix into three bfloat16 pieces in shared memory: piece p, column block a
+// of 64 at dst + (p * kAtoms + a) * R * 128, 128-byte rows, 128-byte swizzle.
+template <int HD, int R, int kThreads>
+struct Stage {
+  static constexpr int kAtoms = HD > 64 ? 2 : 1;
+  static constexpr int kChunks = HD / 8;
+  static constexpr int kTurns = R * kChunks / kThreads;
+  static constexpr uint32_t kPiece = kAtoms * R * 128;
+  static constexpr uint32_t kBytes = 3 * kPiece;
+  static_assert(R * kChunks % kThreads == 0 || R * kChunks < kThreads, "whole turns");
+  static constexpr int kLoops = kTurns > 0 ? kTurns : 1;
+
+  float x[kLoops][8];
+
+  __device__ __forceinline__ void load(const float* src, int first, int rows, int width, bool wide) {
+#pragma unroll
+    for (int n = 0; n < kLoops; ++n) {
+      const int e = threadIdx.x + n * kThreads;
+      if (kTurns == 0 && e >= R * kChunks) break;
+      load8(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width, wide);
+    }
+  }
+  __device__ __forceinline__ void store(uint32_t dst, uint64_t& check) {
+#pragma unroll
+    for (int n = 0; n < kLoops; ++n) {
+      const int e = threadIdx.x + n * kThreads;
+      if (kTurns == 0 && e >= R * kChunks) break;
+      const int r = e / kChunks, chunk = e % kChunks;
+      uint32_t h[4], m[4], l[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split_pair(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
+      const uint32_t at = swizzled_piece(dst + (chunk / 8) * R * 128, r, chunk % 8);
+      st_shared_v4(at, h[0], h[1], h[2], h[3]);
+      st_shared_v4(at + kPiece, m[0], m[1], m[2], m[3]);
+      st_shared_v4(at + 2 * kPiece, l[0], l[1], l[2], l[3]);
+    }
+  }
+};
+
+// The six products in the order they are added, smallest first.
+__device__ __forceinline__ int piece_a(int i) { return (0x001102 >> (4 * i)) & 0xf; }  // l h m m h h
+__device__ __forceinline__ int piece_b(int i) { return (0x010120 >> (4 * i)) & 0xf; }  // h l m h m h
+
+__device__ __forceinline__ uint64_t tile_desc(uint32_t lo) { return (static_cast<uint64_t>(kDescHiSw128) << 32) | lo; }
+
+// D (kRows x kStream) = A (kRows x 16 steps) B^T (kStream x 16 steps), both with the contraction dim contiguous. A lies
+// in shared memory (a0 its address) or in tensor memory (a0 its column, pieces kTmemPiece columns apart).
+template <int HD, bool kTmemA>
+__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0, int steps) {
+  constexpr uint32_t kPieceA = (HD > 64 ? 2 : 1) * kRows * 128, kPieceB = (HD > 64 ? 2 : 1) * kStream * 128;
+  constexpr uint32_t idesc = mma_idesc(kRows, kStream, false, false, false);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    const uint32_t b_lo = desc_lo(b0 + piece_b(i) * kPieceB, 0);
+    const uint32_t a_lo = kTmemA ? a0 + piece_a(i) * (HD / 2) : desc_lo(a0 + piece_a(i) * kPieceA, 0);
+    for (int s = 0; s < steps; ++s) {
+      const uint32_t within = (s & 3) * 2, block = s >> 2;
+      const uint32_t b = b_lo + within + block * (kStream * 128 / 16);
+      if constexpr (kTmemA) mma_ts_lo(d, a_lo + s * 8, b, idesc, i > 0 || s > 0);
+      else mma_ss(d, tile_desc(a_lo + within + block * (kRows * 128 / 16)), tile_desc(b), idesc, i > 0 || s > 0);
+    }
+  }
+}
+
+// D (kRows x HD) = W (kRows x kStream, pieces in tensor memory) X (kStream x HD, rows streamed).
+template <int HD>
+__device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0) {
+  constexpr uint32_t kPiece = (HD > 64 ? 2 : 1) * kStream * 128;
+  constexpr uint32_t idesc = mma_idesc(kRows, HD, false, false, true);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    const uint32_t x_lo = desc_lo(x0 + piece_b(i) * kPiece, kStream * 128);
+    const uint32_t w = w0 + piece_a(i) * kPieceCols;
+#pragma unroll
+    for (int s = 0; s < kStream / 16; ++s) mma_ts_lo(d, w + s * 8, x_lo + s * (16 * 128 / 16), idesc, i > 0 || s > 0);
+  }
+}
+
+// N numbers of one row, split, to tensor memory at `at` (pieces kPieceCols columns apart).
+template <int N>
+__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], uint64_t& check) {
+  uint32_t h[N / 2], m[N / 2], l[N / 2];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) split_pair(w[i], h[i], m[i], l[i], check);
+  tmem_st<N / 2>(at, h);
+  tmem_st<N / 2>(at + kPieceCols, m);
+  tmem_st<N / 2>(at + 2 * kPieceCols, l);
+}
+
+template <int N>
+__device__ __forceinline__ void store_row(float* row, const uint64_t (&acc)[N / 2], int first, int width, bool wide) {
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    float x[4];
+    f2_unpack(acc[i / 2], x[0], x[1]);
+    f2_unpack(acc[i / 2 + 1], x[2], x[3]);
+    if (wide) {
+      if (first + i < width) *reinterpret_cast<float4*>(row + first + i) = make_float4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (first + i + c < width) row[first + i + c] = x[c];
+    }
+  }
+}
+
+__device__ __forceinline__ float warp_sum(float x) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
+  return x;
+}
+
+// ---- the rows of a block that met a non-finite operand, one row per warp. Keys (queries) are walked in the 64-row
+// tiles the row's own tile would see, weight 0 on those it does not, so a hidden infinity gives NaN as it does in the
+// products. ----
+struct Row {
+  float x[4];
+  __device__ __forceinline__ void load(const float* src, int width) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int d = (threadIdx.x & 31) + 32 * c;
+      x[c] = d < width ? src[d] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void zero() { x[0] = x[1] = x[2] = x[3] = 0.f; }
+  __device__ __forceinline__ float dot(const Row& y) const {
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s = fmaf(x[c], y.x[c], s);
+    return warp_sum(s);
+  }
+  __device__ __forceinline__ void add(float w, const Row& y, int width) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if ((threadIdx.x & 31) + 32 * c < width) x[c] = fmaf(w, y.x[c], x[c]);
+  }
+  __device__ __forceinline__ void store(float* dst, int width, float over) const {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int d = (threadIdx.x & 31) + 32 * c;
+      if (d < width) dst[d] = x[c] / over;
+    }
+  }
+};
+
+__device__ __noinline__ void plain_fwd(const Params& g, long long b, int i0, int threads) {
+  for (int i = i0 + (threadIdx.x >> 5); i < min(i0 + kRows, g.t_q); i += threads >> 5) {
+    Row q, k, v, acc;
+    q.load(g.q + (b * g.t_q + i) * g.hd, g.hd);
+    acc.zero();
+    float top = -INFINITY, denom = 0.f;
+    const int end = g.causal ? min(g.t_k, (i / kStream + 1) * kStream) : g.t_k;
+    for (int j = 0; j < end; ++j) {
+      k.load(g.k + (b * g.t_k + j) * g.hd, g.hd);
+      v.load(g.v + (b * g.t_k + j) * g.hd_v, g.hd_v);
+      const bool seen = (!g.causal || j <= i) && (!g.mask || g.mask[b * g.t_k + j] != 0.f);
+      const float s = q.dot(k) * g.scale;
+      float p = 0.f;
+      if (seen) {
+        const float raised = fmaxf(top, s);
+        if (raised == -INFINITY) {
+          p = isnan(s) ? s : 0.f;
+        } else {
+          const float shrink = expf(top - raised);
+          denom *= shrink;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc.x[c] *= shrink;
+          p = expf(s - raised);
+          top = raised;
+        }
+      }
+      denom += p;
+      acc.add(p, v, g.hd_v);
+    }
+    acc.store(g.out + (b * g.t_q + i) * g.hd_v, g.hd_v, denom);
+    if ((threadIdx.x & 31) == 0) g.lse_out[b * g.t_q + i] = top + logf(denom);
+  }
+}
+
+template <bool kKV>
+__device__ __noinline__ void plain_bwd(const Params& g, long long b, int first, int threads) {
+  const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
+  for (int r = first + (threadIdx.x >> 5); r < min(first + kRows, owned); r += threads >> 5) {
+    Row q, k, v, dout, acc0, acc1;
+    acc0.zero();
+    acc1.zero();
+    const int from = kKV && g.causal ? r / kStream * kStream : 0;
+    const int end = !kKV && g.causal ? min(streamed, (r / kStream + 1) * kStream) : streamed;
+    for (int x = from; x < end; ++x) {
+      const long long i = b * g.t_q + (kKV ? x : r), j = b * g.t_k + (kKV ? r : x);
+      q.load(g.q + i * g.hd, g.hd);
+      dout.load(g.dout + i * g.hd_v, g.hd_v);
+      k.load(g.k + j * g.hd, g.hd);
+      v.load(g.v + j * g.hd_v, g.hd_v);
+      const bool seen = (!g.causal || (kKV ? r <= x : x <= r)) && (!g.mask || g.mask[j] != 0.f);
+      const float s = q.dot(k), dp = dout.dot(v);
+      const float p = seen ? expf(s * g.scale - g.lse_in[i]) : 0.f;
+      const float ds = seen ? p * (dp - g.delta[i]) * g.scale : 0.f;
+      if (kKV) {
+        acc0.add(p, dout, g.hd_v);
+        acc1.add(ds, q, g.hd);
+      } else {
+        acc0.add(ds, k, g.hd);
+      }
+    }
+    if (kKV) {
+      acc0.store(g.dv + (b * g.t_k + r) * g.hd_v, g.hd_v, 1.f);
+      acc1.store(g.dk + (b * g.t_k + r) * g.hd, g.hd, 1.f);
+    } else {
+      acc0.store(g.dq + (b * g.t_q + r) * g.hd, g.hd, 1.f);
+    }
+  }
+}
+
+// ---- block set-up and teardown shared by the kernels ----
+// False: an earlier kernel on this device gave up on a wait, take no work.
+template <int kCols, int kBars>
+__device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t* abort_flag, uint64_t* bars, uint32_t& tmem) {
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < kBars; ++i) mbar_init(smem_addr(bars + i), 1);
+    mbar_init_fence();
+  }
+  grid_dependency_wait();
+  if (threadIdx.x == 0) *abort_flag = *reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk;
+  __syncthreads();
+  if (*abort_flag) return false;
+  if (threadIdx.x < 32) {
+    tmem_alloc(smem_addr(slot), kCols);
+    tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  tc_fence_after_sync();
+  grid_launch_dependents();
+  tmem = *slot;
+  return true;
+}
+template <int kCols>
+__device__ __forceinline__ void tear_down(const Params& g, uint32_t tmem) {
+  tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    if (*reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk) {
+      // a wait gave up somewhere: give MMAs still in flight time to land before their memory is released
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    }
+    tc_fence_after_sync();
+    tmem_free(tmem, kCols);
+  }
+}
+
+// The hidden keys of tile [j0, j0 + kStream) as two words in shared memory (bit set = hidden).
+__device__ __forceinline__ void post_hidden(uint32_t* words, const float* mask, int j0, int t_k) {
+  if (threadIdx.x < kStream) {
+    const int j = j0 + threadIdx.x;
+    const unsigned hid = __ballot_sync(kFull, j >= t_k || mask[j] == 0.f);
+    if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = hid;
+  }
+}
+// ... and the part of them a thread with columns [group * N, group * N + N) needs.
+template <int N>
+__device__ __forceinline__ uint32_t my_hidden(const uint32_t* words, int group) {
+  if constexpr (N == 32) return words[group];
+  else return words[group >> 1] >> (16 * (group & 1));
+}
+
+__device__ __forceinline__ uint32_t align_1024(uint32_t addr) { return (addr + 1023u) & ~1023u; }
+
+// ---- forward ----
+template <int HD>
+struct Fwd {
+  static constexpr int kGroups = HD > 64 ? 4 : 2;  // threads to a row
+  static constexpr int kThreads = kRows * kGroups;
+  static constexpr int kBlocks = HD > 64 ? 1 : 2;  // per SM
+  using Held = Stage<HD, kRows, kThreads>;
+  using Tile = Stage<HD, kStream, kThreads>;
+  static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
+  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols;
+  static constexpr int kCols = HD > 64 ? 512 : 256;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
+  using L = Fwd<HD>;
+  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
+  extern __shared__ unsigned char raw[];
+  __shared__ uint32_t slot, abort_flag, hidden[2][2];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ float exchange[G][kRows];
+  uint32_t tmem;
+  if (!set_up<L::kCols, 2>(g, &slot, &abort_flag, bars, tmem)) return;
+  const uint32_t base = align_1024(smem_addr(raw));
+  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1);
+  const int warp = threadIdx.x >> 5, group = warp >> 2;
+  const int row = (warp & 3) * 32 + (threadIdx.x & 31);
+  const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const bool issuer = warp == 0 && elect_one();
+
+  int problem, at;
+  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
+  const int i0 = (g.slots - 1 - at) * kRows;  // long causal rows first
+  const long long b = problem;
+  const float* k = g.k + b * g.t_k * g.hd;
+  const float* v = g.v + b * g.t_k * g.hd_v;
+  const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
+  const int steps = (g.hd + 15) / 16;
+  const int keys_end = g.causal ? min(g.t_k, i0 + kRows) : g.t_k;
+  const int n = (keys_end + kStream - 1) / kStream;
+  const int i = i0 + row;
+
+  uint64_t check = 0;
+  typename L::Tile stage_k, stage_v;
+  stage_k.load(k, 0, g.t_k, g.hd, g.wide_qk);
+  {
+    typename L::Held stage_q;
+    stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd, g.wide_qk);
+    stage_q.store(base + L::kQ, check);
+  }
+  stage_k.store(base + L::kK, check);
+  if (mask) post_hidden(hidden[0], mask, 0, g.t_k);
+  fence_async_shared();
+  __syncthreads();
+  if (issuer) {
+    issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK, steps);
+    mma_commit(scored);
+  }
+  stage_v.load(v, 0, g.t_k, g.hd_v, g.wide_v);
+  stage_v.store(base + L::kV, check);
+  fence_async_shared();
+
+  float top = -INFINITY, shift = 0.f, denom = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
+  uint64_t acc[OW / 2];
+#pragma unroll
+  for (int c = 0; c < OW / 2; ++c) acc[c] = 0;
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo);
+  bool ok = true;
+  for (int j = 0; j < n; ++j) {
+    const int j0 = j * kStream;
+    ok &= mbar_wait(scored, j & 1, g.status, 0x0a00u);
+    tc_fence_after_sync();
+    uint32_t s[CW];
+    tmem_ld<CW>(lanes + L::kS + group * CW, s);
+    tmem_ld_wait();
+    int limit = g.t_k - j0;
+    if (g.causal) limit = min(limit, i - j0 + 1);
+    limit -= group * CW;
+    uint32_t unseen = limit >= CW ? 0u : limit <= 0 ? kFull : ~((1u << limit) - 1u);
+    if (mask) unseen |= my_hidden<CW>(hidden[j & 1], group);
+    if (unseen != 0u) {
+#pragma unroll
+      for (int c = 0; c < CW; ++c)
+        if ((unseen >> c) & 1u) s[c] = 0xff800000u;
+    }
+    float tile_top = -INFINITY;
+#pragma unroll
+    for (int c = 0; c < CW; c += 2) tile_top = max3(tile_top, __uint_as_float(s[c]), __uint_as_float(s[c + 1]));
+    exchange[group][row] = tile_top;
+    __syncthreads();
+    float raised = top;
+#pragma unroll
+    for (int c = 0; c < G; ++c) raised = fmaxf(raised, exchange[c][row]);
+    const float moved = raised == -INFINITY ? 0.f : raised * g.c_hi;
+    const float shrink = top == -INFINITY ? 0.f : exp2_approx(shift - moved);  // nothing gathered yet: nothing to rescale
+    top = raised, shift = moved;
+    const uint64_t minus_shift = f2_pack(-shift, -shift);
+    uint64_t w[CW / 2];
+    uint64_t sum = 0;
+#pragma unroll
+    for (int c = 0; c < CW / 2; ++c) {
+      const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
+      float x0, x1;
+      f2_unpack(f2_fma(s2, c_lo, f2_fma(s2, c_hi, minus_shift)), x0, x1);
+      w[c] = f2_pack(exp2_approx(x0), exp2_approx(x1));
+      sum = f2_add(sum, w[c]);
+    }
+    float sum0, sum1;
+    f2_unpack(sum, sum0, sum1);
+    denom = fmaf(denom, shrink, sum0 + sum1);  // this thread's share; the shares meet after the last tile
+    hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
+    tmem_st_wait();
+    tc_fence_before_sync();
+    if (!__syncthreads_and(ok)) break;
+    if (issuer) {
+      tc_fence_after_sync();
+      issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
+      mma_commit(weighed);
+    }
+    const bool more = j + 1 < n;
+    if (more) {
+      // K's buffer has been read (the scores are there) and so have the scores themselves
+      stage_k.load(k, j0 + kStream, g.t_k, g.hd, g.wide_qk);
+      stage_k.store(base + L::kK, check);
+      if (mask) post_hidden(hidden[(j + 1) & 1], mask, j0 + kStream, g.t_k);
+      fence_async_shared();
+      __syncthreads();
+      if (issuer) {
+        tc_fence_after_sync();
+        issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK, steps);
+        mma_commit(scored);
+      }
+      stage_v.load(v, j0 + kStream, g.t_k, g.hd_v, g.wide_v);
+    }
+    ok &= mbar_wait(weighed, j & 1, g.status, 0x0a01u);
+    tc_fence_after_sync();
+    uint32_t o[OW];
+    tmem_ld<OW>(lanes + L::kO + group * OW, o);
+    tmem_ld_wait();
+    tc_fence_before_sync();
+    const uint64_t shrink2 = f2_pack(shrink, shrink);
+#pragma unroll
+    for (int c = 0; c < OW / 2; ++c) acc[c] = f2_fma(acc[c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
+    if (more) {
+      stage_v.store(base + L::kV, check);  // the weighing has read the tile before this one
+      fence_async_shared();
+    }
+  }
+  ok = __syncthreads_and(ok);
+  if (ok) {
+    if (__syncthreads_or(is_bad(check))) {
+      plain_fwd(g, b, i0, L::kThreads);
+    } else {
+      exchange[group][row] = denom;
+      __syncthreads();
+      float total = 0.f;
+#pragma unroll
+      for (int c = 0; c < G; ++c) total += exchange[c][row];
+      if (i < g.t_q) {
+#pragma unroll
+        for (int c = 0; c < OW / 2; ++c) {
+          float x0, x1;
+          f2_unpack(acc[c], x0, x1);
+          acc[c] = f2_pack(x0 / total, x1 / total);  // 0/0 = NaN for a row with no key, as the oracle has it
+        }
+        store_row<OW>(g.out + (b * g.t_q + i) * g.hd_v, acc, group * OW, g.hd_v, g.wide_out);
+        // once per row, so in double: L is then as good as its sum
+        if (group == 0)
+          g.lse_out[b * g.t_q + i] =
+              top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
+      }
+    }
+  }
+  tear_down<L::kCols>(g, tmem);
+}
+
+// ---- backward: dQ for 128 query rows, or dK and dV for 128 key rows ----
+template <int HD>
+struct Bwd {
+  static constexpr int kGroups = 4;
+  static constexpr int kThreads = kRows * kGroups;
+  // At head dims above 64 two held operands and two streamed tiles do not fit in shared memory twice over: the first
+  // held operand lies in tensor memory, the streamed tiles have one buffer, and the tile's results are written over
+  // the scores they came from.
+  static constexpr bool kWide = HD > 64;
+  static constexpr int kStages = kWide ? 1 : 2;
+  using Held = Stage<HD, kRows, kThreads>;
+  using Tile = Stage<HD, kStream, kThreads>;
+  static constexpr uint32_t kHeld0 = 0, kHeld1 = kWide ? 0 : Held::kBytes, kTiles = kHeld1 + Held::kBytes;
+  static constexpr uint32_t kBytes = kTiles + kStages * 2 * Tile::kBytes + 1024;
+  static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols, kAfter = kP + 3 * kPieceCols;
+  static constexpr uint32_t kOut0 = kWide ? 0 : kAfter, kOut1 = kWide ? 0 : kAfter + HD;
+  static constexpr uint32_t kHeldT = kAfter;  // kWide: the first held operand, three pieces of HD / 2 columns
+  static constexpr int kCols = 512;
+  static_assert(kAfter + (kWide ? 3 * HD / 2 : 2 * HD) <= 512, "tensor memory");
+};
+
+template <int HD, bool kKV>
+__global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
+  using L = Bwd<HD>;
+  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
+  extern __shared__ unsigned char raw[];
+  __shared__ uint32_t slot, abort_flag, hidden[2][2];
+  __shared__ __align__(8) uint64_t bars[3];
+  __shared__ __align__(16) float lse_hi[2][kStream], lse_lo[2][kStream], deltas[2][kStream];  // dK/dV: of the streamed rows
+  uint32_t tmem;
+  if (!set_up<L::kCols, 3>(g, &slot, &abort_flag, bars, tmem)) return;
+  const uint32_t base = align_1024(smem_addr(raw));
+  const uint32_t scored = smem_addr(bars), weighed0 = smem_addr(bars + 1), weighed1 = smem_addr(bars + 2);
+  const int warp = threadIdx.x >> 5, group = warp >> 2;
+  const int row = (warp & 3) * 32 + (threadIdx.x & 31);
+  const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const bool issuer = warp == 0 && elect_one();
+
+  int problem, at;
+  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
+  const int first = (kKV ? at : g.slots - 1 - at) * kRows;  // the longest causal streams first
+  const long long b = problem;
+  // the held pair (against which the tiles are scored) and the streamed pair
+  const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
+  const float* held0 = (kKV ? g.k : g.q) + b * owned * g.hd;
+  const float* held1 = (kKV ? g.v : g.dout) + b * owned * g.hd_v;
+  const float* stream0 = (kKV ? g.q : g.k) + b * streamed * g.hd;
+  const float* stream1 = (kKV ? g.dout : g.v) + b * streamed * g.hd_v;
+  const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
+  const int steps = (g.hd + 15) / 16, steps_v = (g.hd_v + 15) / 16;
+  const int begin = kKV && g.causal ? first : 0;
+  const int end = !kKV && g.causal ? min(streamed, first + kRows) : streamed;
+  const int n = (end - begin + kStream - 1) / kStream;
+  const int mine = first + row;  // this thread's row
+
+  constexpr float kLog2eHi = 1.44269502f, kLog2eLo = 1.92596303e-8f;  // log2(e) in two parts
+  auto to_log2 = [&](float lse, float& hi, float& lo) {
+    hi = lse * kLog2eHi;
+    lo = fmaf(lse, kLog2eHi, -hi) + lse * kLog2eLo;
+  };
+
+  uint64_t check = 0;
+  auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
+  // the streamed tile j, and what goes with its rows
+  auto stage_tile = [&](int j) {
+    const int x0 = begin + j * kStream;
+    typename L::Tile a, c;
+    a.load(stream0, x0, streamed, g.hd, g.wide_qk);
+    c.load(stream1, x0, streamed, g.hd_v, g.wide_v);
+    if (kKV) {
+      if (threadIdx.x < kStream) {
+        const int x = x0 + threadIdx.x;
+        float hi, lo;
+        to_log2(x < streamed ? g.lse_in[b * g.t_q + x] : 0.f, hi, lo);
+        lse_hi[j & 1][threadIdx.x] = hi;
+        lse_lo[j & 1][threadIdx.x] = lo;
+        deltas[j & 1][threadIdx.x] = x < streamed ? g.delta[b * g.t_q + x] : 0.f;
+      }
+    } else if (mask) {
+      post_hidden(hidden[j & 1], mask, x0, g.t_k);
+    }
+    a.store(tile_at(j, 0), check);
+    c.store(tile_at(j, 1), check);
+  };
+  auto issue_tile = [&](int j) {
+    tc_fence_after_sync();
+    issue_scores<HD, L::kWide>(tmem + L::kS, L::kWide ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0), steps);
+    issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, tile_at(j, 1), steps_v);
+    mma_commit(scored);
+  };
+
+  if constexpr (L::kWide) {
+    uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
+#pragma unroll
+    for (int c = 0; c < OW; c += 8) {
+      float x[8];
+      load8(x, held0, mine, owned, group * OW + c, g.hd, g.wide_qk);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[2 * e], x[2 * e + 1]), h[c / 2 + e], m[c / 2 + e], l[c / 2 + e], check);
+    }
+    const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
+    tmem_st<OW / 2>(to, h);
+    tmem_st<OW / 2>(to + HD / 2, m);
+    tmem_st<OW / 2>(to + HD, l);
+    tmem_st_wait();
+    tc_fence_before_sync();
+  } else {
+    typename L::Held stage;
+    stage.load(held0, first, owned, g.hd, g.wide_qk);
+    stage.store(base + L::kHeld0, check);
+  }
+  {
+    typename L::Held stage;
+    stage.load(held1, first, owned, g.hd_v, g.wide_v);
+    stage.store(base + L::kHeld1, check);
+  }
+  if (n > 0) stage_tile(0);
+  fence_async_shared();
+  __syncthreads();
+  if (n > 0 && issuer) issue_tile(0);
+
+  float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
+  bool live = mine < owned;
+  if constexpr (kKV) {
+    if (live && mask) live = mask[mine] != 0.f;
+  } else {
+    if (live) to_log2(g.lse_in[b * g.t_q + mine], my_hi, my_lo);
+    if (live) my_delta = g.delta[b * g.t_q + mine];
+  }
+
+  uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dV and dK
+#pragma unroll
+  for (int c = 0; c < OW / 2; ++c) acc0[c] = acc1[c] = 0;
+  auto gather = [&](uint32_t from, uint64_t(&acc)[OW / 2]) {
+    tc_fence_after_sync();
+    uint32_t o[OW];
+    tmem_ld<OW>(lanes + from + group * OW, o);
+    tmem_ld_wait();
+    tc_fence_before_sync();
+#pragma unroll
+    for (int c = 0; c < OW / 2; ++c) acc[c] = f2_add(acc[c], f2_pack_bits(o[2 * c], o[2 * c + 1]));
+  };
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale2 = f2_pack(g.scale, g.scale);
+  bool ok = true;
+  for (int j = 0; j < n; ++j) {
+    const int x0 = begin + j * kStream;
+    ok &= mbar_wait(scored, j & 1, g.status, 0x0b00u);
+    tc_fence_after_sync();
+    uint32_t s[CW], dp[CW];
+    tmem_ld<CW>(lanes + L::kS + group * CW, s);
+    tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
+    tmem_ld_wait();
+    // columns [from, to) of this thread's CW are seen, less the hidden ones
+    int from = 0, to = streamed - x0 - group * CW;
+    if (g.causal) {
+      if (kKV) from = mine - x0 - group * CW;
+      else to = min(to, mine - x0 - group * CW + 1);
+    }
+    if (!live) to = 0;
+    uint32_t unseen = 0;
+    if (from > 0) unseen |= from >= CW ? kFull : (1u << from) - 1u;
+    if (to < CW) unseen |= to <= 0 ? kFull : ~((1u << to) - 1u);
+    if (!kKV && mask) unseen |= my_hidden<CW>(hidden[j & 1], group);
+    uint64_t p[CW / 2], ds[CW / 2];
+#pragma unroll
+    for (int c = 0; c < CW / 2; ++c) {
+      uint64_t hi, lo, delta;
+      if (kKV) {
+        const int at = group * CW + 2 * c;
+        hi = *reinterpret_cast<const uint64_t*>(&lse_hi[j & 1][at]);
+        lo = *reinterpret_cast<const uint64_t*>(&lse_lo[j & 1][at]);
+        delta = *reinterpret_cast<const uint64_t*>(&deltas[j & 1][at]);
+      } else {
+        hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
+      }
+      const uint64_t minus = f2_pack(-1.f, -1.f);
+      const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
+      uint64_t x = f2_fma(s2, c_hi, hi ^ 0x8000000080000000ull);
+      x = f2_add(x, f2_fma(s2, c_lo, lo ^ 0x8000000080000000ull));
+      float x0_, x1_;
+      f2_unpack(x, x0_, x1_);
+      float p0 = exp2_approx(x0_), p1 = exp2_approx(x1_);
+      if ((unseen >> (2 * c)) & 1u) p0 = 0.f;
+      if ((unseen >> (2 * c + 1)) & 1u) p1 = 0.f;
+      p[c] = f2_pack(p0, p1);
+      const uint64_t d2 = f2_fma(delta, minus, f2_pack_bits(dp[2 * c], dp[2 * c + 1]));
+      float d0, d1;
+      f2_unpack(f2_mul(f2_mul(p[c], d2), scale2), d0, d1);
+      if ((unseen >> (2 * c)) & 1u) d0 = 0.f;  // (delta of a row with no key is NaN)
+      if ((unseen >> (2 * c + 1)) & 1u) d1 = 0.f;
+      ds[c] = f2_pack(d0, d1);
+    }
+    hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, check);
+    if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
+    tmem_st_wait();
+    tc_fence_before_sync();
+    if (!__syncthreads_and(ok)) break;
+    if (issuer) {
+      tc_fence_after_sync();
+      if (kKV) {
+        issue_weigh<HD>(tmem + L::kOut0, tmem + L::kP, tile_at(j, 1));
+        mma_commit(weighed0);
+        if (!L::kWide) {
+          issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
+          mma_commit(weighed1);
+        }
+      } else {
+        issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile_at(j, 0));
+        mma_commit(weighed0);
+      }
+    }
+    const bool more = j + 1 < n;
+    if (!L::kWide && more) {
+      stage_tile(j + 1);  // into the other buffer, whose products were gathered a tile ago
+      fence_async_shared();
+      __syncthreads();
+      if (issuer) issue_tile(j + 1);
+    }
+    ok &= mbar_wait(weighed0, j & 1, g.status, 0x0b01u);
+    gather(L::kOut0, acc0);
+    if (kKV) {
+      if (L::kWide) {
+        if (!__syncthreads_and(ok)) break;
+        if (issuer) {
+          tc_fence_after_sync();
+          issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
+          mma_commit(weighed1);
+        }
+      }
+      ok &= mbar_wait(weighed1, j & 1, g.status, 0x0b02u);
+      gather(L::kOut1, acc1);
+    }
+    if (L::kWide && more) {
+      stage_tile(j + 1);
+      fence_async_shared();
+      if (!__syncthreads_and(ok)) break;
+      if (issuer) issue_tile(j + 1);
+    }
+  }
+  ok = __syncthreads_and(ok);
+  if (ok) {
+    if (__syncthreads_or(is_bad(check))) {
+      plain_bwd<kKV>(g, b, first, L::kThreads);
+    } else if (mine < owned) {
+      if (kKV) {
+        store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);
+        store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc1, group * OW, g.hd, g.wide_out);
+      } else {
+        store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
+      }
+    }
+  }
+  tear_down<L::kCols>(g, tmem);
+}
+
+template <int HD>
+int launch_sized(Op op, const Problem& p) {
+  Params g = {};
+  auto in = [](const void* x) { return static_cast<const float*>(x); };
+  auto aligned = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; };  // (null is)
+  g.q = in(p.q), g.k = in(p.k), g.v = in(p.v), g.mask = in(p.mask), g.dout = in(p.dout), g.lse_in = in(p.lse_in), g.delta = in(p.delta);
+  g.out = static_cast<float*>(p.out), g.lse_out = static_cast<float*>(p.lse_out);
+  g.dq = static_cast<float*>(p.dq), g.dk = static_cast<float*>(p.dk), g.dv = static_cast<float*>(p.dv);
+  g.status = p.status;
+  if (g.status == nullptr)
+    if (int rc = status_word(&g.status)) return rc;
+  g.bh = p.bh;
+  g.slots = ((op == Op::BwdKV ? p.t_k : p.t_q) + kRows - 1) / kRows;
+  g.t_q = p.t_q, g.t_k = p.t_k, g.hd = p.hd, g.hd_v = p.hd_v, g.causal = p.causal ? 1 : 0;
+  g.scale = static_cast<float>(p.scale);
+  const double c = static_cast<double>(g.scale) * 1.4426950408889634;
+  g.c_hi = static_cast<float>(c);
+  if (g.c_hi > c) g.c_hi = nextafterf(g.c_hi, 0.f);
+  g.c_lo = static_cast<float>(c - g.c_hi);
+  if (!(g.c_lo > 0.f)) g.c_lo = 1e-37f;  // a score of -inf has to stay one
+  g.wide_qk = p.hd % 4 == 0 && aligned(p.q) && aligned(p.k);
+  g.wide_v = p.hd_v % 4 == 0 && aligned(p.v) && aligned(p.dout);
+  g.wide_out = p.hd % 4 == 0 && p.hd_v % 4 == 0;
+  if (op == Op::Fwd) g.wide_out = g.wide_out && aligned(p.out);
+  else g.wide_out = g.wide_out && aligned(p.dq) && aligned(p.dk) && aligned(p.dv);
+  const long long blocks = p.bh * g.slots;
+  int sms = 0;
+  if (int rc = sm_count(&sms)) return rc;
+  g.group = work_group(p, blocks, sms);
+  using F = Fwd<HD>;
+  using B = Bwd<HD>;
+  void (*kernel)(const Params) = op == Op::Fwd ? f32_fwd_kernel<HD> : op == Op::BwdQ ? f32_bwd_kernel<HD, false> : f32_bwd_kernel<HD, true>;
+  const uint32_t shared = op == Op::Fwd ? F::kBytes : B::kBytes;
+  // the attribute is per device and per kernel instantiation; set it on first use there
+  static bool sized[64][3] = {};
+  int device = 0;
+  LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");
+  if (device < 0 || device >= 64 || !sized[device][static_cast<int>(op)]) {
+    LIMN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared)),
+              "sizing shared memory for a float32 sdpa kernel");
+    if (device >= 0 && device < 64) sized[device][static_cast<int>(op)] = true;
+  }
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks)), dim3(op == Op::Fwd ? F::kThreads : B::kThreads), shared, p.stream, g),
+            "launching a float32 sdpa kernel");
+  note_launches(1);
+  return LIMN_B200_OK;
+}
+
+}  // namespace
+
+bool f32_split_serves(Op op, const Problem& p) {
+  if (p.dtype != LIMN_B200_F32 || p.hd > 128 || p.hd_v > 128) return false;
+  if (p.layout != LIMN_B200_BHTD || p.strided) return false;
+  if (p.t_q < 16 || p.t_k < 16) return false;  // most of a 128 x 64 tile would be idle
+  // row maxima are taken before scaling, and the scale is folded into exp2 in two parts
+  const float scale = static_cast<float>(p.scale);
+  if (!(scale > 1e-20f && scale < 1e20f)) return false;
+  const long long rows = op == Op::BwdKV ? p.t_k : p.t_q;
+  return p.bh * ((rows + kRows - 1) / kRows) <= 0x7fffffffLL;
+}
+
+int f32_split_launch(Op op, const Problem& p) {
+  const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
+  if (widest <= 32) return launch_sized<32>(op, p);
+  if (widest <= 64) return launch_sized<64>(op, p);
+  return launch_sized<128>(op, p);
+}
+
+}  // namespace limn_b200

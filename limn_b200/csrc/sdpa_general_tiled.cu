@@ -1,8 +1,8 @@
 // Tiled SIMT fused-attention kernels: float32, float16 and bfloat16 storage computed in float32 on the
-// CUDA cores, head dims up to 256, optional key mask, rectangular t_q x t_k. They serve what the tcgen05
-// kernels leave (float32 above all, which has to be computed at its own width to meet the reference's 1e-5
-// check: tests/test_attention.py:250-255) whenever the problem is large enough to fill a tile; the one-row-
-// per-warp kernels in sdpa_general.cu keep float64, wider heads and short sequences.
+// CUDA cores, head dims up to 256, optional key mask, rectangular t_q x t_k. They serve what the tensor-core
+// kernels leave (head dims that are no multiple of 8 in 16 bits, head dims above 128, float32 with a scale that is
+// not positive) whenever the problem is large enough to fill a tile; the one-row-per-warp kernels in
+// sdpa_general.cu keep float64, wider heads and short sequences.
 //
 // Shape of the work: a block of 256 threads owns 64 rows (query rows in the forward and the dQ pass, key rows
 // in the dK/dV pass) and streams the other side through shared memory in tiles of BN rows (64, 32 or 16 of them

@@ -316,6 +316,127 @@ def test_tiled_general_kernels_on_rows_without_a_visible_key(dev):
     assert float(np.abs(lse[:, 5:] - want_lse[:, 5:]).max()) <= 1e-3
 
 
+F32_EDGES = [
+    # t_q, t_k, hd, hd_v, causal, mask kind: the edges of the 128-row blocks, the 64-row tiles, the 16-column steps and
+    # the three widths (32, 64, 128) the float32 tensor-core kernels are built for
+    (16, 16, 8, 8, True, None),
+    (17, 64, 16, 31, False, None),
+    (63, 65, 32, 32, False, "holes"),
+    (64, 64, 33, 33, True, None),
+    (127, 127, 64, 64, True, "pad"),
+    (128, 200, 64, 17, False, None),
+    (129, 129, 65, 65, True, None),
+    (193, 193, 100, 128, True, "holes"),
+    (257, 300, 128, 128, False, "pad"),
+    (1025, 1025, 128, 128, True, None),
+    (1100, 1100, 64, 64, True, None),
+]
+
+
+@pytest.mark.parametrize("case", F32_EDGES, ids=[f"{c[0]}x{c[1]} hd {c[2]}/{c[3]} {'causal' if c[4] else 'full'} {c[5] or ''}" for c in F32_EDGES])
+@pytest.mark.parametrize("shift", [0, 1], ids=["aligned", "bases 4 bytes off"])
+def test_float32_on_the_tensor_cores_keeps_its_width(case, shift):
+    """float32 split into three bfloat16 pieces against float64. A score takes at most hd / 16 truncated additions of
+    its largest partial sum, each below 2^-23 of it, and the probability moves by that times the scaled score; sums over
+    keys are rounded once per 64 of them. 16 * 2^-24 * (1 + max |scaled score|) covers both; plain bfloat16 operands
+    (2^-9) or two pieces (2^-17) do not come near it."""
+    from limn_b200 import runtime
+    from limn_b200._lib import check, lib
+
+    t_q, t_k, hd, hd_v, causal, kind = case
+    bh, L = 3, lib()
+    rng = np.random.default_rng(t_q * 131 + hd)
+    q, k, v, do = (rng.standard_normal((bh, t, w)).astype(np.float32) for t, w in ((t_q, hd), (t_k, hd), (t_k, hd_v), (t_q, hd_v)))
+    mask = None
+    if kind == "holes":
+        mask = (rng.random((bh, t_k)) > 0.3).astype(np.float32)
+        mask[:, 0] = 1
+    elif kind == "pad":
+        mask = np.broadcast_to(np.arange(t_k) < t_k * 2 // 3, (bh, t_k)).astype(np.float32)
+    hold = []
+
+    def put(a):
+        hold.append(runtime.upload(np.concatenate([np.zeros(shift, np.float32), a.ravel()])))
+        return hold[-1].ptr + 4 * shift
+
+    def room(a):
+        hold.append(runtime.empty(a.nbytes + 4 * shift))
+        return hold[-1].ptr + 4 * shift
+
+    def back(ptr, shape):
+        return runtime.download(next(b for b in hold if b.ptr + 4 * shift == ptr), np.float32, (-1,))[shift:].reshape(shape).astype(np.float64)
+
+    rows = np.zeros((bh, t_q), np.float32)
+    pq, pk, pv, pdo = put(q), put(k), put(v), put(do)
+    pm = put(mask) if mask is not None else None
+    po, pl, pd, pdq, pdk, pdv = room(do), room(rows), room(rows), room(q), room(k), room(v)
+    tail = (0, bh, t_q, t_k, hd, hd_v, int(causal), hd**-0.5, None)
+    check(L.limn_b200_sdpa_fwd(pq, pk, pv, pm, po, pl, *tail), "sdpa")
+    check(L.limn_b200_sdpa_bwd_q_fused(pq, pk, pv, po, pdo, pl, pm, pdq, pd, *tail), "sdpa_bwd_q_fused")
+    check(L.limn_b200_sdpa_bwd_kv(pq, pk, pv, pdo, pl, pd, pm, pdk, pdv, *tail), "sdpa_bwd_kv")
+    Q, K, V, DO = (a.astype(np.float64) for a in (q, k, v, do))
+    s = Q @ K.transpose(0, 2, 1) * hd**-0.5
+    biggest = np.abs(s).max()
+    if causal:
+        s = np.where(np.tril(np.ones((t_q, t_k), bool)), s, -np.inf)
+    if mask is not None:
+        s = np.where(mask[:, None, :] != 0, s, -np.inf)
+    top = s.max(-1, keepdims=True)
+    p = np.exp(s - top)
+    total = p.sum(-1, keepdims=True)
+    p /= total
+    o = p @ V
+    ds = p * (DO @ V.transpose(0, 2, 1) - (DO * o).sum(-1, keepdims=True)) * hd**-0.5
+    bound = 16 * 2.0**-24 * (1 + biggest)
+    for ptr, want, what in ((po, o, "O"), (pl, (top + np.log(total))[..., 0], "L"), (pdq, ds @ K, "dQ"),
+                            (pdk, ds.transpose(0, 2, 1) @ Q, "dK"), (pdv, p.transpose(0, 2, 1) @ DO, "dV")):
+        got = back(ptr, want.shape)
+        error = np.linalg.norm(got - want) / np.linalg.norm(want)
+        assert error <= bound, f"{what}: {error:.2e} > {bound:.2e}"
+
+
+@pytest.mark.parametrize("hd", [32, 64, 128])
+def test_float32_infinities_and_nans_come_out_where_float32_arithmetic_puts_them(hd, dev):
+    """Non-finite operands and ones that no bfloat16 holds: an infinite V makes its column of O infinite and leaves the
+    others, a key at -infinity times a positive query weighs nothing, a NaN query is a NaN row, and the largest float32
+    stays finite; the same through both backward passes."""
+    import limn_standin as host
+
+    rng = np.random.default_rng(hd)
+    t = 150
+    q, k, v, do = (rng.standard_normal((4, t, hd)).astype(np.float32) for _ in range(4))
+    q = np.abs(q)
+    v[0, 3, 5] = np.inf
+    k[1, 140] = -np.inf
+    q[2, 70] = np.nan
+    v[3, :, 1] = 3.4e38 / t
+    v[3, 7, 0] = np.finfo(np.float32).max
+    scale = hd**-0.5
+    with np.errstate(all="ignore"):
+        want_out, want_lse = oracle.sdpa_forward(q, k, v, None, causal=False, scale=scale)
+        out, lse = host.Attention(dev, q, k, v, causal=False, key_mask=None).forward()
+        assert np.isinf(want_out[0, :, 5]).all() and np.isnan(want_out[2, 70]).all() and np.isfinite(want_out[1]).all()
+        assert np.array_equal(np.isnan(out), np.isnan(want_out)) and np.array_equal(np.isinf(out), np.isinf(want_out))
+        finite = np.isfinite(want_out)
+        size = np.abs(np.where(finite, want_out, 0)).max(axis=1, keepdims=True)
+        assert (np.abs(out - want_out)[finite] <= 1e-4 * np.broadcast_to(1 + size, out.shape)[finite]).all()
+        assert np.array_equal(np.isnan(lse), np.isnan(want_lse))
+        v[3] = rng.standard_normal((t, hd)).astype(np.float32)
+        v[0, 3, 5] = 0.0
+        do[0, 9, 2] = np.inf
+        att = host.Attention(dev, q, k, v, causal=False, key_mask=None)
+        att.forward()
+        want_out, want_lse = oracle.sdpa_forward(q, k, v, None, causal=False, scale=scale)
+        delta = oracle.row_delta(do, want_out)
+        want = (oracle.sdpa_backward_q(q, k, v, do, want_lse, delta, None, causal=False, scale=scale),
+                *oracle.sdpa_backward_kv(q, k, v, do, want_lse, delta, None, causal=False, scale=scale))
+        for got, wanted, what in zip(att.backward(do), want, ("dQ", "dK", "dV")):
+            assert np.array_equal(np.isnan(got), np.isnan(wanted)), what
+            assert np.array_equal(np.isinf(got), np.isinf(wanted)), what
+            finite = np.isfinite(wanted)
+            assert float(np.abs(got - wanted)[finite].max()) <= 1e-4 * (1 + float(np.abs(wanted[finite]).max())), what
+
+
 FUSED_CASES = [
     # id, dtype, code, shape (q = k = v), causal, key mask?, layout
     ("bf16 d128 causal", BF16, 2, (3, 384, 128), True, False, "bhtd"),
