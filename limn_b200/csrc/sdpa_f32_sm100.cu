@@ -133,26 +133,26 @@ struct Stage {
 };
 
 // The six products in the order they are added, smallest first.
-__device__ __forceinline__ int piece_a(int i) { return (0x001102 >> (4 * i)) & 0xf; }  // l h m m h h
-__device__ __forceinline__ int piece_b(int i) { return (0x010120 >> (4 * i)) & 0xf; }  // h l m h m h
+__device__ __host__ constexpr int piece_a(int i) { return (0x001102 >> (4 * i)) & 0xf; }  // l h m m h h
+__device__ __host__ constexpr int piece_b(int i) { return (0x010120 >> (4 * i)) & 0xf; }  // h l m h m h
 
-__device__ __forceinline__ uint64_t tile_desc(uint32_t lo) { return (static_cast<uint64_t>(kDescHiSw128) << 32) | lo; }
-
-// D (kRows x kStream) = A (kRows x 16 steps) B^T (kStream x 16 steps), both with the contraction dim contiguous. A lies
-// in shared memory (a0 its address) or in tensor memory (a0 its column, pieces kTmemPiece columns apart).
+// D (kRows x kStream) = A (kRows x HD) B^T (kStream x HD), both with the contraction dim contiguous. A lies in shared
+// memory (a0 its address) or in tensor memory (a0 its column, pieces HD / 2 columns apart). Columns past the head dim are
+// zero on both sides. Fully unrolled over compile-time offsets: one thread issues every MMA of the block, and with a
+// loop over the steps it took 115 clocks an MMA instead of the 32 the tensor cores need.
 template <int HD, bool kTmemA>
-__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0, int steps) {
+__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0) {
   constexpr uint32_t kPieceA = (HD > 64 ? 2 : 1) * kRows * 128, kPieceB = (HD > 64 ? 2 : 1) * kStream * 128;
   constexpr uint32_t idesc = mma_idesc(kRows, kStream, false, false, false);
+  const uint32_t a_lo = kTmemA ? a0 : desc_lo(a0, 0), b_lo = desc_lo(b0, 0);
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
-    const uint32_t b_lo = desc_lo(b0 + piece_b(i) * kPieceB, 0);
-    const uint32_t a_lo = kTmemA ? a0 + piece_a(i) * (HD / 2) : desc_lo(a0 + piece_a(i) * kPieceA, 0);
-    for (int s = 0; s < steps; ++s) {
-      const uint32_t within = (s & 3) * 2, block = s >> 2;
-      const uint32_t b = b_lo + within + block * (kStream * 128 / 16);
-      if constexpr (kTmemA) mma_ts_lo(d, a_lo + s * 8, b, idesc, i > 0 || s > 0);
-      else mma_ss(d, tile_desc(a_lo + within + block * (kRows * 128 / 16)), tile_desc(b), idesc, i > 0 || s > 0);
+#pragma unroll
+    for (int s = 0; s < HD / 16; ++s) {
+      const uint32_t b = b_lo + piece_b(i) * (kPieceB / 16) + (s / 4) * (kStream * 128 / 16) + (s % 4) * 2;
+      if constexpr (kTmemA) mma_ts_lo(d, a_lo + piece_a(i) * (HD / 2) + s * 8, b, idesc, i > 0 || s > 0);
+      else if (i == 0 && s == 0) mma_ss_lo<false>(d, a_lo + piece_a(i) * (kPieceA / 16), b, idesc);
+      else mma_ss_lo<true>(d, a_lo + piece_a(i) * (kPieceA / 16) + (s / 4) * (kRows * 128 / 16) + (s % 4) * 2, b, idesc);
     }
   }
 }
@@ -162,12 +162,12 @@ template <int HD>
 __device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0) {
   constexpr uint32_t kPiece = (HD > 64 ? 2 : 1) * kStream * 128;
   constexpr uint32_t idesc = mma_idesc(kRows, HD, false, false, true);
+  const uint32_t x_lo = desc_lo(x0, kStream * 128);
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
-    const uint32_t x_lo = desc_lo(x0 + piece_b(i) * kPiece, kStream * 128);
-    const uint32_t w = w0 + piece_a(i) * kPieceCols;
 #pragma unroll
-    for (int s = 0; s < kStream / 16; ++s) mma_ts_lo(d, w + s * 8, x_lo + s * (16 * 128 / 16), idesc, i > 0 || s > 0);
+    for (int s = 0; s < kStream / 16; ++s)
+      mma_ts_lo(d, w0 + piece_a(i) * kPieceCols + s * 8, x_lo + piece_b(i) * (kPiece / 16) + s * (16 * 128 / 16), idesc, i > 0 || s > 0);
   }
 }
 
@@ -328,7 +328,7 @@ __device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t
   __syncthreads();
   tc_fence_after_sync();
   grid_launch_dependents();
-  tmem = *slot;
+  tmem = __shfl_sync(kFull, *slot, 0);
   return true;
 }
 template <int kCols>
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
   const int warp = threadIdx.x >> 5, group = warp >> 2;
   const int row = (warp & 3) * 32 + (threadIdx.x & 31);
   const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  const bool issuer = warp == 0 && elect_one();
+  const bool issues = __shfl_sync(kFull, warp, 0) == 0;  // the warp that issues, one lane of it elected per bunch
 
   int problem, at;
   cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
@@ -399,7 +399,6 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
   const float* k = g.k + b * g.t_k * g.hd;
   const float* v = g.v + b * g.t_k * g.hd_v;
   const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
-  const int steps = (g.hd + 15) / 16;
   const int keys_end = g.causal ? min(g.t_k, i0 + kRows) : g.t_k;
   const int n = (keys_end + kStream - 1) / kStream;
   const int i = i0 + row;
@@ -416,8 +415,8 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
   if (mask) post_hidden(hidden[0], mask, 0, g.t_k);
   fence_async_shared();
   __syncthreads();
-  if (issuer) {
-    issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK, steps);
+  if (issues && elect_one()) {
+    issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
     mma_commit(scored);
   }
   stage_v.load(v, 0, g.t_k, g.hd_v, g.wide_v);
@@ -476,7 +475,7 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
     tmem_st_wait();
     tc_fence_before_sync();
     if (!__syncthreads_and(ok)) break;
-    if (issuer) {
+    if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
       mma_commit(weighed);
@@ -489,9 +488,9 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
       if (mask) post_hidden(hidden[(j + 1) & 1], mask, j0 + kStream, g.t_k);
       fence_async_shared();
       __syncthreads();
-      if (issuer) {
+      if (issues && elect_one()) {
         tc_fence_after_sync();
-        issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK, steps);
+        issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
         mma_commit(scored);
       }
       stage_v.load(v, j0 + kStream, g.t_k, g.hd_v, g.wide_v);
@@ -574,7 +573,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   const int warp = threadIdx.x >> 5, group = warp >> 2;
   const int row = (warp & 3) * 32 + (threadIdx.x & 31);
   const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  const bool issuer = warp == 0 && elect_one();
+  const bool issues = __shfl_sync(kFull, warp, 0) == 0;  // the warp that issues, one lane of it elected per bunch
 
   int problem, at;
   cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
@@ -587,7 +586,6 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   const float* stream0 = (kKV ? g.q : g.k) + b * streamed * g.hd;
   const float* stream1 = (kKV ? g.dout : g.v) + b * streamed * g.hd_v;
   const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
-  const int steps = (g.hd + 15) / 16, steps_v = (g.hd_v + 15) / 16;
   const int begin = kKV && g.causal ? first : 0;
   const int end = !kKV && g.causal ? min(streamed, first + kRows) : streamed;
   const int n = (end - begin + kStream - 1) / kStream;
@@ -624,8 +622,8 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   };
   auto issue_tile = [&](int j) {
     tc_fence_after_sync();
-    issue_scores<HD, L::kWide>(tmem + L::kS, L::kWide ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0), steps);
-    issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, tile_at(j, 1), steps_v);
+    issue_scores<HD, L::kWide>(tmem + L::kS, L::kWide ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0));
+    issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, tile_at(j, 1));
     mma_commit(scored);
   };
 
@@ -657,7 +655,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   if (n > 0) stage_tile(0);
   fence_async_shared();
   __syncthreads();
-  if (n > 0 && issuer) issue_tile(0);
+  if (n > 0 && issues && elect_one()) issue_tile(0);
 
   float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
   bool live = mine < owned;
@@ -735,7 +733,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
     tmem_st_wait();
     tc_fence_before_sync();
     if (!__syncthreads_and(ok)) break;
-    if (issuer) {
+    if (issues && elect_one()) {
       tc_fence_after_sync();
       if (kKV) {
         issue_weigh<HD>(tmem + L::kOut0, tmem + L::kP, tile_at(j, 1));
@@ -754,14 +752,14 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
       stage_tile(j + 1);  // into the other buffer, whose products were gathered a tile ago
       fence_async_shared();
       __syncthreads();
-      if (issuer) issue_tile(j + 1);
+      if (issues && elect_one()) issue_tile(j + 1);
     }
     ok &= mbar_wait(weighed0, j & 1, g.status, 0x0b01u);
     gather(L::kOut0, acc0);
     if (kKV) {
       if (L::kWide) {
         if (!__syncthreads_and(ok)) break;
-        if (issuer) {
+        if (issues && elect_one()) {
           tc_fence_after_sync();
           issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
           mma_commit(weighed1);
@@ -774,7 +772,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
       stage_tile(j + 1);
       fence_async_shared();
       if (!__syncthreads_and(ok)) break;
-      if (issuer) issue_tile(j + 1);
+      if (issues && elect_one()) issue_tile(j + 1);
     }
   }
   ok = __syncthreads_and(ok);
