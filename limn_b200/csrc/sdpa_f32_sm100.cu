@@ -44,7 +44,7 @@ struct Params {
   int slots, group;  // row tiles per problem; problems scheduled side by side
   int t_q, t_k, hd, hd_v, causal;
   float scale, c_hi, c_lo;  // c_hi + c_lo = scale * log2(e), c_lo > 0
-  bool wide_qk, wide_v, wide_out;  // 16-byte accesses are safe for (q, k), for (v, dO) and for the results
+  bool wide_out;  // the results take 16-byte stores
 };
 
 // ---- x = h + m + l for two floats at a time; `check` becomes NaN when one of them is not finite ----
@@ -79,23 +79,35 @@ __device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&r)[N]) {
   else tmem_st8(addr, r);
 }
 
-// Eight consecutive floats of row `row`, zero beyond the matrix.
-__device__ __forceinline__ void load8(float (&x)[8], const float* src, int row, int rows, int col, int width, bool wide) {
+// Eight consecutive floats of row `row`, zero beyond the matrix. kWide: the width is a multiple of 4 and the base 16-byte
+// aligned. Predicated loads over zeroed registers, in assembly so that they stay that: written as a choice between the
+// loaded value and zero they became a load and a select, which waits for the load where it was issued.
+template <bool kWide>
+__device__ __forceinline__ void load8(float (&x)[8], const float* src, int row, int rows, int col, int width) {
   const float* at = src + static_cast<long long>(row) * width + col;
-  if (wide) {  // the width is a multiple of 4 and the base 16-byte aligned
-    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 a = row < rows && col < width ? *reinterpret_cast<const float4*>(at) : none;
-    const float4 b = row < rows && col + 4 < width ? reinterpret_cast<const float4*>(at)[1] : none;
-    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
-  } else {
+  const int left = row < rows ? width - col : 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = row < rows && col + i < width ? at[i] : 0.f;
+  for (int i = 0; i < 8; i += 4) {
+    if constexpr (kWide) {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %5, 0;\n\t"
+          "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+          "@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+          : "=&f"(x[i]), "=&f"(x[i + 1]), "=&f"(x[i + 2]), "=&f"(x[i + 3])
+          : "l"(at + i), "r"(left - i));
+    } else {
+#pragma unroll
+      for (int e = i; e < i + 4; ++e)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
+                     : "=&f"(x[e])
+                     : "l"(at + e), "r"(left - e));
+    }
   }
 }
 
 // Rows [first, first + R) of a (rows, width) matrix into three bfloat16 pieces in shared memory: piece p, column block a
 // of 64 at dst + (p * kAtoms + a) * R * 128, 128-byte rows, 128-byte swizzle.
-template <int HD, int R, int kThreads>
+template <int HD, int R, int kThreads, bool kWide>
 struct Stage {
   static constexpr int kAtoms = HD > 64 ? 2 : 1;
   static constexpr int kChunks = HD / 8;
@@ -107,12 +119,12 @@ struct Stage {
 
   float x[kLoops][8];
 
-  __device__ __forceinline__ void load(const float* src, int first, int rows, int width, bool wide) {
+  __device__ __forceinline__ void load(const float* src, int first, int rows, int width) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
       const int e = threadIdx.x + n * kThreads;
       if (kTurns == 0 && e >= R * kChunks) break;
-      load8(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width, wide);
+      load8<kWide>(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width);
     }
   }
   __device__ __forceinline__ void store(uint32_t dst, uint64_t& check) {
@@ -363,21 +375,21 @@ __device__ __forceinline__ uint32_t my_hidden(const uint32_t* words, int group) 
 __device__ __forceinline__ uint32_t align_1024(uint32_t addr) { return (addr + 1023u) & ~1023u; }
 
 // ---- forward ----
-template <int HD>
+template <int HD, bool kWide>
 struct Fwd {
   static constexpr int kGroups = HD > 64 ? 4 : 2;  // threads to a row
   static constexpr int kThreads = kRows * kGroups;
   static constexpr int kBlocks = HD > 64 ? 1 : 2;  // per SM
-  using Held = Stage<HD, kRows, kThreads>;
-  using Tile = Stage<HD, kStream, kThreads>;
+  using Held = Stage<HD, kRows, kThreads, kWide>;
+  using Tile = Stage<HD, kStream, kThreads, kWide>;
   static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
   static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols;
   static constexpr int kCols = HD > 64 ? 512 : 256;
 };
 
-template <int HD>
-__global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
-  using L = Fwd<HD>;
+template <int HD, bool kWide>
+__global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
+  using L = Fwd<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
@@ -405,10 +417,10 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
 
   uint64_t check = 0;
   typename L::Tile stage_k, stage_v;
-  stage_k.load(k, 0, g.t_k, g.hd, g.wide_qk);
+  stage_k.load(k, 0, g.t_k, g.hd);
   {
     typename L::Held stage_q;
-    stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd, g.wide_qk);
+    stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd);
     stage_q.store(base + L::kQ, check);
   }
   stage_k.store(base + L::kK, check);
@@ -419,7 +431,7 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
     issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
     mma_commit(scored);
   }
-  stage_v.load(v, 0, g.t_k, g.hd_v, g.wide_v);
+  stage_v.load(v, 0, g.t_k, g.hd_v);
   stage_v.store(base + L::kV, check);
   fence_async_shared();
 
@@ -483,7 +495,7 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
     const bool more = j + 1 < n;
     if (more) {
       // K's buffer has been read (the scores are there) and so have the scores themselves
-      stage_k.load(k, j0 + kStream, g.t_k, g.hd, g.wide_qk);
+      stage_k.load(k, j0 + kStream, g.t_k, g.hd);
       stage_k.store(base + L::kK, check);
       if (mask) post_hidden(hidden[(j + 1) & 1], mask, j0 + kStream, g.t_k);
       fence_async_shared();
@@ -493,7 +505,7 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
         issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
         mma_commit(scored);
       }
-      stage_v.load(v, j0 + kStream, g.t_k, g.hd_v, g.wide_v);
+      stage_v.load(v, j0 + kStream, g.t_k, g.hd_v);
     }
     ok &= mbar_wait(weighed, j & 1, g.status, 0x0a01u);
     tc_fence_after_sync();
@@ -538,29 +550,29 @@ __global__ void __launch_bounds__(Fwd<HD>::kThreads, Fwd<HD>::kBlocks) f32_fwd_k
 }
 
 // ---- backward: dQ for 128 query rows, or dK and dV for 128 key rows ----
-template <int HD>
+template <int HD, bool kWide>
 struct Bwd {
   static constexpr int kGroups = 4;
   static constexpr int kThreads = kRows * kGroups;
   // At head dims above 64 two held operands and two streamed tiles do not fit in shared memory twice over: the first
   // held operand lies in tensor memory, the streamed tiles have one buffer, and the tile's results are written over
   // the scores they came from.
-  static constexpr bool kWide = HD > 64;
-  static constexpr int kStages = kWide ? 1 : 2;
-  using Held = Stage<HD, kRows, kThreads>;
-  using Tile = Stage<HD, kStream, kThreads>;
-  static constexpr uint32_t kHeld0 = 0, kHeld1 = kWide ? 0 : Held::kBytes, kTiles = kHeld1 + Held::kBytes;
+  static constexpr bool kTight = HD > 64;
+  static constexpr int kStages = kTight ? 1 : 2;
+  using Held = Stage<HD, kRows, kThreads, kWide>;
+  using Tile = Stage<HD, kStream, kThreads, kWide>;
+  static constexpr uint32_t kHeld0 = 0, kHeld1 = kTight ? 0 : Held::kBytes, kTiles = kHeld1 + Held::kBytes;
   static constexpr uint32_t kBytes = kTiles + kStages * 2 * Tile::kBytes + 1024;
   static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols, kAfter = kP + 3 * kPieceCols;
-  static constexpr uint32_t kOut0 = kWide ? 0 : kAfter, kOut1 = kWide ? 0 : kAfter + HD;
-  static constexpr uint32_t kHeldT = kAfter;  // kWide: the first held operand, three pieces of HD / 2 columns
+  static constexpr uint32_t kOut0 = kTight ? 0 : kAfter, kOut1 = kTight ? 0 : kAfter + HD;
+  static constexpr uint32_t kHeldT = kAfter;  // kTight: the first held operand, three pieces of HD / 2 columns
   static constexpr int kCols = 512;
-  static_assert(kAfter + (kWide ? 3 * HD / 2 : 2 * HD) <= 512, "tensor memory");
+  static_assert(kAfter + (kTight ? 3 * HD / 2 : 2 * HD) <= 512, "tensor memory");
 };
 
-template <int HD, bool kKV>
-__global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
-  using L = Bwd<HD>;
+template <int HD, bool kKV, bool kWide>
+__global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
+  using L = Bwd<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
@@ -603,8 +615,8 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   auto stage_tile = [&](int j) {
     const int x0 = begin + j * kStream;
     typename L::Tile a, c;
-    a.load(stream0, x0, streamed, g.hd, g.wide_qk);
-    c.load(stream1, x0, streamed, g.hd_v, g.wide_v);
+    a.load(stream0, x0, streamed, g.hd);
+    c.load(stream1, x0, streamed, g.hd_v);
     if (kKV) {
       if (threadIdx.x < kStream) {
         const int x = x0 + threadIdx.x;
@@ -622,17 +634,17 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   };
   auto issue_tile = [&](int j) {
     tc_fence_after_sync();
-    issue_scores<HD, L::kWide>(tmem + L::kS, L::kWide ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0));
+    issue_scores<HD, L::kTight>(tmem + L::kS, L::kTight ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0));
     issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, tile_at(j, 1));
     mma_commit(scored);
   };
 
-  if constexpr (L::kWide) {
+  if constexpr (L::kTight) {
     uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
 #pragma unroll
     for (int c = 0; c < OW; c += 8) {
       float x[8];
-      load8(x, held0, mine, owned, group * OW + c, g.hd, g.wide_qk);
+      load8<kWide>(x, held0, mine, owned, group * OW + c, g.hd);
 #pragma unroll
       for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[2 * e], x[2 * e + 1]), h[c / 2 + e], m[c / 2 + e], l[c / 2 + e], check);
     }
@@ -644,12 +656,12 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
     tc_fence_before_sync();
   } else {
     typename L::Held stage;
-    stage.load(held0, first, owned, g.hd, g.wide_qk);
+    stage.load(held0, first, owned, g.hd);
     stage.store(base + L::kHeld0, check);
   }
   {
     typename L::Held stage;
-    stage.load(held1, first, owned, g.hd_v, g.wide_v);
+    stage.load(held1, first, owned, g.hd_v);
     stage.store(base + L::kHeld1, check);
   }
   if (n > 0) stage_tile(0);
@@ -738,7 +750,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
       if (kKV) {
         issue_weigh<HD>(tmem + L::kOut0, tmem + L::kP, tile_at(j, 1));
         mma_commit(weighed0);
-        if (!L::kWide) {
+        if (!L::kTight) {
           issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
           mma_commit(weighed1);
         }
@@ -748,7 +760,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
       }
     }
     const bool more = j + 1 < n;
-    if (!L::kWide && more) {
+    if (!L::kTight && more) {
       stage_tile(j + 1);  // into the other buffer, whose products were gathered a tile ago
       fence_async_shared();
       __syncthreads();
@@ -757,7 +769,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
     ok &= mbar_wait(weighed0, j & 1, g.status, 0x0b01u);
     gather(L::kOut0, acc0);
     if (kKV) {
-      if (L::kWide) {
+      if (L::kTight) {
         if (!__syncthreads_and(ok)) break;
         if (issues && elect_one()) {
           tc_fence_after_sync();
@@ -768,7 +780,7 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
       ok &= mbar_wait(weighed1, j & 1, g.status, 0x0b02u);
       gather(L::kOut1, acc1);
     }
-    if (L::kWide && more) {
+    if (L::kTight && more) {
       stage_tile(j + 1);
       fence_async_shared();
       if (!__syncthreads_and(ok)) break;
@@ -791,11 +803,12 @@ __global__ void __launch_bounds__(Bwd<HD>::kThreads, 1) f32_bwd_kernel(const __g
   tear_down<L::kCols>(g, tmem);
 }
 
-template <int HD>
+bool aligned(const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; }  // (null is)
+
+template <int HD, bool kWide>
 int launch_sized(Op op, const Problem& p) {
   Params g = {};
   auto in = [](const void* x) { return static_cast<const float*>(x); };
-  auto aligned = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; };  // (null is)
   g.q = in(p.q), g.k = in(p.k), g.v = in(p.v), g.mask = in(p.mask), g.dout = in(p.dout), g.lse_in = in(p.lse_in), g.delta = in(p.delta);
   g.out = static_cast<float*>(p.out), g.lse_out = static_cast<float*>(p.lse_out);
   g.dq = static_cast<float*>(p.dq), g.dk = static_cast<float*>(p.dk), g.dv = static_cast<float*>(p.dv);
@@ -811,8 +824,6 @@ int launch_sized(Op op, const Problem& p) {
   if (g.c_hi > c) g.c_hi = nextafterf(g.c_hi, 0.f);
   g.c_lo = static_cast<float>(c - g.c_hi);
   if (!(g.c_lo > 0.f)) g.c_lo = 1e-37f;  // a score of -inf has to stay one
-  g.wide_qk = p.hd % 4 == 0 && aligned(p.q) && aligned(p.k);
-  g.wide_v = p.hd_v % 4 == 0 && aligned(p.v) && aligned(p.dout);
   g.wide_out = p.hd % 4 == 0 && p.hd_v % 4 == 0;
   if (op == Op::Fwd) g.wide_out = g.wide_out && aligned(p.out);
   else g.wide_out = g.wide_out && aligned(p.dq) && aligned(p.dk) && aligned(p.dv);
@@ -820,9 +831,11 @@ int launch_sized(Op op, const Problem& p) {
   int sms = 0;
   if (int rc = sm_count(&sms)) return rc;
   g.group = work_group(p, blocks, sms);
-  using F = Fwd<HD>;
-  using B = Bwd<HD>;
-  void (*kernel)(const Params) = op == Op::Fwd ? f32_fwd_kernel<HD> : op == Op::BwdQ ? f32_bwd_kernel<HD, false> : f32_bwd_kernel<HD, true>;
+  using F = Fwd<HD, kWide>;
+  using B = Bwd<HD, kWide>;
+  void (*kernel)(const Params) = op == Op::Fwd    ? f32_fwd_kernel<HD, kWide>
+                                : op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide>
+                                                 : f32_bwd_kernel<HD, true, kWide>;
   const uint32_t shared = op == Op::Fwd ? F::kBytes : B::kBytes;
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64][3] = {};
@@ -854,9 +867,10 @@ bool f32_split_serves(Op op, const Problem& p) {
 
 int f32_split_launch(Op op, const Problem& p) {
   const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
-  if (widest <= 32) return launch_sized<32>(op, p);
-  if (widest <= 64) return launch_sized<64>(op, p);
-  return launch_sized<128>(op, p);
+  const bool wide = p.hd % 4 == 0 && p.hd_v % 4 == 0 && aligned(p.q) && aligned(p.k) && aligned(p.v) && aligned(p.dout);
+  if (widest <= 32) return wide ? launch_sized<32, true>(op, p) : launch_sized<32, false>(op, p);
+  if (widest <= 64) return wide ? launch_sized<64, true>(op, p) : launch_sized<64, false>(op, p);
+  return wide ? launch_sized<128, true>(op, p) : launch_sized<128, false>(op, p);
 }
 
 }  // namespace limn_b200
