@@ -152,8 +152,10 @@ __device__ __host__ constexpr int piece_b(int i) { return (0x010120 >> (4 * i)) 
 // memory (a0 its address) or in tensor memory (a0 its column, pieces HD / 2 columns apart). Columns past the head dim are
 // zero on both sides. Fully unrolled over compile-time offsets: one thread issues every MMA of the block, and with a
 // loop over the steps it took 115 clocks an MMA instead of the 32 the tensor cores need.
-template <int HD, bool kTmemA>
-__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0) {
+// kTwo: the last half of the largest products goes to a second accumulator, kStream columns of it at d2, so that a score
+// takes no more than four truncated additions at its full size at head dim 128 either.
+template <int HD, bool kTmemA, bool kTwo = false>
+__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0, uint32_t d2 = 0) {
   constexpr uint32_t kPieceA = (HD > 64 ? 2 : 1) * kRows * 128, kPieceB = (HD > 64 ? 2 : 1) * kStream * 128;
   constexpr uint32_t idesc = mma_idesc(kRows, kStream, false, false, false);
   const uint32_t a_lo = kTmemA ? a0 : desc_lo(a0, 0), b_lo = desc_lo(b0, 0);
@@ -162,9 +164,16 @@ __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b
 #pragma unroll
     for (int s = 0; s < HD / 16; ++s) {
       const uint32_t b = b_lo + piece_b(i) * (kPieceB / 16) + (s / 4) * (kStream * 128 / 16) + (s % 4) * 2;
-      if constexpr (kTmemA) mma_ts_lo(d, a_lo + piece_a(i) * (HD / 2) + s * 8, b, idesc, i > 0 || s > 0);
-      else if (i == 0 && s == 0) mma_ss_lo<false>(d, a_lo + piece_a(i) * (kPieceA / 16), b, idesc);
-      else mma_ss_lo<true>(d, a_lo + piece_a(i) * (kPieceA / 16) + (s / 4) * (kRows * 128 / 16) + (s % 4) * 2, b, idesc);
+      const bool second = kTwo && i == 5 && s >= HD / 32;
+      const bool starts = (i == 0 && s == 0) || (second && s == HD / 32);
+      const uint32_t to = second ? d2 : d;
+      if constexpr (kTmemA) {
+        mma_ts_lo(to, a_lo + piece_a(i) * (HD / 2) + s * 8, b, idesc, starts ? 0u : 1u);
+      } else {
+        const uint32_t a = a_lo + piece_a(i) * (kPieceA / 16) + (s / 4) * (kRows * 128 / 16) + (s % 4) * 2;
+        if (starts) mma_ss_lo<false>(to, a, b, idesc);
+        else mma_ss_lo<true>(to, a, b, idesc);
+      }
     }
   }
 }
@@ -321,11 +330,13 @@ __device__ __noinline__ void plain_bwd(const Params& g, long long b, int first, 
 
 // ---- block set-up and teardown shared by the kernels ----
 // False: an earlier kernel on this device gave up on a wait, take no work.
+// Barriers whose bit is set in `by_warps` expect `warps` arrivals, the others one.
 template <int kCols, int kBars>
-__device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t* abort_flag, uint64_t* bars, uint32_t& tmem) {
+__device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t* abort_flag, uint64_t* bars, uint32_t& tmem,
+                                       uint32_t by_warps = 0u, uint32_t warps = 1u) {
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < kBars; ++i) mbar_init(smem_addr(bars + i), 1);
+    for (int i = 0; i < kBars; ++i) mbar_init(smem_addr(bars + i), (by_warps >> i) & 1u ? warps : 1u);
     mbar_init_fence();
   }
   grid_dependency_wait();
@@ -357,11 +368,19 @@ __device__ __forceinline__ void tear_down(const Params& g, uint32_t tmem) {
   }
 }
 
-// The hidden keys of tile [j0, j0 + kStream) as two words in shared memory (bit set = hidden).
-__device__ __forceinline__ void post_hidden(uint32_t* words, const float* mask, int j0, int t_k) {
+// One float a row of the tile that starts at j0, zero beyond the end: thread i < kStream has row i's.
+__device__ __forceinline__ float row_value(const float* from, int j0, int rows) {
+  const int j = j0 + static_cast<int>(threadIdx.x);
+  float x;  // (as in load8: nothing waits for it here)
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
+               : "=&f"(x)
+               : "l"(from + j), "r"(threadIdx.x < kStream && j < rows ? 1u : 0u));
+  return x;
+}
+// The hidden keys of a tile (flag 0, keys past the end among them) as two words in shared memory, bit set = hidden.
+__device__ __forceinline__ void post_hidden(uint32_t* words, float flag) {
   if (threadIdx.x < kStream) {
-    const int j = j0 + threadIdx.x;
-    const unsigned hid = __ballot_sync(kFull, j >= t_k || mask[j] == 0.f);
+    const unsigned hid = __ballot_sync(kFull, flag == 0.f);
     if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = hid;
   }
 }
@@ -383,7 +402,8 @@ struct Fwd {
   using Held = Stage<HD, kRows, kThreads, kWide>;
   using Tile = Stage<HD, kStream, kThreads, kWide>;
   static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
-  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols;
+  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kS2 = kO + HD;
+  static constexpr bool kTwo = HD > 64;
   static constexpr int kCols = HD > 64 ? 512 : 256;
 };
 
@@ -417,21 +437,23 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
 
   uint64_t check = 0;
   typename L::Tile stage_k, stage_v;
-  stage_k.load(k, 0, g.t_k, g.hd);
   {
+    // every load is on its way before the first one is waited for
     typename L::Held stage_q;
     stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd);
+    stage_k.load(k, 0, g.t_k, g.hd);
+    stage_v.load(v, 0, g.t_k, g.hd_v);
+    const float flag = mask ? row_value(mask, 0, g.t_k) : 0.f;
     stage_q.store(base + L::kQ, check);
+    stage_k.store(base + L::kK, check);
+    if (mask) post_hidden(hidden[0], flag);
   }
-  stage_k.store(base + L::kK, check);
-  if (mask) post_hidden(hidden[0], mask, 0, g.t_k);
   fence_async_shared();
   __syncthreads();
   if (issues && elect_one()) {
-    issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
+    issue_scores<HD, false, L::kTwo>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
     mma_commit(scored);
   }
-  stage_v.load(v, 0, g.t_k, g.hd_v);
   stage_v.store(base + L::kV, check);
   fence_async_shared();
 
@@ -447,7 +469,15 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     tc_fence_after_sync();
     uint32_t s[CW];
     tmem_ld<CW>(lanes + L::kS + group * CW, s);
-    tmem_ld_wait();
+    if constexpr (L::kTwo) {
+      uint32_t more_s[CW];
+      tmem_ld<CW>(lanes + L::kS2 + group * CW, more_s);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < CW; ++c) s[c] = __float_as_uint(__uint_as_float(s[c]) + __uint_as_float(more_s[c]));
+    } else {
+      tmem_ld_wait();
+    }
     int limit = g.t_k - j0;
     if (g.causal) limit = min(limit, i - j0 + 1);
     limit -= group * CW;
@@ -496,13 +526,14 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     if (more) {
       // K's buffer has been read (the scores are there) and so have the scores themselves
       stage_k.load(k, j0 + kStream, g.t_k, g.hd);
+      const float flag = mask ? row_value(mask, j0 + kStream, g.t_k) : 0.f;
       stage_k.store(base + L::kK, check);
-      if (mask) post_hidden(hidden[(j + 1) & 1], mask, j0 + kStream, g.t_k);
+      if (mask) post_hidden(hidden[(j + 1) & 1], flag);
       fence_async_shared();
       __syncthreads();
       if (issues && elect_one()) {
         tc_fence_after_sync();
-        issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
+        issue_scores<HD, false, L::kTwo>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
         mma_commit(scored);
       }
       stage_v.load(v, j0 + kStream, g.t_k, g.hd_v);
@@ -549,9 +580,305 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   tear_down<L::kCols>(g, tmem);
 }
 
+// log2(e) in two parts: a log-sum-exp in log2 units, as hi + lo
+__device__ __forceinline__ void to_log2(const float lse, float& hi, float& lo) {
+  constexpr float kHi = 1.44269502f, kLo = 1.92596303e-8f;
+  hi = lse * kHi;
+  lo = fmaf(lse, kHi, -hi) + lse * kLo;
+}
+
+// What both backward kernels do with the scores of a row: P = 2^(s c - L), dS = P (dP - delta) scale, 0 where unseen.
+// `hi`, `lo`, `delta` give a column's L (in log2 units) and delta; a row's own ones repeated in the dQ pass.
+template <int CW, typename Columns>
+__device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s)[CW], const uint32_t (&dp)[CW], uint32_t unseen,
+                                             Columns columns, uint64_t (&p)[CW / 2], uint64_t (&ds)[CW / 2]) {
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale = f2_pack(g.scale, g.scale);
+  const uint64_t minus = f2_pack(-1.f, -1.f);
+#pragma unroll
+  for (int c = 0; c < CW / 2; ++c) {
+    uint64_t hi, lo, delta;
+    columns(2 * c, hi, lo, delta);
+    const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
+    const uint64_t x = f2_add(f2_fma(s2, c_hi, hi ^ 0x8000000080000000ull), f2_fma(s2, c_lo, lo ^ 0x8000000080000000ull));
+    float a, b;
+    f2_unpack(x, a, b);
+    p[c] = f2_pack(exp2_approx(a), exp2_approx(b));
+    ds[c] = f2_mul(f2_mul(p[c], f2_fma(delta, minus, f2_pack_bits(dp[2 * c], dp[2 * c + 1]))), scale);
+  }
+  if (unseen != 0u) {  // (dS too: delta of a row with no key is NaN)
+#pragma unroll
+    for (int c = 0; c < CW / 2; ++c) {
+      float a, b;
+      f2_unpack(p[c], a, b);
+      p[c] = f2_pack((unseen >> (2 * c)) & 1u ? 0.f : a, (unseen >> (2 * c + 1)) & 1u ? 0.f : b);
+      f2_unpack(ds[c], a, b);
+      ds[c] = f2_pack((unseen >> (2 * c)) & 1u ? 0.f : a, (unseen >> (2 * c + 1)) & 1u ? 0.f : b);
+    }
+  }
+}
+
+// The columns of a thread's CW that its row does not see: outside [from, to), as bits.
+template <int CW>
+__device__ __forceinline__ uint32_t outside(int from, int to) {
+  uint32_t unseen = 0;
+  if (from > 0) unseen |= from >= CW ? kFull : (1u << from) - 1u;
+  if (to < CW) unseen |= to <= 0 ? kFull : ~((1u << to) - 1u);
+  return unseen;
+}
+
+// ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
+// Sixteen row warps (four threads to a row) load, split, weigh and sum; a seventeenth issues every MMA. It used to be one
+// of the sixteen: issuing a tile's MMAs takes as long as the tensor cores take to run them (2400 + 1160 clocks of the
+// 5200 a dQ tile took at head dim 64), the other fifteen had nothing to do meanwhile, and the tensor cores nothing while
+// the sixteenth caught up. Now a tile's scores run while the tile before it is weighed. Rows and issuer tell each other
+// through mbarriers whose waits are bounded; no barrier of the block stands inside the loop, so a warp that gave up on a
+// wait cannot hang the others.
+template <int HD, bool kKV, bool kWide>
+struct Pipe {
+  static constexpr int kGroups = 4, kRowThreads = kRows * kGroups, kThreads = kRowThreads + 32;
+  using Held = Stage<HD, kRows, kRowThreads, kWide>;
+  using Tile = Stage<HD, kStream, kRowThreads, kWide>;
+  // tensor memory: scores, dP, the pieces of dS and (dK/dV) of P, a tile's products, and the held operands if they fit:
+  // they are the A side of the scores, an MMA then only reads the streamed tile from shared memory (whose bandwidth
+  // bounds it at 48 clocks with both there, for 32), and shared memory holds four tiles instead of two
+  static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols;
+  static constexpr uint32_t kOut0 = kKV ? kP + 3 * kPieceCols : kP, kOut1 = kOut0 + HD, kHeldCol = kKV ? kOut1 + HD : kOut1;
+  static constexpr bool kHeldT = kHeldCol + 3 * HD <= 512;
+  static constexpr int kStages = kHeldT ? 4 : 2;
+  static constexpr uint32_t kHeld0 = 0, kHeld1 = Held::kBytes, kTiles = kHeldT ? 0 : 2 * Held::kBytes;
+  static constexpr uint32_t kBytes = kTiles + kStages * 2 * Tile::kBytes + 1024;
+  static constexpr int kCols = 512;
+};
+
+template <int HD, bool kKV, bool kWide>
+__global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
+  using L = Pipe<HD, kKV, kWide>;
+  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G, kRowWarps = L::kRowThreads / 32;
+  extern __shared__ unsigned char raw[];
+  __shared__ uint32_t slot, abort_flag, hidden[L::kStages][2];
+  __shared__ __align__(8) uint64_t bars[8];
+  __shared__ __align__(16) float lse_hi[L::kStages][kStream], lse_lo[L::kStages][kStream], deltas[L::kStages][kStream];
+  uint32_t tmem;
+  // scored, weighed: by the tensor cores; free (the scores have been read), handed (P, dS are there), staged[stage]: by the row warps
+  if (!set_up<L::kCols, 8>(g, &slot, &abort_flag, bars, tmem, 0xfcu, kRowWarps)) return;
+  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1), free_ = smem_addr(bars + 2), handed = smem_addr(bars + 3);
+  auto staged = [&](int j) { return smem_addr(bars + 4 + j % L::kStages); };
+  auto staged_parity = [&](int j) { return static_cast<uint32_t>(j / L::kStages) & 1u; };
+  const uint32_t base = align_1024(smem_addr(raw));
+  const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  int problem, at;
+  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
+  const int first = (kKV ? at : g.slots - 1 - at) * kRows;  // the longest causal streams first
+  const long long b = problem;
+  // the held pair (against which the tiles are scored) and the streamed pair
+  const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
+  const int begin = kKV && g.causal ? first : 0;
+  const int end = !kKV && g.causal ? min(streamed, first + kRows) : streamed;
+  const int n = (end - begin + kStream - 1) / kStream;
+  auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
+  bool ok = true;
+  uint64_t check = 0;
+
+  if (warp == kRowWarps) {
+    // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
+    for (int j = -1; j < n; ++j) {
+      if (j + 1 < n) {
+        ok = mbar_wait(staged(j + 1), staged_parity(j + 1), g.status, 0x0b10u);
+        if (j >= 0) ok = ok && mbar_wait(free_, j & 1, g.status, 0x0b11u);
+        ok = __all_sync(kFull, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_scores<HD, L::kHeldT>(tmem + L::kS, L::kHeldT ? tmem + L::kHeldCol : base + L::kHeld0, tile_at(j + 1, 0));
+          issue_scores<HD, L::kHeldT>(tmem + L::kDp, L::kHeldT ? tmem + L::kHeldCol + 3 * HD / 2 : base + L::kHeld1, tile_at(j + 1, 1));
+          mma_commit(scored);
+        }
+        __syncwarp();
+      }
+      if (j >= 0) {
+        ok = __all_sync(kFull, mbar_wait(handed, j & 1, g.status, 0x0b12u));
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          if (kKV) issue_weigh<HD>(tmem + L::kOut1, tmem + L::kP, tile_at(j, 1));
+          issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile_at(j, 0));
+          mma_commit(weighed);
+        }
+        __syncwarp();
+      }
+    }
+    ok = __syncthreads_and(ok);
+    __syncthreads_or(0);
+  } else {
+    // ================= row warps =================
+    const int group = warp >> 2;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const float* held0 = (kKV ? g.k : g.q) + b * owned * g.hd;
+    const float* held1 = (kKV ? g.v : g.dout) + b * owned * g.hd_v;
+    const float* stream0 = (kKV ? g.q : g.k) + b * streamed * g.hd;
+    const float* stream1 = (kKV ? g.dout : g.v) + b * streamed * g.hd_v;
+    const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
+    const int mine = first + row;  // this thread's row
+    auto arrive = [&](uint32_t bar) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    // the streamed tile j, and what goes with its rows: to registers, and from there to shared memory
+    typename L::Tile tile0, tile1;
+    float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
+    auto load_tile = [&](int j) {
+      const int x0 = begin + j * kStream;
+      tile0.load(stream0, x0, streamed, g.hd);
+      tile1.load(stream1, x0, streamed, g.hd_v);
+      if (kKV) {
+        row_a = row_value(g.lse_in + b * g.t_q, x0, streamed);
+        row_b = row_value(g.delta + b * g.t_q, x0, streamed);
+      } else if (mask) {
+        row_a = row_value(mask, x0, streamed);
+      }
+    };
+    auto store_tile = [&](int j) {
+      if (kKV) {
+        if (threadIdx.x < kStream) {
+          float hi, lo;
+          to_log2(row_a, hi, lo);
+          lse_hi[j % L::kStages][threadIdx.x] = hi;
+          lse_lo[j % L::kStages][threadIdx.x] = lo;
+          deltas[j % L::kStages][threadIdx.x] = row_b;
+        }
+      } else if (mask) {
+        post_hidden(hidden[j % L::kStages], row_a);
+      }
+      tile0.store(tile_at(j, 0), check);
+      tile1.store(tile_at(j, 1), check);
+      fence_async_shared();
+      arrive(staged(j));
+    };
+
+    // every load is on its way before the first one is waited for
+    float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
+    bool live = mine < owned;
+    if constexpr (L::kHeldT) {
+      float x[2][OW / 8][8];
+#pragma unroll
+      for (int c = 0; c < OW / 8; ++c) {
+        load8<kWide>(x[0][c], held0, mine, owned, group * OW + 8 * c, g.hd);
+        load8<kWide>(x[1][c], held1, mine, owned, group * OW + 8 * c, g.hd_v);
+      }
+      load_tile(0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int c = 0; c < OW / 8; ++c) {
+          uint32_t hi[4], mi[4], lo[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
+          const uint32_t to = lanes + L::kHeldCol + h * (3 * HD / 2) + group * (OW / 2) + 4 * c;
+          tmem_st4(to, hi);
+          tmem_st4(to + HD / 2, mi);
+          tmem_st4(to + HD, lo);
+        }
+      tmem_st_wait();
+      tc_fence_before_sync();
+    } else {
+      typename L::Held stage0, stage1;
+      stage0.load(held0, first, owned, g.hd);
+      stage1.load(held1, first, owned, g.hd_v);
+      load_tile(0);
+      stage0.store(base + L::kHeld0, check);
+      stage1.store(base + L::kHeld1, check);
+    }
+    if constexpr (kKV) {
+      if (live && mask) live = mask[mine] != 0.f;
+    } else if (live) {
+      to_log2(g.lse_in[b * g.t_q + mine], my_hi, my_lo);
+      my_delta = g.delta[b * g.t_q + mine];
+    }
+    store_tile(0);  // (says that the held rows are there, too)
+    if (n > 1) {
+      load_tile(1);
+      store_tile(1);
+    }
+    if (n > 2) load_tile(2);
+
+    uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dK and dV
+#pragma unroll
+    for (int c = 0; c < OW / 2; ++c) acc0[c] = acc1[c] = 0;
+    auto gather = [&](uint32_t from, uint64_t(&acc)[OW / 2]) {
+      uint32_t o[OW];
+      tmem_ld<OW>(lanes + from + group * OW, o);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < OW / 2; ++c) acc[c] = f2_add(acc[c], f2_pack_bits(o[2 * c], o[2 * c + 1]));
+    };
+    for (int j = 0; j < n; ++j) {
+      const int x0 = begin + j * kStream;
+      if (kKV || mask) ok = mbar_wait(staged(j), staged_parity(j), g.status, 0x0b20u);
+      ok = __all_sync(kFull, ok && mbar_wait(scored, j & 1, g.status, 0x0b21u));
+      if (!ok) break;
+      tc_fence_after_sync();
+      uint32_t s[CW], dp[CW];
+      tmem_ld<CW>(lanes + L::kS + group * CW, s);
+      tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      arrive(free_);
+      int from = 0, to = streamed - x0 - group * CW;
+      if (g.causal) {
+        if (kKV) from = mine - x0 - group * CW;
+        else to = min(to, mine - x0 - group * CW + 1);
+      }
+      uint32_t unseen = outside<CW>(from, live ? to : 0);
+      if (!kKV && mask) unseen |= my_hidden<CW>(hidden[j % L::kStages], group);
+      uint64_t p[CW / 2], ds[CW / 2];
+      weigh_scores<CW>(g, s, dp, unseen, [&](int c, uint64_t& hi, uint64_t& lo, uint64_t& delta) {
+        if (kKV) {
+          hi = *reinterpret_cast<const uint64_t*>(&lse_hi[j % L::kStages][group * CW + c]);
+          lo = *reinterpret_cast<const uint64_t*>(&lse_lo[j % L::kStages][group * CW + c]);
+          delta = *reinterpret_cast<const uint64_t*>(&deltas[j % L::kStages][group * CW + c]);
+        } else {
+          hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
+        }
+      }, p, ds);
+      // (the products of the tile before have been gathered, so its P and dS have been read)
+      hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, check);
+      if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      arrive(handed);
+      // tile j + 2 takes the place of tile j + 2 - kStages: gathered already, or now about to be
+      if (L::kStages > 2 && j + 2 < n) store_tile(j + 2);
+      if (L::kStages > 2 && j + 3 < n) load_tile(j + 3);
+      ok = __all_sync(kFull, mbar_wait(weighed, j & 1, g.status, 0x0b22u));
+      if (!ok) break;
+      tc_fence_after_sync();
+      gather(L::kOut0, acc0);
+      if (kKV) gather(L::kOut1, acc1);
+      tc_fence_before_sync();
+      if (L::kStages == 2 && j + 2 < n) store_tile(j + 2);
+      if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
+    }
+    ok = __syncthreads_and(ok);
+    const bool bad = __syncthreads_or(is_bad(check));
+    if (ok && bad) {
+      plain_bwd<kKV>(g, b, first, L::kRowThreads);
+    } else if (ok && mine < owned) {
+      if (kKV) {
+        store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
+        store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc1, group * OW, g.hd_v, g.wide_out);
+      } else {
+        store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
+      }
+    }
+  }
+  tear_down<L::kCols>(g, tmem);
+}
+
 // ---- backward: dQ for 128 query rows, or dK and dV for 128 key rows ----
 template <int HD, bool kWide>
-struct Bwd {
+struct BwdWide {
   static constexpr int kGroups = 4;
   static constexpr int kThreads = kRows * kGroups;
   // At head dims above 64 two held operands and two streamed tiles do not fit in shared memory twice over: the first
@@ -571,8 +898,8 @@ struct Bwd {
 };
 
 template <int HD, bool kKV, bool kWide>
-__global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
-  using L = Bwd<HD, kWide>;
+__global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_kernel(const __grid_constant__ Params g) {
+  using L = BwdWide<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
@@ -603,34 +930,37 @@ __global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(co
   const int n = (end - begin + kStream - 1) / kStream;
   const int mine = first + row;  // this thread's row
 
-  constexpr float kLog2eHi = 1.44269502f, kLog2eLo = 1.92596303e-8f;  // log2(e) in two parts
-  auto to_log2 = [&](float lse, float& hi, float& lo) {
-    hi = lse * kLog2eHi;
-    lo = fmaf(lse, kLog2eHi, -hi) + lse * kLog2eLo;
-  };
-
   uint64_t check = 0;
   auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
-  // the streamed tile j, and what goes with its rows
-  auto stage_tile = [&](int j) {
+  // the streamed tile j, and what goes with its rows: to registers, and from there to shared memory
+  typename L::Tile tile0, tile1;
+  float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
+  auto load_tile = [&](int j) {
     const int x0 = begin + j * kStream;
-    typename L::Tile a, c;
-    a.load(stream0, x0, streamed, g.hd);
-    c.load(stream1, x0, streamed, g.hd_v);
+    tile0.load(stream0, x0, streamed, g.hd);
+    tile1.load(stream1, x0, streamed, g.hd_v);
+    if (kKV) {
+      row_a = row_value(g.lse_in + b * g.t_q, x0, streamed);
+      row_b = row_value(g.delta + b * g.t_q, x0, streamed);
+    } else if (mask) {
+      row_a = row_value(mask, x0, streamed);
+    }
+  };
+  auto store_tile = [&](int j) {
     if (kKV) {
       if (threadIdx.x < kStream) {
-        const int x = x0 + threadIdx.x;
         float hi, lo;
-        to_log2(x < streamed ? g.lse_in[b * g.t_q + x] : 0.f, hi, lo);
+        to_log2(row_a, hi, lo);
         lse_hi[j & 1][threadIdx.x] = hi;
         lse_lo[j & 1][threadIdx.x] = lo;
-        deltas[j & 1][threadIdx.x] = x < streamed ? g.delta[b * g.t_q + x] : 0.f;
+        deltas[j & 1][threadIdx.x] = row_b;
       }
     } else if (mask) {
-      post_hidden(hidden[j & 1], mask, x0, g.t_k);
+      post_hidden(hidden[j & 1], row_a);
     }
-    a.store(tile_at(j, 0), check);
-    c.store(tile_at(j, 1), check);
+    tile0.store(tile_at(j, 0), check);
+    tile1.store(tile_at(j, 1), check);
+    fence_async_shared();
   };
   auto issue_tile = [&](int j) {
     tc_fence_after_sync();
@@ -639,44 +969,47 @@ __global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(co
     mma_commit(scored);
   };
 
-  if constexpr (L::kTight) {
-    uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
-#pragma unroll
-    for (int c = 0; c < OW; c += 8) {
-      float x[8];
-      load8<kWide>(x, held0, mine, owned, group * OW + c, g.hd);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[2 * e], x[2 * e + 1]), h[c / 2 + e], m[c / 2 + e], l[c / 2 + e], check);
-    }
-    const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
-    tmem_st<OW / 2>(to, h);
-    tmem_st<OW / 2>(to + HD / 2, m);
-    tmem_st<OW / 2>(to + HD, l);
-    tmem_st_wait();
-    tc_fence_before_sync();
-  } else {
-    typename L::Held stage;
-    stage.load(held0, first, owned, g.hd);
-    stage.store(base + L::kHeld0, check);
-  }
-  {
-    typename L::Held stage;
-    stage.load(held1, first, owned, g.hd_v);
-    stage.store(base + L::kHeld1, check);
-  }
-  if (n > 0) stage_tile(0);
-  fence_async_shared();
-  __syncthreads();
-  if (n > 0 && issues && elect_one()) issue_tile(0);
-
+  // every load is on its way before the first one is waited for
   float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
   bool live = mine < owned;
-  if constexpr (kKV) {
-    if (live && mask) live = mask[mine] != 0.f;
-  } else {
-    if (live) to_log2(g.lse_in[b * g.t_q + mine], my_hi, my_lo);
-    if (live) my_delta = g.delta[b * g.t_q + mine];
+  {
+    typename L::Held stage1;
+    if constexpr (L::kTight) {
+      float x[OW / 8][8];
+#pragma unroll
+      for (int c = 0; c < OW / 8; ++c) load8<kWide>(x[c], held0, mine, owned, group * OW + 8 * c, g.hd);
+      stage1.load(held1, first, owned, g.hd_v);
+      uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
+#pragma unroll
+      for (int e = 0; e < OW / 2; ++e) split_pair(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
+      const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
+      tmem_st<OW / 2>(to, h);
+      tmem_st<OW / 2>(to + HD / 2, m);
+      tmem_st<OW / 2>(to + HD, l);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      load_tile(0);
+    } else {
+      typename L::Held stage0;
+      stage0.load(held0, first, owned, g.hd);
+      stage1.load(held1, first, owned, g.hd_v);
+      load_tile(0);
+      stage0.store(base + L::kHeld0, check);
+    }
+    if constexpr (kKV) {
+      if (live && mask) live = mask[mine] != 0.f;
+    } else if (live) {
+      my_hi = g.lse_in[b * g.t_q + mine];
+      my_delta = g.delta[b * g.t_q + mine];
+    }
+    stage1.store(base + L::kHeld1, check);
   }
+  store_tile(0);  // (fences the held rows too)
+  __syncthreads();
+  if (issues && elect_one()) issue_tile(0);
+  if (!L::kTight && n > 1) load_tile(1);
+
+  if constexpr (!kKV) to_log2(my_hi, my_hi, my_lo);
 
   uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dV and dK
 #pragma unroll
@@ -700,6 +1033,15 @@ __global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(co
     tmem_ld<CW>(lanes + L::kS + group * CW, s);
     tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
     tmem_ld_wait();
+    const bool more = j + 1 < n;
+    if (!L::kTight && more) {
+      // the scores' place is free, and so is the other buffer, whose products were gathered a tile ago: the next tile's
+      // scores are on their way before this one's dS is worked out
+      tc_fence_before_sync();
+      store_tile(j + 1);
+      __syncthreads();
+      if (issues && elect_one()) issue_tile(j + 1);
+    }
     // columns [from, to) of this thread's CW are seen, less the hidden ones
     int from = 0, to = streamed - x0 - group * CW;
     if (g.causal) {
@@ -759,13 +1101,7 @@ __global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(co
         mma_commit(weighed0);
       }
     }
-    const bool more = j + 1 < n;
-    if (!L::kTight && more) {
-      stage_tile(j + 1);  // into the other buffer, whose products were gathered a tile ago
-      fence_async_shared();
-      __syncthreads();
-      if (issues && elect_one()) issue_tile(j + 1);
-    }
+    if (!L::kTight && j + 2 < n) load_tile(j + 2);
     ok &= mbar_wait(weighed0, j & 1, g.status, 0x0b01u);
     gather(L::kOut0, acc0);
     if (kKV) {
@@ -781,8 +1117,8 @@ __global__ void __launch_bounds__(Bwd<HD, kWide>::kThreads, 1) f32_bwd_kernel(co
       gather(L::kOut1, acc1);
     }
     if (L::kTight && more) {
-      stage_tile(j + 1);
-      fence_async_shared();
+      load_tile(j + 1);
+      store_tile(j + 1);
       if (!__syncthreads_and(ok)) break;
       if (issues && elect_one()) issue_tile(j + 1);
     }
@@ -832,11 +1168,20 @@ int launch_sized(Op op, const Problem& p) {
   if (int rc = sm_count(&sms)) return rc;
   g.group = work_group(p, blocks, sms);
   using F = Fwd<HD, kWide>;
-  using B = Bwd<HD, kWide>;
-  void (*kernel)(const Params) = op == Op::Fwd    ? f32_fwd_kernel<HD, kWide>
-                                : op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide>
-                                                 : f32_bwd_kernel<HD, true, kWide>;
-  const uint32_t shared = op == Op::Fwd ? F::kBytes : B::kBytes;
+  void (*kernel)(const Params) = f32_fwd_kernel<HD, kWide>;
+  uint32_t shared = F::kBytes, threads = F::kThreads;
+  if (op != Op::Fwd) {
+    if constexpr (HD > 64) {
+      using B = BwdWide<HD, kWide>;
+      kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
+      shared = B::kBytes, threads = B::kThreads;
+    } else {
+      using Q = Pipe<HD, false, kWide>;
+      using KV = Pipe<HD, true, kWide>;
+      kernel = op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide> : f32_bwd_kernel<HD, true, kWide>;
+      shared = op == Op::BwdQ ? Q::kBytes : KV::kBytes, threads = Q::kThreads;
+    }
+  }
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64][3] = {};
   int device = 0;
@@ -846,7 +1191,7 @@ int launch_sized(Op op, const Problem& p) {
               "sizing shared memory for a float32 sdpa kernel");
     if (device >= 0 && device < 64) sized[device][static_cast<int>(op)] = true;
   }
-  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks)), dim3(op == Op::Fwd ? F::kThreads : B::kThreads), shared, p.stream, g),
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks)), dim3(threads), shared, p.stream, g),
             "launching a float32 sdpa kernel");
   note_launches(1);
   return LIMN_B200_OK;
