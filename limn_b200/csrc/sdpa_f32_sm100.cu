@@ -656,12 +656,13 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G, kRowWarps = L::kRowThreads / 32;
   extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[L::kStages][2];
-  __shared__ __align__(8) uint64_t bars[8];
+  __shared__ __align__(8) uint64_t bars[9];
   __shared__ __align__(16) float lse_hi[L::kStages][kStream], lse_lo[L::kStages][kStream], deltas[L::kStages][kStream];
   uint32_t tmem;
-  // scored, weighed: by the tensor cores; free (the scores have been read), handed (P, dS are there), staged[stage]: by the row warps
-  if (!set_up<L::kCols, 8>(g, &slot, &abort_flag, bars, tmem, 0xfcu, kRowWarps)) return;
-  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1), free_ = smem_addr(bars + 2), handed = smem_addr(bars + 3);
+  // scored, weighed, weighed_p (dK/dV: dV's products, the first of the two): by the tensor cores; free (the scores have
+  // been read), handed (P, dS are there), staged[stage]: by the row warps
+  if (!set_up<L::kCols, 9>(g, &slot, &abort_flag, bars, tmem, 0xfcu, kRowWarps)) return;
+  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1), weighed_p = smem_addr(bars + 8), free_ = smem_addr(bars + 2), handed = smem_addr(bars + 3);
   auto staged = [&](int j) { return smem_addr(bars + 4 + j % L::kStages); };
   auto staged_parity = [&](int j) { return static_cast<uint32_t>(j / L::kStages) & 1u; };
   const uint32_t base = align_1024(smem_addr(raw));
@@ -701,7 +702,10 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
         if (!ok) break;
         tc_fence_after_sync();
         if (elect_one()) {
-          if (kKV) issue_weigh<HD>(tmem + L::kOut1, tmem + L::kP, tile_at(j, 1));
+          if (kKV) {
+            issue_weigh<HD>(tmem + L::kOut1, tmem + L::kP, tile_at(j, 1));
+            mma_commit(weighed_p);
+          }
           issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile_at(j, 0));
           mma_commit(weighed);
         }
@@ -739,7 +743,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
         row_a = row_value(mask, x0, streamed);
       }
     };
-    auto store_tile = [&](int j) {
+    auto store_tile = [&](int j, bool split = false) {  // split: the second operand and the rows' values only
       if (kKV) {
         if (threadIdx.x < kStream) {
           float hi, lo;
@@ -751,10 +755,12 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       } else if (mask) {
         post_hidden(hidden[j % L::kStages], row_a);
       }
-      tile0.store(tile_at(j, 0), check);
       tile1.store(tile_at(j, 1), check);
-      fence_async_shared();
-      arrive(staged(j));
+      if (!split) {
+        tile0.store(tile_at(j, 0), check);
+        fence_async_shared();
+        arrive(staged(j));
+      }
     };
 
     // every load is on its way before the first one is waited for
@@ -851,13 +857,23 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       // tile j + 2 takes the place of tile j + 2 - kStages: gathered already, or now about to be
       if (L::kStages > 2 && j + 2 < n) store_tile(j + 2);
       if (L::kStages > 2 && j + 3 < n) load_tile(j + 3);
+      if constexpr (kKV) {  // dV's part while the tensor cores are at dK's
+        ok = __all_sync(kFull, mbar_wait(weighed_p, j & 1, g.status, 0x0b23u));
+        if (!ok) break;
+        tc_fence_after_sync();
+        gather(L::kOut1, acc1);
+        if (L::kStages == 2 && j + 2 < n) store_tile(j + 2, true);
+      }
       ok = __all_sync(kFull, mbar_wait(weighed, j & 1, g.status, 0x0b22u));
       if (!ok) break;
       tc_fence_after_sync();
       gather(L::kOut0, acc0);
-      if (kKV) gather(L::kOut1, acc1);
       tc_fence_before_sync();
-      if (L::kStages == 2 && j + 2 < n) store_tile(j + 2);
+      if (L::kStages == 2 && j + 2 < n) {
+        tile0.store(tile_at(j + 2, 0), check);
+        fence_async_shared();
+        arrive(staged(j + 2));
+      }
       if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
     }
     ok = __syncthreads_and(ok);
