@@ -437,23 +437,21 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
 
   uint64_t check = 0;
   typename L::Tile stage_k, stage_v;
+  stage_k.load(k, 0, g.t_k, g.hd);
   {
-    // every load is on its way before the first one is waited for
     typename L::Held stage_q;
     stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd);
-    stage_k.load(k, 0, g.t_k, g.hd);
-    stage_v.load(v, 0, g.t_k, g.hd_v);
-    const float flag = mask ? row_value(mask, 0, g.t_k) : 0.f;
     stage_q.store(base + L::kQ, check);
-    stage_k.store(base + L::kK, check);
-    if (mask) post_hidden(hidden[0], flag);
   }
+  stage_k.store(base + L::kK, check);
+  if (mask) post_hidden(hidden[0], row_value(mask, 0, g.t_k));
   fence_async_shared();
   __syncthreads();
   if (issues && elect_one()) {
     issue_scores<HD, false, L::kTwo>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
     mma_commit(scored);
   }
+  stage_v.load(v, 0, g.t_k, g.hd_v);
   stage_v.store(base + L::kV, check);
   fence_async_shared();
 
