@@ -119,18 +119,22 @@ struct Stage {
 
   float x[kLoops][8];
 
-  __device__ __forceinline__ void load(const float* src, int first, int rows, int width) {
+  // `thread`: which of the kThreads the calling one counts as. A tile with fewer pieces than threads is done by the first
+  // ones only; the dQ pass gives two such tiles to different halves of the block (290 -> 283 us for 6 x 8192 x 32; in the
+  // dK/dV pass it costs registers, 400 -> 420).
+  __device__ __forceinline__ static int second_half() { return kTurns == 0 ? threadIdx.x ^ (kThreads / 2) : threadIdx.x; }
+  __device__ __forceinline__ void load(const float* src, int first, int rows, int width, int thread = threadIdx.x) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
-      const int e = threadIdx.x + n * kThreads;
+      const int e = thread + n * kThreads;
       if (kTurns == 0 && e >= R * kChunks) break;
       load8<kWide>(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width);
     }
   }
-  __device__ __forceinline__ void store(uint32_t dst, uint64_t& check) {
+  __device__ __forceinline__ void store(uint32_t dst, uint64_t& check, int thread = threadIdx.x) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
-      const int e = threadIdx.x + n * kThreads;
+      const int e = thread + n * kThreads;
       if (kTurns == 0 && e >= R * kChunks) break;
       const int r = e / kChunks, chunk = e % kChunks;
       uint32_t h[4], m[4], l[4];
@@ -733,7 +737,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
     auto load_tile = [&](int j) {
       const int x0 = begin + j * kStream;
       tile0.load(stream0, x0, streamed, g.hd);
-      tile1.load(stream1, x0, streamed, g.hd_v);
+      tile1.load(stream1, x0, streamed, g.hd_v, kKV ? threadIdx.x : L::Tile::second_half());
       if (kKV) {
         row_a = row_value(g.lse_in + b * g.t_q, x0, streamed);
         row_b = row_value(g.delta + b * g.t_q, x0, streamed);
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       } else if (mask) {
         post_hidden(hidden[j % L::kStages], row_a);
       }
-      tile1.store(tile_at(j, 1), check);
+      tile1.store(tile_at(j, 1), check, kKV ? threadIdx.x : L::Tile::second_half());
       if (!split) {
         tile0.store(tile_at(j, 0), check);
         fence_async_shared();
@@ -890,25 +894,22 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
   tear_down<L::kCols>(g, tmem);
 }
 
-// ---- backward: dQ for 128 query rows, or dK and dV for 128 key rows ----
+// ---- backward at head dims above 64 ----
+// Two held operands and two streamed tiles do not fit in shared memory: the first held operand lies in tensor memory, the
+// streamed tiles have one buffer, and a tile's products are written over the scores they came from. What is left to run
+// side by side is little, so the row warps also issue.
 template <int HD, bool kWide>
 struct BwdWide {
   static constexpr int kGroups = 4;
   static constexpr int kThreads = kRows * kGroups;
-  // At head dims above 64 two held operands and two streamed tiles do not fit in shared memory twice over: the first
-  // held operand lies in tensor memory, the streamed tiles have one buffer, and the tile's results are written over
-  // the scores they came from.
-  static constexpr bool kTight = HD > 64;
-  static constexpr int kStages = kTight ? 1 : 2;
   using Held = Stage<HD, kRows, kThreads, kWide>;
   using Tile = Stage<HD, kStream, kThreads, kWide>;
-  static constexpr uint32_t kHeld0 = 0, kHeld1 = kTight ? 0 : Held::kBytes, kTiles = kHeld1 + Held::kBytes;
-  static constexpr uint32_t kBytes = kTiles + kStages * 2 * Tile::kBytes + 1024;
-  static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols, kAfter = kP + 3 * kPieceCols;
-  static constexpr uint32_t kOut0 = kTight ? 0 : kAfter, kOut1 = kTight ? 0 : kAfter + HD;
-  static constexpr uint32_t kHeldT = kAfter;  // kTight: the first held operand, three pieces of HD / 2 columns
+  static constexpr uint32_t kHeld1 = 0, kTile0 = Held::kBytes, kTile1 = kTile0 + Tile::kBytes;
+  static constexpr uint32_t kBytes = kTile1 + Tile::kBytes + 1024;
+  static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols, kHeldT = kP + 3 * kPieceCols;
+  static constexpr uint32_t kOut = 0;
   static constexpr int kCols = 512;
-  static_assert(kAfter + (kTight ? 3 * HD / 2 : 2 * HD) <= 512, "tensor memory");
+  static_assert(kHeldT + 3 * HD / 2 <= kCols && kOut + HD <= kDs, "tensor memory");
 };
 
 template <int HD, bool kKV, bool kWide>
@@ -916,9 +917,9 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   using L = BwdWide<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ unsigned char raw[];
-  __shared__ uint32_t slot, abort_flag, hidden[2][2];
+  __shared__ uint32_t slot, abort_flag, hidden[2];
   __shared__ __align__(8) uint64_t bars[3];
-  __shared__ __align__(16) float lse_hi[2][kStream], lse_lo[2][kStream], deltas[2][kStream];  // dK/dV: of the streamed rows
+  __shared__ __align__(16) float lse_hi[kStream], lse_lo[kStream], deltas[kStream];  // dK/dV: of the streamed rows
   uint32_t tmem;
   if (!set_up<L::kCols, 3>(g, &slot, &abort_flag, bars, tmem)) return;
   const uint32_t base = align_1024(smem_addr(raw));
@@ -945,99 +946,76 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   const int mine = first + row;  // this thread's row
 
   uint64_t check = 0;
-  auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
-  // the streamed tile j, and what goes with its rows: to registers, and from there to shared memory
-  typename L::Tile tile0, tile1;
-  float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
-  auto load_tile = [&](int j) {
+  // the streamed tile j, and what goes with its rows
+  auto stage_tile = [&](int j) {
     const int x0 = begin + j * kStream;
+    typename L::Tile tile0, tile1;
     tile0.load(stream0, x0, streamed, g.hd);
     tile1.load(stream1, x0, streamed, g.hd_v);
     if (kKV) {
-      row_a = row_value(g.lse_in + b * g.t_q, x0, streamed);
-      row_b = row_value(g.delta + b * g.t_q, x0, streamed);
-    } else if (mask) {
-      row_a = row_value(mask, x0, streamed);
-    }
-  };
-  auto store_tile = [&](int j) {
-    if (kKV) {
+      const float lse = row_value(g.lse_in + b * g.t_q, x0, streamed), delta = row_value(g.delta + b * g.t_q, x0, streamed);
       if (threadIdx.x < kStream) {
         float hi, lo;
-        to_log2(row_a, hi, lo);
-        lse_hi[j & 1][threadIdx.x] = hi;
-        lse_lo[j & 1][threadIdx.x] = lo;
-        deltas[j & 1][threadIdx.x] = row_b;
+        to_log2(lse, hi, lo);
+        lse_hi[threadIdx.x] = hi;
+        lse_lo[threadIdx.x] = lo;
+        deltas[threadIdx.x] = delta;
       }
     } else if (mask) {
-      post_hidden(hidden[j & 1], row_a);
+      post_hidden(hidden, row_value(mask, x0, streamed));
     }
-    tile0.store(tile_at(j, 0), check);
-    tile1.store(tile_at(j, 1), check);
+    tile0.store(base + L::kTile0, check);
+    tile1.store(base + L::kTile1, check);
     fence_async_shared();
   };
-  auto issue_tile = [&](int j) {
+  auto issue_tile = [&]() {
     tc_fence_after_sync();
-    issue_scores<HD, L::kTight>(tmem + L::kS, L::kTight ? tmem + L::kHeldT : base + L::kHeld0, tile_at(j, 0));
-    issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, tile_at(j, 1));
+    issue_scores<HD, true>(tmem + L::kS, tmem + L::kHeldT, base + L::kTile0);
+    issue_scores<HD, false>(tmem + L::kDp, base + L::kHeld1, base + L::kTile1);
     mma_commit(scored);
   };
 
-  // every load is on its way before the first one is waited for
   float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
   bool live = mine < owned;
   {
+    float x[OW / 8][8];
+#pragma unroll
+    for (int c = 0; c < OW / 8; ++c) load8<kWide>(x[c], held0, mine, owned, group * OW + 8 * c, g.hd);
     typename L::Held stage1;
-    if constexpr (L::kTight) {
-      float x[OW / 8][8];
+    stage1.load(held1, first, owned, g.hd_v);
+    uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
 #pragma unroll
-      for (int c = 0; c < OW / 8; ++c) load8<kWide>(x[c], held0, mine, owned, group * OW + 8 * c, g.hd);
-      stage1.load(held1, first, owned, g.hd_v);
-      uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
-#pragma unroll
-      for (int e = 0; e < OW / 2; ++e) split_pair(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
-      const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
-      tmem_st<OW / 2>(to, h);
-      tmem_st<OW / 2>(to + HD / 2, m);
-      tmem_st<OW / 2>(to + HD, l);
-      tmem_st_wait();
-      tc_fence_before_sync();
-      load_tile(0);
-    } else {
-      typename L::Held stage0;
-      stage0.load(held0, first, owned, g.hd);
-      stage1.load(held1, first, owned, g.hd_v);
-      load_tile(0);
-      stage0.store(base + L::kHeld0, check);
-    }
+    for (int e = 0; e < OW / 2; ++e) split_pair(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
+    const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
+    tmem_st<OW / 2>(to, h);
+    tmem_st<OW / 2>(to + HD / 2, m);
+    tmem_st<OW / 2>(to + HD, l);
+    tmem_st_wait();
+    tc_fence_before_sync();
     if constexpr (kKV) {
       if (live && mask) live = mask[mine] != 0.f;
     } else if (live) {
-      my_hi = g.lse_in[b * g.t_q + mine];
+      to_log2(g.lse_in[b * g.t_q + mine], my_hi, my_lo);
       my_delta = g.delta[b * g.t_q + mine];
     }
     stage1.store(base + L::kHeld1, check);
   }
-  store_tile(0);  // (fences the held rows too)
+  stage_tile(0);  // (fences the held rows too)
   __syncthreads();
-  if (issues && elect_one()) issue_tile(0);
-  if (!L::kTight && n > 1) load_tile(1);
-
-  if constexpr (!kKV) to_log2(my_hi, my_hi, my_lo);
+  if (issues && elect_one()) issue_tile();
 
   uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dV and dK
 #pragma unroll
   for (int c = 0; c < OW / 2; ++c) acc0[c] = acc1[c] = 0;
-  auto gather = [&](uint32_t from, uint64_t(&acc)[OW / 2]) {
+  auto gather = [&](uint64_t(&acc)[OW / 2]) {
     tc_fence_after_sync();
     uint32_t o[OW];
-    tmem_ld<OW>(lanes + from + group * OW, o);
+    tmem_ld<OW>(lanes + L::kOut + group * OW, o);
     tmem_ld_wait();
     tc_fence_before_sync();
 #pragma unroll
     for (int c = 0; c < OW / 2; ++c) acc[c] = f2_add(acc[c], f2_pack_bits(o[2 * c], o[2 * c + 1]));
   };
-  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale2 = f2_pack(g.scale, g.scale);
   bool ok = true;
   for (int j = 0; j < n; ++j) {
     const int x0 = begin + j * kStream;
@@ -1047,55 +1025,23 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     tmem_ld<CW>(lanes + L::kS + group * CW, s);
     tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
     tmem_ld_wait();
-    const bool more = j + 1 < n;
-    if (!L::kTight && more) {
-      // the scores' place is free, and so is the other buffer, whose products were gathered a tile ago: the next tile's
-      // scores are on their way before this one's dS is worked out
-      tc_fence_before_sync();
-      store_tile(j + 1);
-      __syncthreads();
-      if (issues && elect_one()) issue_tile(j + 1);
-    }
-    // columns [from, to) of this thread's CW are seen, less the hidden ones
     int from = 0, to = streamed - x0 - group * CW;
     if (g.causal) {
       if (kKV) from = mine - x0 - group * CW;
       else to = min(to, mine - x0 - group * CW + 1);
     }
-    if (!live) to = 0;
-    uint32_t unseen = 0;
-    if (from > 0) unseen |= from >= CW ? kFull : (1u << from) - 1u;
-    if (to < CW) unseen |= to <= 0 ? kFull : ~((1u << to) - 1u);
-    if (!kKV && mask) unseen |= my_hidden<CW>(hidden[j & 1], group);
+    uint32_t unseen = outside<CW>(from, live ? to : 0);
+    if (!kKV && mask) unseen |= my_hidden<CW>(hidden, group);
     uint64_t p[CW / 2], ds[CW / 2];
-#pragma unroll
-    for (int c = 0; c < CW / 2; ++c) {
-      uint64_t hi, lo, delta;
+    weigh_scores<CW>(g, s, dp, unseen, [&](int c, uint64_t& hi, uint64_t& lo, uint64_t& delta) {
       if (kKV) {
-        const int at = group * CW + 2 * c;
-        hi = *reinterpret_cast<const uint64_t*>(&lse_hi[j & 1][at]);
-        lo = *reinterpret_cast<const uint64_t*>(&lse_lo[j & 1][at]);
-        delta = *reinterpret_cast<const uint64_t*>(&deltas[j & 1][at]);
+        hi = *reinterpret_cast<const uint64_t*>(&lse_hi[group * CW + c]);
+        lo = *reinterpret_cast<const uint64_t*>(&lse_lo[group * CW + c]);
+        delta = *reinterpret_cast<const uint64_t*>(&deltas[group * CW + c]);
       } else {
         hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
       }
-      const uint64_t minus = f2_pack(-1.f, -1.f);
-      const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
-      uint64_t x = f2_fma(s2, c_hi, hi ^ 0x8000000080000000ull);
-      x = f2_add(x, f2_fma(s2, c_lo, lo ^ 0x8000000080000000ull));
-      float x0_, x1_;
-      f2_unpack(x, x0_, x1_);
-      float p0 = exp2_approx(x0_), p1 = exp2_approx(x1_);
-      if ((unseen >> (2 * c)) & 1u) p0 = 0.f;
-      if ((unseen >> (2 * c + 1)) & 1u) p1 = 0.f;
-      p[c] = f2_pack(p0, p1);
-      const uint64_t d2 = f2_fma(delta, minus, f2_pack_bits(dp[2 * c], dp[2 * c + 1]));
-      float d0, d1;
-      f2_unpack(f2_mul(f2_mul(p[c], d2), scale2), d0, d1);
-      if ((unseen >> (2 * c)) & 1u) d0 = 0.f;  // (delta of a row with no key is NaN)
-      if ((unseen >> (2 * c + 1)) & 1u) d1 = 0.f;
-      ds[c] = f2_pack(d0, d1);
-    }
+    }, p, ds);
     hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, check);
     if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
     tmem_st_wait();
@@ -1103,51 +1049,37 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     if (!__syncthreads_and(ok)) break;
     if (issues && elect_one()) {
       tc_fence_after_sync();
-      if (kKV) {
-        issue_weigh<HD>(tmem + L::kOut0, tmem + L::kP, tile_at(j, 1));
-        mma_commit(weighed0);
-        if (!L::kTight) {
-          issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
-          mma_commit(weighed1);
-        }
-      } else {
-        issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile_at(j, 0));
-        mma_commit(weighed0);
-      }
+      issue_weigh<HD>(tmem + L::kOut, tmem + (kKV ? L::kP : L::kDs), base + (kKV ? L::kTile1 : L::kTile0));
+      mma_commit(weighed0);
     }
-    if (!L::kTight && j + 2 < n) load_tile(j + 2);
     ok &= mbar_wait(weighed0, j & 1, g.status, 0x0b01u);
-    gather(L::kOut0, acc0);
+    gather(acc0);
     if (kKV) {
-      if (L::kTight) {
-        if (!__syncthreads_and(ok)) break;
-        if (issues && elect_one()) {
-          tc_fence_after_sync();
-          issue_weigh<HD>(tmem + L::kOut1, tmem + L::kDs, tile_at(j, 0));
-          mma_commit(weighed1);
-        }
+      if (!__syncthreads_and(ok)) break;
+      if (issues && elect_one()) {
+        tc_fence_after_sync();
+        issue_weigh<HD>(tmem + L::kOut, tmem + L::kDs, base + L::kTile0);
+        mma_commit(weighed1);
       }
       ok &= mbar_wait(weighed1, j & 1, g.status, 0x0b02u);
-      gather(L::kOut1, acc1);
+      gather(acc1);
     }
-    if (L::kTight && more) {
-      load_tile(j + 1);
-      store_tile(j + 1);
+    if (j + 1 < n) {
+      stage_tile(j + 1);
       if (!__syncthreads_and(ok)) break;
-      if (issues && elect_one()) issue_tile(j + 1);
+      if (issues && elect_one()) issue_tile();
     }
   }
   ok = __syncthreads_and(ok);
-  if (ok) {
-    if (__syncthreads_or(is_bad(check))) {
-      plain_bwd<kKV>(g, b, first, L::kThreads);
-    } else if (mine < owned) {
-      if (kKV) {
-        store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);
-        store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc1, group * OW, g.hd, g.wide_out);
-      } else {
-        store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
-      }
+  const bool bad = __syncthreads_or(is_bad(check));
+  if (ok && bad) {
+    plain_bwd<kKV>(g, b, first, L::kThreads);
+  } else if (ok && mine < owned) {
+    if (kKV) {
+      store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);
+      store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc1, group * OW, g.hd, g.wide_out);
+    } else {
+      store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
     }
   }
   tear_down<L::kCols>(g, tmem);
