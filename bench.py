@@ -550,10 +550,11 @@ def decode_cases(args, world: int, torch, device, barrier, max_over_ranks) -> di
 
 def off_grid_cases(args, world: int, torch, device, barrier, max_over_ranks) -> dict:
     """Shapes outside the four BASELINE configurations that the ops are still called with, device-resident, forward and
-    forward+backward (row dot as its own launch). "float32": float32 storage, computed at float32 on the CUDA cores
+    forward+backward (row dot as its own launch). "float32": float32 storage and accuracy, each operand in three
+    bfloat16 pieces on the tensor cores
     (limn's numpy and c devices run BASELINE's first configuration this way, and a model kept in float32 calls the
-    ops like this), against the float32 multiply-add rate of the part (SMs x 128 lanes x 2 x the maximum SM clock: a
-    nominal figure, nothing measures it here). "narrow_heads": bfloat16 with head dims that are not 64 or 128, which
+    ops like this), set against the float32 multiply-add rate of the CUDA cores (SMs x 128 lanes x 2 x the maximum SM
+    clock: a nominal figure, nothing measures it here, and no bound on this path). "narrow_heads": bfloat16 with head dims that are not 64 or 128, which
     run zero-padded in the tensor-core kernels; credited with the flops of the real head dim."""
     from limn_b200._lib import lib
 

@@ -9,11 +9,15 @@
 // added to the row's total in registers, rounded to nearest, as the CUDA-core kernels in sdpa_general_tiled.cu do.
 //
 // What bounds it: six bfloat16 products at 4096 multiply-adds a clock and SM are 683 float32 multiply-adds a clock,
-// against 128 on the CUDA cores. Measured on B200 (forward / dQ / dK and dV, us, causal; the CUDA-core kernels in
-// brackets): 256 x 256 keys x 64: 42 / 72 / 96 (121 / 166 / 219); 6 x 8192 x 32: 379 / 651 / 901 (1333 / 1777 / 2402);
-// 64 x 1024 x 128: 189 / 267 / 341 (813 / 1117 / 1714). Against float64 every result is as close as before or closer
-// (8192 keys x 32: O 1.6e-7 for 5.8e-7, dK 4.3e-7 for 2.2e-6 in the 2-norm). A block owns 128 rows (query rows in the forward and the dQ pass, key rows in the
-// dK/dV pass), one row to each tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
+// against 128 on the CUDA cores; the split, the softmax and the running totals stay there and take about as long as the
+// MMAs (dQ at head dim 64: 2 300 and 2 500 clocks of a tile's 3 700). Measured on B200 (forward / dQ / dK and dV, us, causal;
+// the CUDA-core kernels in brackets): 256 x 256 keys x 64: 38 / 55 / 71 (121 / 166 / 219); 6 x 8192 x 32: 282 / 286 / 399
+// (1333 / 1777 / 2402); 64 x 1024 x 128: 170 / 224 / 289 (813 / 1117 / 1714); 64 x 32 x 64: 7.3 / 7.6 / 9.2 (10.8 / 12.4 /
+// 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.6e-7 for 5.8e-7, dK 4.3e-7 for 2.2e-6
+// in the 2-norm), L is at the rounding of a float32 like theirs.
+//
+// A block owns 128 rows (query rows in the forward and the dQ pass, key rows in the dK/dV pass), one row to each
+// tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
 // with ordinary loads (the split has to pass through registers anyway), split and left in shared memory in the
 // 128-byte-swizzled layout; probabilities and dS are split in registers and go to tensor memory as the A operand.
 //
