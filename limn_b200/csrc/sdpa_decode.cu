@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   const unsigned char* v_base = static_cast<const unsigned char*>(prm.v) + (batch * prm.v_strides.batch + head * prm.v_strides.head) * kBytes;
   const long long k_row = prm.k_strides.row * kBytes, v_row = prm.v_strides.row * kBytes;  // bytes between keys
   const void* flags = kMask ? static_cast<const unsigned char*>(prm.mask) + static_cast<long long>(problem) * prm.t_k * kBytes : nullptr;
-  // Lanes beyond a row's columns (a head narrower than D) read the row's first piece again: their q is zero, and what
-  // they gather of V is never stored.
+  // Lanes beyond a row's columns (a head narrower than D) read the row's first piece again: what they make of K is
+  // replaced by zero (their q is zero too, but an infinity in K times that is NaN), and what they gather of V is never stored.
   const bool real = gl < prm.pieces;
   const int k_at = (real ? gl : 0) * 8 * kBytes, v_at = (gl < prm.pieces_v ? gl : 0) * 8 * kBytes;
 
@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
         float dot = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) dot = fmaf(q[r][i], kf[i], dot);
+        dot = real ? dot : 0.f;
 #pragma unroll
         for (int step = kLanesPerKey / 2; step > 0; step >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, step);
         s[r][u] = visible ? dot : -INFINITY;

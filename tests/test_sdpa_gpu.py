@@ -589,6 +589,35 @@ def test_decode_shapes_in_float32_and_at_every_width(case, dev):
         np.testing.assert_array_equal(a.view(np.uint8), b.view(np.uint8))
 
 
+DECODE_WIDTHS = [(np.float32, 24, 24), (np.float32, 64, 128), (np.float32, 64, 64), (BF16, 40, 40), (BF16, 64, 128), (BF16, 64, 64), (np.float16, 128, 128)]
+DECODE_WIDTH_IDS = [f"{np.dtype(d).name} hd {a} hd_v {b}" for d, a, b in DECODE_WIDTHS]
+
+
+def _decode_forward(dev, q, k, v, mask=None):
+    """The forward of one query row per problem, having made sure that the streaming kernel serves it."""
+    import limn_standin as host
+    from limn_b200._lib import PATH_DECODE, lib
+
+    code = {"float32": 0, "float16": 1, "bfloat16": 2}[q.dtype.name]
+    assert lib().limn_b200_sdpa_path(code, q.shape[0], q.shape[1], k.shape[1], q.shape[2], v.shape[2], 0, int(mask is not None), q.shape[2] ** -0.5) == PATH_DECODE
+    return host.Attention(dev, q, k, v, key_mask=mask).forward()
+
+
+@pytest.mark.parametrize(("dtype", "hd", "hd_v"), DECODE_WIDTHS, ids=DECODE_WIDTH_IDS)
+def test_decode_with_a_key_at_minus_infinity(dtype, hd, hd_v, dev):
+    """A key at -infinity times a positive query weighs nothing, wherever the infinity stands in the row: the lanes a
+    narrow head leaves over must not meet it."""
+    q, k, v, _ = _random_case(900 + hd, dtype, (4, 1, hd), (4, 300, hd), (4, 300, hd_v))
+    q = np.abs(q)
+    for p, (key, col) in enumerate(((0, 0), (299, 7), (150, hd - 1), (10, 3))):
+        k[p, key, col] = -np.inf
+    want_out, want_lse = oracle.sdpa_forward(q, k, v, causal=False, scale=hd**-0.5)
+    assert np.isfinite(want_out.astype(np.float32)).all() and np.isfinite(want_lse).all()
+    out, lse = _decode_forward(dev, q, k, v)
+    close(out, want_out, FWD_TOL[np.dtype(dtype).name], "O")
+    close(lse, want_lse, LSE_TOL, "L")
+
+
 def test_two_runs_give_the_same_bits(dev):
     import limn_standin as host
 
