@@ -210,14 +210,15 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
       float mx = s[r][0];
 #pragma unroll
       for (int u = 1; u < kUnroll; ++u) mx = fmaxf(mx, s[r][u]);
-      const float m_new = fmaxf(m[r], mx);
-      if (m_new == -INFINITY) continue;  // nothing visible yet: p would be exp2(-inf + inf)
-      const float alpha = exp2f((m[r] - m_new) * sl2);  // 0 at the first visible key, where m is -inf
+      const float m_new = fmaxf(m[r], mx);  // (passes a NaN by: the weight below has it)
+      // as long as nothing is visible the weights are taken against 0: exp2(-inf), and NaN for a NaN score
+      const float base = m_new == -INFINITY ? 0.f : m_new;
+      const float alpha = exp2f((m[r] - base) * sl2);  // 0 while m is -inf
       m[r] = m_new;
       float p[kUnroll], sum = 0.f;
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        p[u] = exp2f((s[r][u] - m_new) * sl2);
+        p[u] = exp2f((s[r][u] - base) * sl2);
         sum += p[u];
       }
       l[r] = l[r] * alpha + sum;

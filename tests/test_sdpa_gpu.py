@@ -618,6 +618,28 @@ def test_decode_with_a_key_at_minus_infinity(dtype, hd, hd_v, dev):
     close(lse, want_lse, LSE_TOL, "L")
 
 
+@pytest.mark.parametrize(("dtype", "hd", "hd_v"), DECODE_WIDTHS, ids=DECODE_WIDTH_IDS)
+def test_decode_with_nan_scores(dtype, hd, hd_v, dev):
+    """A NaN key or query is a NaN row of O and L, also where the other keys of the same lanes are hidden or past the
+    end; the problems beside it keep their numbers."""
+    q, k, v, _ = _random_case(910 + hd, dtype, (5, 1, hd), (5, 260, hd), (5, 260, hd_v))
+    mask = np.ones((5, 260), dtype=dtype)
+    k[0, 259, 2] = np.nan  # the last pass, beside slots past the end
+    k[1, 7, hd - 1] = np.nan
+    mask[1, 8:] = 0
+    q[2, 0, 1] = np.nan
+    k[3, 100, 0] = np.nan  # a hidden key's score is no score
+    mask[3, 100] = 0
+    with np.errstate(invalid="ignore"):
+        want_out, want_lse = oracle.sdpa_forward(q, k, v, mask, causal=False, scale=hd**-0.5)
+    for problems in (0, 1, 2):
+        assert np.isnan(want_out[problems].astype(np.float32)).all() and np.isnan(want_lse[problems]).all()
+    out, lse = _decode_forward(dev, q, k, v, mask)
+    assert np.isnan(out[:3].astype(np.float32)).all() and np.isnan(lse[:3]).all()
+    close(out[3:], want_out[3:], FWD_TOL[np.dtype(dtype).name], "O")
+    close(lse[3:], want_lse[3:], LSE_TOL, "L")
+
+
 def test_two_runs_give_the_same_bits(dev):
     import limn_standin as host
 
