@@ -187,13 +187,21 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
       const int at = min(key[u], prm.t_k - 1);
       v_raw[u] = load8<kKind>(v_base + at * v_row + v_at);
     }
+    const bool ragged = first + kPerPass > prm.t_k;  // some of this pass's slots lie past the end
     float s[R][kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       float kf[8];
       widen8<kKind>(k_raw[u], kf);
       bool visible = key[u] < prm.t_k;
-      if (kMask && visible) visible = key_visible<kKind>(flags, key[u]);
+      // a key that does not exist has no V: the last key's would meet a weight of 0, and 0 * inf is NaN. In float32 a
+      // hidden key's V does not count either (as in the one-row-per-warp kernel), so the empty slots of a cache may hold
+      // anything; in 16 bits it does, as in the tensor-core kernels and the oracle, where 0 * NaN is NaN.
+      if (ragged && !visible) v_raw[u] = Raw8<kKind>{};
+      if (kMask && visible) {
+        visible = key_visible<kKind>(flags, key[u]);
+        if (kKind == kF32 && !visible) v_raw[u] = Raw8<kKind>{};
+      }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         float dot = 0.f;

@@ -640,6 +640,39 @@ def test_decode_with_nan_scores(dtype, hd, hd_v, dev):
     close(lse[3:], want_lse[3:], LSE_TOL, "L")
 
 
+@pytest.mark.parametrize(("dtype", "hd", "hd_v"), DECODE_WIDTHS, ids=DECODE_WIDTH_IDS)
+def test_decode_with_values_no_weight_reaches(dtype, hd, hd_v, dev):
+    """An infinity in the last V row stays one (the slots past the end have no V), at lengths that end inside a pass. The V
+    of a hidden key does not count in float32, so the empty slots of a cache may hold anything; in 16 bits it does, as in
+    the oracle, where a weight of 0 times NaN is NaN."""
+    name = np.dtype(dtype).name
+    for t_k in (300, 513, 1025):
+        q, k, v, _ = _random_case(920 + t_k, dtype, (3, 1, hd), (3, t_k, hd), (3, t_k, hd_v))
+        v[0, -1, 3] = np.inf
+        v[1, -1, hd_v - 1] = -np.inf
+        want_out, want_lse = oracle.sdpa_forward(q, k, v, causal=False, scale=hd**-0.5)
+        out, lse = _decode_forward(dev, q, k, v)
+        assert out[0, 0, 3] == np.inf and out[1, 0, hd_v - 1] == -np.inf
+        finite = np.isfinite(want_out.astype(np.float32))
+        assert finite.sum() == finite.size - 2
+        close(out[finite], want_out[finite], FWD_TOL[name], "O")
+        close(lse, want_lse, LSE_TOL, "L")
+        v[0, -1, 3] = v[1, -1, hd_v - 1] = 0
+        mask = np.ones((3, t_k), dtype=dtype)
+        mask[1, t_k // 2 :] = 0  # slots not filled yet, and problem 2 with one hole
+        mask[2, 20] = 0
+        clean_out, clean_lse = oracle.sdpa_forward(q, k, v, mask, causal=False, scale=hd**-0.5)
+        v[1, t_k // 2 :] = np.nan
+        v[2, 20] = np.inf
+        out, lse = _decode_forward(dev, q, k, v, mask)
+        close(lse, clean_lse, LSE_TOL, "L")
+        close(out[:1], clean_out[:1], FWD_TOL[name], "O")
+        if name == "float32":
+            close(out[1:], clean_out[1:], FWD_TOL[name], "O")
+        else:
+            assert np.isnan(out[1:].astype(np.float32)).all()
+
+
 def test_two_runs_give_the_same_bits(dev):
     import limn_standin as host
 
