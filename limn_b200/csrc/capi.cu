@@ -20,6 +20,10 @@ thread_local int g_launches = 0;
 constexpr int kMaxDevices = 64;
 std::mutex g_status_mutex;
 unsigned int* g_status_words[kMaxDevices] = {};
+// The status word is part of the library's device image, zero when it is loaded: the float32 kernels need it and nothing
+// else besides their operands, and a first call under stream capture, or with all memory given away, may not allocate.
+// (In host code the name is only a handle for cudaGetSymbolAddress.)
+__device__ __align__(256) unsigned int g_status_image[64];
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -51,10 +55,10 @@ int status_word(unsigned int** word) {
   if (device < 0 || device >= kMaxDevices) return fail(LIMN_B200_UNSUPPORTED, "device ordinal %d out of range", device);
   std::lock_guard<std::mutex> lock(g_status_mutex);
   if (g_status_words[device] == nullptr) {
-    unsigned int* fresh = nullptr;
-    LIMN_CUDA(cudaMalloc(&fresh, 256), "allocating the device status word");
-    LIMN_CUDA(cudaMemset(fresh, 0, 256), "clearing the device status word");
-    g_status_words[device] = fresh;
+    void* image = nullptr;
+    LIMN_CUDA(cudaGetSymbolAddress(&image, g_status_image), "looking up the device status word");
+    if (image == nullptr) return fail(LIMN_B200_CUDA_ERROR, "cuda: the device status word has no address");
+    g_status_words[device] = static_cast<unsigned int*>(image);
   }
   *word = g_status_words[device];
   return LIMN_B200_OK;

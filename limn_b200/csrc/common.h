@@ -50,7 +50,7 @@ struct Problem {
   // dQ pass only: compute delta from `out` (the forward's O) and dO on the way and write it to `delta`, instead of
   // reading it. Served by the tensor-core kernels; the general family runs the row-dot kernel first.
   bool fuse_delta = false;
-  // Where kernels that wait record giving up. Null means the per-device word status_word() allocates.
+  // Where kernels that wait record giving up. Null means the per-device word of status_word().
   unsigned int* status = nullptr;
   // Two zeroed words for the kernels' work counters. Null means a pair from schedule_words().
   unsigned int* schedule = nullptr;
@@ -72,8 +72,8 @@ int cuda_fail(cudaError_t err, const char* doing);
     if (err__ != cudaSuccess) return ::limn_b200::cuda_fail(err__, doing); \
   } while (0)
 
-// Device address of the current device's status word (allocated on first use, one per
-// device, zero-initialised). Kernels that wait write a non-zero code there when they give up.
+// Device address of the current device's status word (part of the library's device image, one per
+// device, zero-initialised; nothing is allocated). Kernels that wait write a non-zero code there when they give up.
 int status_word(unsigned int** word);
 // Two zeroed words (next work item, CTAs finished) for one launch of a kernel whose CTAs fetch their
 // work items themselves. A kernel leaves its pair zeroed again, so the pairs are handed out in turn from
