@@ -23,16 +23,12 @@
 //
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
 // number (inf - inf in the split, inf * 0 between pieces). The split notices (its remainder is NaN), and a block that
-// met one computes its rows again on the CUDA cores, with the code of the tiled kernels there (a step whose every block
-// does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 507 / 1 984 / 2 556, the tiled kernels alone 1 340 / 1 790 / 2 410;
-// one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above head dim 64 leave their loop when
-// they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
+// met one computes its rows again, one row per warp, in plain float32.
 #include <cmath>
 #include <cstdint>
 
 #include "common.h"
 #include "sm100_ptx.cuh"
-#include "tiled_rows.cuh"
 
 namespace limn_b200 {
 namespace {
@@ -42,9 +38,6 @@ using namespace ptx;
 constexpr int kRows = 128;    // rows a block owns
 constexpr int kStream = 64;   // rows of a streamed tile
 constexpr unsigned kFull = 0xffffffffu;
-// dS goes to the tensor cores this much larger: its third piece is then a bfloat16 wherever dS is a float32, however small
-// the gradients (an overflow shows in the split or in the sums, which are divided by it again).
-constexpr float kDsUp = 65536.f;
 constexpr int kPieceCols = kStream / 2;  // tensor-memory columns of one 16-bit piece of a (kRows x kStream) matrix
 
 struct Params {
@@ -54,25 +47,12 @@ struct Params {
   long long bh;
   int slots, group;  // row tiles per problem; problems scheduled side by side
   int t_q, t_k, hd, hd_v, causal;
-  float scale, ds_scale, c_hi, c_lo;  // ds_scale = scale * kDsUp; c_hi + c_lo = scale * log2(e), c_lo > 0
+  float scale, c_hi, c_lo;  // c_hi + c_lo = scale * log2(e), c_lo > 0
   bool wide_out;  // the results take 16-byte stores
 };
 
-// ---- x = h + m + l for two floats at a time ----
-// What an operand's split shows. Of a float32 of ordinary size the second remainder has eight bits at most and is its own
-// third piece, so the low half of its word is zero. It is not for an infinity or a NaN (the remainder is the NaN 0x7fffffff) and for
-// a number so small (below about 2^-110) that pieces fall under bfloat16's 2^-133 and bits would be lost.
-struct Check {
-  uint32_t words = 0;   // all second remainders of operands
-  uint64_t weights = 0; // NaN once a weight (P or dS) was not finite
-  __device__ __forceinline__ bool bad() const {
-    float a, b;
-    f2_unpack(weights, a, b);
-    return (words & 0xffffu) != 0u || !(a == 0.f && b == 0.f);
-  }
-};
-template <bool kOperand>
-__device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, Check& check) {
+// ---- x = h + m + l for two floats at a time; `check` becomes NaN when one of them is not finite ----
+__device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, uint64_t& check) {
   const uint64_t minus = f2_pack(-1.f, -1.f);
   float a, b;
   f2_unpack(x, a, b);
@@ -83,8 +63,12 @@ __device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m,
   x = f2_fma(f2_pack_bits(m << 16, m & 0xffff0000u), minus, x);  // exact
   f2_unpack(x, a, b);
   l = pack_bf16(a, b);
-  if (kOperand) check.words |= __float_as_uint(a) | __float_as_uint(b);
-  else check.weights = f2_fma(x, 0ull, check.weights);
+  check = f2_fma(x, 0ull, check);
+}
+__device__ __forceinline__ bool is_bad(uint64_t check) {
+  float a, b;
+  f2_unpack(check, a, b);
+  return !(a == 0.f && b == 0.f);
 }
 
 template <int N>
@@ -151,7 +135,7 @@ struct Stage {
       load8<kWide>(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width);
     }
   }
-  __device__ __forceinline__ void store(uint32_t dst, Check& check, int thread = threadIdx.x) {
+  __device__ __forceinline__ void store(uint32_t dst, uint64_t& check, int thread = threadIdx.x) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
       const int e = thread + n * kThreads;
@@ -159,7 +143,7 @@ struct Stage {
       const int r = e / kChunks, chunk = e % kChunks;
       uint32_t h[4], m[4], l[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) split_pair<true>(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
+      for (int i = 0; i < 4; ++i) split_pair(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
       const uint32_t at = swizzled_piece(dst + (chunk / 8) * R * 128, r, chunk % 8);
       st_shared_v4(at, h[0], h[1], h[2], h[3]);
       st_shared_v4(at + kPiece, m[0], m[1], m[2], m[3]);
@@ -218,10 +202,10 @@ __device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0
 
 // N numbers of one row, split, to tensor memory at `at` (pieces kPieceCols columns apart).
 template <int N>
-__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], Check& check) {
+__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], uint64_t& check) {
   uint32_t h[N / 2], m[N / 2], l[N / 2];
 #pragma unroll
-  for (int i = 0; i < N / 2; ++i) split_pair<false>(w[i], h[i], m[i], l[i], check);
+  for (int i = 0; i < N / 2; ++i) split_pair(w[i], h[i], m[i], l[i], check);
   tmem_st<N / 2>(at, h);
   tmem_st<N / 2>(at + kPieceCols, m);
   tmem_st<N / 2>(at + 2 * kPieceCols, l);
@@ -244,34 +228,111 @@ __device__ __forceinline__ void store_row(float* row, const uint64_t (&acc)[N / 
   }
 }
 
-// ---- the rows of a block whose operands do not split, on the CUDA cores (tiled_rows.cuh): each 256 threads of the block
-// take 64 rows at a time. Streamed tiles are as long as the block's shared memory allows for all its groups together. ----
-template <int HD, Op kOp, int kGroups, uint32_t kBytes>
-constexpr int again_tile() {
-  constexpr uint32_t kShare = kBytes / kGroups & ~15u;
-  if (HD <= 64 && tiled::shared_bytes<HD, 64>(kOp) <= kShare) return 64;
-  if (tiled::shared_bytes<HD, 32>(kOp) <= kShare) return 32;
-  return 16;
+__device__ __forceinline__ float warp_sum(float x) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
+  return x;
 }
-template <int HD, Op kOp, int kGroups, uint32_t kBytes, bool kWide>
-__device__ __noinline__ void rows_again(const Params& g, long long b, int first, unsigned char* shared) {
-  constexpr int BN = again_tile<HD, kOp, kGroups, kBytes>();
-  constexpr uint32_t kShare = kBytes / kGroups & ~15u;
-  static_assert(tiled::shared_bytes<HD, BN>(kOp) <= kShare, "shared memory");
-  tiled::Args a = {};
-  a.q = g.q, a.k = g.k, a.v = g.v, a.mask = g.mask, a.dout = g.dout, a.lse_in = g.lse_in, a.delta = g.delta;
-  a.out = g.out, a.dq = g.dq, a.dk = g.dk, a.dv = g.dv, a.lse_out = g.lse_out;
-  a.t_q = g.t_q, a.t_k = g.t_k, a.hd = g.hd, a.hd_v = g.hd_v, a.causal = g.causal, a.scale = g.scale;
-  a.wide_qk = a.wide_v = kWide;
-  const int group = threadIdx.x / tiled::kThreads, thread = threadIdx.x % tiled::kThreads;
-  float* mine = reinterpret_cast<float*>(shared + group * kShare);
-  auto sync = [group] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(tiled::kThreads) : "memory"); };
-  const int owned = kOp == Op::BwdKV ? g.t_k : g.t_q;
-  for (int at = first + group * tiled::kBM; at < min(first + kRows, owned); at += kGroups * tiled::kBM) {
-    if constexpr (kOp == Op::Fwd) tiled::fwd_rows<float, HD, BN>(a, b, at, mine, thread, sync);
-    else if constexpr (kOp == Op::BwdQ) tiled::bwd_q_rows<float, HD, BN>(a, b, at, mine, thread, sync);
-    else tiled::bwd_kv_rows<float, HD, BN>(a, b, at, mine, thread, sync);
-    sync();  // its shared memory has been read
+
+// ---- the rows of a block that met a non-finite operand, one row per warp. Keys (queries) are walked in the 64-row
+// tiles the row's own tile would see, weight 0 on those it does not, so a hidden infinity gives NaN as it does in the
+// products. ----
+struct Row {
+  float x[4];
+  __device__ __forceinline__ void load(const float* src, int width) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int d = (threadIdx.x & 31) + 32 * c;
+      x[c] = d < width ? src[d] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void zero() { x[0] = x[1] = x[2] = x[3] = 0.f; }
+  __device__ __forceinline__ float dot(const Row& y) const {
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s = fmaf(x[c], y.x[c], s);
+    return warp_sum(s);
+  }
+  __device__ __forceinline__ void add(float w, const Row& y, int width) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if ((threadIdx.x & 31) + 32 * c < width) x[c] = fmaf(w, y.x[c], x[c]);
+  }
+  __device__ __forceinline__ void store(float* dst, int width, float over) const {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int d = (threadIdx.x & 31) + 32 * c;
+      if (d < width) dst[d] = x[c] / over;
+    }
+  }
+};
+
+__device__ __noinline__ void plain_fwd(const Params& g, long long b, int i0, int threads) {
+  for (int i = i0 + (threadIdx.x >> 5); i < min(i0 + kRows, g.t_q); i += threads >> 5) {
+    Row q, k, v, acc;
+    q.load(g.q + (b * g.t_q + i) * g.hd, g.hd);
+    acc.zero();
+    float top = -INFINITY, denom = 0.f;
+    const int end = g.causal ? min(g.t_k, (i / kStream + 1) * kStream) : g.t_k;
+    for (int j = 0; j < end; ++j) {
+      k.load(g.k + (b * g.t_k + j) * g.hd, g.hd);
+      v.load(g.v + (b * g.t_k + j) * g.hd_v, g.hd_v);
+      const bool seen = (!g.causal || j <= i) && (!g.mask || g.mask[b * g.t_k + j] != 0.f);
+      const float s = q.dot(k) * g.scale;
+      float p = 0.f;
+      if (seen) {
+        const float raised = fmaxf(top, s);
+        if (raised == -INFINITY) {
+          p = isnan(s) ? s : 0.f;
+        } else {
+          const float shrink = expf(top - raised);
+          denom *= shrink;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc.x[c] *= shrink;
+          p = expf(s - raised);
+          top = raised;
+        }
+      }
+      denom += p;
+      acc.add(p, v, g.hd_v);
+    }
+    acc.store(g.out + (b * g.t_q + i) * g.hd_v, g.hd_v, denom);
+    if ((threadIdx.x & 31) == 0) g.lse_out[b * g.t_q + i] = top + logf(denom);
+  }
+}
+
+template <bool kKV>
+__device__ __noinline__ void plain_bwd(const Params& g, long long b, int first, int threads) {
+  const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
+  for (int r = first + (threadIdx.x >> 5); r < min(first + kRows, owned); r += threads >> 5) {
+    Row q, k, v, dout, acc0, acc1;
+    acc0.zero();
+    acc1.zero();
+    const int from = kKV && g.causal ? r / kStream * kStream : 0;
+    const int end = !kKV && g.causal ? min(streamed, (r / kStream + 1) * kStream) : streamed;
+    for (int x = from; x < end; ++x) {
+      const long long i = b * g.t_q + (kKV ? x : r), j = b * g.t_k + (kKV ? r : x);
+      q.load(g.q + i * g.hd, g.hd);
+      dout.load(g.dout + i * g.hd_v, g.hd_v);
+      k.load(g.k + j * g.hd, g.hd);
+      v.load(g.v + j * g.hd_v, g.hd_v);
+      const bool seen = (!g.causal || (kKV ? r <= x : x <= r)) && (!g.mask || g.mask[j] != 0.f);
+      const float s = q.dot(k), dp = dout.dot(v);
+      const float p = seen ? expf(s * g.scale - g.lse_in[i]) : 0.f;
+      const float ds = seen ? p * (dp - g.delta[i]) * g.scale : 0.f;
+      if (kKV) {
+        acc0.add(p, dout, g.hd_v);
+        acc1.add(ds, q, g.hd);
+      } else {
+        acc0.add(ds, k, g.hd);
+      }
+    }
+    if (kKV) {
+      acc0.store(g.dv + (b * g.t_k + r) * g.hd_v, g.hd_v, 1.f);
+      acc1.store(g.dk + (b * g.t_k + r) * g.hd, g.hd, 1.f);
+    } else {
+      acc0.store(g.dq + (b * g.t_q + r) * g.hd, g.hd, 1.f);
+    }
   }
 }
 
@@ -358,7 +419,7 @@ template <int HD, bool kWide>
 __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
   using L = Fwd<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
-  extern __shared__ __align__(16) unsigned char raw[];
+  extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ float exchange[G][kRows];
@@ -382,7 +443,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   const int n = (keys_end + kStream - 1) / kStream;
   const int i = i0 + row;
 
-  Check check;
+  uint64_t check = 0;
   typename L::Tile stage_k, stage_v;
   stage_k.load(k, 0, g.t_k, g.hd);
   {
@@ -461,7 +522,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
+    if (!__syncthreads_and(ok)) break;
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
@@ -499,8 +560,8 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   }
   ok = __syncthreads_and(ok);
   if (ok) {
-    if (__syncthreads_or(check.bad())) {
-      rows_again<HD, Op::Fwd, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, i0, raw);
+    if (__syncthreads_or(is_bad(check))) {
+      plain_fwd(g, b, i0, L::kThreads);
     } else {
       exchange[group][row] = denom;
       __syncthreads();
@@ -532,13 +593,12 @@ __device__ __forceinline__ void to_log2(const float lse, float& hi, float& lo) {
   lo = fmaf(lse, kHi, -hi) + lse * kLo;
 }
 
-// What both backward kernels do with the scores of a row: P = 2^(s c - L), kDsUp dS = P (dP - delta) scale kDsUp, 0 where
-// unseen.
+// What both backward kernels do with the scores of a row: P = 2^(s c - L), dS = P (dP - delta) scale, 0 where unseen.
 // `hi`, `lo`, `delta` give a column's L (in log2 units) and delta; a row's own ones repeated in the dQ pass.
 template <int CW, typename Columns>
 __device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s)[CW], const uint32_t (&dp)[CW], uint32_t unseen,
                                              Columns columns, uint64_t (&p)[CW / 2], uint64_t (&ds)[CW / 2]) {
-  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale = f2_pack(g.ds_scale, g.ds_scale);
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale = f2_pack(g.scale, g.scale);
   const uint64_t minus = f2_pack(-1.f, -1.f);
 #pragma unroll
   for (int c = 0; c < CW / 2; ++c) {
@@ -560,16 +620,6 @@ __device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s
       f2_unpack(ds[c], a, b);
       ds[c] = f2_pack((unseen >> (2 * c)) & 1u ? 0.f : a, (unseen >> (2 * c + 1)) & 1u ? 0.f : b);
     }
-  }
-}
-
-// The sums over dS at their own size again. One that overflowed at kDsUp times it counts as a weight that was not finite.
-template <int N>
-__device__ __forceinline__ void settle(uint64_t (&acc)[N], Check& check) {
-#pragma unroll
-  for (int c = 0; c < N; ++c) {
-    check.weights = f2_fma(acc[c], 0ull, check.weights);
-    acc[c] = f2_mul(acc[c], f2_pack(1.f / kDsUp, 1.f / kDsUp));
   }
 }
 
@@ -610,7 +660,7 @@ template <int HD, bool kKV, bool kWide>
 __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
   using L = Pipe<HD, kKV, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G, kRowWarps = L::kRowThreads / 32;
-  extern __shared__ __align__(16) unsigned char raw[];
+  extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[L::kStages][2];
   __shared__ __align__(8) uint64_t bars[9];
   __shared__ __align__(16) float lse_hi[L::kStages][kStream], lse_lo[L::kStages][kStream], deltas[L::kStages][kStream];
@@ -635,7 +685,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
   const int n = (end - begin + kStream - 1) / kStream;
   auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
   bool ok = true;
-  Check check;
+  uint64_t check = 0;
 
   if (warp == kRowWarps) {
     // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
@@ -736,7 +786,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
         for (int c = 0; c < OW / 8; ++c) {
           uint32_t hi[4], mi[4], lo[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split_pair<true>(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
+          for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
           const uint32_t to = lanes + L::kHeldCol + h * (3 * HD / 2) + group * (OW / 2) + 4 * c;
           tmem_st4(to, hi);
           tmem_st4(to + HD / 2, mi);
@@ -832,11 +882,10 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       }
       if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
     }
-    settle(acc0, check);
     ok = __syncthreads_and(ok);
-    const bool bad = __syncthreads_or(check.bad());
+    const bool bad = __syncthreads_or(is_bad(check));
     if (ok && bad) {
-      rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
+      plain_bwd<kKV>(g, b, first, L::kRowThreads);
     } else if (ok && mine < owned) {
       if (kKV) {
         store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
@@ -871,7 +920,7 @@ template <int HD, bool kKV, bool kWide>
 __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_kernel(const __grid_constant__ Params g) {
   using L = BwdWide<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
-  extern __shared__ __align__(16) unsigned char raw[];
+  extern __shared__ unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2];
   __shared__ __align__(8) uint64_t bars[3];
   __shared__ __align__(16) float lse_hi[kStream], lse_lo[kStream], deltas[kStream];  // dK/dV: of the streamed rows
@@ -900,7 +949,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   const int n = (end - begin + kStream - 1) / kStream;
   const int mine = first + row;  // this thread's row
 
-  Check check;
+  uint64_t check = 0;
   // the streamed tile j, and what goes with its rows
   auto stage_tile = [&](int j) {
     const int x0 = begin + j * kStream;
@@ -940,7 +989,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     stage1.load(held1, first, owned, g.hd_v);
     uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
 #pragma unroll
-    for (int e = 0; e < OW / 2; ++e) split_pair<true>(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
+    for (int e = 0; e < OW / 2; ++e) split_pair(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
     const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
     tmem_st<OW / 2>(to, h);
     tmem_st<OW / 2>(to + HD / 2, m);
@@ -1001,7 +1050,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
+    if (!__syncthreads_and(ok)) break;
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kOut, tmem + (kKV ? L::kP : L::kDs), base + (kKV ? L::kTile1 : L::kTile0));
@@ -1025,12 +1074,10 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
       if (issues && elect_one()) issue_tile();
     }
   }
-  if (kKV) settle(acc1, check);
-  else settle(acc0, check);
   ok = __syncthreads_and(ok);
-  const bool bad = __syncthreads_or(check.bad());
+  const bool bad = __syncthreads_or(is_bad(check));
   if (ok && bad) {
-    rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
+    plain_bwd<kKV>(g, b, first, L::kThreads);
   } else if (ok && mine < owned) {
     if (kKV) {
       store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);
@@ -1058,7 +1105,6 @@ int launch_sized(Op op, const Problem& p) {
   g.slots = ((op == Op::BwdKV ? p.t_k : p.t_q) + kRows - 1) / kRows;
   g.t_q = p.t_q, g.t_k = p.t_k, g.hd = p.hd, g.hd_v = p.hd_v, g.causal = p.causal ? 1 : 0;
   g.scale = static_cast<float>(p.scale);
-  g.ds_scale = g.scale * kDsUp;
   const double c = static_cast<double>(g.scale) * 1.4426950408889634;
   g.c_hi = static_cast<float>(c);
   if (g.c_hi > c) g.c_hi = nextafterf(g.c_hi, 0.f);
