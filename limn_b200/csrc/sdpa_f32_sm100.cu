@@ -23,12 +23,16 @@
 //
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
 // number (inf - inf in the split, inf * 0 between pieces). The split notices (its remainder is NaN), and a block that
-// met one computes its rows again, one row per warp, in plain float32.
+// met one computes its rows again on the CUDA cores, with the code of the tiled kernels there (a step whose every block
+// does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 507 / 1 984 / 2 556, the tiled kernels alone 1 340 / 1 790 / 2 410;
+// one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above head dim 64 leave their loop when
+// they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
 #include <cmath>
 #include <cstdint>
 
 #include "common.h"
 #include "sm100_ptx.cuh"
+#include "tiled_rows.cuh"
 
 namespace limn_b200 {
 namespace {
@@ -228,111 +232,34 @@ __device__ __forceinline__ void store_row(float* row, const uint64_t (&acc)[N / 
   }
 }
 
-__device__ __forceinline__ float warp_sum(float x) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
-  return x;
+// ---- the rows of a block whose operands do not split, on the CUDA cores (tiled_rows.cuh): each 256 threads of the block
+// take 64 rows at a time. Streamed tiles are as long as the block's shared memory allows for all its groups together. ----
+template <int HD, Op kOp, int kGroups, uint32_t kBytes>
+constexpr int again_tile() {
+  constexpr uint32_t kShare = kBytes / kGroups & ~15u;
+  if (HD <= 64 && tiled::shared_bytes<HD, 64>(kOp) <= kShare) return 64;
+  if (tiled::shared_bytes<HD, 32>(kOp) <= kShare) return 32;
+  return 16;
 }
-
-// ---- the rows of a block that met a non-finite operand, one row per warp. Keys (queries) are walked in the 64-row
-// tiles the row's own tile would see, weight 0 on those it does not, so a hidden infinity gives NaN as it does in the
-// products. ----
-struct Row {
-  float x[4];
-  __device__ __forceinline__ void load(const float* src, int width) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int d = (threadIdx.x & 31) + 32 * c;
-      x[c] = d < width ? src[d] : 0.f;
-    }
-  }
-  __device__ __forceinline__ void zero() { x[0] = x[1] = x[2] = x[3] = 0.f; }
-  __device__ __forceinline__ float dot(const Row& y) const {
-    float s = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) s = fmaf(x[c], y.x[c], s);
-    return warp_sum(s);
-  }
-  __device__ __forceinline__ void add(float w, const Row& y, int width) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-      if ((threadIdx.x & 31) + 32 * c < width) x[c] = fmaf(w, y.x[c], x[c]);
-  }
-  __device__ __forceinline__ void store(float* dst, int width, float over) const {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int d = (threadIdx.x & 31) + 32 * c;
-      if (d < width) dst[d] = x[c] / over;
-    }
-  }
-};
-
-__device__ __noinline__ void plain_fwd(const Params& g, long long b, int i0, int threads) {
-  for (int i = i0 + (threadIdx.x >> 5); i < min(i0 + kRows, g.t_q); i += threads >> 5) {
-    Row q, k, v, acc;
-    q.load(g.q + (b * g.t_q + i) * g.hd, g.hd);
-    acc.zero();
-    float top = -INFINITY, denom = 0.f;
-    const int end = g.causal ? min(g.t_k, (i / kStream + 1) * kStream) : g.t_k;
-    for (int j = 0; j < end; ++j) {
-      k.load(g.k + (b * g.t_k + j) * g.hd, g.hd);
-      v.load(g.v + (b * g.t_k + j) * g.hd_v, g.hd_v);
-      const bool seen = (!g.causal || j <= i) && (!g.mask || g.mask[b * g.t_k + j] != 0.f);
-      const float s = q.dot(k) * g.scale;
-      float p = 0.f;
-      if (seen) {
-        const float raised = fmaxf(top, s);
-        if (raised == -INFINITY) {
-          p = isnan(s) ? s : 0.f;
-        } else {
-          const float shrink = expf(top - raised);
-          denom *= shrink;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc.x[c] *= shrink;
-          p = expf(s - raised);
-          top = raised;
-        }
-      }
-      denom += p;
-      acc.add(p, v, g.hd_v);
-    }
-    acc.store(g.out + (b * g.t_q + i) * g.hd_v, g.hd_v, denom);
-    if ((threadIdx.x & 31) == 0) g.lse_out[b * g.t_q + i] = top + logf(denom);
-  }
-}
-
-template <bool kKV>
-__device__ __noinline__ void plain_bwd(const Params& g, long long b, int first, int threads) {
-  const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
-  for (int r = first + (threadIdx.x >> 5); r < min(first + kRows, owned); r += threads >> 5) {
-    Row q, k, v, dout, acc0, acc1;
-    acc0.zero();
-    acc1.zero();
-    const int from = kKV && g.causal ? r / kStream * kStream : 0;
-    const int end = !kKV && g.causal ? min(streamed, (r / kStream + 1) * kStream) : streamed;
-    for (int x = from; x < end; ++x) {
-      const long long i = b * g.t_q + (kKV ? x : r), j = b * g.t_k + (kKV ? r : x);
-      q.load(g.q + i * g.hd, g.hd);
-      dout.load(g.dout + i * g.hd_v, g.hd_v);
-      k.load(g.k + j * g.hd, g.hd);
-      v.load(g.v + j * g.hd_v, g.hd_v);
-      const bool seen = (!g.causal || (kKV ? r <= x : x <= r)) && (!g.mask || g.mask[j] != 0.f);
-      const float s = q.dot(k), dp = dout.dot(v);
-      const float p = seen ? expf(s * g.scale - g.lse_in[i]) : 0.f;
-      const float ds = seen ? p * (dp - g.delta[i]) * g.scale : 0.f;
-      if (kKV) {
-        acc0.add(p, dout, g.hd_v);
-        acc1.add(ds, q, g.hd);
-      } else {
-        acc0.add(ds, k, g.hd);
-      }
-    }
-    if (kKV) {
-      acc0.store(g.dv + (b * g.t_k + r) * g.hd_v, g.hd_v, 1.f);
-      acc1.store(g.dk + (b * g.t_k + r) * g.hd, g.hd, 1.f);
-    } else {
-      acc0.store(g.dq + (b * g.t_q + r) * g.hd, g.hd, 1.f);
-    }
+template <int HD, Op kOp, int kGroups, uint32_t kBytes, bool kWide>
+__device__ __noinline__ void rows_again(const Params& g, long long b, int first, unsigned char* shared) {
+  constexpr int BN = again_tile<HD, kOp, kGroups, kBytes>();
+  constexpr uint32_t kShare = kBytes / kGroups & ~15u;
+  static_assert(tiled::shared_bytes<HD, BN>(kOp) <= kShare, "shared memory");
+  tiled::Args a = {};
+  a.q = g.q, a.k = g.k, a.v = g.v, a.mask = g.mask, a.dout = g.dout, a.lse_in = g.lse_in, a.delta = g.delta;
+  a.out = g.out, a.dq = g.dq, a.dk = g.dk, a.dv = g.dv, a.lse_out = g.lse_out;
+  a.t_q = g.t_q, a.t_k = g.t_k, a.hd = g.hd, a.hd_v = g.hd_v, a.causal = g.causal, a.scale = g.scale;
+  a.wide_qk = a.wide_v = kWide;
+  const int group = threadIdx.x / tiled::kThreads, thread = threadIdx.x % tiled::kThreads;
+  float* mine = reinterpret_cast<float*>(shared + group * kShare);
+  auto sync = [group] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(tiled::kThreads) : "memory"); };
+  const int owned = kOp == Op::BwdKV ? g.t_k : g.t_q;
+  for (int at = first + group * tiled::kBM; at < min(first + kRows, owned); at += kGroups * tiled::kBM) {
+    if constexpr (kOp == Op::Fwd) tiled::fwd_rows<float, HD, BN>(a, b, at, mine, thread, sync);
+    else if constexpr (kOp == Op::BwdQ) tiled::bwd_q_rows<float, HD, BN>(a, b, at, mine, thread, sync);
+    else tiled::bwd_kv_rows<float, HD, BN>(a, b, at, mine, thread, sync);
+    sync();  // its shared memory has been read
   }
 }
 
@@ -419,7 +346,7 @@ template <int HD, bool kWide>
 __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
   using L = Fwd<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
-  extern __shared__ unsigned char raw[];
+  extern __shared__ __align__(16) unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ float exchange[G][kRows];
@@ -522,7 +449,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok)) break;
+    if (!__syncthreads_and(ok && !is_bad(check))) break;  // (nothing is in flight here)
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
@@ -561,7 +488,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   ok = __syncthreads_and(ok);
   if (ok) {
     if (__syncthreads_or(is_bad(check))) {
-      plain_fwd(g, b, i0, L::kThreads);
+      rows_again<HD, Op::Fwd, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, i0, raw);
     } else {
       exchange[group][row] = denom;
       __syncthreads();
@@ -660,7 +587,7 @@ template <int HD, bool kKV, bool kWide>
 __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
   using L = Pipe<HD, kKV, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G, kRowWarps = L::kRowThreads / 32;
-  extern __shared__ unsigned char raw[];
+  extern __shared__ __align__(16) unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[L::kStages][2];
   __shared__ __align__(8) uint64_t bars[9];
   __shared__ __align__(16) float lse_hi[L::kStages][kStream], lse_lo[L::kStages][kStream], deltas[L::kStages][kStream];
@@ -885,7 +812,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
     ok = __syncthreads_and(ok);
     const bool bad = __syncthreads_or(is_bad(check));
     if (ok && bad) {
-      plain_bwd<kKV>(g, b, first, L::kRowThreads);
+      rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
     } else if (ok && mine < owned) {
       if (kKV) {
         store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
@@ -920,7 +847,7 @@ template <int HD, bool kKV, bool kWide>
 __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_kernel(const __grid_constant__ Params g) {
   using L = BwdWide<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
-  extern __shared__ unsigned char raw[];
+  extern __shared__ __align__(16) unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2];
   __shared__ __align__(8) uint64_t bars[3];
   __shared__ __align__(16) float lse_hi[kStream], lse_lo[kStream], deltas[kStream];  // dK/dV: of the streamed rows
@@ -1050,7 +977,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok)) break;
+    if (!__syncthreads_and(ok && !is_bad(check))) break;  // (nothing is in flight here)
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kOut, tmem + (kKV ? L::kP : L::kDs), base + (kKV ? L::kTile1 : L::kTile0));
@@ -1077,7 +1004,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   ok = __syncthreads_and(ok);
   const bool bad = __syncthreads_or(is_bad(check));
   if (ok && bad) {
-    plain_bwd<kKV>(g, b, first, L::kThreads);
+    rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
   } else if (ok && mine < owned) {
     if (kKV) {
       store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);

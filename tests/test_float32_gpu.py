@@ -7,6 +7,7 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -45,3 +46,86 @@ def test_the_first_float32_call_on_a_device_may_be_under_stream_capture():
     """Nothing is allocated and nothing waited for by a float32 forward and backward, the first call of a process included."""
     done = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+def _problem(seed, bh, t_q, t_k, hd, hd_v):
+    rng = np.random.default_rng(seed)
+    return [rng.standard_normal((bh, t, w)).astype(np.float32) for t, w in ((t_q, hd), (t_k, hd), (t_k, hd_v), (t_q, hd_v))]
+
+
+def _step(q, k, v, do, mask, causal, scale):
+    """One training step's three calls; O, L, dQ, dK, dV."""
+    from limn_b200 import runtime
+    from limn_b200._lib import check, lib
+
+    L = lib()
+    (bh, t_q, hd), (t_k, hd_v) = q.shape, v.shape[1:]
+    pq, pk, pv, pdo = (runtime.upload(a) for a in (q, k, v, do))
+    pm = runtime.upload(mask) if mask is not None else None
+    po, pl, pd, pdq, pdk, pdv = (runtime.empty(n) for n in (do.nbytes, 4 * bh * t_q, 4 * bh * t_q, q.nbytes, k.nbytes, v.nbytes))
+    m = pm.ptr if pm is not None else None
+    tail = (0, bh, t_q, t_k, hd, hd_v, int(causal), scale, None)
+    check(L.limn_b200_sdpa_fwd(pq.ptr, pk.ptr, pv.ptr, m, po.ptr, pl.ptr, *tail), "sdpa")
+    check(L.limn_b200_sdpa_bwd_q_fused(pq.ptr, pk.ptr, pv.ptr, po.ptr, pdo.ptr, pl.ptr, m, pdq.ptr, pd.ptr, *tail), "sdpa_bwd_q_fused")
+    check(L.limn_b200_sdpa_bwd_kv(pq.ptr, pk.ptr, pv.ptr, pdo.ptr, pl.ptr, pd.ptr, m, pdk.ptr, pdv.ptr, *tail), "sdpa_bwd_kv")
+    shapes = ((po, do.shape), (pl, (bh, t_q)), (pdq, q.shape), (pdk, k.shape), (pdv, v.shape))
+    return [runtime.download(buf, np.float32, shape).astype(np.float64) for buf, shape in shapes]
+
+
+def _step64(q, k, v, do, mask, causal, scale):
+    q, k, v, do = (a.astype(np.float64) for a in (q, k, v, do))
+    s = q @ k.transpose(0, 2, 1) * scale
+    seen = np.ones(s.shape, bool)
+    if causal:
+        seen &= np.tril(np.ones(s.shape[1:], bool))
+    if mask is not None:
+        seen &= mask[:, None, :] != 0
+    s = np.where(seen, s, -np.inf)
+    top = s.max(-1, keepdims=True)
+    p = np.exp(s - top)
+    total = p.sum(-1, keepdims=True)
+    p /= total
+    out = p @ v
+    ds = np.where(seen, p * (do @ v.transpose(0, 2, 1) - (do * out).sum(-1, keepdims=True)) * scale, 0)
+    return [out, (top + np.log(total))[..., 0], ds @ k, ds.transpose(0, 2, 1) @ q, p.transpose(0, 2, 1) @ do]
+
+
+def _compare(got, want, bound):
+    for g, w, what in zip(got, want, ("O", "L", "dQ", "dK", "dV")):
+        error = np.linalg.norm(g - w) / np.linalg.norm(w)
+        assert error <= bound, f"{what}: {error:.2e} > {bound:.2e}"
+
+
+BLOCKS = [(16, 40, 32, 32, False), (130, 130, 32, 24, True), (200, 200, 64, 64, True), (257, 300, 64, 33, False), (193, 193, 128, 128, True), (64, 129, 100, 128, False)]
+BLOCK_IDS = [f"{a}x{b} hd {c}/{d} {'causal' if e else 'full'}" for a, b, c, d, e in BLOCKS]
+
+
+@pytest.mark.parametrize("case", BLOCKS, ids=BLOCK_IDS)
+def test_blocks_that_leave_the_tensor_cores_match_the_others(case):
+    """An operand that has no bfloat16 pieces (here the largest float32, in hidden rows of V, where it counts for nothing)
+    sends the blocks that meet it to the CUDA cores: every row of theirs, ragged ends and hidden keys included, against float64.
+    The bound is that of the CUDA-core sums: sqrt(300) roundings of 2^-24, times 8."""
+    t_q, t_k, hd, hd_v, causal = case
+    q, k, v, do = _problem(t_q + hd, 3, t_q, t_k, hd, hd_v)
+    mask = (np.random.default_rng(t_k).random((3, t_k)) > 0.2).astype(np.float32)
+    mask[:, 0] = 1
+    want = _step64(q, k, v, do, mask, causal, hd**-0.5)
+    v[mask == 0] = np.finfo(np.float32).max
+    got = _step(q, k, v, do, mask, causal, hd**-0.5)
+    _compare(got, want, 8 * 300**0.5 * 2.0**-24)
+    assert (got[3][mask == 0] == 0).all() and (got[4][mask == 0] == 0).all()
+
+
+@pytest.mark.parametrize(("hd", "dtype"), [(32, np.float32), (64, np.float32), (128, np.float32), (192, np.float32), (36, np.float16)])
+def test_a_row_whose_only_key_is_nan(hd, dtype, dev):
+    """No running maximum sees a NaN score; the weight must."""
+    import limn_standin as host
+
+    q, k, v, _ = (a.astype(dtype) for a in _problem(hd, 2, 40, 40, hd, hd))
+    k[0, 3, 1] = np.nan
+    mask = np.ones((2, 40), dtype)
+    mask[0, :3] = 0
+    mask[0, 4:] = 0
+    out, lse = host.Attention(dev, q, k, v, causal=True, key_mask=mask).forward()
+    assert np.isnan(out[0].astype(np.float32)).all() and np.isnan(lse[0, 3:]).all() and np.isneginf(lse[0, :3]).all()
+    assert np.isfinite(out[1].astype(np.float32)).all() and np.isfinite(lse[1]).all()
