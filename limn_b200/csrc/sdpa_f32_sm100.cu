@@ -55,8 +55,21 @@ struct Params {
   bool wide_out;  // the results take 16-byte stores
 };
 
-// ---- x = h + m + l for two floats at a time; `check` becomes NaN when one of them is not finite ----
-__device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, uint64_t& check) {
+// ---- x = h + m + l for two floats at a time ----
+// What an operand's split shows. Of a float32 of ordinary size the second remainder has eight bits at most and is its own
+// third piece, so the low half of its word is zero. It is not for an infinity or a NaN (the remainder is the NaN 0x7fffffff) and for
+// a number so small (below about 2^-110) that pieces fall under bfloat16's 2^-133 and bits would be lost.
+struct Check {
+  uint32_t words = 0;   // all second remainders of operands
+  uint64_t weights = 0; // NaN once a weight (P or dS) was not finite
+  __device__ __forceinline__ bool bad() const {
+    float a, b;
+    f2_unpack(weights, a, b);
+    return (words & 0xffffu) != 0u || !(a == 0.f && b == 0.f);
+  }
+};
+template <bool kOperand>
+__device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, Check& check) {
   const uint64_t minus = f2_pack(-1.f, -1.f);
   float a, b;
   f2_unpack(x, a, b);
@@ -67,12 +80,8 @@ __device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m,
   x = f2_fma(f2_pack_bits(m << 16, m & 0xffff0000u), minus, x);  // exact
   f2_unpack(x, a, b);
   l = pack_bf16(a, b);
-  check = f2_fma(x, 0ull, check);
-}
-__device__ __forceinline__ bool is_bad(uint64_t check) {
-  float a, b;
-  f2_unpack(check, a, b);
-  return !(a == 0.f && b == 0.f);
+  if (kOperand) check.words |= __float_as_uint(a) | __float_as_uint(b);
+  else check.weights = f2_fma(x, 0ull, check.weights);
 }
 
 template <int N>
@@ -139,7 +148,7 @@ struct Stage {
       load8<kWide>(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width);
     }
   }
-  __device__ __forceinline__ void store(uint32_t dst, uint64_t& check, int thread = threadIdx.x) {
+  __device__ __forceinline__ void store(uint32_t dst, Check& check, int thread = threadIdx.x) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
       const int e = thread + n * kThreads;
@@ -147,7 +156,7 @@ struct Stage {
       const int r = e / kChunks, chunk = e % kChunks;
       uint32_t h[4], m[4], l[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) split_pair(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
+      for (int i = 0; i < 4; ++i) split_pair<true>(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
       const uint32_t at = swizzled_piece(dst + (chunk / 8) * R * 128, r, chunk % 8);
       st_shared_v4(at, h[0], h[1], h[2], h[3]);
       st_shared_v4(at + kPiece, m[0], m[1], m[2], m[3]);
@@ -206,10 +215,10 @@ __device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0
 
 // N numbers of one row, split, to tensor memory at `at` (pieces kPieceCols columns apart).
 template <int N>
-__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], uint64_t& check) {
+__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], Check& check) {
   uint32_t h[N / 2], m[N / 2], l[N / 2];
 #pragma unroll
-  for (int i = 0; i < N / 2; ++i) split_pair(w[i], h[i], m[i], l[i], check);
+  for (int i = 0; i < N / 2; ++i) split_pair<false>(w[i], h[i], m[i], l[i], check);
   tmem_st<N / 2>(at, h);
   tmem_st<N / 2>(at + kPieceCols, m);
   tmem_st<N / 2>(at + 2 * kPieceCols, l);
@@ -370,7 +379,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   const int n = (keys_end + kStream - 1) / kStream;
   const int i = i0 + row;
 
-  uint64_t check = 0;
+  Check check;
   typename L::Tile stage_k, stage_v;
   stage_k.load(k, 0, g.t_k, g.hd);
   {
@@ -449,7 +458,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok && !is_bad(check))) break;  // (nothing is in flight here)
+    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
@@ -487,7 +496,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   }
   ok = __syncthreads_and(ok);
   if (ok) {
-    if (__syncthreads_or(is_bad(check))) {
+    if (__syncthreads_or(check.bad())) {
       rows_again<HD, Op::Fwd, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, i0, raw);
     } else {
       exchange[group][row] = denom;
@@ -612,7 +621,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
   const int n = (end - begin + kStream - 1) / kStream;
   auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
   bool ok = true;
-  uint64_t check = 0;
+  Check check;
 
   if (warp == kRowWarps) {
     // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
@@ -713,7 +722,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
         for (int c = 0; c < OW / 8; ++c) {
           uint32_t hi[4], mi[4], lo[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split_pair(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
+          for (int e = 0; e < 4; ++e) split_pair<true>(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
           const uint32_t to = lanes + L::kHeldCol + h * (3 * HD / 2) + group * (OW / 2) + 4 * c;
           tmem_st4(to, hi);
           tmem_st4(to + HD / 2, mi);
@@ -810,7 +819,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
     }
     ok = __syncthreads_and(ok);
-    const bool bad = __syncthreads_or(is_bad(check));
+    const bool bad = __syncthreads_or(check.bad());
     if (ok && bad) {
       rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
     } else if (ok && mine < owned) {
@@ -876,7 +885,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   const int n = (end - begin + kStream - 1) / kStream;
   const int mine = first + row;  // this thread's row
 
-  uint64_t check = 0;
+  Check check;
   // the streamed tile j, and what goes with its rows
   auto stage_tile = [&](int j) {
     const int x0 = begin + j * kStream;
@@ -916,7 +925,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     stage1.load(held1, first, owned, g.hd_v);
     uint32_t h[OW / 2], m[OW / 2], l[OW / 2];
 #pragma unroll
-    for (int e = 0; e < OW / 2; ++e) split_pair(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
+    for (int e = 0; e < OW / 2; ++e) split_pair<true>(f2_pack(x[e / 4][2 * (e % 4)], x[e / 4][2 * (e % 4) + 1]), h[e], m[e], l[e], check);
     const uint32_t to = lanes + L::kHeldT + group * (OW / 2);
     tmem_st<OW / 2>(to, h);
     tmem_st<OW / 2>(to + HD / 2, m);
@@ -977,7 +986,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
     tmem_st_wait();
     tc_fence_before_sync();
-    if (!__syncthreads_and(ok && !is_bad(check))) break;  // (nothing is in flight here)
+    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
     if (issues && elect_one()) {
       tc_fence_after_sync();
       issue_weigh<HD>(tmem + L::kOut, tmem + (kKV ? L::kP : L::kDs), base + (kKV ? L::kTile1 : L::kTile0));
@@ -1002,7 +1011,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
     }
   }
   ok = __syncthreads_and(ok);
-  const bool bad = __syncthreads_or(is_bad(check));
+  const bool bad = __syncthreads_or(check.bad());
   if (ok && bad) {
     rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
   } else if (ok && mine < owned) {

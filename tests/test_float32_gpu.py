@@ -129,3 +129,21 @@ def test_a_row_whose_only_key_is_nan(hd, dtype, dev):
     out, lse = host.Attention(dev, q, k, v, causal=True, key_mask=mask).forward()
     assert np.isnan(out[0].astype(np.float32)).all() and np.isnan(lse[0, 3:]).all() and np.isneginf(lse[0, :3]).all()
     assert np.isfinite(out[1].astype(np.float32)).all() and np.isfinite(lse[1]).all()
+
+
+@pytest.mark.parametrize("hd", [32, 64, 128])
+@pytest.mark.parametrize(("which", "power"), [("q", -118), ("v", -118), ("do", -118)])
+def test_small_operands_keep_their_bits(which, power, hd):
+    """Operands near the end of float32's range, whose third piece would lie below bfloat16's: the results keep the
+    accuracy of float32 sums (the bound above; two pieces alone would leave 2^-17 of every operand)."""
+    q, k, v, do = _problem(7 + hd, 2, 150, 150, hd, hd)
+    scale = hd**-0.5
+    small = np.float32(2.0**power)
+    if which == "q":
+        q, scale = q * small, scale * 2.0**60
+        k = k * np.float32(2.0**58)
+    elif which == "v":
+        v = v * small
+    else:
+        do = do * small
+    _compare(_step(q, k, v, do, None, True, scale), _step64(q, k, v, do, None, True, scale), 8 * 150**0.5 * 2.0**-24)
