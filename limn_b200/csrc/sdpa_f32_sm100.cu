@@ -42,6 +42,9 @@ using namespace ptx;
 constexpr int kRows = 128;    // rows a block owns
 constexpr int kStream = 64;   // rows of a streamed tile
 constexpr unsigned kFull = 0xffffffffu;
+// dS goes to the tensor cores this much larger: its third piece is then a bfloat16 wherever dS is a float32, however small
+// the gradients (an overflow shows in the split or in the sums, which are divided by it again).
+constexpr float kDsUp = 65536.f;
 constexpr int kPieceCols = kStream / 2;  // tensor-memory columns of one 16-bit piece of a (kRows x kStream) matrix
 
 struct Params {
@@ -51,7 +54,7 @@ struct Params {
   long long bh;
   int slots, group;  // row tiles per problem; problems scheduled side by side
   int t_q, t_k, hd, hd_v, causal;
-  float scale, c_hi, c_lo;  // c_hi + c_lo = scale * log2(e), c_lo > 0
+  float scale, ds_scale, c_hi, c_lo;  // ds_scale = scale * kDsUp; c_hi + c_lo = scale * log2(e), c_lo > 0
   bool wide_out;  // the results take 16-byte stores
 };
 
@@ -529,12 +532,13 @@ __device__ __forceinline__ void to_log2(const float lse, float& hi, float& lo) {
   lo = fmaf(lse, kHi, -hi) + lse * kLo;
 }
 
-// What both backward kernels do with the scores of a row: P = 2^(s c - L), dS = P (dP - delta) scale, 0 where unseen.
+// What both backward kernels do with the scores of a row: P = 2^(s c - L), kDsUp dS = P (dP - delta) scale kDsUp, 0 where
+// unseen.
 // `hi`, `lo`, `delta` give a column's L (in log2 units) and delta; a row's own ones repeated in the dQ pass.
 template <int CW, typename Columns>
 __device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s)[CW], const uint32_t (&dp)[CW], uint32_t unseen,
                                              Columns columns, uint64_t (&p)[CW / 2], uint64_t (&ds)[CW / 2]) {
-  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale = f2_pack(g.scale, g.scale);
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo), scale = f2_pack(g.ds_scale, g.ds_scale);
   const uint64_t minus = f2_pack(-1.f, -1.f);
 #pragma unroll
   for (int c = 0; c < CW / 2; ++c) {
@@ -556,6 +560,16 @@ __device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s
       f2_unpack(ds[c], a, b);
       ds[c] = f2_pack((unseen >> (2 * c)) & 1u ? 0.f : a, (unseen >> (2 * c + 1)) & 1u ? 0.f : b);
     }
+  }
+}
+
+// The sums over dS at their own size again. One that overflowed at kDsUp times it counts as a weight that was not finite.
+template <int N>
+__device__ __forceinline__ void settle(uint64_t (&acc)[N], Check& check) {
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    check.weights = f2_fma(acc[c], 0ull, check.weights);
+    acc[c] = f2_mul(acc[c], f2_pack(1.f / kDsUp, 1.f / kDsUp));
   }
 }
 
@@ -818,6 +832,7 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
       }
       if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
     }
+    settle(acc0, check);
     ok = __syncthreads_and(ok);
     const bool bad = __syncthreads_or(check.bad());
     if (ok && bad) {
@@ -1010,6 +1025,8 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
       if (issues && elect_one()) issue_tile();
     }
   }
+  if (kKV) settle(acc1, check);
+  else settle(acc0, check);
   ok = __syncthreads_and(ok);
   const bool bad = __syncthreads_or(check.bad());
   if (ok && bad) {
@@ -1041,6 +1058,7 @@ int launch_sized(Op op, const Problem& p) {
   g.slots = ((op == Op::BwdKV ? p.t_k : p.t_q) + kRows - 1) / kRows;
   g.t_q = p.t_q, g.t_k = p.t_k, g.hd = p.hd, g.hd_v = p.hd_v, g.causal = p.causal ? 1 : 0;
   g.scale = static_cast<float>(p.scale);
+  g.ds_scale = g.scale * kDsUp;
   const double c = static_cast<double>(g.scale) * 1.4426950408889634;
   g.c_hi = static_cast<float>(c);
   if (g.c_hi > c) g.c_hi = nextafterf(g.c_hi, 0.f);

@@ -147,3 +147,12 @@ def test_small_operands_keep_their_bits(which, power, hd):
     else:
         do = do * small
     _compare(_step(q, k, v, do, None, True, scale), _step64(q, k, v, do, None, True, scale), 8 * 150**0.5 * 2.0**-24)
+
+
+@pytest.mark.parametrize("hd", [32, 64, 128])
+def test_small_gradients_keep_their_bits(hd):
+    """dO is still large enough for its three pieces, dS (smaller by a probability and the scale) is not."""
+    q, k, v, do = _problem(17 + hd, 2, 300, 300, hd, hd)
+    do = (np.sign(do) * (1 + np.abs(do) % 1) * 2.0**-108).astype(np.float32)
+    scale = hd**-0.5 / 256
+    _compare(_step(q, k, v, do, None, False, scale), _step64(q, k, v, do, None, False, scale), 1.5e-6)
