@@ -89,7 +89,7 @@ int work_group(const Problem& p, long long items, int sms) {
   // Otherwise by locality: the items running side by side should share few enough K and V tiles for L2
   // (256 problems of S = 4096, D = 128: groups of 8 to 16 are 1.5 % faster than 32, 10 % faster than one group).
   constexpr long long kL2Share = 32LL << 20;  // of B200's 126 MB
-  const long long streamed = static_cast<long long>(p.t_k) * (p.hd + p.hd_v) * 2;  // K and V of one problem, 16-bit
+  const long long streamed = static_cast<long long>(p.t_k) * (p.hd + p.hd_v) * (p.dtype == LIMN_B200_F32 ? 4 : 2);  // K and V of one problem
   long long group = streamed > 0 ? kL2Share / streamed : 1;
   if (group < 1) group = 1;
   if (group > all) group = all;
