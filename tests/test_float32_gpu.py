@@ -156,3 +156,15 @@ def test_small_gradients_keep_their_bits(hd):
     do = (np.sign(do) * (1 + np.abs(do) % 1) * 2.0**-108).astype(np.float32)
     scale = hd**-0.5 / 256
     _compare(_step(q, k, v, do, None, False, scale), _step64(q, k, v, do, None, False, scale), 1.5e-6)
+
+
+@pytest.mark.parametrize("hd", [24, 64, 100])
+@pytest.mark.parametrize("scale", [-0.1, 0.0])
+def test_scales_that_are_not_positive(scale, hd):
+    """These stay on the tiled CUDA-core kernels at every width."""
+    q, k, v, do = _problem(27 + hd, 2, 130, 130, hd, hd)
+    got, want = _step(q, k, v, do, None, True, scale), _step64(q, k, v, do, None, True, scale)
+    if scale == 0.0:
+        assert (got[2] == 0).all() and (got[3] == 0).all()
+        got[2], want[2], got[3], want[3] = got[0], want[0], got[0], want[0]
+    _compare(got, want, 8 * 130**0.5 * 2.0**-24)
