@@ -549,19 +549,18 @@ def decode_cases(args, world: int, torch, device, barrier, max_over_ranks) -> di
 
 
 def off_grid_cases(args, world: int, torch, device, barrier, max_over_ranks) -> dict:
-    """Shapes outside the four BASELINE configurations that the ops are still called with, device-resident, forward and
-    forward+backward (row dot as its own launch). "float32": float32 storage and accuracy, each operand in three
-    bfloat16 pieces on the tensor cores
-    (limn's numpy and c devices run BASELINE's first configuration this way, and a model kept in float32 calls the
-    ops like this), set against the float32 multiply-add rate of the CUDA cores (SMs x 128 lanes x 2 x the maximum SM
-    clock: a nominal figure, nothing measures it here, and no bound on this path). "narrow_heads": bfloat16 with head dims that are not 64 or 128, which
-    run zero-padded in the tensor-core kernels; credited with the flops of the real head dim."""
+    """Shapes outside the four headline configurations that the ops are still called with, device-resident, forward and
+    forward+backward (row dot as its own launch). "float32": float32 storage and accuracy (limn's numpy and c devices run
+    the smallest configuration this way, and a model kept in float32 calls the ops like this), each operand in three
+    bfloat16 pieces on the tensor cores: six products for one, so its bound is a sixth of the measured bfloat16 rate.
+    "narrow_heads": bfloat16 with head dims that are not 64 or 128, which run zero-padded in the tensor-core kernels;
+    credited with the flops of the real head dim."""
     from limn_b200._lib import lib
 
     L = lib()
-    props = torch.cuda.get_device_properties(device)
-    fma_peak = props.multi_processor_count * 128 * 2 * 1.965e9 / 1e12
-    found = {"float32": {"fp32_fma_tflops_nominal": fma_peak}, "narrow_heads": {}}
+    peak, _ = peaks()
+    split_peak = float(peak.get("bf16_tflops", FALLBACK_PEAKS["bf16_tflops"])) / 6
+    found = {"float32": {"sixth_of_measured_bf16_tflops": split_peak}, "narrow_heads": {}}
     cases = (("float32", "reference_cpu_case_B1_H2_S128_D32_causal", 2, 128, 32, True),
              ("float32", "gpt_layer_in_float32_B32_H8_S256_D64_causal", 256, 256, 64, True),
              ("float32", "B4_H16_S1024_D128_causal", 64, 1024, 128, True),
@@ -602,7 +601,7 @@ def off_grid_cases(args, world: int, torch, device, barrier, max_over_ranks) -> 
             entry[key + "_tflops"] = credit * fwd_flops(bh * world, s, d, causal) / (ms * 1e-3) / 1e12
             if f32:
                 executed = (1.0 if key == "fwd" else 4.5) * fwd_flops(bh, s, d, causal) / (ms * 1e-3) / 1e12
-                entry[key + "_executed_frac_of_fp32_fma_nominal"] = executed / fma_peak
+                entry[key + "_executed_frac_of_sixth_of_measured_bf16"] = executed / split_peak
         found[family][name] = entry
     return found
 

@@ -39,10 +39,12 @@ enum limn_b200_status {
 
 /* Which kernel family served (or would serve) a problem. */
 enum limn_b200_path {
-  LIMN_B200_PATH_GENERAL = 0,  /* SIMT kernels: any float dtype, any hd/hd_v */
+  LIMN_B200_PATH_GENERAL = 0,  /* everything else, any float dtype, any hd/hd_v: SIMT kernels, except that float32 with hd and hd_v up
+                                  to 128 and sides of 16 rows and more runs on the tensor cores where that is faster, at float32
+                                  accuracy (this query does not tell the two apart) */
   LIMN_B200_PATH_TCGEN05 = 1,  /* TMA + tcgen05 kernels: f16/bf16, hd and hd_v multiples of 8 up to 128 (run as 64 or 128), any t_q/t_k, with or without key mask */
   LIMN_B200_PATH_DECODE = 2    /* forward only, no causal mask (the step of a kv cache), hd and hd_v multiples of 8 up to 128,
-                                  dense or strided rows on 16-byte boundaries: t_q <= 4 in f16/bf16, t_q < 16 in float32. One CTA
+                                  rows on 16-byte boundaries: t_q <= 4 in f16/bf16 (dense or strided), t_q < 16 in float32 (dense). One CTA
                                   or cluster streams a problem's keys and values once, bound by HBM, no tensor cores */
 };
 

@@ -3,10 +3,11 @@
 // float32 has to keep its own width (the reference checks it at 1e-5: tests/test_attention.py:250-255), and the tensor
 // cores multiply 8-bit significands in bfloat16. Three of those hold a float32: x = h + m + l, each the bfloat16
 // nearest to what the ones before left, 8 + 8 + 8 bits and two signs. A product of two float32 matrices is then the
-// sum of six bfloat16 products, h h + (h m + m h) + (m m + h l + l h); what is left out (m l, l m, l l) is 2^-26 of it,
-// less than float32's own rounding. The accumulator adds in float32 but truncates, so the six are issued smallest
-// first, and no total stays in tensor memory for longer than one tile: every tile's product starts from zero and is
-// added to the row's total in registers, rounded to nearest, as the CUDA-core kernels in sdpa_general_tiled.cu do.
+// sum of six bfloat16 products, h h + (h m + m h) + (m m + h l + l h); what is left out (m l, l m, l l) is 2^-24.3 of it at
+// most and 2^-27.5 in the root mean square, about float32's own rounding. The accumulator adds in float32 but truncates,
+// so the six are issued smallest first, and no total stays in tensor memory for longer than one tile: every tile's
+// product starts from zero and is added to the row's total in registers, rounded to nearest, as the CUDA-core kernels
+// (tiled_rows.cuh) do.
 //
 // What bounds it: six bfloat16 products at 4096 multiply-adds a clock and SM are 683 float32 multiply-adds a clock,
 // against 128 on the CUDA cores; the split, the softmax and the running totals stay there and take about as long as the
@@ -22,11 +23,11 @@
 // 128-byte-swizzled layout; probabilities and dS are split in registers and go to tensor memory as the A operand.
 //
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
-// number (inf - inf in the split, inf * 0 between pieces). The split notices (its remainder is NaN), and a block that
-// met one computes its rows again on the CUDA cores, with the code of the tiled kernels there (a step whose every block
-// does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 507 / 1 984 / 2 556, the tiled kernels alone 1 340 / 1 790 / 2 410;
-// one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above head dim 64 leave their loop when
-// they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
+// number (inf - inf in the split, inf * 0 between pieces), and one below about 2^-110 would lose its last bits. The split
+// notices both, and a block that met one computes its rows again on the CUDA cores, with the code of the tiled kernels
+// there (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 507 / 1 984 / 2 556, the tiled
+// kernels alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above
+// head dim 64 leave their loop when they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
 #include <cmath>
 #include <cstdint>
 
@@ -583,10 +584,10 @@ __device__ __forceinline__ uint32_t outside(int from, int to) {
 }
 
 // ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
-// Sixteen row warps (four threads to a row) load, split, weigh and sum; a seventeenth issues every MMA. It used to be one
-// of the sixteen: issuing a tile's MMAs takes as long as the tensor cores take to run them (2400 + 1160 clocks of the
-// 5200 a dQ tile took at head dim 64), the other fifteen had nothing to do meanwhile, and the tensor cores nothing while
-// the sixteenth caught up. Now a tile's scores run while the tile before it is weighed. Rows and issuer tell each other
+// Sixteen row warps (four threads to a row) load, split, weigh and sum; a seventeenth issues every MMA, so that a tile's
+// scores run while the tile before it is weighed. Issuing a tile's MMAs takes as long as the tensor cores take to run them: with
+// one of the sixteen as issuer that was 2400 + 1160 clocks of the 5200 a dQ tile took at head dim 64, in which the other fifteen
+// had nothing to do, and the tensor cores nothing while the issuer caught up. Rows and issuer tell each other
 // through mbarriers whose waits are bounded; no barrier of the block stands inside the loop, so a warp that gave up on a
 // wait cannot hang the others.
 template <int HD, bool kKV, bool kWide>

@@ -332,8 +332,8 @@ row_dot16_kernel(const uint4* __restrict__ out, const uint4* __restrict__ dout, 
   }
 }
 
-// The same for float32: four elements of a row to a thread. One warp to a row, each lane striding through it, took 10.3 us
-// for 65536 rows of 64; the two operands are 5 us of reading.
+// The same for float32: four elements of a row to a thread, 5.2 us for 65536 rows of 64, which is the time to read the two
+// operands (one warp to a row, each lane striding through it: 10.3 us).
 template <int kLanes>
 __global__ void __launch_bounds__(256)
 row_dot32_kernel(const float4* __restrict__ out, const float4* __restrict__ dout, float* __restrict__ delta, long long rows, int pieces) {
