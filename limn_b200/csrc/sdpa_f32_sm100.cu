@@ -1102,6 +1102,25 @@ int launch_sized(Op op, const Problem& p) {
   return LIMN_B200_OK;
 }
 
+// Many short problems are better off in the tiled CUDA-core kernels: with both sides inside one 64-row tile half of a block's
+// 128 rows are empty, a head dim below the kernel's width is padding, and a block's fixed cost is all there is, while several
+// of their 256-thread blocks share an SM. Measured on B200 as time here over time there, from 16 x 16 to 64 x 64 rows, at 512 /
+// 2048 / 8192 problems: dQ 1.2-1.4 / 1.4-1.6 / 1.4-1.7 at head dim 8, 1.1-1.3 / 1.3-1.4 / 1.1-1.5 at 16, 0.95-1.05 / 1.1-1.2 /
+// 1.0-1.2 at 32; dK and dV 1.1-1.2 / 1.2-1.4 / 1.2-1.4, 1.0-1.1 / 1.1-1.2 / 1.1-1.3, and at 32 with up to 32 queries 0.9-1.05 /
+// 1.04-1.1 / 1.1; the forward 1.0-1.2 at head dim 8, at 16 up to 16 x 64 rows 1.0-1.1, at 32 0.65-0.8. At head dim 64 all
+// three gain here (0.5-1.0); at 128 the forward loses up to 32 keys (1.05-1.35) and dQ up to 16 (1.04-1.1, 0.9 at 64 x 16). At
+// 128 problems and fewer, one block to an SM, and from 65 rows on everything gains here (0.3-0.9).
+bool short_rows(Op op, const Problem& p) {
+  if (p.t_q > 64 || p.t_k > 64) return false;
+  int sms = 0;
+  if (sm_count(&sms) != LIMN_B200_OK || p.bh <= 3LL * sms) return false;
+  const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
+  if (widest <= 16) return op != Op::Fwd || widest * p.t_q * p.t_k <= 8 * 64 * 64;
+  if (widest <= 32) return p.bh > 4LL * sms && (op == Op::BwdQ || (op == Op::BwdKV && p.t_q <= 32));
+  if (widest <= 64) return false;
+  return op == Op::Fwd ? p.t_k <= 32 : op == Op::BwdQ && p.t_k <= 16;
+}
+
 }  // namespace
 
 bool f32_split_serves(Op op, const Problem& p) {
@@ -1112,7 +1131,7 @@ bool f32_split_serves(Op op, const Problem& p) {
   const float scale = static_cast<float>(p.scale);
   if (!(scale > 1e-20f && scale < 1e20f)) return false;
   const long long rows = op == Op::BwdKV ? p.t_k : p.t_q;
-  return p.bh * ((rows + kRows - 1) / kRows) <= 0x7fffffffLL;
+  return p.bh * ((rows + kRows - 1) / kRows) <= 0x7fffffffLL && !short_rows(op, p);
 }
 
 int f32_split_launch(Op op, const Problem& p) {

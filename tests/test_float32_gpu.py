@@ -168,3 +168,17 @@ def test_scales_that_are_not_positive(scale, hd):
         assert (got[2] == 0).all() and (got[3] == 0).all()
         got[2], want[2], got[3], want[3] = got[0], want[0], got[0], want[0]
     _compare(got, want, 8 * 130**0.5 * 2.0**-24)
+
+
+@pytest.mark.parametrize("hd", [8, 16, 24, 32, 72, 128])
+def test_many_short_problems(hd):
+    """Which kernels take a few hundred short problems depends on their number, sides and width: the edges of that rule, with
+    and without masks, all against float64 (and so against one another)."""
+    for bh, t_q, t_k, causal, masked in ((700, 16, 16, True, False), (700, 32, 33, False, True), (460, 64, 64, True, True), (700, 17, 64, False, False),
+                                         (700, 64, 32, False, True), (440, 33, 16, False, False), (600, 65, 64, False, False)):
+        q, k, v, do = _problem(hd + t_q, bh, t_q, t_k, hd, hd)
+        mask = None
+        if masked:
+            mask = (np.random.default_rng(t_k).random((bh, t_k)) > 0.2).astype(np.float32)
+            mask[:, 0] = 1
+        _compare(_step(q, k, v, do, mask, causal, hd**-0.5), _step64(q, k, v, do, mask, causal, hd**-0.5), 8 * 64**0.5 * 2.0**-24)
