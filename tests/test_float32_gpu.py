@@ -182,3 +182,13 @@ def test_many_short_problems(hd):
             mask = (np.random.default_rng(t_k).random((bh, t_k)) > 0.2).astype(np.float32)
             mask[:, 0] = 1
         _compare(_step(q, k, v, do, mask, causal, hd**-0.5), _step64(q, k, v, do, mask, causal, hd**-0.5), 8 * 64**0.5 * 2.0**-24)
+
+
+@pytest.mark.parametrize(("t_q", "t_k", "hd"), [(256, 256, 64), (256, 256, 48), (131, 200, 37)])
+def test_truncated_scores_do_not_show_in_l(t_q, t_k, hd):
+    """L against float64 over 32 problems: rounding it once leaves 2.6e-8; without the mean of what the scores' additions
+    truncate put back it is 3.6e-8."""
+    q, k, v, do = _problem(37 + hd, 32, t_q, t_k, hd, hd)
+    causal = t_q == t_k
+    got, want = (f(q, k, v, do, None, causal, hd**-0.5)[1] for f in (_step, _step64))
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 3.2e-8
