@@ -13,6 +13,14 @@ import pytest
 pytestmark = pytest.mark.gpu
 ROOT = Path(__file__).resolve().parent.parent
 
+
+@pytest.fixture(scope="module")
+def dev():
+    import limn_standin as host
+
+    return host.Device()
+
+
 FIRST_CALLS = """
 import torch
 from limn_b200._lib import check, lib
