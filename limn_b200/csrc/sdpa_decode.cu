@@ -314,7 +314,11 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
         else if (kKind == kF16) *reinterpret_cast<__half*>(dst) = __float2half_rn(value);
         else *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(value);
       }
-      if (d == 0) prm.lse[static_cast<long long>(problem) * prm.t_q + row] = m_tot * prm.scale + logf(l_tot);
+      if (d == 0) {  // in float32 once per row in double: L is then as good as its sum
+        const long long to = static_cast<long long>(problem) * prm.t_q + row;
+        if (kKind == kF32) prm.lse[to] = static_cast<float>(static_cast<double>(m_tot) * prm.scale + log(static_cast<double>(l_tot)));
+        else prm.lse[to] = m_tot * prm.scale + logf(l_tot);
+      }
     }
   }
   if (split > 1) cluster_sync();  // no CTA leaves while CTA 0 may still be reading its shared memory
