@@ -1107,21 +1107,25 @@ int launch_sized(Op op, const Problem& p) {
 
 // Many short problems are better off in the tiled CUDA-core kernels: with both sides inside one 64-row tile half of a block's
 // 128 rows are empty, a head dim below the kernel's width is padding, and a block's fixed cost is all there is, while several
-// of their 256-thread blocks share an SM. Measured on B200 as time here over time there, from 16 x 16 to 64 x 64 rows, at 512 /
-// 2048 / 8192 problems: dQ 1.2-1.4 / 1.4-1.6 / 1.4-1.7 at head dim 8, 1.1-1.3 / 1.3-1.4 / 1.1-1.5 at 16, 0.95-1.05 / 1.1-1.2 /
-// 1.0-1.2 at 32; dK and dV 1.1-1.2 / 1.2-1.4 / 1.2-1.4, 1.0-1.1 / 1.1-1.2 / 1.1-1.3, and at 32 with up to 32 queries 0.9-1.05 /
-// 1.04-1.1 / 1.1; the forward 1.0-1.2 at head dim 8, at 16 up to 16 x 64 rows 1.0-1.1, at 32 0.65-0.8. At head dim 64 all
-// three gain here (0.5-1.0); at 128 the forward loses up to 32 keys (1.05-1.35) and dQ up to 16 (1.04-1.1, 0.9 at 64 x 16). At
-// 128 problems and fewer, one block to an SM, and from 65 rows on everything gains here (0.3-0.9).
+// of their 256-thread blocks share an SM. Measured on B200 as time here over time there, 16 x 16 to 64 x 64 rows:
+//   forward  head dims 8 and 16: 0.9-1.1 at 256 problems, 1.2-1.5 at 384 and more; 24: 1.07-1.2 from 384 on; 32: 0.65-0.8;
+//            72 to 128 with up to 32 keys: 1.1-1.8 from 256 problems on (beyond 32 keys 1.1 at 72, 0.7 at 128)
+//   dQ       8 and 16: 1.0-1.3 at 256 and 384 problems, 1.1-1.7 beyond; 32: 0.95-1.05 at 512, 1.0-1.2 beyond; 72 and 100 with
+//            up to 32 keys 1.04-1.4; 128 with up to 16 keys 0.9-1.1
+//   dK, dV   8: 1.0-1.1 at 384; 8 and 16: 1.0-1.2 at 512, 1.1-1.4 beyond; 32 with up to 32 queries 0.9-1.05 at 512, 1.04-1.13
+//            beyond; 72 to 128: 0.5-0.9
+// At head dim 64 all three gain here (0.5-1.0), at 40 all but dQ of thousands of problems of 16 rows (1.1); so does everything at
+// 128 problems, one block to an SM (0.5-0.9, the forward at 72 with up to 32 keys 1.1), and nearly everything from 65 rows on.
 bool short_rows(Op op, const Problem& p) {
   if (p.t_q > 64 || p.t_k > 64) return false;
   int sms = 0;
-  if (sm_count(&sms) != LIMN_B200_OK || p.bh <= 3LL * sms) return false;
+  if (sm_count(&sms) != LIMN_B200_OK || p.bh <= sms) return false;
   const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
-  if (widest <= 16) return op != Op::Fwd || widest * p.t_q * p.t_k <= 8 * 64 * 64;
-  if (widest <= 32) return p.bh > 4LL * sms && (op == Op::BwdQ || (op == Op::BwdKV && p.t_q <= 32));
-  if (widest <= 64) return false;
-  return op == Op::Fwd ? p.t_k <= 32 : op == Op::BwdQ && p.t_k <= 16;
+  if (widest > 64) return op == Op::Fwd ? p.t_k <= 32 : op == Op::BwdQ && p.t_k <= (widest <= 100 ? 32 : 16);
+  if (widest > 32) return false;
+  if (widest <= 16) return op == Op::BwdQ || p.bh > (op == Op::Fwd ? 2LL : 3LL) * sms;
+  if (op == Op::Fwd) return widest <= 24 && p.bh > 2LL * sms;
+  return p.bh > 4LL * sms && (op == Op::BwdQ || p.t_q <= 32);
 }
 
 }  // namespace

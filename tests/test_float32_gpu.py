@@ -183,7 +183,7 @@ def test_many_short_problems(hd):
     """Which kernels take a few hundred short problems depends on their number, sides and width: the edges of that rule, with
     and without masks, all against float64 (and so against one another)."""
     for bh, t_q, t_k, causal, masked in ((700, 16, 16, True, False), (700, 32, 33, False, True), (460, 64, 64, True, True), (700, 17, 64, False, False),
-                                         (700, 64, 32, False, True), (440, 33, 16, False, False), (600, 65, 64, False, False)):
+                                         (700, 64, 32, False, True), (160, 33, 16, False, False), (320, 64, 64, True, False), (600, 65, 64, False, False)):
         q, k, v, do = _problem(hd + t_q, bh, t_q, t_k, hd, hd)
         mask = None
         if masked:
