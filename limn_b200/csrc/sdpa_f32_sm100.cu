@@ -14,8 +14,8 @@
 // MMAs (dQ at head dim 64: 2 300 and 2 500 clocks of a tile's 3 700). Measured on B200 (forward / dQ / dK and dV, us, causal;
 // the CUDA-core kernels in brackets): 256 x 256 keys x 64: 38 / 55 / 71 (121 / 166 / 219); 6 x 8192 x 32: 282 / 286 / 399
 // (1333 / 1777 / 2402); 64 x 1024 x 128: 170 / 224 / 289 (813 / 1117 / 1714); 64 x 32 x 64: 7.3 / 7.6 / 9.2 (10.8 / 12.4 /
-// 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.6e-7 for 5.8e-7, dK 4.3e-7 for 2.2e-6
-// in the 2-norm), L is at the rounding of a float32 like theirs.
+// 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.4e-7 for 6.1e-7, dQ 3.2e-7 for 7.6e-7
+// in the 2-norm), and so is L (256 x 256 x 64: 2.9e-8 for 3.5e-8; rounding it once is 2.6e-8).
 //
 // A block owns 128 rows (query rows in the forward and the dQ pass, key rows in the dK/dV pass), one row to each
 // tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
@@ -25,7 +25,7 @@
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
 // number (inf - inf in the split, inf * 0 between pieces), and one below about 2^-110 would lose its last bits. The split
 // notices both, and a block that met one computes its rows again on the CUDA cores, with the code of the tiled kernels
-// there (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 507 / 1 984 / 2 556, the tiled
+// there (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 213 / 1 984 / 2 548, the tiled
 // kernels alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above
 // head dim 64 leave their loop when they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
 #include <cmath>
