@@ -44,28 +44,26 @@ namespace {
 using namespace ptx;
 
 constexpr int kTile = 128;
-// Ten warps work; the CTA is launched with twelve because the compiler spills less in the elementwise loop at
-// this block size (measured: 1 to 2 % faster). Warps 10 and 11 go straight to the final barrier.
-constexpr int kThreads = 384;
-#ifndef LIMN_BWD_KV_THREADS
-#define LIMN_BWD_KV_THREADS 352
-#endif
-// The dK/dV pass never uses warps 10 and 11 (the dQ pass does, when it computes the row statistics itself), and
-// its elementwise loop comes out of the compiler a little better with one spare warp than with two (1 % at head dim
-// 64, nothing at 128; the dQ pass is 2 to 4 % slower that way and keeps its twelve).
-template <bool kKV>
+// Ten warps work, but the block size decides what the compiler spills where in the elementwise loop. The dQ pass takes
+// twelve (warps 10 and 11 compute the row statistics of the fused entry point, or go straight to the final barrier). The dK/dV
+// pass at head dim 64 ten under a key mask, twelve under a causal one, else eleven; measured with 10, 11 and 12 warps, us: 192
+// padded problems of 500 38.8, 41.9, 42.5; 128 causal of 2048 175.6, 179.1, 162.8; encoder_2k 564, 564, 573; at head dim 128 all
+// three are the same.
+template <int D, bool kCausal, bool kKV, bool kMask>
 constexpr int bwd_threads() {
-  return kKV ? LIMN_BWD_KV_THREADS : kThreads;
+  if (!kKV) return 384;
+  return D == 64 && kMask ? 320 : D == 64 && kCausal ? 384 : 352;
 }
 constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
-// Early schedule: of every 8 pairs of scores, how many take exp2 as a cubic on the FMA pipe instead of on the
-// special-function unit. Measured on B200 with the work-fetching kernels: 1 or 2 of 8 lose 3 to 5 % in the dQ
-// pass and 7 % or more in the dK/dV pass at head dim 64, so the default is none.
+// dQ pass at head dim 64: of every 8 pairs of scores, how many take exp2 as a polynomial (of degree 4: 3e-6, the probability is
+// rounded to 16 bits at once) on the FMA pipe instead of on the special-function unit. Measured with the elected issue, one /
+// two / three of 8 over none: encoder_2k 0.955 / 0.945 / 0.97, 64 problems of 100 x 1500 0.95 / 0.93 / 0.96. Not at head dim 128 (1.02 to
+// 1.04), nor in the dK/dV pass, which spills (1.7).
 #ifndef LIMN_BWD_POLY_PAIRS
-#define LIMN_BWD_POLY_PAIRS 0
+#define LIMN_BWD_POLY_PAIRS 2
 #endif
 constexpr int kPolyPairsOf8 = LIMN_BWD_POLY_PAIRS;
 
@@ -230,7 +228,7 @@ __device__ __forceinline__ float row_dot(const void* a_row, const void* b_row, i
 // S^T and dP^T take turns in one 128-column region, S^T first, dP^T as soon as S^T is in registers, so that
 // 128 columns are left for the operands and every MMA is full width.
 template <int D, bool kCausal, bool kFp16, bool kKV, bool kEarly, bool kSeq, bool kMask>
-__global__ void __launch_bounds__((bwd_threads<kKV>()), 1)
+__global__ void __launch_bounds__((bwd_threads<D, kCausal, kKV, kMask>()), 1)
 sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                 const __grid_constant__ CUtensorMap map_out0, const __grid_constant__ CUtensorMap map_out1, const BwdParams prm) {
@@ -283,7 +281,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     return item;
   };
 
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == kProducerWarp * 32) {
     for (int i = 0; i < B::count; ++i) {
       uint32_t arrivals = 1u;
       if (kSeq) {
@@ -302,17 +300,25 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(bar(i), arrivals);
     }
     mbar_init_fence();
+    tma_prefetch_descriptor(&map_q);
+    tma_prefetch_descriptor(&map_k);
+    tma_prefetch_descriptor(&map_v);
+    tma_prefetch_descriptor(&map_do);
   }
   // up to here nothing has touched global memory, so all of it may run under the tail of the kernel before this one
   grid_dependency_wait();
   grid_launch_dependents();
+  // What is left of the set-up runs side by side: the status word is read, tensor memory allocated (a block that stands
+  // down frees it again), and the producer, which initialised the barriers itself, does not wait for either: its first loads are
+  // on their way. (Once the status word is found set its waits return, and its loads are given time to land at the end.)
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk;
-  if (warp == kMmaWarp) {  // (beside the read of the status word: a block that stands down frees it again)
+  if (warp == kMmaWarp) {
     tmem_alloc(smem_addr(&tmem_slot), kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if (warp == kProducerWarp) named_barrier_arrive(1, bwd_threads<D, kCausal, kKV, kMask>());
+  else named_barrier_sync(1, bwd_threads<D, kCausal, kKV, kMask>());
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
@@ -332,7 +338,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   auto a_wrap = [&](int it) { return static_cast<uint32_t>((it / L::kStagesA) & 1); };
   auto b_wrap = [&](int it) { return static_cast<uint32_t>((it / L::kStagesB) & 1); };
 
-  bool ok = !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
+  bool ok = warp == kProducerWarp || !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
 #ifdef LIMN_TRACE
   int trace_n = 0;
 #endif
@@ -362,10 +368,6 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (warp == kProducerWarp) {
     // ================= TMA producer, work fetcher =================
     if (lane == 0 && ok) {
-      tma_prefetch_descriptor(held_a);
-      tma_prefetch_descriptor(held_b);
-      tma_prefetch_descriptor(stream_a);
-      tma_prefetch_descriptor(stream_b);
       int done = 0;
       for (unsigned n_item = 0; ok; ++n_item) {
         const unsigned ring = n_item & 1u;
@@ -856,8 +858,8 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
             const uint64_t x2 = f2_fma(f2_pack_bits(s[c][e], s[c][e + 1]), sl2_2, neg_l2);
             float p0, p1;
-            if (((e >> 1) & 7) < kPolyPairsOf8) {
-              exp2_poly2(x2, p0, p1);  // on the FMA pipe, beside the special-function unit
+            if (!kKV && D == 64 && ((e >> 1) & 7) < kPolyPairsOf8) {
+              exp2_poly2<4>(x2, p0, p1);  // on the FMA pipe, beside the special-function unit
             } else {
               f2_unpack(x2, p0, p1);
               p0 = exp2_approx(p0), p1 = exp2_approx(p1);
@@ -1099,7 +1101,7 @@ int launch_bwd(const Problem& p) {
               "sizing shared memory for an sdpa backward kernel");
     sized[device] = true;
   }
-  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(bwd_threads<kKV>()), L::kBytes, p.stream, map_q, map_k, map_v, map_do, map_out0, map_out1, prm),
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(bwd_threads<D, kCausal, kKV, kMask>()), L::kBytes, p.stream, map_q, map_k, map_v, map_do, map_out0, map_out1, prm),
             "launching an sdpa backward kernel");
   note_launches(1);
   return LIMN_B200_OK;

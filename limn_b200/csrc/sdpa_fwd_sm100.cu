@@ -509,7 +509,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             // (not under a key mask: the cubic turns a hidden key's -inf into 2^-125 rather than 0, which a row
             // with no visible key at all would then mistake for a denominator)
             if (!kMask && ((i >> 1) & 7) < poly_pairs_of_8<D, kCausal>()) {
-              exp2_poly2(x2, p0, p1);
+              exp2_poly2<3>(x2, p0, p1);
             } else {
               f2_unpack(x2, p0, p1);
               p0 = exp2_approx(p0);
