@@ -39,29 +39,31 @@ using namespace ptx;
 constexpr int kTileRows = 128;   // query rows per Q tile, keys per K/V tile
 constexpr int kQTiles = 2;       // Q tiles per CTA
 // Ten warps work, but the block size decides how the compiler allocates registers in the softmax loop (all sizes
-// end at 168 registers; what differs is what is spilled where), and the best size differs by instantiation.
-// Measured on B200: head dim 128 under a causal mask, 11 warps (0.7 % over 12, 8 % over 10); without a key mask
-// otherwise, 10 warps (head dim 64: 1 to 5 % over 12; head dim 128 without a causal mask: 1 %); the key-mask kernels
-// stay at the 12 they were tuned with. The spare warps go straight to the final barrier.
-template <int D, bool kCausal, bool kMask>
+// end at 168 registers; what differs is what is spilled where). Measured on B200 with the elected issue: head dim 128 under a
+// causal mask 10 warps, 5 % over 11 and 12 (prefill_4k 0.912, 0.964 and 0.957 ms); the key-mask kernels stay at the 12 they were
+// tuned with. The spare warps go straight to the final barrier.
+template <bool kMask>
 constexpr int fwd_threads() {
-  return kMask ? 384 : (D == 128 && kCausal) ? 352 : 320;
+  return kMask ? 384 : 320;
 }
 constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleSlack = 8.f;   // log2 units a row maximum may outgrow its reference before O is rescaled
-// Of every 8 pairs of scores, how many take exp2 as a cubic on the FMA pipe instead of on the special-function
-// unit. Measured on B200: one pair is best at head dim 64 and without a causal mask (1 to 2.5 % over none or two),
-// none under a causal mask at head dim 128 (1 to 2 % over one or two); three or more are slower everywhere.
-// LIMN_POLY_PAIRS overrides the choice for experiments.
-template <int D, bool kCausal>
+// Of every 8 pairs of scores, how many take exp2 as a polynomial on the FMA pipe instead of on the special-function
+// unit. Measured on B200 with the elected issue, as time over that without any: head dim 64 two pairs 0.95 to 0.98 (one 1.0,
+// three 1.0), under a key mask two 0.95 but 1.03 with a causal mask on top; head dim 128 without a mask one pair of degree 3 0.96
+// (degree 4 or 5 gain nothing), with any mask 1.0 to 1.02. Degree 5 at head dim 64 keeps the log-sum-exp at float32's own
+// accuracy, 4e-8 (a cubic in one pair of eight: 1e-7 to 1.6e-6), for 1 % of the time. LIMN_POLY_PAIRS overrides the choice for
+// experiments.
+template <int D, bool kCausal, bool kMask>
 constexpr int poly_pairs_of_8() {
 #ifdef LIMN_POLY_PAIRS
   return LIMN_POLY_PAIRS;
 #else
-  return (D == 128 && kCausal) ? 0 : 1;
+  if (D == 64) return kCausal && kMask ? 0 : 2;
+  return kCausal || kMask ? 0 : 1;
 #endif
 }
 
@@ -108,7 +110,8 @@ struct FwdBars {
   static constexpr int work_empty = work_full + 2;  // + slot: every consumer has read it
   static constexpr int stage_full = work_empty + 2;   // + t: every row of a staging block is written (128 arrivals)
   static constexpr int stage_free = stage_full + 2;   // + t: the tile store has read the block
-  static constexpr int count = stage_free + 2;
+  static constexpr int merge_full = stage_free + 2;   // shared item: Q tile 1's part of every row is complete (128 arrivals)
+  static constexpr int count = merge_full + 1;
 };
 
 // Build-time diagnostic (-DLIMN_TRACE): one CTA records clock64() at each step of its pipeline into a
@@ -140,8 +143,8 @@ struct FwdParams {
   float scale;
 };
 
-template <int D, bool kCausal, bool kFp16, bool kMask>
-__global__ void __launch_bounds__((fwd_threads<D, kCausal, kMask>()), 1)
+template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared>
+__global__ void __launch_bounds__((fwd_threads<kMask>()), 1)
 sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const FwdParams prm) {
   using L = FwdLayout<D, kCausal, kMask>;
@@ -150,13 +153,14 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __shared__ uint32_t tmem_slot;
   __shared__ uint32_t abort_flag;
   __shared__ unsigned work_ring[2];
+  __shared__ float merge_m[kTileRows], merge_l[kTileRows];  // shared item: from Q tile 1's softmax group to the other
 
   const uint32_t raw = smem_addr(smem_unaligned);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const uint32_t bars = base + L::kBarOff;
   auto bar = [&](int i) { return bars + 8u * i; };
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (the same in every lane, and known to be)
   const int lane = threadIdx.x & 31;
 
   // ---- which rows a work item covers ----
@@ -165,7 +169,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     int head, batch;    // the problem's coordinates in the operands
     int q0[kQTiles];    // first query row of each Q tile
     int n_kv[kQTiles];  // key tiles each Q tile consumes
-    int n_max;
+    int n_max;          // the larger of the two
+    int loads;          // key tiles the item streams
   };
   auto decode = [&](unsigned index) {
     Item it;
@@ -181,37 +186,50 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (kCausal) n = min(n, pair * kQTiles + t + 1);
       it.n_kv[t] = it.q0[t] < prm.t_q ? n : 0;
     }
+    it.loads = max(it.n_kv[0], it.n_kv[1]);
+    if (kShared) {
+      it.q0[1] = it.q0[0];
+      it.n_kv[1] = it.loads / 2;
+      it.n_kv[0] = it.loads - it.n_kv[1];
+    }
     it.n_max = max(it.n_kv[0], it.n_kv[1]);
     return it;
   };
 
   // ---- set-up: barriers, tensor memory ----
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == kProducerWarp * 32) {
     for (int i = 0; i < B::count; ++i) {
       unsigned arrivals = 1u;
       if ((i >= B::p_full && i < B::p_full + 2) || (i >= B::p_half && i < B::p_half + 2) || (i >= B::o_free && i < B::o_free + 2) ||
-          (i >= B::stage_full && i < B::stage_full + 2))
+          (i >= B::stage_full && i < B::stage_full + 2) || i == B::merge_full)
         arrivals = 128u;                                           // every thread of a softmax group
       if (i >= B::work_empty && i < B::work_empty + 2) arrivals = 9u;  // the MMA warp and the eight softmax warps
       mbar_init(bar(i), arrivals);
     }
     mbar_init_fence();
+    tma_prefetch_descriptor(&map_q);
+    tma_prefetch_descriptor(&map_k);
+    tma_prefetch_descriptor(&map_v);
   }
   // up to here nothing has touched global memory, so all of it may run under the tail of the kernel before this one
   grid_dependency_wait();
   grid_launch_dependents();
+  // What is left of the set-up runs side by side: the status word is read, tensor memory allocated (a block that stands
+  // down frees it again), and the producer, which initialised the barriers itself, does not wait for either: its first loads are
+  // on their way. (Once the status word is found set its waits return, and its loads are given time to land at the end.) A
+  // kernel of one tile: 6.0 -> 5.5 us.
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk;
-  __syncthreads();
-  if (warp == kMmaWarp && !abort_flag) {
+  if (warp == kMmaWarp) {  // (beside the read of the status word: a block that stands down frees it again)
     tmem_alloc(smem_addr(&tmem_slot), kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if (warp == kProducerWarp) named_barrier_arrive(1, fwd_threads<kMask>());
+  else named_barrier_sync(1, fwd_threads<kMask>());
   tc_fence_after_sync();
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
-  bool ok = !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
+  bool ok = warp == kProducerWarp || !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
 #ifdef LIMN_TRACE
   int trace_n = 0;
 #endif
@@ -230,9 +248,6 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (warp == kProducerWarp) {
     // ================= TMA producer, work fetcher =================
     if (lane == 0 && ok) {
-      tma_prefetch_descriptor(&map_q);
-      tma_prefetch_descriptor(&map_k);
-      tma_prefetch_descriptor(&map_v);
       unsigned q_uses[kQTiles] = {0u, 0u};  // items so far in which Q tile t had rows
       unsigned step = 0;                    // key tiles loaded so far, over all items
       for (unsigned n_item = 0; ok; ++n_item) {
@@ -258,7 +273,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             tma_load_4d(base + L::kQOff + t * L::kTileBytes + a * L::kAtomBytes, &map_q, bar(B::q_full + t), a * 64,
                         item.q0[t], item.head, item.batch);
         }
-        for (int j = 0; j < item.n_max && ok; ++j, ++step) {
+        for (int j = 0; j < item.loads && ok; ++j, ++step) {
           const int stage = step % L::kStages;
           const uint32_t wrap = (step / L::kStages) & 1;
           ok = mbar_wait(bar(B::k_empty + stage), wrap ^ 1u, prm.status, 0x0100u | stage);
@@ -280,7 +295,12 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
   } else if (warp == kMmaWarp) {
     // ================= MMA issuer =================
-    if (lane == 0 && ok) {
+    // The warp stays together and one lane of it is elected for each bunch of MMAs: what the instructions take from uniform
+    // registers is then computed there. A lane 0 on its own took 240 to 560 clocks to issue four MMAs and the barriers
+    // around them, now 130 to 400, and what the issue takes lies in the chain from one tile's probabilities to the next one's
+    // scores. Measured, with the set-up below: encoder_2k 0.376 -> 0.350 ms, 64 problems of 2048 x 2048 x 128 without a
+    // mask 0.137 -> 0.127, under one 48.3 -> 43.6 us (1024 keys), prefill_4k 0.934 -> 0.911 ms.
+    if (ok) {
       constexpr uint32_t idesc_s = mma_idesc(kTileRows, kTileRows, kFp16, false, false);
       constexpr uint32_t idesc_pv = mma_idesc(kTileRows, D, kFp16, false, true);
       // S_t = Q_t K^T over the head dim, 16 elements per instruction
@@ -308,79 +328,102 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       unsigned q_uses[kQTiles] = {0u, 0u};  // items finished in which Q tile t had rows
       unsigned tiles[kQTiles] = {0u, 0u};   // key tiles Q tile t has been through, over all items
       unsigned step = 0;                    // key tiles consumed so far, over all items
+      auto wait = [&](int i, uint32_t parity, unsigned tag) { return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, prm.status, tag)); };
       for (unsigned n_item = 0; ok; ++n_item) {
         unsigned index;
-        ok = next_item(n_item, index);
+        ok = __all_sync(0xffffffffu, next_item(n_item, index));
         if (!ok) break;
-        mbar_arrive(bar(B::work_empty + (n_item & 1u)));
+        index = __shfl_sync(0xffffffffu, index, 0);
+        if (elect_one()) mbar_arrive(bar(B::work_empty + (n_item & 1u)));
+        __syncwarp();
         if (index >= prm.items) break;
         const Item item = decode(index);
+        auto at = [&](int t, int j) { return step + (kShared ? 2 * j + t : j); };  // Q tile t's j-th key tile, over all items
 #pragma unroll
         for (int t = 0; t < kQTiles; ++t)
-          if (item.n_kv[t] > 0 && ok) ok = mbar_wait(bar(B::q_full + t), q_uses[t] & 1u, prm.status, 0x0200u | t);
+          if (item.n_kv[t] > 0 && ok) ok = wait(B::q_full + t, q_uses[t] & 1u, 0x0200u | t);
         if (!ok) break;
         if (item.n_max > 0) {
-          const int stage = step % L::kStages;
-          ok = mbar_wait(bar(B::k_full + stage), (step / L::kStages) & 1, prm.status, 0x0210u);
-          if (!ok) break;
-          tc_fence_after_sync();
 #pragma unroll
           for (int t = 0; t < kQTiles; ++t)
-            if (item.n_kv[t] > 0) {
+            if (item.n_kv[t] > 0 && ok) {
+              const unsigned first = at(t, 0);
+              const int stage = first % L::kStages;
+              ok = wait(B::k_full + stage, (first / L::kStages) & 1, 0x0210u);
+              if (!ok) break;
+              tc_fence_after_sync();
               // (the S_t region is free: the MMAs run in issue order, and the last one issued for this tile was
               // the product that consumed the P_t stored there)
-              issue_s(t, stage);
-              mma_commit(bar(B::s_full + t));
-              if (item.n_kv[t] == 1) mma_commit(bar(B::q_empty + t));
+              if (elect_one()) {
+                issue_s(t, stage);
+                mma_commit(bar(B::s_full + t));
+                if (item.n_kv[t] == 1) mma_commit(bar(B::q_empty + t));
+                if (kShared) mma_commit(bar(B::k_empty + stage));
+              }
+              __syncwarp();
             }
-          mma_commit(bar(B::k_empty + stage));
+          if (!ok) break;
+          if (!kShared && elect_one()) mma_commit(bar(B::k_empty + step % L::kStages));
+          __syncwarp();
         }
-        for (int j = 0; j < item.n_max && ok; ++j, ++step) {
-          const int stage = step % L::kStages;
-          const uint32_t wrap = (step / L::kStages) & 1;
-          const int next = (step + 1) % L::kStages;
-          const uint32_t next_wrap = ((step + 1) / L::kStages) & 1;
-          ok = mbar_wait(bar(B::v_full + stage), wrap, prm.status, 0x0220u | stage);
+        for (int j = 0; j < item.n_max && ok; ++j) {
           bool issued_next = false;
 #pragma unroll
           for (int t = 0; t < kQTiles; ++t) {
             if (!ok || j >= item.n_kv[t]) continue;
+            const unsigned here = at(t, j), then = at(t, j + 1);
+            const int stage = here % L::kStages, next = then % L::kStages;
+            ok = wait(B::v_full + stage, (here / L::kStages) & 1, 0x0220u | stage);
+            if (!ok) break;
             TRACE_EVENT(100 + t);
             const uint32_t phase = tiles[t] & 1u;
             // the product starts on the first 64 keys while the softmax is still on the last 64
-            ok = mbar_wait(bar(B::p_half + t), phase, prm.status, 0x0260u | t);
+            ok = wait(B::p_half + t, phase, 0x0260u | t);
             if (!ok) break;
             // the item's first product overwrites O_t: the previous item's epilogue must have read it
-            if (j == 0) ok = mbar_wait(bar(B::o_free + t), (q_uses[t] & 1u) ^ 1u, prm.status, 0x0270u | t);
+            if (j == 0) ok = wait(B::o_free + t, (q_uses[t] & 1u) ^ 1u, 0x0270u | t);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_pv(t, stage, 0, j == 0);
-            ok = mbar_wait(bar(B::p_full + t), phase, prm.status, 0x0230u | t);
+            if (elect_one()) issue_pv(t, stage, 0, j == 0);
+            __syncwarp();
+            ok = wait(B::p_full + t, phase, 0x0230u | t);
             if (!ok) break;
             TRACE_EVENT(110 + t);
             tc_fence_after_sync();
-            issue_pv(t, stage, 1, j == 0);
+            const bool last = j + 1 >= item.n_kv[t];
+            if (elect_one()) {
+              issue_pv(t, stage, 1, j == 0);
+              if (last) mma_commit(bar(B::o_full + t));
+              if (kShared) mma_commit(bar(B::v_empty + stage));
+            }
+            __syncwarp();
             TRACE_EVENT(120 + t);
             ++tiles[t];
-            if (j + 1 < item.n_kv[t]) {
+            if (!last) {
               // the scores can only follow the product that consumed the P_t lying over them; s_full then also
               // tells the softmax that O_t is settled
-              ok = mbar_wait(bar(B::k_full + next), next_wrap, prm.status, 0x0240u | next);
+              ok = wait(B::k_full + next, (then / L::kStages) & 1, 0x0240u | next);
               if (!ok) break;
               tc_fence_after_sync();
-              issue_s(t, next);
-              mma_commit(bar(B::s_full + t));
-              if (j + 2 == item.n_kv[t]) mma_commit(bar(B::q_empty + t));
+              if (elect_one()) {
+                issue_s(t, next);
+                mma_commit(bar(B::s_full + t));
+                if (j + 2 == item.n_kv[t]) mma_commit(bar(B::q_empty + t));
+                if (kShared) mma_commit(bar(B::k_empty + next));
+              }
+              __syncwarp();
               TRACE_EVENT(130 + t);
               issued_next = true;
-            } else {
-              mma_commit(bar(B::o_full + t));
             }
           }
           if (!ok) break;
-          mma_commit(bar(B::v_empty + stage));
-          if (issued_next) mma_commit(bar(B::k_empty + next));
+          if (!kShared && elect_one()) {
+            mma_commit(bar(B::v_empty + (step + j) % L::kStages));
+            if (issued_next) mma_commit(bar(B::k_empty + (step + j + 1) % L::kStages));
+          }
+          __syncwarp();
         }
+        step += item.loads;
 #pragma unroll
         for (int t = 0; t < kQTiles; ++t)
           if (item.n_kv[t] > 0) ++q_uses[t];
@@ -402,6 +445,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     unsigned tiles = 0;   // key tiles this group has been through, over all items
     unsigned o_uses = 0;  // items this group has finished
     unsigned stores = 0;  // staging blocks this group has handed to TMA
+    unsigned merges = 0;  // shared items so far
     // Key mask: a hidden key is a score of -inf for every row. Each lane fetches four of a tile's 128 flags one tile
     // ahead of their use; a ballot per 32 keys then gives every thread all of them.
     // (the flags stay as loaded until the next tile needs them: a warp issues in order, so turning them into anything
@@ -427,7 +471,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int row = item.q0[t] + row_in_tile;
     float m = -INFINITY, l = 0.f;
     unsigned flags[4] = {1u, 1u, 1u, 1u};
-    if (kMask) fetch_flags(problem, 0, flags);
+    auto key0 = [&](int j) { return (kShared ? 2 * j + t : j) * kTileRows; };  // first key of this Q tile's j-th key tile
+    if (kMask) fetch_flags(problem, key0(0), flags);
     for (int j = 0; j < n; ++j, ++tiles) {
       // Key mask: which of the tile's 128 keys are hidden, as four ballot words in registers (each lane fetched four
       // of the flags a tile ahead). A tile none of whose keys is hidden (every tile but the last few of a padded
@@ -438,7 +483,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
         for (int c = 0; c < 4; ++c) hid[c] = __ballot_sync(0xffffffffu, (flags[c] & 0x7fffu) == 0u);
         any_hidden = ((hid[0] | hid[1]) | (hid[2] | hid[3])) != 0u;
-        if (j + 1 < n) fetch_flags(problem, (j + 1) * kTileRows, flags);
+        if (j + 1 < n) fetch_flags(problem, key0(j + 1), flags);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(bar(B::s_full + t), tiles & 1u, prm.status, 0x0300u | t));  // warp-uniform: the tensor-memory ops below are warp-wide
       if (!ok) break;
@@ -449,7 +494,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       for (int c = 0; c < 4; ++c) tmem_ld32(t_s + 32 * c, s[c]);
       tmem_ld_wait();
       TRACE_EVENT(3);
-      const int kv0 = j * kTileRows;
+      const int kv0 = key0(j);
       const bool diagonal = kCausal && kv0 + kTileRows > item.q0[t];     // some key of this tile is right of some row
       const bool ragged = kv0 + kTileRows > prm.t_k;                // some key of this tile does not exist
       if (diagonal || ragged || (kMask && any_hidden)) {
@@ -477,7 +522,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         m = mx;
       }
       TRACE_EVENT(4);
-      const float shift = (kMask && m == -INFINITY) ? 0.f : -m * sl2;
+      // (the same for half of a shared item's keys, which may all have scores of -inf)
+      const float shift = ((kMask || kShared) && m == -INFINITY) ? 0.f : -m * sl2;
       const uint64_t shift2 = f2_pack(shift, shift);
       uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
@@ -506,10 +552,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           for (int i = 0; i < 32; i += 2) {
             const uint64_t x2 = f2_fma(f2_pack_bits(s[c][i], s[c][i + 1]), sl2_2, shift2);
             float p0, p1;
-            // (not under a key mask: the cubic turns a hidden key's -inf into 2^-125 rather than 0, which a row
-            // with no visible key at all would then mistake for a denominator)
-            if (!kMask && ((i >> 1) & 7) < poly_pairs_of_8<D, kCausal>()) {
-              exp2_poly2<3>(x2, p0, p1);
+            if (((i >> 1) & 7) < poly_pairs_of_8<D, kCausal, kMask>()) {
+              exp2_poly2<D == 64 ? 5 : 3>(x2, p0, p1);
             } else {
               f2_unpack(x2, p0, p1);
               p0 = exp2_approx(p0);
@@ -540,7 +584,48 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(B::o_full + t), o_uses & 1u, prm.status, 0x0310u | t));
     if (ok) {
       tc_fence_after_sync();
+      float from_1 = 0.f;  // shared item: what Q tile 1's part of this row counts relative to this one's (already in l and O_0's factor)
+      float keep = 1.f;
+      if (kShared) {
+        // a group for Q tile 1 leaves its maximum and sum and lets the other one read O_1
+        if (t == 1) {
+          merge_m[row_in_tile] = m, merge_l[row_in_tile] = l;
+          tc_fence_before_sync();
+          mbar_arrive(bar(B::merge_full));
+          ++o_uses;
+          continue;
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(B::merge_full), merges & 1u, prm.status, 0x0340u));
+        if (!ok) break;
+        ++merges;
+        tc_fence_after_sync();
+        const float m_1 = *const_cast<volatile float*>(&merge_m[row_in_tile]), l_1 = *const_cast<volatile float*>(&merge_l[row_in_tile]);
+        const float top = fmaxf(m, m_1);
+        // (a part that has seen no visible key has m = -inf and l = 0, and counts nothing)
+        keep = m == -INFINITY ? 0.f : exp2_approx((m - top) * sl2);
+        from_1 = m_1 == -INFINITY ? 0.f : exp2_approx((m_1 - top) * sl2);
+        l = l * keep + l_1 * from_1;
+        m = top;
+      }
       const float inv = 1.f / l;
+      // 32 columns of the row, as they leave (16 bits later)
+      auto take = [&](int col, uint32_t (&o)[32]) {
+        tmem_ld32(t_o + col, o);
+        if (kShared) {
+          uint32_t o_1[32];
+          tmem_ld32(t_o + D + col, o_1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * keep + __uint_as_float(o_1[i]) * from_1);
+        } else {
+          tmem_ld_wait();
+        }
+      };
+      auto free_o = [&] {
+        tc_fence_before_sync();
+        mbar_arrive(bar(B::o_free + t));
+        if (kShared) mbar_arrive(bar(B::o_free + 1));
+      };
       const long long out_row = static_cast<long long>(problem) * prm.t_q + row;  // in L, which is always dense
       if constexpr (L::kTileStore) {
         // O goes out as tile stores: every thread leaves its row, rounded, in the group's staging block (in the
@@ -562,8 +647,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
             uint32_t o[32];
-            tmem_ld32(t_o + 64 * blk + 32 * cc, o);
-            tmem_ld_wait();
+            take(64 * blk + 32 * cc, o);
 #pragma unroll
             for (int v4 = 0; v4 < 4; ++v4) {
               uint32_t w[4];
@@ -578,8 +662,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
           if (blk == D / 64 - 1) {
             // O_t is in registers or staged: the next item's first product may overwrite it
-            tc_fence_before_sync();
-            mbar_arrive(bar(B::o_free + t));
+            free_o();
           }
           fence_async_shared();
           mbar_arrive(bar(B::stage_full + t));
@@ -596,8 +679,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
-        tmem_ld32(t_o + 32 * c, o);
-        tmem_ld_wait();
+        take(32 * c, o);
         if (row < prm.t_q) {
           uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(prm.out) + (out_at + 32 * c) * 2);
 #pragma unroll
@@ -615,8 +697,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
       if (row < prm.t_q) prm.lse[out_row] = m * prm.scale + logf(l);
       // O_t is in registers or stored: the next item's first product may overwrite it
-      tc_fence_before_sync();
-      mbar_arrive(bar(B::o_free + t));
+      free_o();
       }
       ++o_uses;
     }
@@ -628,7 +709,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // ---- teardown ----
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kMmaWarp && !abort_flag) {
+  if (warp == kMmaWarp) {
     if (*reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk) {
       // a wait gave up somewhere: give copies and MMAs still in flight time to land before the
       // tensor memory and shared memory they target are released
@@ -645,8 +726,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 }
 
-template <int D, bool kCausal, bool kFp16, bool kMask>
-int launch_fwd(const Problem& p) {
+template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared>
+int launch_fwd_s(const Problem& p) {
   using L = FwdLayout<D, kCausal, kMask>;
   CUtensorMap map_q, map_k, map_v, map_o;
   const int heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh), batch = static_cast<int>(p.bh / heads);
@@ -685,7 +766,7 @@ int launch_fwd(const Problem& p) {
   if (int rc = sm_count(&sms)) return rc;
   prm.group = work_group(p, items, sms);
   const long long ctas = items < sms ? items : sms;  // one CTA per SM (shared and tensor memory allow no more), each fetching items until none is left
-  auto kernel = sdpa_fwd_kernel<D, kCausal, kFp16, kMask>;
+  auto kernel = sdpa_fwd_kernel<D, kCausal, kFp16, kMask, kShared>;
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64] = {};
   int device = 0;
@@ -695,10 +776,24 @@ int launch_fwd(const Problem& p) {
               "sizing shared memory for the sdpa kernel");
     sized[device] = true;
   }
-  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(fwd_threads<D, kCausal, kMask>()), L::kBytes, p.stream, map_q, map_k, map_v, map_o, prm),
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(fwd_threads<kMask>()), L::kBytes, p.stream, map_q, map_k, map_v, map_o, prm),
             "launching the sdpa kernel");
   note_launches(1);
   return LIMN_B200_OK;
+}
+
+// A problem with one Q tile: its tile goes into both places, the even key tiles to the first and the odd ones to the second,
+// whose softmax group would be idle otherwise, and the epilogue puts the two parts of every row together. That halves the
+// chain of key tiles, which is all there is to such an item. Measured: 64 problems of 100 x 1500 keys x 64 21.7 -> 14.3 us (18.8
+// without), 8 of 128 x 4096 x 128 52.5 -> 30.4, 192 of 100 x 700 x 64 under a mask 27.8 -> 19.2. The line lies where it does not
+// depend on how many problems there are: a row's bits must not. (The last, single tile of an odd number of them was tried
+// too: a gain of 3 % at head dim 64, a loss of up to 24 % at 128, where the kernel then spills.)
+template <int D, bool kCausal, bool kFp16, bool kMask>
+int launch_fwd(const Problem& p) {
+  if constexpr (!kCausal) {  // (a causal problem of one Q tile has one key tile)
+    if (p.t_q <= kTileRows && p.t_k > kTileRows) return launch_fwd_s<D, kCausal, kFp16, kMask, true>(p);
+  }
+  return launch_fwd_s<D, kCausal, kFp16, kMask, false>(p);
 }
 
 template <int D, bool kMask>

@@ -1,0 +1,101 @@
+"""The 16-bit forward for problems of at most 128 query rows, whose key tiles both softmax groups share (even ones to the first,
+odd ones to the second), and scores that are infinite or NaN on either of the two ways exp2 is taken."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import BF16, parity
+from oracle import sdpa_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    import limn_standin as host
+
+    return host.Device()
+
+
+def _check(dev, q, k, v, do, mask=None):
+    """Forward and backward against the oracle, at the tolerances of the other kernel tests."""
+    import limn_standin as host
+
+    half = q.dtype == np.dtype(np.float16)
+    scale = q.shape[-1] ** -0.5
+    att = host.Attention(dev, q, k, v, causal=False, key_mask=mask)
+    out, lse = att.forward()
+    want_out, want_lse = oracle.sdpa_forward(q, k, v, mask, causal=False, scale=scale)
+    parity(out, want_out, 2e-3 if half else 2e-2, "O")
+    parity(lse, want_lse, 1e-3, "L")
+    dq, dk, dv = att.backward(do)
+    delta = oracle.row_delta(do, want_out)
+    want = (oracle.sdpa_backward_q(q, k, v, do, want_lse, delta, mask, causal=False, scale=scale),
+            *oracle.sdpa_backward_kv(q, k, v, do, want_lse, delta, mask, causal=False, scale=scale))
+    for got, ref, what in zip((dq, dk, dv), want, ("dQ", "dK", "dV")):
+        parity(got, ref, 4e-3 if half else 2e-2, what)
+
+
+def _problem(seed, bh, t_q, t_k, hd, dtype=BF16):
+    rng = np.random.default_rng(seed)
+    return [rng.standard_normal((bh, t, hd)).astype(np.float32).astype(dtype) for t in (t_q, t_k, t_k, t_q)]
+
+
+# bh, t_q, t_k, hd: two key tiles (the second of a single key), three, an even number, more problems than SMs, t_q at and beside 128
+SHARED = [(2, 5, 129, 64), (3, 100, 300, 64), (2, 128, 512, 128), (2, 127, 257, 96), (200, 6, 260, 64), (3, 129, 300, 64), (2, 64, 128, 64), (160, 33, 385, 32)]
+
+
+@pytest.mark.parametrize("case", SHARED, ids=[f"{c[0]} x {c[1]}x{c[2]} hd {c[3]}" for c in SHARED])
+@pytest.mark.parametrize("dtype", [BF16, np.float16], ids=["bf16", "f16"])
+def test_problems_of_one_query_tile(case, dtype, dev):
+    _check(dev, *_problem(sum(case), *case, dtype))
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("hidden", ["even tiles", "odd tiles", "all but one key"])
+def test_a_group_whose_keys_are_all_hidden(hd, hidden, dev):
+    t_k = 640
+    q, k, v, do = _problem(hd, 2, 40, t_k, hd)
+    tile = np.arange(t_k) // 128
+    keep = {"even tiles": tile % 2 == 1, "odd tiles": tile % 2 == 0, "all but one key": np.arange(t_k) == 300}[hidden]
+    mask = np.broadcast_to(keep, (2, t_k)).astype(np.float32).astype(BF16)
+    _check(dev, q, k, v, do, mask)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("first", [0, 128], ids=["first tile", "second tile"])
+def test_a_group_whose_scores_are_all_minus_infinity(hd, first, dev):
+    """One part of every row counts nothing; with a single tile per group nothing else would bring its maximum up."""
+    import limn_standin as host
+
+    q, k, v, _ = _problem(hd + first, 2, 40, 256, hd)
+    q = np.abs(q.astype(np.float32)).astype(BF16)
+    k[:, first : first + 128] = -np.inf
+    if first == 0:  # (without the sharing a first tile of such keys is NaN, as it always was)
+        assert q.shape[1] <= 128
+    out, lse = host.Attention(dev, q, k, v, causal=False).forward()
+    want_out, want_lse = oracle.sdpa_forward(q, k, v, causal=False, scale=hd**-0.5)
+    parity(out, want_out, 2e-2, "O")
+    parity(lse, want_lse, 1e-3, "L")
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("t_q", [40, 200])
+@pytest.mark.parametrize("masked", [False, True], ids=["", "masked"])
+def test_a_nan_key_makes_every_row_nan(hd, t_q, masked, dev):
+    """Whichever of a tile's columns it falls on: some take exp2 as a polynomial, the others on the special-function unit."""
+    import limn_standin as host
+
+    t_k = 300
+    q, k, v, do = _problem(hd + t_q, 16, t_q, t_k, hd)
+    for p in range(16):
+        k[p, 17 * p] = np.nan  # the 16 residues of a column index mod 16, over all three tiles
+    mask = np.ones((16, t_k), np.float32).astype(BF16) if masked else None
+    att = host.Attention(dev, q, k, v, causal=False, key_mask=mask)
+    out, lse = att.forward()
+    assert np.isnan(out.astype(np.float32)).all()
+    assert np.isnan(lse.astype(np.float32)).all()
+    dq, _, _ = att.backward(do)
+    assert np.isnan(dq.astype(np.float32)).all()
