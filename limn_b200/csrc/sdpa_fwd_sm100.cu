@@ -10,6 +10,7 @@
 //   P_t = exp2(S_t - m_t)    128 softmax threads per Q tile, one row each; P_t overwrites S_t as 16-bit
 //   O_t += P_t V_j           tcgen05.mma, A = P_t from tensor memory, B = V_j (MN-major) from shared memory
 // Two Q tiles per item keep the tensor pipe busy on one while the other is in its softmax.
+// (A problem with a single Q tile puts it in both places and deals its key tiles out between them: launch_fwd below.)
 // Each output row has exactly one owner and is accumulated in a fixed key order, so two
 // runs give the same bits, as the kernel this replaces promises (limn/cuda_emit.py:748-752).
 //
