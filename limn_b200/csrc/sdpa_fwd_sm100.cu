@@ -41,11 +41,12 @@ constexpr int kTileRows = 128;   // query rows per Q tile, keys per K/V tile
 constexpr int kQTiles = 2;       // Q tiles per CTA
 // Ten warps work, but the block size decides how the compiler allocates registers in the softmax loop (all sizes
 // end at 168 registers; what differs is what is spilled where). Measured on B200 with the elected issue: head dim 128 under a
-// causal mask 10 warps, 5 % over 11 and 12 (prefill_4k 0.912, 0.964 and 0.957 ms); the key-mask kernels stay at the 12 they were
-// tuned with. The spare warps go straight to the final barrier.
-template <bool kMask>
+// causal mask 10 warps, 5 % over 11 and 12 (prefill_4k 0.912, 0.964 and 0.957 ms), without one 10 by 1 and 6 %; head dim 64 10 by 2
+// to 5 %; under a key mask at head dim 64 11 (192 padded problems of 500 33.5 us, 34.6 with 12; causal on top 25.3, 25.6), at 128 no
+// difference. The spare warps go straight to the final barrier.
+template <int D, bool kMask>
 constexpr int fwd_threads() {
-  return kMask ? 384 : 320;
+  return kMask ? (D == 64 ? 352 : 384) : 320;
 }
 constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
@@ -73,7 +74,7 @@ struct FwdLayout {
   static constexpr int kTileBytes = kTileRows * D * 2;
   static constexpr int kAtomBytes = kTileRows * 128;        // one 64-element-wide column block of a tile
   // K and V rings, each this deep. Shared memory would hold more at head dim 64, but deeper rings are slower there
-  // (measured 3: +1.5 %, 5: +4 %): two tiles in flight cover the load latency, more only put TMA's writes in the MMAs' way.
+  // (measured 5: +4 %; 3: +1.5 % once, no difference with the elected issue): two tiles in flight cover the load latency.
   static constexpr int kStages = 2;
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + kQTiles * kTileBytes;
@@ -145,7 +146,7 @@ struct FwdParams {
 };
 
 template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared>
-__global__ void __launch_bounds__((fwd_threads<kMask>()), 1)
+__global__ void __launch_bounds__((fwd_threads<D, kMask>()), 1)
 sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const FwdParams prm) {
   using L = FwdLayout<D, kCausal, kMask>;
@@ -225,8 +226,8 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  if (warp == kProducerWarp) named_barrier_arrive(1, fwd_threads<kMask>());
-  else named_barrier_sync(1, fwd_threads<kMask>());
+  if (warp == kProducerWarp) named_barrier_arrive(1, fwd_threads<D, kMask>());
+  else named_barrier_sync(1, fwd_threads<D, kMask>());
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
@@ -777,7 +778,7 @@ int launch_fwd_s(const Problem& p) {
               "sizing shared memory for the sdpa kernel");
     sized[device] = true;
   }
-  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(fwd_threads<kMask>()), L::kBytes, p.stream, map_q, map_k, map_v, map_o, prm),
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(fwd_threads<D, kMask>()), L::kBytes, p.stream, map_q, map_k, map_v, map_o, prm),
             "launching the sdpa kernel");
   note_launches(1);
   return LIMN_B200_OK;
