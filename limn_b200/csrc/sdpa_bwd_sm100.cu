@@ -58,10 +58,11 @@ constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
-// dQ pass at head dim 64: of every 8 pairs of scores, how many take exp2 as a polynomial (of degree 4: 3e-6, the probability is
-// rounded to 16 bits at once) on the FMA pipe instead of on the special-function unit. Measured with the elected issue, one /
-// two / three of 8 over none: encoder_2k 0.955 / 0.945 / 0.97, 64 problems of 100 x 1500 0.95 / 0.93 / 0.96. Not at head dim 128 (1.02 to
-// 1.04), nor in the dK/dV pass, which spills (1.7).
+// dQ pass at head dim 64: of every 8 pairs of scores, how many take exp2 as a polynomial on the FMA pipe instead of on the
+// special-function unit. Of degree 5, as accurate as ex2.approx: degree 4 (3e-6) takes the same time. Measured with the elected
+// issue, two of 8 over none: encoder_2k 0.95, 64 problems of 100 x 1500 0.95, 32 of 777 0.96, 32 causal of 2048 0.97, 256 causal of
+// 256 1.01; one or three of 8 0.01 to 0.03 worse at the first two. Not at head dim 128 (1.02 to 1.04), nor in the dK/dV pass, which
+// spills (1.7).
 #ifndef LIMN_BWD_POLY_PAIRS
 #define LIMN_BWD_POLY_PAIRS 2
 #endif
@@ -859,7 +860,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const uint64_t x2 = f2_fma(f2_pack_bits(s[c][e], s[c][e + 1]), sl2_2, neg_l2);
             float p0, p1;
             if (!kKV && D == 64 && ((e >> 1) & 7) < kPolyPairsOf8) {
-              exp2_poly2<4>(x2, p0, p1);  // on the FMA pipe, beside the special-function unit
+              exp2_poly2<5>(x2, p0, p1);  // on the FMA pipe, beside the special-function unit
             } else {
               f2_unpack(x2, p0, p1);
               p0 = exp2_approx(p0), p1 = exp2_approx(p1);

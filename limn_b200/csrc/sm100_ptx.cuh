@@ -382,15 +382,15 @@ __device__ __forceinline__ float max_nan(float a, float b) {  // a NaN if either
 // 2^x for two values on the FMA pipe instead of the special-function unit: round x to the
 // nearest integer n with the 1.5 * 2^23 trick, evaluate a polynomial for 2^(x - n) on [-0.5, 0.5], and multiply by 2^n. The
 // polynomials are relative minimax fits; largest and root-mean-square relative error as evaluated in float32: degree 3
-// 7.5e-5 and 5.2e-5, degree 4 2.9e-6 and 1.8e-6, degree 5 1.7e-7 and 7e-8 (what ex2.approx has). x is clamped at -127, where
+// 7.5e-5 and 5.2e-5, degree 5 1.7e-7 and 7e-8 (what ex2.approx has). x is clamped at -127, where
 // 2^n comes out as 0: a score of -inf gives exactly 0 and what lies below the normal range is 0 or close to it, as with
 // ex2.approx.ftz. A NaN stays one.
 template <int kDegree>
 __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& lo, float& hi) {
-  static_assert(kDegree >= 3 && kDegree <= 5, "the fits there are");
-  constexpr float c[3][6] = {{9.9992805719e-01f, 6.9326096773e-01f, 2.4261112511e-01f, 5.5171668530e-02f, 0.f, 0.f},
-                             {1.0000000000e+00f, 6.9312417507e-01f, 2.4024099112e-01f, 5.5906426162e-02f, 9.5828529447e-03f, 0.f},
-                             {1.0000000000e+00f, 6.9314700365e-01f, 2.4022242427e-01f, 5.5507335812e-02f, 9.6715129912e-03f, 1.3264727313e-03f}};
+  static_assert(kDegree == 3 || kDegree == 5, "the fits there are");
+  constexpr float c[6] = {kDegree == 3 ? 9.9992805719e-01f : 1.0000000000e+00f, kDegree == 3 ? 6.9326096773e-01f : 6.9314700365e-01f,
+                          kDegree == 3 ? 2.4261112511e-01f : 2.4022242427e-01f, kDegree == 3 ? 5.5171668530e-02f : 5.5507335812e-02f,
+                          9.6715129912e-03f, 1.3264727313e-03f};
   float x0, x1;
   f2_unpack(x2, x0, x1);
   x2 = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
@@ -398,9 +398,9 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& lo, float& hi) {
   const uint64_t t2 = f2_add(x2, magic);
   const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
   const uint64_t r2 = f2_fma(n2, f2_pack(-1.f, -1.f), x2);
-  uint64_t p2 = f2_pack(c[kDegree - 3][kDegree], c[kDegree - 3][kDegree]);
+  uint64_t p2 = f2_pack(c[kDegree], c[kDegree]);
 #pragma unroll
-  for (int i = kDegree - 1; i >= 0; --i) p2 = f2_fma(p2, r2, f2_pack(c[kDegree - 3][i], c[kDegree - 3][i]));
+  for (int i = kDegree - 1; i >= 0; --i) p2 = f2_fma(p2, r2, f2_pack(c[i], c[i]));
   float t0, t1;
   f2_unpack(t2, t0, t1);
   const uint32_t one = 0x3f800000u;
