@@ -374,17 +374,26 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-__device__ __forceinline__ float max_nan(float a, float b) {  // a NaN if either is
+__device__ __forceinline__ uint64_t f2_mul_ftz(uint64_t a, uint64_t b) {  // a product below the normal range is 0
+  uint64_t r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// x held to [-bound, bound] (bound > 0) in one instruction; a NaN stays one
+__device__ __forceinline__ float held_within(float x, float bound) {
   float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(bound));
   return r;
 }
 // 2^x for two values on the FMA pipe instead of the special-function unit: round x to the
 // nearest integer n with the 1.5 * 2^23 trick, evaluate a polynomial for 2^(x - n) on [-0.5, 0.5], and multiply by 2^n. The
 // polynomials are relative minimax fits; largest and root-mean-square relative error as evaluated in float32: degree 3
-// 7.5e-5 and 5.2e-5, degree 5 1.7e-7 and 7e-8 (what ex2.approx has). x is clamped at -127, where
-// 2^n comes out as 0: a score of -inf gives exactly 0 and what lies below the normal range is 0 or close to it, as with
-// ex2.approx.ftz. A NaN stays one.
+// 7.5e-5 and 5.2e-5, degree 5 1.7e-7 and 7e-8 (what ex2.approx has). x is held to
+// [-127, 127], for any x to come out as it does from ex2.approx.ftz: the polynomial gives 2^(x - n - 1) and the factor is 2^(n + 1),
+// whose exponent field is 255, infinity, at n = 127, and 1 at n = -127, where the product lies below the normal range and is
+// flushed to 0. So -inf and what lies below 2^-126 give exactly 0, 126.5 and more give +inf (ex2.approx from 128 on), a
+// NaN stays one. (Without the upper bound the exponent field wraps from 128.5 on, which a caller's L can reach in the dQ pass.
+// A maximum and a minimum instead of held_within: 1 to 4 % on the kernels that use this.)
 template <int kDegree>
 __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& lo, float& hi) {
   static_assert(kDegree == 3 || kDegree == 5, "the fits there are");
@@ -393,18 +402,18 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& lo, float& hi) {
                           9.6715129912e-03f, 1.3264727313e-03f};
   float x0, x1;
   f2_unpack(x2, x0, x1);
-  x2 = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
+  x2 = f2_pack(held_within(x0, 127.f), held_within(x1, 127.f));
   const uint64_t magic = f2_pack(12582912.f, 12582912.f);
   const uint64_t t2 = f2_add(x2, magic);
   const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
   const uint64_t r2 = f2_fma(n2, f2_pack(-1.f, -1.f), x2);
-  uint64_t p2 = f2_pack(c[kDegree], c[kDegree]);
+  uint64_t p2 = f2_pack(0.5f * c[kDegree], 0.5f * c[kDegree]);
 #pragma unroll
-  for (int i = kDegree - 1; i >= 0; --i) p2 = f2_fma(p2, r2, f2_pack(c[i], c[i]));
+  for (int i = kDegree - 1; i >= 0; --i) p2 = f2_fma(p2, r2, f2_pack(0.5f * c[i], 0.5f * c[i]));
   float t0, t1;
   f2_unpack(t2, t0, t1);
-  const uint32_t one = 0x3f800000u;
-  f2_unpack(f2_mul(p2, f2_pack_bits((__float_as_uint(t0) << 23) + one, (__float_as_uint(t1) << 23) + one)), lo, hi);
+  const uint32_t two = 0x40000000u;
+  f2_unpack(f2_mul_ftz(p2, f2_pack_bits((__float_as_uint(t0) << 23) + two, (__float_as_uint(t1) << 23) + two)), lo, hi);
 }
 
 // Which (problem, slot) work item `index` is. Items are fetched in index order, so the order is the schedule:

@@ -1,5 +1,5 @@
 """The probabilities of the 16-bit dQ pass, some of which take exp2 as a polynomial and the others on the special-function unit:
-as accurate as each other. What the pass computes is dS = P (dP - delta); with one
+as accurate as each other, and infinite where the row's L makes them so. What the pass computes is dS = P (dP - delta); with one
 key whose dP is 1, delta 0 and K a unit vector, a row's dQ is that key's P rounded to 16 bits."""
 
 from __future__ import annotations
@@ -66,3 +66,50 @@ def test_probabilities_are_as_good_as_float32_exp2(width, dtype):
     wrong = (got != want) & sure
     assert not wrong.any(), f"{wrong.sum()} of {16 * sure.sum()}: P is off by up to {np.abs(np.broadcast_to(off, got.shape)[wrong]).max():.1e}"
     assert (np.abs(got - middle * 0.125) <= step * 0.0626).all()  # (the unsure ones are one of the two values)
+
+
+@HALVES
+@WIDTHS
+def test_a_probability_beyond_float32_is_not_finite(width, dtype):
+    """An L far below the row's scores, which cannot be this row's: exp2 of 128.4 and more. The gradient must show it."""
+    c = np.array([89, 89.5, 90, 92, 96, 104, 128, 136, 160, 176, 200, 256, 264, 354, 512, 1024, 5000, 8000], np.float64)
+    assert c[0] * 8 * 0.125 * np.log2(np.e) > 128
+    q, k, v, do = _one_key_each(width, dtype, c.size)
+    q[:, :, 1] = c.astype(dtype)
+    k[:, :, 1] = -8
+    for p, key in enumerate(KEYS):
+        k[p, key, 1] = 8  # (the other keys' P is 0)
+    got = _dq(q, k, v, do, np.zeros((16, c.size), np.float32))
+    assert not np.isfinite(got).any()
+
+
+@HALVES
+@WIDTHS
+def test_a_probability_below_float32_is_zero(width, dtype):
+    """Down to 2^-126 a P is a number, below it nothing: not a subnormal one, whatever it is multiplied by."""
+    c = np.array([0, 1, 80, 89, 89.5, 90, 96, 128, 200, 256, 354, 1024, 8000], np.float64)
+    q, k, v, do = _one_key_each(width, dtype, c.size)
+    q[:, :, 1] = c.astype(dtype)
+    k[:, :, 1] = -8  # x from 0 to -1.4 c
+    for p, key in enumerate(KEYS):
+        do[p, :, 0] = 2.0**14  # dP as large as float16 has it
+    got = _dq(q, k, v, do, np.zeros((16, c.size), np.float32))
+    q64 = q[0, :, 1].astype(np.float64)
+    p64 = np.exp(-q64)
+    gone = q64 * np.log2(np.e) > 126.5
+    assert gone.sum() >= 6
+    assert (got[:, gone] == 0).all()
+    kept = q64 * np.log2(np.e) < 10
+    assert np.allclose(got[:, kept, 0], (p64 * 2.0**14 * 0.125)[kept], rtol=2**-8)
+
+
+@HALVES
+@WIDTHS
+def test_a_nan_score_or_l_makes_the_row_nan(width, dtype):
+    q, k, v, do = _one_key_each(width, dtype, 4)
+    lse = np.zeros((16, 4), np.float32)
+    lse[:, 1] = np.nan
+    q[:, 2, 2] = np.nan
+    got = _dq(q, k, v, do, lse)
+    assert np.isnan(got[:, 1]).all() and np.isnan(got[:, 2]).all()
+    assert np.isfinite(got[:, [0, 3]]).all()
