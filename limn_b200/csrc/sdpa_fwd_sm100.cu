@@ -514,18 +514,17 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
         for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      // Without a key mask the first tile always has a visible key (key 0), so mx is finite from the start.
-      // With one, a row may have met no visible key yet: then mx and m are both -inf, nothing moves, and the
-      // exponentials are measured against 0 so that they come out exp2(-inf) = 0 instead of NaN.
-      const bool moves = (mx - m) * sl2 > kRescaleSlack;  // true at the first visible key, where m is -inf
+      // A row may have met nothing but scores of -inf yet, be it that its keys are hidden or that the operands make them so:
+      // then mx and m are both -inf, nothing moves, and the exponentials are measured against 0 so that they come out
+      // exp2(-inf) = 0 instead of NaN.
+      const bool moves = (mx - m) * sl2 > kRescaleSlack;  // true at the first score above -inf, where m is -inf
       float alpha = 1.f;
       if (moves) {
         alpha = exp2_approx((m - mx) * sl2);
         m = mx;
       }
       TRACE_EVENT(4);
-      // (the same for half of a shared item's keys, which may all have scores of -inf)
-      const float shift = ((kMask || kShared) && m == -INFINITY) ? 0.f : -m * sl2;
+      const float shift = m == -INFINITY ? 0.f : -m * sl2;
       const uint64_t shift2 = f2_pack(shift, shift);
       uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll

@@ -64,19 +64,27 @@ def test_a_group_whose_keys_are_all_hidden(hd, hidden, dev):
     _check(dev, q, k, v, do, mask)
 
 
+# t_q, t_k, causal: both parts of a shared problem; a tile and a row more than sharing takes; two Q tiles; three key tiles; causal
+# rows that see the first tile whole, in part and as all there is
+ROWS = [(40, 256, False), (128, 256, False), (129, 256, False), (200, 384, False), (300, 300, True)]
+
+
+@pytest.mark.parametrize("masked", [False, True], ids=["", "masked"])
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("first", [0, 128], ids=["first tile", "second tile"])
-def test_a_group_whose_scores_are_all_minus_infinity(hd, first, dev):
-    """One part of every row counts nothing; with a single tile per group nothing else would bring its maximum up."""
+@pytest.mark.parametrize("rows", ROWS, ids=[f"{r[0]}x{r[1]}{' causal' if r[2] else ''}" for r in ROWS])
+def test_a_tile_whose_scores_are_all_minus_infinity(rows, first, hd, masked, dev):
+    """It counts nothing, whether it is the first a row meets, one of two parts of the row, or all the row has."""
     import limn_standin as host
 
-    q, k, v, _ = _problem(hd + first, 2, 40, 256, hd)
+    t_q, t_k, causal = rows
+    q, k, v, _ = _problem(hd + first, 2, t_q, t_k, hd)
     q = np.abs(q.astype(np.float32)).astype(BF16)
     k[:, first : first + 128] = -np.inf
-    if first == 0:  # (without the sharing a first tile of such keys is NaN, as it always was)
-        assert q.shape[1] <= 128
-    out, lse = host.Attention(dev, q, k, v, causal=False).forward()
-    want_out, want_lse = oracle.sdpa_forward(q, k, v, causal=False, scale=hd**-0.5)
+    mask = np.ones((2, t_k), np.float32).astype(BF16) if masked else None
+    out, lse = host.Attention(dev, q, k, v, causal=causal, key_mask=mask).forward()
+    want_out, want_lse = oracle.sdpa_forward(q, k, v, mask, causal=causal, scale=hd**-0.5)
+    assert np.isfinite(want_lse[:, 128 if first == 0 and causal else 0 :]).all()
     parity(out, want_out, 2e-2, "O")
     parity(lse, want_lse, 1e-3, "L")
 
