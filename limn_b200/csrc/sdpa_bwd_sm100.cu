@@ -311,15 +311,19 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   grid_launch_dependents();
   // What is left of the set-up runs side by side: the status word is read, tensor memory allocated (a block that stands
   // down frees it again), and the producer, which initialised the barriers itself, does not wait for either: its first loads are
-  // on their way. (Once the status word is found set its waits return, and its loads are given time to land at the end.)
+  // on their way.
+  // Whether the block stands down, because an earlier kernel on this device gave up, is decided by thread 0's one reading of
+  // the word and holds for all of the block, also when the host clears the word meanwhile: no item is computed, nothing is stored
+  // or drawn from the work counter, and the producer's first loads are given time to land at the end.
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk;
+  if (warp == 0) named_barrier_arrive(kDecided, 64);
   if (warp == kMmaWarp) {
     tmem_alloc(smem_addr(&tmem_slot), kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  if (warp == kProducerWarp) named_barrier_arrive(1, bwd_threads<D, kCausal, kKV, kMask>());
-  else named_barrier_sync(1, bwd_threads<D, kCausal, kKV, kMask>());
+  if (warp == kProducerWarp) named_barrier_arrive(kSetUp, bwd_threads<D, kCausal, kKV, kMask>());
+  else named_barrier_sync(kSetUp, bwd_threads<D, kCausal, kKV, kMask>());
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
@@ -339,7 +343,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   auto a_wrap = [&](int it) { return static_cast<uint32_t>((it / L::kStagesA) & 1); };
   auto b_wrap = [&](int it) { return static_cast<uint32_t>((it / L::kStagesB) & 1); };
 
-  bool ok = warp == kProducerWarp || !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
+  bool ok = warp == kProducerWarp || !abort_flag;  // (the producer asks once its first loads are out)
 #ifdef LIMN_TRACE
   int trace_n = 0;
 #endif
@@ -368,49 +372,77 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   if (warp == kProducerWarp) {
     // ================= TMA producer, work fetcher =================
-    if (lane == 0 && ok) {
-      int done = 0;
-      for (unsigned n_item = 0; ok; ++n_item) {
-        const unsigned ring = n_item & 1u;
-        ok = mbar_wait(bar(B::work_empty + ring), ((n_item >> 1) & 1u) ^ 1u, prm.status, 0x1120u | ring);
-        if (!ok) break;
-        // a CTA's first item is its own number (no round trip to the counter on the way to the first load); the
-        // counter hands out what lies beyond the grid
-        const unsigned index = n_item == 0 ? blockIdx.x : gridDim.x + atomicAdd(prm.schedule, 1u);
-        Item item = {0, 0, 0, 0, 0, 0};
-        if (index < prm.items) item = decode(index);
-        if constexpr (kKV) {
-          volatile int* f = work_items[ring];
-          f[0] = item.problem, f[1] = item.head, f[2] = item.batch, f[3] = item.own0, f[4] = item.first, f[5] = item.count;
-        }
-        *reinterpret_cast<volatile unsigned*>(&work_ring[ring]) = index;
-        mbar_arrive(bar(B::work_full + ring));
-        if (index >= prm.items) break;
-        ok = mbar_wait(bar(B::held_empty), (n_item & 1u) ^ 1u, prm.status, 0x1130u);
-        if (!ok) break;
-        mbar_expect_tx(bar(B::held_full), 2 * L::kTileBytes);
+    auto publish = [&](unsigned n_item, unsigned index, const Item& item) {
+      const unsigned ring = n_item & 1u;
+      if constexpr (kKV) {
+        volatile int* f = work_items[ring];
+        f[0] = item.problem, f[1] = item.head, f[2] = item.batch, f[3] = item.own0, f[4] = item.first, f[5] = item.count;
+      }
+      *reinterpret_cast<volatile unsigned*>(&work_ring[ring]) = index;
+      mbar_arrive(bar(B::work_full + ring));
+    };
+    auto load_held = [&](const Item& item) {
+      mbar_expect_tx(bar(B::held_full), 2 * L::kTileBytes);
 #pragma unroll
-        for (int a = 0; a < D / 64; ++a) {
-          tma_load_4d(held_a_smem + a * L::kAtomBytes, held_a, bar(B::held_full), a * 64, item.own0, item.head, item.batch);
-          tma_load_4d(held_b_smem + a * L::kAtomBytes, held_b, bar(B::held_full), a * 64, item.own0, item.head, item.batch);
-        }
-        for (int it = 0; it < item.count; ++it) {
+      for (int a = 0; a < D / 64; ++a) {
+        tma_load_4d(held_a_smem + a * L::kAtomBytes, held_a, bar(B::held_full), a * 64, item.own0, item.head, item.batch);
+        tma_load_4d(held_b_smem + a * L::kAtomBytes, held_b, bar(B::held_full), a * 64, item.own0, item.head, item.batch);
+      }
+    };
+    // the item's `it`-th streamed tile, the g-th over all items
+    auto load_a = [&](const Item& item, int it, int g) {
+      mbar_expect_tx(a_full(g), L::kTileBytes);
+#pragma unroll
+      for (int a = 0; a < D / 64; ++a)
+        tma_load_4d(stream_a_smem(g) + a * L::kAtomBytes, stream_a, a_full(g), a * 64, (item.first + it) * kTile, item.head, item.batch);
+    };
+    auto load_b = [&](const Item& item, int it, int g) {
+      mbar_expect_tx(b_full(g), L::kTileBytes);
+#pragma unroll
+      for (int a = 0; a < D / 64; ++a)
+        tma_load_4d(stream_b_smem(g) + a * L::kAtomBytes, stream_b, b_full(g), a * 64, (item.first + it) * kTile, item.head, item.batch);
+    };
+    // a CTA's first item is its own number (no round trip to the counter on the way to the first load); the counter hands out
+    // what lies beyond the grid
+    Item item = {0, 0, 0, 0, 0, 0};
+    if (kKV) item = decode(blockIdx.x);
+    if (lane == 0) publish(0u, blockIdx.x, item);
+    if (!kKV) item = decode(blockIdx.x);
+    int done = 0, it = 0;
+    if (lane == 0) {
+      load_held(item);
+      // (as many as have room: with one of them ahead of the decision the dQ pass of 256 causal problems of 256 x 64 took 19.2 us, 18.5 so)
+      for (; it < min(item.count, min(L::kStagesA, L::kStagesB)); ++it) {
+        load_a(item, it, it);
+        load_b(item, it, it);
+      }
+    }
+    __syncwarp();
+    named_barrier_sync(kDecided, 64);
+    if (lane == 0 && !abort_flag) {
+      for (unsigned n_item = 1;; ++n_item) {
+        for (; it < item.count && ok; ++it) {
           const int g = done + it;
-          const int row0 = (item.first + it) * kTile;
           ok = mbar_wait(a_empty(g), a_wrap(g) ^ 1u, prm.status, 0x1100u);
           if (!ok) break;
-          mbar_expect_tx(a_full(g), L::kTileBytes);
-#pragma unroll
-          for (int a = 0; a < D / 64; ++a)
-            tma_load_4d(stream_a_smem(g) + a * L::kAtomBytes, stream_a, a_full(g), a * 64, row0, item.head, item.batch);
+          load_a(item, it, g);
           ok = mbar_wait(b_empty(g), b_wrap(g) ^ 1u, prm.status, 0x1110u);
           if (!ok) break;
-          mbar_expect_tx(b_full(g), L::kTileBytes);
-#pragma unroll
-          for (int a = 0; a < D / 64; ++a)
-            tma_load_4d(stream_b_smem(g) + a * L::kAtomBytes, stream_b, b_full(g), a * 64, row0, item.head, item.batch);
+          load_b(item, it, g);
         }
         done += item.count;
+        const unsigned ring = n_item & 1u;
+        if (ok) ok = mbar_wait(bar(B::work_empty + ring), ((n_item >> 1) & 1u) ^ 1u, prm.status, 0x1120u | ring);
+        if (!ok) break;
+        const unsigned index = gridDim.x + atomicAdd(prm.schedule, 1u);
+        if (kKV && index < prm.items) item = decode(index);
+        publish(n_item, index, item);
+        if (index >= prm.items) break;
+        if (!kKV) item = decode(index);
+        ok = mbar_wait(bar(B::held_empty), (n_item & 1u) ^ 1u, prm.status, 0x1130u);
+        if (!ok) break;
+        load_held(item);
+        it = 0;
       }
     }
   } else if (warp == kMmaWarp) {
@@ -1012,7 +1044,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kMmaWarp) {
-    if (*reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk) {
+    if (abort_flag || *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk) {
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // let copies and MMAs still in flight land
     }
     tc_fence_after_sync();

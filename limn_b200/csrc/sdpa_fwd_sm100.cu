@@ -218,20 +218,23 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   grid_launch_dependents();
   // What is left of the set-up runs side by side: the status word is read, tensor memory allocated (a block that stands
   // down frees it again), and the producer, which initialised the barriers itself, does not wait for either: its first loads are
-  // on their way. (Once the status word is found set its waits return, and its loads are given time to land at the end.) A
-  // kernel of one tile: 6.0 -> 5.5 us.
+  // on their way. A kernel of one tile: 6.0 -> 5.5 us.
+  // Whether the block stands down, because an earlier kernel on this device gave up, is decided by thread 0's one reading of
+  // the word and holds for all of the block, also when the host clears the word meanwhile: no item is computed, nothing is stored
+  // or drawn from the work counter, and the producer's first loads are given time to land at the end.
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk;
-  if (warp == kMmaWarp) {  // (beside the read of the status word: a block that stands down frees it again)
+  if (warp == 0) named_barrier_arrive(kDecided, 64);
+  if (warp == kMmaWarp) {
     tmem_alloc(smem_addr(&tmem_slot), kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  if (warp == kProducerWarp) named_barrier_arrive(1, fwd_threads<D, kMask>());
-  else named_barrier_sync(1, fwd_threads<D, kMask>());
+  if (warp == kProducerWarp) named_barrier_arrive(kSetUp, fwd_threads<D, kMask>());
+  else named_barrier_sync(kSetUp, fwd_threads<D, kMask>());
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
-  bool ok = warp == kProducerWarp || !abort_flag;  // an earlier kernel on this device gave up: take no work, only leave the counters as found
+  bool ok = warp == kProducerWarp || !abort_flag;  // (the producer asks once its first loads are out)
 #ifdef LIMN_TRACE
   int trace_n = 0;
 #endif
@@ -249,50 +252,73 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   if (warp == kProducerWarp) {
     // ================= TMA producer, work fetcher =================
-    if (lane == 0 && ok) {
-      unsigned q_uses[kQTiles] = {0u, 0u};  // items so far in which Q tile t had rows
-      unsigned step = 0;                    // key tiles loaded so far, over all items
-      for (unsigned n_item = 0; ok; ++n_item) {
-        const unsigned slot = n_item & 1u;
-        ok = mbar_wait(bar(B::work_empty + slot), ((n_item >> 1) & 1u) ^ 1u, prm.status, 0x0120u | slot);
-        if (!ok) break;
-        // a CTA's first item is its own number (no round trip to the counter on the way to the first load); the
-        // counter hands out what lies beyond the grid
-        const unsigned index = n_item == 0 ? blockIdx.x : gridDim.x + atomicAdd(prm.schedule, 1u);
-        *reinterpret_cast<volatile unsigned*>(&work_ring[slot]) = index;
-        mbar_arrive(bar(B::work_full + slot));
-        if (index >= prm.items) break;
-        const Item item = decode(index);
+    unsigned q_uses[kQTiles] = {0u, 0u};  // items so far in which Q tile t had rows
+    auto publish = [&](unsigned n_item, unsigned index) {
+      *reinterpret_cast<volatile unsigned*>(&work_ring[n_item & 1u]) = index;
+      mbar_arrive(bar(B::work_full + (n_item & 1u)));
+    };
+    auto load_q = [&](const Item& item, int t) {
+      ++q_uses[t];
+      mbar_expect_tx(bar(B::q_full + t), L::kTileBytes);
 #pragma unroll
-        for (int t = 0; t < kQTiles; ++t) {
-          if (item.n_kv[t] == 0 || !ok) continue;
-          ok = mbar_wait(bar(B::q_empty + t), (q_uses[t] & 1u) ^ 1u, prm.status, 0x0130u | t);
-          if (!ok) break;
-          ++q_uses[t];
-          mbar_expect_tx(bar(B::q_full + t), L::kTileBytes);
+      for (int a = 0; a < D / 64; ++a)
+        tma_load_4d(base + L::kQOff + t * L::kTileBytes + a * L::kAtomBytes, &map_q, bar(B::q_full + t), a * 64, item.q0[t], item.head, item.batch);
+    };
+    auto load_k = [&](const Item& item, int j, int stage) {
+      mbar_expect_tx(bar(B::k_full + stage), L::kTileBytes);
 #pragma unroll
-          for (int a = 0; a < D / 64; ++a)
-            tma_load_4d(base + L::kQOff + t * L::kTileBytes + a * L::kAtomBytes, &map_q, bar(B::q_full + t), a * 64,
-                        item.q0[t], item.head, item.batch);
-        }
-        for (int j = 0; j < item.loads && ok; ++j, ++step) {
+      for (int a = 0; a < D / 64; ++a)
+        tma_load_4d(base + L::kKOff + stage * L::kTileBytes + a * L::kAtomBytes, &map_k, bar(B::k_full + stage), a * 64, j * kTileRows, item.head, item.batch);
+    };
+    auto load_v = [&](const Item& item, int j, int stage) {
+      mbar_expect_tx(bar(B::v_full + stage), L::kTileBytes);
+#pragma unroll
+      for (int a = 0; a < D / 64; ++a)
+        tma_load_4d(base + L::kVOff + stage * L::kTileBytes + a * L::kAtomBytes, &map_v, bar(B::v_full + stage), a * 64, j * kTileRows, item.head, item.batch);
+    };
+    // a CTA's first item is its own number (no round trip to the counter on the way to the first load); the counter hands out
+    // what lies beyond the grid
+    if (lane == 0) publish(0u, blockIdx.x);
+    Item item = decode(blockIdx.x);
+    unsigned step = 0;  // key tiles loaded so far, over all items
+    int j = 0;
+    if (lane == 0) {
+#pragma unroll
+      for (int t = 0; t < kQTiles; ++t)
+        if (item.n_kv[t] > 0) load_q(item, t);
+      for (; j < min(item.loads, L::kStages); ++j, ++step) {  // (as many as have room)
+        load_k(item, j, j);
+        load_v(item, j, j);
+      }
+    }
+    __syncwarp();
+    named_barrier_sync(kDecided, 64);
+    if (lane == 0 && !abort_flag) {
+      for (unsigned n_item = 1;; ++n_item) {
+        for (; j < item.loads && ok; ++j, ++step) {
           const int stage = step % L::kStages;
           const uint32_t wrap = (step / L::kStages) & 1;
           ok = mbar_wait(bar(B::k_empty + stage), wrap ^ 1u, prm.status, 0x0100u | stage);
           if (!ok) break;
-          mbar_expect_tx(bar(B::k_full + stage), L::kTileBytes);
-#pragma unroll
-          for (int a = 0; a < D / 64; ++a)
-            tma_load_4d(base + L::kKOff + stage * L::kTileBytes + a * L::kAtomBytes, &map_k, bar(B::k_full + stage), a * 64,
-                        j * kTileRows, item.head, item.batch);
+          load_k(item, j, stage);
           ok = mbar_wait(bar(B::v_empty + stage), wrap ^ 1u, prm.status, 0x0110u | stage);
           if (!ok) break;
-          mbar_expect_tx(bar(B::v_full + stage), L::kTileBytes);
-#pragma unroll
-          for (int a = 0; a < D / 64; ++a)
-            tma_load_4d(base + L::kVOff + stage * L::kTileBytes + a * L::kAtomBytes, &map_v, bar(B::v_full + stage), a * 64,
-                        j * kTileRows, item.head, item.batch);
+          load_v(item, j, stage);
         }
+        const unsigned slot = n_item & 1u;
+        if (ok) ok = mbar_wait(bar(B::work_empty + slot), ((n_item >> 1) & 1u) ^ 1u, prm.status, 0x0120u | slot);
+        if (!ok) break;
+        const unsigned index = gridDim.x + atomicAdd(prm.schedule, 1u);
+        publish(n_item, index);
+        if (index >= prm.items) break;
+        item = decode(index);
+#pragma unroll
+        for (int t = 0; t < kQTiles; ++t) {
+          if (item.n_kv[t] == 0 || !ok) continue;
+          ok = mbar_wait(bar(B::q_empty + t), (q_uses[t] & 1u) ^ 1u, prm.status, 0x0130u | t);
+          if (ok) load_q(item, t);
+        }
+        j = 0;
       }
     }
   } else if (warp == kMmaWarp) {
@@ -711,7 +737,7 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kMmaWarp) {
-    if (*reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk) {
+    if (abort_flag || *reinterpret_cast<volatile unsigned*>(prm.status) != kStatusOk) {
       // a wait gave up somewhere: give copies and MMAs still in flight time to land before the
       // tensor memory and shared memory they target are released
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);

@@ -102,6 +102,8 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- named barriers of a CTA (0 is __syncthreads): take part and wait, or take part and go on ----
+// In the set-up of the 16-bit kernels: everything the roles need is in place; thread 0 has decided whether the block stands down.
+enum : int { kSetUp = 1, kDecided = 2 };
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void named_barrier_arrive(int id, int threads) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 

@@ -60,6 +60,59 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_recovers():
     assert runtime.device_status() == 0
 
 
+# bh, t_q, t_k, width, causal: more items than SMs, of one and two tiles, so that a producer draws from the work counter before it
+# has to wait; one query tile against two key tiles (shared keys); long streams, which it has to wait in at its first item
+STANDING_DOWN = [(300, 100, 100, 64, 0), (300, 100, 100, 128, 1), (200, 100, 200, 64, 0), (200, 60, 250, 128, 0), (20, 900, 900, 64, 1), (20, 900, 900, 128, 0)]
+
+
+@pytest.mark.parametrize("shape", STANDING_DOWN, ids=[f"{s[0]} x {s[1]}x{s[2]} width {s[3]}{' causal' if s[4] else ''}" for s in STANDING_DOWN])
+def test_every_kernel_stands_down_and_leaves_nothing_behind(shape):
+    from limn_b200 import runtime
+    from limn_b200._lib import DEVICE_TIMEOUT, check, lib
+
+    L = lib()
+    runtime.set_device(0)
+    assert runtime.device_status() == 0
+    bh, t_q, t_k, width, causal = shape
+    rng = np.random.default_rng(sum(shape))
+    q, k, v, do = (runtime.upload(rng.standard_normal((bh, t, width)).astype(np.float32).astype(BF16)) for t in (t_q, t_k, t_k, t_q))
+    tail = (2, bh, t_q, t_k, width, width, causal, width**-0.5, None)
+    rows, keys = bh * t_q, bh * t_k
+    sizes = {"out": rows * width * 2, "lse": rows * 4, "delta": rows * 4, "dq": rows * width * 2, "fused_delta": rows * 4,
+             "fused_dq": rows * width * 2, "dk": keys * width * 2, "dv": keys * width * 2}
+    known = {}
+
+    def launch(poison):
+        """All four calls; the backward ones on the first launch's O, L and delta."""
+        to = {name: runtime.empty(size, poison=poison) for name, size in sizes.items()}
+        o = known or to
+        check(L.limn_b200_sdpa_fwd(q.ptr, k.ptr, v.ptr, None, to["out"].ptr, to["lse"].ptr, *tail), "sdpa")
+        if not known:
+            check(L.limn_b200_sdpa_delta(o["out"].ptr, do.ptr, to["delta"].ptr, 2, rows, width, None), "row dot")
+        check(L.limn_b200_sdpa_bwd_q(q.ptr, k.ptr, v.ptr, do.ptr, o["lse"].ptr, o["delta"].ptr, None, to["dq"].ptr, *tail), "dq")
+        check(L.limn_b200_sdpa_bwd_q_fused(q.ptr, k.ptr, v.ptr, o["out"].ptr, do.ptr, o["lse"].ptr, None, to["fused_dq"].ptr, to["fused_delta"].ptr, *tail), "dq")
+        check(L.limn_b200_sdpa_bwd_kv(q.ptr, k.ptr, v.ptr, do.ptr, o["lse"].ptr, o["delta"].ptr, None, to["dk"].ptr, to["dv"].ptr, *tail), "dk, dv")
+        runtime.synchronize()
+        return to
+
+    def bytes_of(buffers):
+        return {name: runtime.download(buffers[name], np.uint8, (size,)) for name, size in sizes.items() if name != "delta"}
+
+    known.update(launch(0xFF))
+    good = bytes_of(known)
+    check(L.limn_b200_wait_probe(20000, None, None), "wait probe")
+    for name, seen in bytes_of(launch(0xAB)).items():
+        if name == "fused_delta" and t_k > 512:
+            continue  # (long dense problems have a kernel of their own for it, which waits for nothing and runs regardless)
+        assert (seen == 0xAB).all(), f"{name} was written although an earlier kernel had given up"
+    word = ctypes.c_uint(0)
+    assert L.limn_b200_device_status(ctypes.byref(word)) == DEVICE_TIMEOUT and word.value == 0x57417E57
+    for _ in range(2):
+        for name, seen in bytes_of(launch(0xAB)).items():
+            np.testing.assert_array_equal(seen, good[name], err_msg=name)
+    assert runtime.device_status() == 0
+
+
 def test_finish_raises_like_a_failed_kernel_of_the_reference():
     """limn_b200.install() wraps the device's finish(): after a batch in which one of our Runners ran, a set
     status word surfaces as RuntimeError("cuda: ..."), where limn raises for a failed kernel of its own."""
