@@ -811,14 +811,21 @@ int launch_fwd_s(const Problem& p) {
 
 // A problem with one Q tile: its tile goes into both places, the even key tiles to the first and the odd ones to the second,
 // whose softmax group would be idle otherwise, and the epilogue puts the two parts of every row together. That halves the
-// chain of key tiles, which is all there is to such an item. Measured: 64 problems of 100 x 1500 keys x 64 21.7 -> 14.3 us (18.8
-// without), 8 of 128 x 4096 x 128 52.5 -> 30.4, 192 of 100 x 700 x 64 under a mask 27.8 -> 19.2. The line lies where it does not
-// depend on how many problems there are: a row's bits must not. (The last, single tile of an odd number of them was tried
-// too: a gain of 3 % at head dim 64, a loss of up to 24 % at 128, where the kernel then spills.)
+// chain of key tiles, which is all there is to such an item. Measured, us without / with: 64 problems of 100 x 1500 keys x 64
+// 18.6 / 14.1, 8 of 128 x 4096 x 128 46.9 / 30.7, 192 of 100 x 700 x 64 under a mask 22.8 / 19.0.
+// The line, without / with: what sharing costs is a second copy of Q and the merge, so it pays from some number of key tiles on.
+//   two tiles at width 128 without a mask, not shared: 1600 of 16 x 160 48.0 / 58.8, 320 15.0 / 16.7, 32 6.8 / 6.9; 32 of 100 x 256 6.9 / 7.3
+//   two at width 64, shared: 32 of 16 x 160 6.1 / 5.8, 96 6.5 / 6.8, 320 13.0 / 13.9, 1600 41.3 / 47.6; of 100 rows 6.4 / 6.0, 6.7 / 7.1, 13.9 / 14.2, 44.9 / 48.4
+//   two under a mask, shared: width 64 8 to 1600 of 100 x 160 7.3 / 7.1 to 60.7 / 55.9, width 128 8.2 / 8.1 to 71.3 / 64.7
+//   three at width 128 (384 keys), shared: 32 of 100 rows 8.3 / 8.3, 320 20.1 / 18.7, 1600 70.1 / 70.4; of 16 rows 7.8 / 7.9, 17.8 / 17.7, 61.0 / 63.4
+//   four (512 keys): 9.6 / 9.1, 25.0 / 23.0, 88.0 / 87.3
+// It does not depend on how many problems there are: a row's bits must not. (The last, single tile of an odd number of them was
+// tried too: a gain of 3 % at head dim 64, a loss of up to 24 % at 128, where the kernel then spills.)
 template <int D, bool kCausal, bool kFp16, bool kMask>
 int launch_fwd(const Problem& p) {
   if constexpr (!kCausal) {  // (a causal problem of one Q tile has one key tile)
-    if (p.t_q <= kTileRows && p.t_k > kTileRows) return launch_fwd_s<D, kCausal, kFp16, kMask, true>(p);
+    constexpr int kAlone = (D == 128 && !kMask) ? 2 * kTileRows : kTileRows;  // keys up to which one group takes them all
+    if (p.t_q <= kTileRows && p.t_k > kAlone) return launch_fwd_s<D, kCausal, kFp16, kMask, true>(p);
   }
   return launch_fwd_s<D, kCausal, kFp16, kMask, false>(p);
 }

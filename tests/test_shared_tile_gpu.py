@@ -53,6 +53,24 @@ def test_problems_of_one_query_tile(case, dtype, dev):
     _check(dev, *_problem(sum(case), *case, dtype))
 
 
+def _rows_and_lse(dev, q, k, v, mask=None):
+    import limn_standin as host
+
+    out, lse = host.Attention(dev, q, k, v, causal=False, key_mask=mask).forward()
+    return out.view(np.uint16), lse.view(np.uint32)
+
+
+@pytest.mark.parametrize("t_k", [129, 256], ids=["129 keys", "256 keys"])
+@pytest.mark.parametrize("t_q", [16, 128])
+def test_two_key_tiles_at_width_128_are_not_shared(t_q, t_k, dev):
+    """Sharing those costs more than it saves. Unshared rows are those of a problem of two query tiles, bit for bit."""
+    q, k, v, _ = _problem(t_q + t_k, 3, 200, t_k, 128)
+    out, lse = _rows_and_lse(dev, q, k, v)
+    head_out, head_lse = _rows_and_lse(dev, np.ascontiguousarray(q[:, :t_q]), k, v)
+    np.testing.assert_array_equal(head_out, out[:, :t_q])
+    np.testing.assert_array_equal(head_lse, lse[:, :t_q])
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("hidden", ["even tiles", "odd tiles", "all but one key"])
 def test_a_group_whose_keys_are_all_hidden(hd, hidden, dev):
