@@ -71,6 +71,27 @@ def test_two_key_tiles_at_width_128_are_not_shared(t_q, t_k, dev):
     np.testing.assert_array_equal(head_lse, lse[:, :t_q])
 
 
+@pytest.mark.parametrize("t_k,hd", [(300, 128), (1300, 128), (200, 64), (700, 64)])
+def test_l_of_shared_rows_is_as_good_as_of_unshared_ones(t_k, hd, dev):
+    """Against float64, as a root mean square over 16 000 rows: the same rows in problems of 100 query rows, which are shared, and of
+    200, which are not. Under a mask, where all exponentials are as good as float32's. 1 % for the rows' chance (1 / sqrt(2 x 16000))."""
+    rng = np.random.default_rng(t_k + hd)
+    bh, t_q = 160, 100
+    q, k, v = (rng.standard_normal((bh, t, hd)).astype(np.float32).astype(np.float16) for t in (2 * t_q, t_k, t_k))
+    keep = np.arange(t_k) < rng.integers(t_k // 2, t_k + 1, (bh, 1))
+    mask = keep.astype(np.float16)
+    scores = np.where(keep[:, None], np.matmul(q[:, :t_q].astype(np.float64), k.astype(np.float64).transpose(0, 2, 1)) * hd**-0.5, -np.inf)
+    top = scores.max(-1, keepdims=True)
+    want = (top + np.log(np.exp(scores - top).sum(-1, keepdims=True)))[..., 0]
+
+    def off(rows):
+        lse = _rows_and_lse(dev, np.ascontiguousarray(q[:, :rows]), k, v, mask)[1].view(np.float32)
+        return np.sqrt(np.mean((lse.reshape(bh, rows)[:, :t_q] - want) ** 2))
+
+    shared, alone = off(t_q), off(2 * t_q)
+    assert shared <= 1.01 * alone, f"{shared:.3e} against {alone:.3e}"
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("hidden", ["even tiles", "odd tiles", "all but one key"])
 def test_a_group_whose_keys_are_all_hidden(hd, hidden, dev):
