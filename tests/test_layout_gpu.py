@@ -25,6 +25,8 @@ CASES = [
     (3, 4, 128, 128, 64, False, BF16),
     (2, 3, 200, 200, 96, True, BF16),  # narrower heads run zero-padded in the 128 and the 64 kernel
     (2, 2, 150, 150, 40, False, np.dtype(np.float16)),
+    (2, 3, 100, 300, 64, False, BF16),  # one query tile, key tiles shared by the two softmax groups
+    (3, 2, 128, 400, 96, False, np.dtype(np.float16)),
 ]
 
 
@@ -152,6 +154,35 @@ def test_slices_of_one_projection_buffer_give_the_dense_bits(hd, causal, t):
     assert L.limn_b200_sdpa_fwd_strided(q_ptr, k_ptr, v_ptr, None, out.ptr, lse.ptr, None, *tail) == 1
     assert L.limn_b200_sdpa_fwd_strided(q_ptr, k_ptr, v_ptr, None, out.ptr, lse.ptr, arr(in_qkv, in_qkv, in_qkv, token_major),
                                         0, batch, heads, t, t, hd, hd, int(causal), hd**-0.5, None) == 2  # float32: not served strided
+
+
+@pytest.mark.parametrize("t_q,t_k,hd", [(100, 300, 64), (128, 520, 128), (33, 129, 40)])
+@pytest.mark.parametrize("masked", [False, True], ids=["", "masked"])
+def test_cross_attention_out_of_a_key_value_projection_gives_the_dense_bits(t_q, t_k, hd, masked):
+    """The strided forward where the two softmax groups share a problem's keys: q and O token-major, k and v slices of one
+    (batch, t_k, 2, heads, hd) projection output."""
+    import ctypes
+
+    from limn_b200 import runtime
+    from limn_b200._lib import check, lib
+
+    L = lib()
+    batch, heads = 3, 2
+    q, k, v, do = _inputs(36, batch, heads, t_q, t_k, hd, BF16)
+    mask = (np.arange(t_k) % 7 != 3).astype(np.float32).astype(BF16) * np.ones((batch, heads, 1), BF16) if masked else None
+    want = _run("bhtd", (q, k, v, do), mask, batch, heads, t_q, t_k, hd, False, BF16)
+    q_dev = runtime.upload(np.ascontiguousarray(q.transpose(0, 2, 1, 3)))
+    kv_dev = runtime.upload(np.ascontiguousarray(np.stack([a.transpose(0, 2, 1, 3) for a in (k, v)], axis=2)))
+    m_dev = runtime.upload(mask) if masked else None
+    row1, row2 = heads * hd, 2 * heads * hd
+    strides = (ctypes.c_longlong * 12)(*[t_q * row1, hd, row1], *[t_k * row2, hd, row2] * 2, *[t_q * row1, hd, row1])
+    out, lse = runtime.empty(q.nbytes), runtime.empty(batch * heads * t_q * 4)
+    check(L.limn_b200_sdpa_fwd_strided(q_dev.ptr, kv_dev.ptr, kv_dev.ptr + row1 * 2, m_dev.ptr if masked else None, out.ptr, lse.ptr, strides, 2, batch, heads,
+                                       t_q, t_k, hd, hd, 0, hd**-0.5, None), "sdpa")
+    assert runtime.device_status() == 0
+    got = runtime.download(out, BF16, (batch, t_q, heads, hd)).transpose(0, 2, 1, 3)
+    np.testing.assert_array_equal(got.view(np.uint16), want["out"].view(np.uint16))
+    np.testing.assert_array_equal(runtime.download(lse, np.uint32, (batch, heads, t_q)), want["lse"].view(np.uint32))
 
 
 def test_dense_layout_code_is_the_dense_entry_point():

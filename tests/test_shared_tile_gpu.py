@@ -71,6 +71,37 @@ def test_two_key_tiles_at_width_128_are_not_shared(t_q, t_k, dev):
     np.testing.assert_array_equal(head_lse, lse[:, :t_q])
 
 
+# bh, t_q, t_k, hd: more problems than SMs, so that a CTA has shared items one after the other; odd and even numbers of key tiles
+MANY = [(333, 60, 300, 64), (333, 20, 130, 64), (200, 100, 400, 128)]
+
+
+@pytest.mark.parametrize("masked", [False, True], ids=["", "masked"])
+@pytest.mark.parametrize("case", MANY, ids=[f"{c[0]} x {c[1]}x{c[2]} hd {c[3]}" for c in MANY])
+def test_many_shared_problems(case, masked, dev):
+    bh, t_q, t_k, hd = case
+    operands = _problem(sum(case), *case)
+    mask = None
+    if masked:
+        rng = np.random.default_rng(bh + t_k)
+        mask = ((np.arange(t_k) < rng.integers(1, t_k + 1, (bh, 1))) & (rng.random((bh, t_k)) < 0.9)).astype(np.float32)
+        mask[:, 0] = 1
+        mask = mask.astype(BF16)
+    _check(dev, *operands, mask)
+
+
+@pytest.mark.parametrize("masked", [False, True], ids=["", "masked"])
+@pytest.mark.parametrize("case", MANY, ids=[f"{c[0]} x {c[1]}x{c[2]} hd {c[3]}" for c in MANY])
+def test_a_row_has_the_same_bits_however_many_problems_there_are(case, masked, dev):
+    bh, t_q, t_k, hd = case
+    q, k, v, _ = _problem(sum(case), *case)
+    mask = (np.arange(t_k) < 1 + np.arange(bh)[:, None] * t_k // bh).astype(np.float32).astype(BF16) if masked else None
+    out, lse = _rows_and_lse(dev, q, k, v, mask)
+    for p in (0, 150, bh - 1):
+        alone_out, alone_lse = _rows_and_lse(dev, *(np.ascontiguousarray(a[p : p + 1]) for a in (q, k, v)), None if mask is None else mask[p : p + 1])
+        np.testing.assert_array_equal(alone_out[0], out[p])
+        np.testing.assert_array_equal(alone_lse[0], lse[p])
+
+
 @pytest.mark.parametrize("t_k,hd", [(300, 128), (1300, 128), (200, 64), (700, 64)])
 def test_l_of_shared_rows_is_as_good_as_of_unshared_ones(t_k, hd, dev):
     """Against float64, as a root mean square over 16 000 rows: the same rows in problems of 100 query rows, which are shared, and of
@@ -138,7 +169,7 @@ def test_a_nan_key_makes_every_row_nan(hd, t_q, masked, dev):
     t_k = 300
     q, k, v, do = _problem(hd + t_q, 16, t_q, t_k, hd)
     for p in range(16):
-        k[p, 17 * p] = np.nan  # the 16 residues of a column index mod 16, over all three tiles
+        k[p, 19 * p] = np.nan  # the 16 residues of a column index mod 16, over all three tiles (up to key 285)
     mask = np.ones((16, t_k), np.float32).astype(BF16) if masked else None
     att = host.Attention(dev, q, k, v, causal=False, key_mask=mask)
     out, lse = att.forward()
