@@ -162,9 +162,6 @@ struct BwdParams {
   float scale;
 };
 
-// barrier among the 128 threads of one group (ids 1 and 2; 0 is __syncthreads)
-__device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
-
 // One accumulator row slice (32 fp32 columns) scaled, rounded and written as 64 bytes, or as many 16-byte pieces
 // of them as the row has columns left.
 template <bool kFp16>

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   __shared__ float part_acc[kWarps][R][D];
   __shared__ float peer_m[kMaxSplit - 1][R], peer_l[kMaxSplit - 1][R], peer_o[kMaxSplit - 1][R][D];  // in CTA 0: the other CTAs' shares
 
-  constexpr int kFolds = (R * D + kThreads - 1) / kThreads;  // output elements of a thread
+  static_assert(R * D <= kThreads, "a thread folds one output element");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = lane / kLanesPerKey, gl = lane % kLanesPerKey;
   const int split = prm.split;
@@ -286,23 +286,18 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   // ---- the 16 warps: thread (r, d) folds them in warp order; the CTAs of a cluster leave their shares with CTA 0, which
   // folds those in rank order. One element per thread, rounded once. ----
   if (split > 1) cluster_wait();  // every CTA of the cluster has started
-  float m_at[kFolds], l_at[kFolds], o_at[kFolds];
-#pragma unroll
-  for (int n = 0; n < kFolds; ++n) {
-    const int at = threadIdx.x + n * kThreads;
-    if (at >= R * D) break;
-    const int r = at / D, d = at - r * D;
-    float m_tot = -INFINITY;
+  const int r = threadIdx.x / D, d = threadIdx.x - r * D;
+  const bool mine = threadIdx.x < R * D;
+  float m_tot = -INFINITY, l_tot = 0.f, o = 0.f;
+  if (mine) {
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) m_tot = fmaxf(m_tot, part_m[w][r]);
-    float l_tot = 0.f, o = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
       const float f = part_m[w][r] == -INFINITY ? 0.f : exp2f((part_m[w][r] - m_tot) * sl2);
       l_tot = fmaf(part_l[w][r], f, l_tot);
       o = fmaf(part_acc[w][r][d], f, o);
     }
-    m_at[n] = m_tot, l_at[n] = l_tot, o_at[n] = o;
     if (rank > 0) {
       store_at_first(&peer_o[rank - 1][r][d], o);
       if (d == 0) store_at_first(&peer_m[rank - 1][r], m_tot), store_at_first(&peer_l[rank - 1][r], l_tot);
@@ -310,42 +305,32 @@ __global__ void __launch_bounds__(kThreads, R <= 2 ? 2 : 1) sdpa_decode_kernel(c
   }
   if (split > 1) {
     cluster_arrive();
-    if (rank > 0) {
-      cluster_wait();  // (a CTA may not leave before the barrier is complete)
-      return;
-    }
-    cluster_wait();
+    cluster_wait();  // (also in the CTAs that are done: none may leave before the barrier is complete)
+    if (rank > 0) return;
   }
-#pragma unroll
-  for (int n = 0; n < kFolds; ++n) {
-    const int at = threadIdx.x + n * kThreads;
-    if (at >= R * D) break;
-    const int r = at / D, d = at - r * D;
-    float m_tot = m_at[n], l_tot = l_at[n], o = o_at[n];
-    for (int c = 1; c < split; ++c) {
-      const float m_c = peer_m[c - 1][r], l_c = peer_l[c - 1][r], o_c = peer_o[c - 1][r][d];
-      const float m_new = fmaxf(m_tot, m_c);
-      const float fa = m_tot == -INFINITY ? 0.f : exp2f((m_tot - m_new) * sl2);
-      const float fc = m_c == -INFINITY ? 0.f : exp2f((m_c - m_new) * sl2);
-      l_tot = l_tot * fa + l_c * fc;
-      o = o * fa + o_c * fc;
-      m_tot = m_new;
-    }
-    const int row = row0 + r;
-    if (row >= prm.t_q) continue;
-    const float value = o / l_tot;  // 0 / 0 = NaN for a row with no visible key, as the oracle gives
-    unsigned char* dst = static_cast<unsigned char*>(prm.out) +
-                         (batch * prm.o_strides.batch + head * prm.o_strides.head + static_cast<long long>(row) * prm.o_strides.row + d) * kBytes;
-    if (d < prm.pieces_v * 8) {
-      if (kKind == kF32) *reinterpret_cast<float*>(dst) = value;
-      else if (kKind == kF16) *reinterpret_cast<__half*>(dst) = __float2half_rn(value);
-      else *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(value);
-    }
-    if (d == 0) {  // in float32 once per row in double: L is then as good as its sum
-      const long long to = static_cast<long long>(problem) * prm.t_q + row;
-      if (kKind == kF32) prm.lse[to] = static_cast<float>(static_cast<double>(m_tot) * prm.scale + log(static_cast<double>(l_tot)));
-      else prm.lse[to] = m_tot * prm.scale + logf(l_tot);
-    }
+  const int row = row0 + r;
+  if (!mine || row >= prm.t_q) return;
+  for (int c = 1; c < split; ++c) {
+    const float m_c = peer_m[c - 1][r], l_c = peer_l[c - 1][r], o_c = peer_o[c - 1][r][d];
+    const float m_new = fmaxf(m_tot, m_c);
+    const float fa = m_tot == -INFINITY ? 0.f : exp2f((m_tot - m_new) * sl2);
+    const float fc = m_c == -INFINITY ? 0.f : exp2f((m_c - m_new) * sl2);
+    l_tot = l_tot * fa + l_c * fc;
+    o = o * fa + o_c * fc;
+    m_tot = m_new;
+  }
+  const float value = o / l_tot;  // 0 / 0 = NaN for a row with no visible key, as the oracle gives
+  unsigned char* dst = static_cast<unsigned char*>(prm.out) +
+                       (batch * prm.o_strides.batch + head * prm.o_strides.head + static_cast<long long>(row) * prm.o_strides.row + d) * kBytes;
+  if (d < prm.pieces_v * 8) {
+    if (kKind == kF32) *reinterpret_cast<float*>(dst) = value;
+    else if (kKind == kF16) *reinterpret_cast<__half*>(dst) = __float2half_rn(value);
+    else *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(value);
+  }
+  if (d == 0) {  // in float32 once per row in double: L is then as good as its sum
+    const long long to = static_cast<long long>(problem) * prm.t_q + row;
+    if (kKind == kF32) prm.lse[to] = static_cast<float>(static_cast<double>(m_tot) * prm.scale + log(static_cast<double>(l_tot)));
+    else prm.lse[to] = m_tot * prm.scale + logf(l_tot);
   }
 }
 
