@@ -194,8 +194,9 @@ const char* limn_b200_last_error(void);
 int limn_b200_version(void);
 
 /* Kernels that wait (on TMA or tensor-core completion) give up after a bounded time and
- * record a code in a per-device status word instead of hanging; kernels launched on that device
- * afterwards return at once, writing nothing, until the word has been read. This synchronises the
+ * record a code in a per-device status word instead of hanging; kernels of that kind launched on that
+ * device afterwards return within some milliseconds, writing nothing, until the word has been read
+ * (the float64, CUDA-core, decode and row-dot kernels wait for nothing and run). This synchronises the
  * current device, reads its word into *status and clears it. Returns LIMN_B200_OK with *status == 0
  * when no kernel gave up, LIMN_B200_DEVICE_TIMEOUT with *status = 0x5741rrbb (role rr, barrier bb)
  * when one did. The reference reports a failed kernel from its batch barrier

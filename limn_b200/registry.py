@@ -266,8 +266,8 @@ def check_device_status(doing: str = "waiting for the batch") -> None:
 
     A kernel that waits (on a TMA copy or on the tensor pipe) does so for a bounded time; when
     the time runs out it records a code in a per-device status word and returns, and every
-    later kernel on that device returns at once without writing its outputs until the word has
-    been read. The reference turns a failed kernel into a RuntimeError at its batch barrier
+    later kernel of that kind on that device returns without writing its outputs until the word
+    has been read. The reference turns a failed kernel into a RuntimeError at its batch barrier
     (limn/backend_cuda.py:349 through check(), :154-162); this is the same for ours."""
     global _launched_since_check
     if not _launched_since_check:

@@ -2,7 +2,7 @@
 
 Every wait in the tensor-core kernels (on a TMA copy, on the tensor pipe, on another warp) is bounded: when
 its budget runs out the kernel records 0x5741rrbb in the device's status word and returns, and kernels that
-start while the word is set stand down at once. limn_b200_wait_probe makes exactly that happen with a
+start while the word is set stand down. limn_b200_wait_probe makes exactly that happen with a
 one-warp kernel of its own that waits a few microseconds on a barrier nobody arrives at; the production
 kernels are not touched. The test then checks what the rest of the library promises about that state."""
 
