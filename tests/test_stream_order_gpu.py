@@ -54,3 +54,50 @@ def test_a_decode_step_between_the_kernel_that_writes_its_cache_and_the_one_that
         for got, ref in zip(run(lambda: None), want, strict=True):
             np.testing.assert_array_equal(got, ref)
     assert runtime.device_status() == 0
+
+
+@pytest.mark.parametrize("name", list(NAMES))
+@pytest.mark.parametrize("shape", DECODE, ids=[f"{s[0]} x {s[1]} x {s[2]}" for s in DECODE])
+def test_the_same_three_calls_as_a_graph(shape, name):
+    """Captured once and replayed over buffers that were filled with something else: the edges between the calls hold there too."""
+    import torch
+
+    from limn_b200._lib import DTYPE_CODES, check, lib
+
+    L = lib()
+    bh, t, width = shape
+    dtype = {"bfloat16": torch.bfloat16, "float16": torch.float16, "float32": torch.float32}[name]
+    gen = torch.Generator(device="cuda").manual_seed(sum(shape))
+    q, k, v, one, last = (torch.randn((bh, n, width), generator=gen, device="cuda").to(dtype) for n in (t, t, t, 1, 40))
+    cache, step, end = torch.empty_like(q), torch.empty_like(one), torch.empty_like(last)
+    lse = [torch.empty((bh, n), device="cuda") for n in (t, 1, 40)]
+
+    def forward(q, k, v, out, lse_out, causal):
+        stream = torch.cuda.current_stream().cuda_stream
+        check(L.limn_b200_sdpa_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), None, out.data_ptr(), lse_out.data_ptr(), DTYPE_CODES[name], bh, q.shape[1],
+                                   k.shape[1], width, width, causal, width**-0.5, stream), "sdpa")
+
+    def run():
+        forward(q, k, v, cache, lse[0], 1)
+        forward(one, cache, cache, step, lse[1], 0)
+        forward(last, step, step, end, lse[2], 0)
+
+    results = (cache, step, end, *lse)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        run()
+        stream.synchronize()
+        want = [r.clone() for r in results]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run()
+            run()
+        for value in (0.0, 3.5, float("nan")):
+            for r in results:
+                r.fill_(value)
+            graph.replay()
+            stream.synchronize()
+            for got, ref in zip(results, want, strict=True):
+                assert torch.equal(got, ref)
+    graph.reset()
