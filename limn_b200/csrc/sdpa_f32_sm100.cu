@@ -62,30 +62,26 @@ struct Params {
 // ---- x = h + m + l for two floats at a time ----
 // What an operand's split shows. Of a float32 of ordinary size the second remainder has eight bits at most and is its own
 // third piece, so the low half of its word is zero. It is not for an infinity or a NaN (the remainder is the NaN 0x7fffffff) and for
-// a number so small (below about 2^-110) that pieces fall under bfloat16's 2^-133 and bits would be lost.
+// a number so small (below about 2^-110) that pieces fall under bfloat16's 2^-133 and bits would be lost. Weights (P and dS) are
+// not looked at one by one: one that is not finite makes a NaN of its row's sums, where it is noticed.
 struct Check {
-  uint32_t words = 0;   // all second remainders of operands
-  uint64_t weights = 0; // NaN once a weight (P or dS) was not finite
-  __device__ __forceinline__ bool bad() const {
-    float a, b;
-    f2_unpack(weights, a, b);
-    return (words & 0xffffu) != 0u || !(a == 0.f && b == 0.f);
-  }
+  uint32_t words = 0;  // all second remainders of operands
+  bool sums = false;   // a sum was not finite
+  __device__ __forceinline__ bool bad() const { return (words & 0xffffu) != 0u || sums; }
 };
+// The middle piece is left as -m, the way the subtractions give it, and the products with one of it turn its sign round
+// (piece_minus). Both remainders are exact. Eight clocks a pair and scheduler; with the pieces unpacked to float32 and a packed FMA
+// for each remainder it was eleven.
 template <bool kOperand>
 __device__ __forceinline__ void split_pair(uint64_t x, uint32_t& h, uint32_t& m, uint32_t& l, Check& check) {
-  const uint64_t minus = f2_pack(-1.f, -1.f);
   float a, b;
   f2_unpack(x, a, b);
   h = pack_bf16(a, b);
-  x = f2_fma(f2_pack_bits(h << 16, h & 0xffff0000u), minus, x);  // exact
-  f2_unpack(x, a, b);
+  a = sub_bf16_lo(h, a), b = sub_bf16_hi(h, b);  // h - x
   m = pack_bf16(a, b);
-  x = f2_fma(f2_pack_bits(m << 16, m & 0xffff0000u), minus, x);  // exact
-  f2_unpack(x, a, b);
+  a = sub_bf16_lo(m, a), b = sub_bf16_hi(m, b);  // x - h - m
   l = pack_bf16(a, b);
   if (kOperand) check.words |= __float_as_uint(a) | __float_as_uint(b);
-  else check.weights = f2_fma(x, 0ull, check.weights);
 }
 
 template <int N>
@@ -172,6 +168,7 @@ struct Stage {
 // The six products in the order they are added, smallest first.
 __device__ __host__ constexpr int piece_a(int i) { return (0x001102 >> (4 * i)) & 0xf; }  // l h m m h h
 __device__ __host__ constexpr int piece_b(int i) { return (0x010120 >> (4 * i)) & 0xf; }  // h l m h m h
+__device__ __host__ constexpr bool piece_minus(int i) { return (piece_a(i) == 1) != (piece_b(i) == 1); }
 
 // D (kRows x kStream) = A (kRows x HD) B^T (kStream x HD), both with the contraction dim contiguous. A lies in shared
 // memory (a0 its address) or in tensor memory (a0 its column, pieces HD / 2 columns apart). Columns past the head dim are
@@ -182,10 +179,10 @@ __device__ __host__ constexpr int piece_b(int i) { return (0x010120 >> (4 * i)) 
 template <int HD, bool kTmemA, bool kTwo = false>
 __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b0, uint32_t d2 = 0) {
   constexpr uint32_t kPieceA = (HD > 64 ? 2 : 1) * kRows * 128, kPieceB = (HD > 64 ? 2 : 1) * kStream * 128;
-  constexpr uint32_t idesc = mma_idesc(kRows, kStream, false, false, false);
   const uint32_t a_lo = kTmemA ? a0 : desc_lo(a0, 0), b_lo = desc_lo(b0, 0);
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
+    const uint32_t idesc = mma_idesc(kRows, kStream, false, false, false, piece_minus(i));
 #pragma unroll
     for (int s = 0; s < HD / 16; ++s) {
       const uint32_t b = b_lo + piece_b(i) * (kPieceB / 16) + (s / 4) * (kStream * 128 / 16) + (s % 4) * 2;
@@ -207,10 +204,10 @@ __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t a0, uint32_t b
 template <int HD>
 __device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0) {
   constexpr uint32_t kPiece = (HD > 64 ? 2 : 1) * kStream * 128;
-  constexpr uint32_t idesc = mma_idesc(kRows, HD, false, false, true);
   const uint32_t x_lo = desc_lo(x0, kStream * 128);
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
+    const uint32_t idesc = mma_idesc(kRows, HD, false, false, true, piece_minus(i));
 #pragma unroll
     for (int s = 0; s < kStream / 16; ++s)
       mma_ts_lo(d, w0 + piece_a(i) * kPieceCols + s * 8, x_lo + piece_b(i) * (kPiece / 16) + s * (16 * 128 / 16), idesc, i > 0 || s > 0);
@@ -459,6 +456,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     float sum0, sum1;
     f2_unpack(sum, sum0, sum1);
     denom = fmaf(denom, shrink, sum0 + sum1);  // this thread's share; the shares meet after the last tile
+    check.sums |= !(denom < INFINITY);
     hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
     tmem_st_wait();
     tc_fence_before_sync();
@@ -564,14 +562,20 @@ __device__ __forceinline__ void weigh_scores(const Params& g, const uint32_t (&s
   }
 }
 
-// The sums over dS at their own size again. One that overflowed at kDsUp times it counts as a weight that was not finite.
+// The sums over dS at their own size again, and whether they are finite: one is not where one of them overflowed at kDsUp times
+// its size, and a whole row is not where a P or a dS of it was not (dS is P times something, and the products of a piece that is
+// infinite are infinite or NaN for every column).
 template <int N>
 __device__ __forceinline__ void settle(uint64_t (&acc)[N], Check& check) {
+  uint64_t zero = 0;
 #pragma unroll
   for (int c = 0; c < N; ++c) {
-    check.weights = f2_fma(acc[c], 0ull, check.weights);
+    zero = f2_fma(acc[c], 0ull, zero);
     acc[c] = f2_mul(acc[c], f2_pack(1.f / kDsUp, 1.f / kDsUp));
   }
+  float a, b;
+  f2_unpack(zero, a, b);
+  check.sums |= !(a == 0.f && b == 0.f);
 }
 
 // The columns of a thread's CW that its row does not see: outside [from, to), as bits.

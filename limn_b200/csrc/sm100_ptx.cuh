@@ -184,11 +184,12 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lead
 }
 
 // Instruction descriptor for tcgen05.mma.kind::f16: fp32 accumulate, A and B both bf16 or
-// both fp16. a_mn / b_mn say the operand is MN-major (0 = K-major).
-__host__ __device__ constexpr uint32_t mma_idesc(int m, int n, bool fp16, bool a_mn, bool b_mn) {
+
+__host__ __device__ constexpr uint32_t mma_idesc(int m, int n, bool fp16, bool a_mn, bool b_mn, bool a_minus = false) {
   return (1u << 4)                      // D format: f32
          | ((fp16 ? 0u : 1u) << 7)      // A format: f16 = 0, bf16 = 1
          | ((fp16 ? 0u : 1u) << 10)     // B format
+         | ((a_minus ? 1u : 0u) << 13)  // negate A
          | ((a_mn ? 1u : 0u) << 15)     // A major
          | ((b_mn ? 1u : 0u) << 16)     // B major
          | (static_cast<uint32_t>(n >> 3) << 17)
@@ -338,6 +339,18 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
+// h - x, h being the bfloat16 in the low or high half of `pair`: the mixed-precision subtraction reads the half-word as it lies.
+__device__ __forceinline__ float sub_bf16_lo(uint32_t pair, float x) {
+  float r;
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tsub.rn.f32.bf16 %0, lo, %2;\n\t}" : "=f"(r) : "r"(pair), "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sub_bf16_hi(uint32_t pair, float x) {
+  float r;
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tsub.rn.f32.bf16 %0, hi, %2;\n\t}" : "=f"(r) : "r"(pair), "f"(x));
   return r;
 }
 
