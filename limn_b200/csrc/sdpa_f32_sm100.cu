@@ -225,19 +225,58 @@ __device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2
   tmem_st<N / 2>(at + 2 * kPieceCols, l);
 }
 
+// B lanes of a warp (B = 2 or 4) hold B pieces of 16 bytes each of a row of their own; afterwards x[r] is piece (lane % B) of the
+// row of lane r of the B.
+template <int B>
+__device__ __forceinline__ void swap_rows_for_pieces(float (&x)[B][4]) {
+  const uint32_t lane = lane_id();
+#pragma unroll
+  for (int d = 1; d < B; d *= 2) {
+    const bool upper = (lane & d) != 0;
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      if (i & d) continue;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float got = __shfl_xor_sync(kFull, upper ? x[i][c] : x[i | d][c], d);
+        if (upper) x[i][c] = got;
+        else x[i | d][c] = got;
+      }
+    }
+  }
+}
+
+// The N columns from `col` on of a warp's 32 rows from `first` on, a row to a thread, into a matrix of (rows, width). A row's
+// own 16-byte pieces, stored one after the other, are 32 lines of memory an instruction, and the load/store unit takes a clock for
+// each (a block's 128 x 64 results 2 000 to 6 000 clocks); with the pieces of B neighbouring rows exchanged first, an instruction
+// writes 64 bytes (N = 8: 32) of each row it touches.
 template <int N>
-__device__ __forceinline__ void store_row(float* row, const uint64_t (&acc)[N / 2], int first, int width, bool wide) {
+__device__ __forceinline__ void store_rows(float* dst, const uint64_t (&acc)[N / 2], int first, int rows, int col, int width, bool wide) {
+  const int lane = static_cast<int>(lane_id());
+  if (wide) {
+    constexpr int B = N / 4 < 4 ? N / 4 : 4;
+    const int top = first + (lane & ~(B - 1)), at = col + 4 * (lane & (B - 1));
 #pragma unroll
-  for (int i = 0; i < N; i += 4) {
-    float x[4];
-    f2_unpack(acc[i / 2], x[0], x[1]);
-    f2_unpack(acc[i / 2 + 1], x[2], x[3]);
-    if (wide) {
-      if (first + i < width) *reinterpret_cast<float4*>(row + first + i) = make_float4(x[0], x[1], x[2], x[3]);
-    } else {
+    for (int set = 0; set < N / 4; set += B) {
+      float x[B][4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (first + i + c < width) row[first + i + c] = x[c];
+      for (int i = 0; i < B; ++i) {
+        f2_unpack(acc[2 * (set + i)], x[i][0], x[i][1]);
+        f2_unpack(acc[2 * (set + i) + 1], x[i][2], x[i][3]);
+      }
+      swap_rows_for_pieces<B>(x);
+#pragma unroll
+      for (int r = 0; r < B; ++r)
+        if (top + r < rows && at + 4 * set < width)
+          *reinterpret_cast<float4*>(dst + static_cast<long long>(top + r) * width + at + 4 * set) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
+    }
+  } else if (first + lane < rows) {
+    float* row = dst + static_cast<long long>(first + lane) * width;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float x[2];
+      f2_unpack(acc[i / 2], x[0], x[1]);
+      if (col + i < width) row[col + i] = x[i & 1];
     }
   }
 }
@@ -506,19 +545,17 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
       float total = 0.f;
 #pragma unroll
       for (int c = 0; c < G; ++c) total += exchange[c][row];
-      if (i < g.t_q) {
 #pragma unroll
-        for (int c = 0; c < OW / 2; ++c) {
-          float x0, x1;
-          f2_unpack(acc[c], x0, x1);
-          acc[c] = f2_pack(x0 / total, x1 / total);  // 0/0 = NaN for a row with no key, as the oracle has it
-        }
-        store_row<OW>(g.out + (b * g.t_q + i) * g.hd_v, acc, group * OW, g.hd_v, g.wide_out);
-        // once per row, so in double: L is then as good as its sum
-        if (group == 0)
-          g.lse_out[b * g.t_q + i] =
-              top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
+      for (int c = 0; c < OW / 2; ++c) {
+        float x0, x1;
+        f2_unpack(acc[c], x0, x1);
+        acc[c] = f2_pack(x0 / total, x1 / total);  // 0/0 = NaN for a row with no key, as the oracle has it
       }
+      store_rows<OW>(g.out + b * g.t_q * g.hd_v, acc, i0 + (warp & 3) * 32, g.t_q, group * OW, g.hd_v, g.wide_out);
+      // once per row, so in double: L is then as good as its sum
+      if (group == 0 && i < g.t_q)
+        g.lse_out[b * g.t_q + i] =
+            top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
     }
   }
   tear_down<L::kCols>(g, tmem);
@@ -842,12 +879,13 @@ __global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_ker
     const bool bad = __syncthreads_or(check.bad());
     if (ok && bad) {
       rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
-    } else if (ok && mine < owned) {
+    } else if (ok) {
+      const int top = first + (warp & 3) * 32;
       if (kKV) {
-        store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
-        store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc1, group * OW, g.hd_v, g.wide_out);
+        store_rows<OW>(g.dk + b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
+        store_rows<OW>(g.dv + b * owned * g.hd_v, acc1, top, owned, group * OW, g.hd_v, g.wide_out);
       } else {
-        store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
+        store_rows<OW>(g.dq + b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
       }
     }
   }
@@ -1036,12 +1074,13 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
   const bool bad = __syncthreads_or(check.bad());
   if (ok && bad) {
     rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
-  } else if (ok && mine < owned) {
+  } else if (ok) {
+    const int top = first + (warp & 3) * 32;
     if (kKV) {
-      store_row<OW>(g.dv + (b * owned + mine) * g.hd_v, acc0, group * OW, g.hd_v, g.wide_out);
-      store_row<OW>(g.dk + (b * owned + mine) * g.hd, acc1, group * OW, g.hd, g.wide_out);
+      store_rows<OW>(g.dv + b * owned * g.hd_v, acc0, top, owned, group * OW, g.hd_v, g.wide_out);
+      store_rows<OW>(g.dk + b * owned * g.hd, acc1, top, owned, group * OW, g.hd, g.wide_out);
     } else {
-      store_row<OW>(g.dq + (b * owned + mine) * g.hd, acc0, group * OW, g.hd, g.wide_out);
+      store_rows<OW>(g.dq + b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
     }
   }
   tear_down<L::kCols>(g, tmem);
