@@ -28,6 +28,7 @@
 // there (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 213 / 1 984 / 2 548, the tiled
 // kernels alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above
 // head dim 64 leave their loop when they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -136,22 +137,18 @@ struct Stage {
 
   float x[kLoops][8];
 
-  // `thread`: which of the kThreads the calling one counts as. A tile with fewer pieces than threads is done by the first
-  // ones only; the dQ pass gives two such tiles to different halves of the block (290 -> 283 us for 6 x 8192 x 32; in the
-  // dK/dV pass it costs registers, 400 -> 420).
-  __device__ __forceinline__ static int second_half() { return kTurns == 0 ? threadIdx.x ^ (kThreads / 2) : threadIdx.x; }
-  __device__ __forceinline__ void load(const float* src, int first, int rows, int width, int thread = threadIdx.x) {
+  __device__ __forceinline__ void load(const float* src, int first, int rows, int width) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
-      const int e = thread + n * kThreads;
+      const int e = threadIdx.x + n * kThreads;
       if (kTurns == 0 && e >= R * kChunks) break;
       load8<kWide>(x[n], src, first + e / kChunks, rows, (e % kChunks) * 8, width);
     }
   }
-  __device__ __forceinline__ void store(uint32_t dst, Check& check, int thread = threadIdx.x) {
+  __device__ __forceinline__ void store(uint32_t dst, Check& check) {
 #pragma unroll
     for (int n = 0; n < kLoops; ++n) {
-      const int e = thread + n * kThreads;
+      const int e = threadIdx.x + n * kThreads;
       if (kTurns == 0 && e >= R * kChunks) break;
       const int r = e / kChunks, chunk = e % kChunks;
       uint32_t h[4], m[4], l[4];
@@ -338,11 +335,11 @@ __device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t
   tmem = __shfl_sync(kFull, *slot, 0);
   return true;
 }
-template <int kCols>
+template <int kCols, int kWarp = 0>
 __device__ __forceinline__ void tear_down(const Params& g, uint32_t tmem) {
   tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < 32) {
+  if (threadIdx.x / 32 == kWarp) {
     if (*reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk) {
       // a wait gave up somewhere: give MMAs still in flight time to land before their memory is released
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
@@ -353,19 +350,19 @@ __device__ __forceinline__ void tear_down(const Params& g, uint32_t tmem) {
 }
 
 // One float a row of the tile that starts at j0, zero beyond the end: thread i < kStream has row i's.
-__device__ __forceinline__ float row_value(const float* from, int j0, int rows) {
-  const int j = j0 + static_cast<int>(threadIdx.x);
+__device__ __forceinline__ float row_value(const float* from, int j0, int rows, int thread = threadIdx.x) {
+  const int j = j0 + thread;
   float x;  // (as in load8: nothing waits for it here)
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
                : "=&f"(x)
-               : "l"(from + j), "r"(threadIdx.x < kStream && j < rows ? 1u : 0u));
+               : "l"(from + j), "r"(thread < kStream && j < rows ? 1u : 0u));
   return x;
 }
 // The hidden keys of a tile (flag 0, keys past the end among them) as two words in shared memory, bit set = hidden.
-__device__ __forceinline__ void post_hidden(uint32_t* words, float flag) {
-  if (threadIdx.x < kStream) {
+__device__ __forceinline__ void post_hidden(uint32_t* words, float flag, int thread = threadIdx.x) {
+  if (thread < kStream) {
     const unsigned hid = __ballot_sync(kFull, flag == 0.f);
-    if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = hid;
+    if ((thread & 31) == 0) words[thread >> 5] = hid;
   }
 }
 // ... and the part of them a thread with columns [group * N, group * N + N) needs.
@@ -624,272 +621,461 @@ __device__ __forceinline__ uint32_t outside(int from, int to) {
   return unseen;
 }
 
+// ---- the kernels that work in roles: sixteen row warps, three splitting warps, one issuing warp ----
+// Four row threads to a row take scores out of tensor memory, turn them into weights, split those and sum a tile's products; the
+// splitting warps bring the streamed operands into shared memory in pieces, a few tiles ahead; the issuing warp issues every MMA.
+// The roles meet at mbarriers whose waits are bounded; no barrier of the block stands inside their loops, so a warp that gave up on a
+// wait cannot hang the others. A block goes through several work items: the splitting warps run ahead into the next item while the
+// row warps end this one.
+constexpr int kRowWarps = 16, kSplitWarps = 3, kIssuer = kRowWarps + kSplitWarps;
+constexpr int kRowThreads = 32 * kRowWarps, kSplitThreads = 32 * kSplitWarps, kRoleThreads = 32 * (kIssuer + 1);
+constexpr int kRowGroups = kRowThreads / kRows;  // threads to a row
+constexpr int kMostItems = 32;                   // work items of a block: each has a bit of a word
+
+// Work item `k` of this block. Blocks take turns, there and back: items are in the order of their length under a causal mask, and a
+// block that got a long one in one turn gets a short one in the next.
+__device__ __forceinline__ bool work_item(const Params& g, int k, int& problem, int& slot) {
+  const long long grid = gridDim.x, within = (k & 1) ? grid - 1 - blockIdx.x : blockIdx.x, index = k * grid + within;
+  if (k >= kMostItems || index >= g.bh * g.slots) return false;
+  cta_work(static_cast<int>(index), g.slots, g.bh, g.group, problem, slot);
+  return true;
+}
+
+// What the splitting warps carry from global memory to pieces in shared memory, half a streamed tile (one operand) at a time, and in
+// registers meanwhile: a thread that has split one of its eighths of a row loads the next half's in its place.
+template <int HD, bool kWide>
+struct Carry {
+  static constexpr int kChunks = HD / 8, kStep = kSplitThreads / kChunks;  // rows from one turn to the next
+  static constexpr int kTurns = (kStream + kStep - 1) / kStep;
+  static constexpr uint32_t kPiece = kStream * 128;
+  static_assert(HD <= 64 && kSplitThreads % kChunks == 0, "a thread keeps its columns");
+  float x[kTurns][8];
+  int row, chunk;  // of the first turn
+
+  __device__ __forceinline__ explicit Carry(int thread) : row(thread / kChunks), chunk(thread % kChunks) {}
+  __device__ __forceinline__ void load(int n, const float* src, int first, int rows, int width) {
+    if (n * kStep + kStep <= kStream || n * kStep + row < kStream) load8<kWide>(x[n], src, first + n * kStep + row, rows, chunk * 8, width);
+  }
+  __device__ __forceinline__ void store(int n, uint32_t dst, Check& check) {
+    if (n * kStep + kStep <= kStream || n * kStep + row < kStream) {
+      uint32_t h[4], m[4], l[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split_pair<true>(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
+      const uint32_t at = swizzled_piece(dst, n * kStep + row, chunk);
+      st_shared_v4(at, h[0], h[1], h[2], h[3]);
+      st_shared_v4(at + kPiece, m[0], m[1], m[2], m[3]);
+      st_shared_v4(at + 2 * kPiece, l[0], l[1], l[2], l[3]);
+    }
+  }
+};
+
+__device__ __forceinline__ void warp_arrives(uint32_t bar) {
+  __syncwarp();
+  if (lane_id() == 0) mbar_arrive(bar);
+}
+// Every lane waits, and the warp goes on together: false for all of it if one of them gave up.
+__device__ __forceinline__ bool warp_waits(uint32_t bar, uint32_t parity, unsigned* status, unsigned tag) {
+  return __all_sync(kFull, mbar_wait(bar, parity, status, tag));
+}
+
+// 16 bytes (4, where rows are not whole 16-byte pieces) from global to shared memory without registers; zero where `left` <= 0.
+template <bool kWide>
+__device__ __forceinline__ void copy_async16(uint32_t dst, const float* src, int left) {
+  if constexpr (kWide) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(left > 0 ? 16 : 0) : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * i), "l"(left > i ? src + i : src), "r"(left > i ? 4 : 0) : "memory");
+  }
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Where a row warp's part of a held operand (its 32 rows, its group's HD / 4 columns) waits, as float32, for its turn in tensor
+// memory: only that warp touches it. 16-byte piece p of row r; eight rows' pieces lie on distinct banks.
+template <int HD>
+__device__ __forceinline__ uint32_t held_piece(uint32_t at, int r, int p) {
+  constexpr int kPieces = HD / 16;  // of a row
+  static_assert(kPieces == 4 || kPieces == 2, "head dims 64 and 32");
+  const int where = kPieces == 4 ? p ^ ((r >> 1) & 3) : p ^ ((r >> 2) & 1);
+  return at + static_cast<uint32_t>(r * kPieces + where) * 16u;
+}
+template <int HD, bool kWide>
+__device__ __forceinline__ void fetch_held(uint32_t at, const float* src, int first, int rows, int col, int width) {
+  constexpr int kPieces = HD / 16;
+  const int lane = static_cast<int>(lane_id());
+#pragma unroll
+  for (int n = 0; n < kPieces; ++n) {
+    const int e = lane + 32 * n, r = e / kPieces, p = e % kPieces;
+    const bool there = first + r < rows;
+    const int c = col + 4 * p;
+    copy_async16<kWide>(held_piece<HD>(at, r, p), there && c < width ? src + static_cast<long long>(first + r) * width + c : src, there ? width - c : 0);
+  }
+}
+// ... and from there, split, to this thread's lane of tensor memory at column `to` (pieces HD / 2 columns apart).
+template <int HD>
+__device__ __forceinline__ void place_held(uint32_t to, uint32_t at, Check& check) {
+  constexpr int kPieces = HD / 16;
+  const int lane = static_cast<int>(lane_id());
+  float x[4 * kPieces];
+#pragma unroll
+  for (int p = 0; p < kPieces; ++p)
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(x[4 * p]), "=f"(x[4 * p + 1]), "=f"(x[4 * p + 2]), "=f"(x[4 * p + 3])
+                 : "r"(held_piece<HD>(at, lane, p)) : "memory");
+  uint32_t h[2 * kPieces], m[2 * kPieces], l[2 * kPieces];
+#pragma unroll
+  for (int e = 0; e < 2 * kPieces; ++e) split_pair<true>(f2_pack(x[2 * e], x[2 * e + 1]), h[e], m[e], l[e], check);
+  if constexpr (kPieces == 4) {
+    tmem_st8(to, h), tmem_st8(to + HD / 2, m), tmem_st8(to + HD, l);
+  } else {
+    tmem_st4(to, h), tmem_st4(to + HD / 2, m), tmem_st4(to + HD, l);
+  }
+}
+
 // ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
-// Sixteen row warps (four threads to a row) load, split, weigh and sum; a seventeenth issues every MMA, so that a tile's
-// scores run while the tile before it is weighed. Issuing a tile's MMAs takes as long as the tensor cores take to run them: with
-// one of the sixteen as issuer that was 2400 + 1160 clocks of the 5200 a dQ tile took at head dim 64, in which the other fifteen
-// had nothing to do, and the tensor cores nothing while the issuer caught up. Rows and issuer tell each other
-// through mbarriers whose waits are bounded; no barrier of the block stands inside the loop, so a warp that gave up on a
-// wait cannot hang the others.
-template <int HD, bool kKV, bool kWide>
+// A tile's scores are computed while the row warps are at the tile before it, and its products are gathered while the next tile's
+// are: a row warp comes to each of its waits with the answer there, as long as the tensor cores keep up.
+template <int HD, bool kKV>
 struct Pipe {
-  static constexpr int kGroups = 4, kRowThreads = kRows * kGroups, kThreads = kRowThreads + 32;
-  using Held = Stage<HD, kRows, kRowThreads, kWide>;
-  using Tile = Stage<HD, kStream, kRowThreads, kWide>;
   // tensor memory: scores, dP, the pieces of dS and (dK/dV) of P, a tile's products, and the held operands if they fit:
   // they are the A side of the scores, an MMA then only reads the streamed tile from shared memory (whose bandwidth
-  // bounds it at 48 clocks with both there, for 32), and shared memory holds four tiles instead of two
+  // bounds it at 48 clocks with both there, for 32)
   static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols;
   static constexpr uint32_t kOut0 = kKV ? kP + 3 * kPieceCols : kP, kOut1 = kOut0 + HD, kHeldCol = kKV ? kOut1 + HD : kOut1;
   static constexpr bool kHeldT = kHeldCol + 3 * HD <= 512;
-  static constexpr int kStages = kHeldT ? 4 : 2;
-  static constexpr uint32_t kHeld0 = 0, kHeld1 = Held::kBytes, kTiles = kHeldT ? 0 : 2 * Held::kBytes;
-  static constexpr uint32_t kBytes = kTiles + kStages * 2 * Tile::kBytes + 1024;
   static constexpr int kCols = 512;
+  // shared memory: places for the first streamed operand, which the products need, and for the second; the held operands, in
+  // pieces or, where those are in tensor memory, as the next item's float32. The first operand has three places: with two, a tile
+  // could not be brought in before the products of the tile two before it were done.
+  static constexpr int kPlaces0 = 3, kPlaces1 = HD > 32 ? 2 : 3;
+  static constexpr uint32_t kTile = 3 * kStream * 128, kHeldPieces = 3 * kRows * 128, kHeldRaw = kRows * HD * 4;
+  static constexpr uint32_t kTile0 = 0, kTile1 = kPlaces0 * kTile, kHeld0 = kTile1 + kPlaces1 * kTile, kHeld1 = kHeld0 + (kHeldT ? kHeldRaw : kHeldPieces);
+  static constexpr uint32_t kBytes = kHeld1 + (kHeldT ? kHeldRaw : kHeldPieces) + 1024;
 };
 
 template <int HD, bool kKV, bool kWide>
-__global__ void __launch_bounds__(Pipe<HD, kKV, kWide>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
-  using L = Pipe<HD, kKV, kWide>;
-  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G, kRowWarps = L::kRowThreads / 32;
+__global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
+  using L = Pipe<HD, kKV>;
+  using Held = Stage<HD, kRows, kRowThreads, kWide>;
+  constexpr int CW = kStream / kRowGroups, OW = HD / kRowGroups;
   extern __shared__ __align__(16) unsigned char raw[];
-  __shared__ uint32_t slot, abort_flag, hidden[L::kStages][2];
-  __shared__ __align__(8) uint64_t bars[9];
-  __shared__ __align__(16) float lse_hi[L::kStages][kStream], lse_lo[L::kStages][kStream], deltas[L::kStages][kStream];
-  uint32_t tmem;
-  // scored, weighed, weighed_p (dK/dV: dV's products, the first of the two): by the tensor cores; free (the scores have
-  // been read), handed (P, dS are there), staged[stage]: by the row warps
-  if (!set_up<L::kCols, 9>(g, &slot, &abort_flag, bars, tmem, 0xfcu, kRowWarps)) return;
-  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1), weighed_p = smem_addr(bars + 8), free_ = smem_addr(bars + 2), handed = smem_addr(bars + 3);
-  auto staged = [&](int j) { return smem_addr(bars + 4 + j % L::kStages); };
-  auto staged_parity = [&](int j) { return static_cast<uint32_t>(j / L::kStages) & 1u; };
-  const uint32_t base = align_1024(smem_addr(raw));
+  __shared__ uint32_t slot, abort_flag, again_all, hidden[L::kPlaces0][2];
+  // by the tensor cores: scored, weighed, and a place's tile no longer needed (done0, done1); by the row warps: held operands there,
+  // scores read (free), P and dS there (handed); by the splitting warps: a tile there (staged0, staged1)
+  enum { kScored, kWeighed, kHeldThere, kFree, kHanded, kDone0, kDone1 = kDone0 + L::kPlaces0, kStaged0 = kDone1 + L::kPlaces1, kStaged1 = kStaged0 + L::kPlaces0, kBars = kStaged1 + L::kPlaces1 };
+  __shared__ __align__(8) uint64_t bars[kBars];
+  __shared__ __align__(16) float lse_hi[kKV ? L::kPlaces0 : 1][kStream], lse_lo[kKV ? L::kPlaces0 : 1][kStream], deltas[kKV ? L::kPlaces0 : 1][kStream];
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < kBars; ++i)
+      mbar_init(smem_addr(bars + i), i >= kStaged0 ? kSplitWarps : i == kHeldThere || i == kFree || i == kHanded ? kRowWarps : 1);
+    mbar_init_fence();
+    again_all = 0;
+  }
+  auto bar = [&](int i) { return smem_addr(bars + i); };
+  auto place = [](int t, int places) { return t % places; };
+  auto round = [](int t, int places) { return static_cast<uint32_t>(t / places) & 1u; };
+  const uint32_t base = align_1024(smem_addr(raw));
+  auto tile0_at = [&](int t) { return base + L::kTile0 + place(t, L::kPlaces0) * L::kTile; };
+  auto tile1_at = [&](int t) { return base + L::kTile1 + place(t, L::kPlaces1) * L::kTile; };
 
-  int problem, at;
-  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
-  const int first = (kKV ? at : g.slots - 1 - at) * kRows;  // the longest causal streams first
-  const long long b = problem;
   // the held pair (against which the tiles are scored) and the streamed pair
   const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
-  const int begin = kKV && g.causal ? first : 0;
-  const int end = !kKV && g.causal ? min(streamed, first + kRows) : streamed;
-  const int n = (end - begin + kStream - 1) / kStream;
-  auto tile_at = [&](int j, int which) { return base + L::kTiles + ((j % L::kStages) * 2 + which) * L::Tile::kBytes; };
-  bool ok = true;
-  Check check;
+  struct Item {
+    long long b;
+    int first, begin, tiles;  // first own row; first streamed row, tiles of them
+  };
+  auto item = [&](int k, Item& it) {
+    int problem = 0, at = 0;
+    if (!work_item(g, k, problem, at)) return false;
+    it.b = problem;
+    it.first = (kKV ? at : g.slots - 1 - at) * kRows;  // the longest causal streams first
+    it.begin = kKV && g.causal ? it.first : 0;
+    const int end = !kKV && g.causal ? min(streamed, it.first + kRows) : streamed;
+    it.tiles = (end - it.begin + kStream - 1) / kStream;
+    return true;
+  };
+  auto held0 = [&](const Item& it) { return (kKV ? g.k : g.q) + it.b * owned * g.hd; };
+  auto held1 = [&](const Item& it) { return (kKV ? g.v : g.dout) + it.b * owned * g.hd_v; };
+  auto stream0 = [&](const Item& it) { return (kKV ? g.q : g.k) + it.b * streamed * g.hd; };
+  auto stream1 = [&](const Item& it) { return (kKV ? g.dout : g.v) + it.b * streamed * g.hd_v; };
 
-  if (warp == kRowWarps) {
-    // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
-    for (int j = -1; j < n; ++j) {
-      if (j + 1 < n) {
-        ok = mbar_wait(staged(j + 1), staged_parity(j + 1), g.status, 0x0b10u);
-        if (j >= 0) ok = ok && mbar_wait(free_, j & 1, g.status, 0x0b11u);
-        ok = __all_sync(kFull, ok);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (elect_one()) {
-          issue_scores<HD, L::kHeldT>(tmem + L::kS, L::kHeldT ? tmem + L::kHeldCol : base + L::kHeld0, tile_at(j + 1, 0));
-          issue_scores<HD, L::kHeldT>(tmem + L::kDp, L::kHeldT ? tmem + L::kHeldCol + 3 * HD / 2 : base + L::kHeld1, tile_at(j + 1, 1));
-          mma_commit(scored);
-        }
-        __syncwarp();
-      }
-      if (j >= 0) {
-        ok = __all_sync(kFull, mbar_wait(handed, j & 1, g.status, 0x0b12u));
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (elect_one()) {
-          if (kKV) {
-            issue_weigh<HD>(tmem + L::kOut1, tmem + L::kP, tile_at(j, 1));
-            mma_commit(weighed_p);
-          }
-          issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile_at(j, 0));
-          mma_commit(weighed);
-        }
-        __syncwarp();
-      }
-    }
-    ok = __syncthreads_and(ok);
-    __syncthreads_or(0);
-  } else {
-    // ================= row warps =================
-    const int group = warp >> 2;
-    const int row = (warp & 3) * 32 + lane;
-    const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    const float* held0 = (kKV ? g.k : g.q) + b * owned * g.hd;
-    const float* held1 = (kKV ? g.v : g.dout) + b * owned * g.hd_v;
-    const float* stream0 = (kKV ? g.q : g.k) + b * streamed * g.hd;
-    const float* stream1 = (kKV ? g.dout : g.v) + b * streamed * g.hd_v;
-    const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
-    const int mine = first + row;  // this thread's row
-    auto arrive = [&](uint32_t bar) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar);
-    };
-    // the streamed tile j, and what goes with its rows: to registers, and from there to shared memory
-    typename L::Tile tile0, tile1;
-    float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
-    auto load_tile = [&](int j) {
-      const int x0 = begin + j * kStream;
-      tile0.load(stream0, x0, streamed, g.hd);
-      tile1.load(stream1, x0, streamed, g.hd_v, kKV ? threadIdx.x : L::Tile::second_half());
-      if (kKV) {
-        row_a = row_value(g.lse_in + b * g.t_q, x0, streamed);
-        row_b = row_value(g.delta + b * g.t_q, x0, streamed);
-      } else if (mask) {
-        row_a = row_value(mask, x0, streamed);
-      }
-    };
-    auto store_tile = [&](int j, bool split = false) {  // split: the second operand and the rows' values only
-      if (kKV) {
-        if (threadIdx.x < kStream) {
-          float hi, lo;
-          to_log2(row_a, hi, lo);
-          lse_hi[j % L::kStages][threadIdx.x] = hi;
-          lse_lo[j % L::kStages][threadIdx.x] = lo;
-          deltas[j % L::kStages][threadIdx.x] = row_b;
-        }
-      } else if (mask) {
-        post_hidden(hidden[j % L::kStages], row_a);
-      }
-      tile1.store(tile_at(j, 1), check, kKV ? threadIdx.x : L::Tile::second_half());
-      if (!split) {
-        tile0.store(tile_at(j, 0), check);
-        fence_async_shared();
-        arrive(staged(j));
-      }
-    };
+  // a row warp's part of the held operands
+  const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+  const uint32_t raw0 = base + L::kHeld0 + warp * (32 * OW * 4), raw1 = base + L::kHeld1 + warp * (32 * OW * 4);
+  auto fetch = [&](const Item& it) {
+    fetch_held<HD, kWide>(raw0, held0(it), it.first + quarter * 32, owned, group * OW, g.hd);
+    fetch_held<HD, kWide>(raw1, held1(it), it.first + quarter * 32, owned, group * OW, g.hd_v);
+  };
 
-    // every load is on its way before the first one is waited for
-    float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
-    bool live = mine < owned;
-    if constexpr (L::kHeldT) {
-      float x[2][OW / 8][8];
-#pragma unroll
-      for (int c = 0; c < OW / 8; ++c) {
-        load8<kWide>(x[0][c], held0, mine, owned, group * OW + 8 * c, g.hd);
-        load8<kWide>(x[1][c], held1, mine, owned, group * OW + 8 * c, g.hd_v);
-      }
-      load_tile(0);
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int c = 0; c < OW / 8; ++c) {
-          uint32_t hi[4], mi[4], lo[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) split_pair<true>(f2_pack(x[h][c][2 * e], x[h][c][2 * e + 1]), hi[e], mi[e], lo[e], check);
-          const uint32_t to = lanes + L::kHeldCol + h * (3 * HD / 2) + group * (OW / 2) + 4 * c;
-          tmem_st4(to, hi);
-          tmem_st4(to + HD / 2, mi);
-          tmem_st4(to + HD, lo);
-        }
-      tmem_st_wait();
-      tc_fence_before_sync();
-    } else {
-      typename L::Held stage0, stage1;
-      stage0.load(held0, first, owned, g.hd);
-      stage1.load(held1, first, owned, g.hd_v);
-      load_tile(0);
-      stage0.store(base + L::kHeld0, check);
-      stage1.store(base + L::kHeld1, check);
-    }
-    if constexpr (kKV) {
-      if (live && mask) live = mask[mine] != 0.f;
-    } else if (live) {
-      to_log2(g.lse_in[b * g.t_q + mine], my_hi, my_lo);
-      my_delta = g.delta[b * g.t_q + mine];
-    }
-    store_tile(0);  // (says that the held rows are there, too)
-    if (n > 1) {
-      load_tile(1);
-      store_tile(1);
-    }
-    if (n > 2) load_tile(2);
+  // the held operands of an item into L2, a 128-byte line to a thread
+  auto prefetch_held = [&](const Item& it) {
+    constexpr int kLines = HD / 32;
+    const int e = threadIdx.x, r = it.first + (e % (kRows * kLines)) / kLines, c = (e % kLines) * 32;
+    const bool second = e >= kRows * kLines;
+    const int width = second ? g.hd_v : g.hd;
+    if (e < 2 * kRows * kLines && r < owned && c < width)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"((second ? held1(it) : held0(it)) + static_cast<long long>(r) * width + c));
+  };
 
-    uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dK and dV
-#pragma unroll
-    for (int c = 0; c < OW / 2; ++c) acc0[c] = acc1[c] = 0;
-    auto gather = [&](uint32_t from, uint64_t(&acc)[OW / 2]) {
-      uint32_t o[OW];
-      tmem_ld<OW>(lanes + from + group * OW, o);
-      tmem_ld_wait();
-#pragma unroll
-      for (int c = 0; c < OW / 2; ++c) acc[c] = f2_add(acc[c], f2_pack_bits(o[2 * c], o[2 * c + 1]));
-    };
-    for (int j = 0; j < n; ++j) {
-      const int x0 = begin + j * kStream;
-      if (kKV || mask) ok = mbar_wait(staged(j), staged_parity(j), g.status, 0x0b20u);
-      ok = __all_sync(kFull, ok && mbar_wait(scored, j & 1, g.status, 0x0b21u));
-      if (!ok) break;
-      tc_fence_after_sync();
-      uint32_t s[CW], dp[CW];
-      tmem_ld<CW>(lanes + L::kS + group * CW, s);
-      tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      arrive(free_);
-      int from = 0, to = streamed - x0 - group * CW;
-      if (g.causal) {
-        if (kKV) from = mine - x0 - group * CW;
-        else to = min(to, mine - x0 - group * CW + 1);
-      }
-      uint32_t unseen = outside<CW>(from, live ? to : 0);
-      if (!kKV && mask) unseen |= my_hidden<CW>(hidden[j % L::kStages], group);
-      uint64_t p[CW / 2], ds[CW / 2];
-      weigh_scores<CW>(g, s, dp, unseen, [&](int c, uint64_t& hi, uint64_t& lo, uint64_t& delta) {
-        if (kKV) {
-          hi = *reinterpret_cast<const uint64_t*>(&lse_hi[j % L::kStages][group * CW + c]);
-          lo = *reinterpret_cast<const uint64_t*>(&lse_lo[j % L::kStages][group * CW + c]);
-          delta = *reinterpret_cast<const uint64_t*>(&deltas[j % L::kStages][group * CW + c]);
-        } else {
-          hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
-        }
-      }, p, ds);
-      // (the products of the tile before have been gathered, so its P and dS have been read)
-      hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, check);
-      if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
-      tmem_st_wait();
-      tc_fence_before_sync();
-      arrive(handed);
-      // tile j + 2 takes the place of tile j + 2 - kStages: gathered already, or now about to be
-      if (L::kStages > 2 && j + 2 < n) store_tile(j + 2);
-      if (L::kStages > 2 && j + 3 < n) load_tile(j + 3);
-      if constexpr (kKV) {  // dV's part while the tensor cores are at dK's
-        ok = __all_sync(kFull, mbar_wait(weighed_p, j & 1, g.status, 0x0b23u));
-        if (!ok) break;
-        tc_fence_after_sync();
-        gather(L::kOut1, acc1);
-        if (L::kStages == 2 && j + 2 < n) store_tile(j + 2, true);
-      }
-      ok = __all_sync(kFull, mbar_wait(weighed, j & 1, g.status, 0x0b22u));
-      if (!ok) break;
-      tc_fence_after_sync();
-      gather(L::kOut0, acc0);
-      tc_fence_before_sync();
-      if (L::kStages == 2 && j + 2 < n) {
-        tile0.store(tile_at(j + 2, 0), check);
-        fence_async_shared();
-        arrive(staged(j + 2));
-      }
-      if (L::kStages == 2 && j + 3 < n) load_tile(j + 3);
-    }
-    settle(acc0, check);
-    ok = __syncthreads_and(ok);
-    const bool bad = __syncthreads_or(check.bad());
-    if (ok && bad) {
-      rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, L::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, b, first, raw);
-    } else if (ok) {
-      const int top = first + (warp & 3) * 32;
-      if (kKV) {
-        store_rows<OW>(g.dk + b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
-        store_rows<OW>(g.dv + b * owned * g.hd_v, acc1, top, owned, group * OW, g.hd_v, g.wide_out);
-      } else {
-        store_rows<OW>(g.dq + b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
-      }
-    }
+  Item it;
+  const bool any = item(0, it);
+  grid_dependency_wait();
+  if (warp == kIssuer) {
+    tmem_alloc(smem_addr(&slot), L::kCols);
+    tmem_relinquish();
   }
-  tear_down<L::kCols>(g, tmem);
+  if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk;
+  // the first operands set out before the block is set up
+  Carry<HD, kWide> carry(threadIdx.x - kRowThreads);
+  if (any && warp < kRowWarps) {
+    if (L::kHeldT) fetch(it);
+  } else if (any && warp < kIssuer) {
+#pragma unroll
+    for (int n = 0; n < carry.kTurns; ++n) carry.load(n, stream0(it), it.begin, streamed, g.hd);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(kFull, slot, 0);
+  bool ok = true;
+  uint32_t again = 0;  // items in which this thread met something that does not split
+  if (abort_flag) {
+    // an earlier kernel on this device gave up on a wait: take no work
+    copy_async_wait();
+  } else if (warp == kIssuer) {
+    // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
+    grid_launch_dependents();
+    int t = 0;  // tiles so far
+    auto weigh = [&](int t) {
+      ok = ok && warp_waits(bar(kHanded), t & 1, g.status, 0x0b12u);
+      if (!ok) return;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        if (kKV) {
+          issue_weigh<HD>(tmem + L::kOut1, tmem + L::kP, tile1_at(t));
+          mma_commit(bar(kDone1 + place(t, L::kPlaces1)));
+        }
+        issue_weigh<HD>(tmem + L::kOut0, tmem + L::kDs, tile0_at(t));
+        mma_commit(bar(kWeighed));
+        mma_commit(bar(kDone0 + place(t, L::kPlaces0)));
+      }
+      __syncwarp();
+    };
+    for (int k = 0; ok && item(k, it); ++k) {
+      ok = warp_waits(bar(kHeldThere), k & 1, g.status, 0x0b13u);
+      for (int j = 0; ok && j < it.tiles; ++j, ++t) {
+        ok = warp_waits(bar(kStaged0 + place(t, L::kPlaces0)), round(t, L::kPlaces0), g.status, 0x0b10u);
+        if (t > 0) ok = ok && warp_waits(bar(kFree), (t - 1) & 1, g.status, 0x0b11u);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) issue_scores<HD, L::kHeldT>(tmem + L::kS, L::kHeldT ? tmem + L::kHeldCol : base + L::kHeld0, tile0_at(t));
+        __syncwarp();
+        ok = warp_waits(bar(kStaged1 + place(t, L::kPlaces1)), round(t, L::kPlaces1), g.status, 0x0b14u);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_scores<HD, L::kHeldT>(tmem + L::kDp, L::kHeldT ? tmem + L::kHeldCol + 3 * HD / 2 : base + L::kHeld1, tile1_at(t));
+          mma_commit(bar(kScored));
+          if (!kKV) mma_commit(bar(kDone1 + place(t, L::kPlaces1)));
+        }
+        __syncwarp();
+        if (j > 0) weigh(t - 1);
+      }
+      if (ok) weigh(t - 1);
+    }
+  } else if (warp >= kRowWarps) {
+    // ================= splitting warps =================
+    const int thread = threadIdx.x - kRowThreads;
+    const float* mask = g.mask;
+    float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
+    auto load_rows = [&](const Item& it, int x0) {
+      if (kKV) {
+        row_a = row_value(g.lse_in + it.b * g.t_q, x0, streamed, thread);
+        row_b = row_value(g.delta + it.b * g.t_q, x0, streamed, thread);
+      } else if (mask) {
+        row_a = row_value(mask + it.b * g.t_k, x0, streamed, thread);
+      }
+    };
+    if (any) load_rows(it, it.begin);
+    int t = 0;
+    bool more = any;
+    for (int k = 0; ok && more; ++k) {
+      Check check;
+      Item next = it;
+      more = item(k + 1, next);
+      for (int j = 0; j < it.tiles; ++j, ++t) {
+        const int x0 = it.begin + j * kStream;
+        if (t >= L::kPlaces0) ok = ok && warp_waits(bar(kDone0 + place(t, L::kPlaces0)), round(t, L::kPlaces0) ^ 1u, g.status, 0x0b30u);
+        if (!ok) break;
+        if (kKV) {
+          if (thread < kStream) {
+            float hi, lo;
+            to_log2(row_a, hi, lo);
+            lse_hi[place(t, L::kPlaces0)][thread] = hi;
+            lse_lo[place(t, L::kPlaces0)][thread] = lo;
+            deltas[place(t, L::kPlaces0)][thread] = row_b;
+          }
+        } else if (mask) {
+          post_hidden(hidden[place(t, L::kPlaces0)], row_a, thread);
+        }
+#pragma unroll
+        for (int n = 0; n < carry.kTurns; ++n) {
+          carry.store(n, tile0_at(t), check);
+          carry.load(n, stream1(it), x0, streamed, g.hd_v);
+        }
+        fence_async_shared();
+        warp_arrives(bar(kStaged0 + place(t, L::kPlaces0)));
+        if (t >= L::kPlaces1) ok = ok && warp_waits(bar(kDone1 + place(t, L::kPlaces1)), round(t, L::kPlaces1) ^ 1u, g.status, 0x0b31u);
+        if (!ok) break;
+        const bool last = j + 1 == it.tiles;
+        const Item& then = last ? next : it;
+        const int x1 = last ? next.begin : x0 + kStream;
+        const float* from = stream0(then);
+        const int rows = last && !more ? 0 : streamed;  // nothing left to load
+        if (rows > 0) load_rows(then, x1);
+#pragma unroll
+        for (int n = 0; n < carry.kTurns; ++n) {
+          carry.store(n, tile1_at(t), check);
+          carry.load(n, from, x1, rows, g.hd);
+        }
+        fence_async_shared();
+        warp_arrives(bar(kStaged1 + place(t, L::kPlaces1)));
+      }
+      if (check.bad()) again |= 1u << k;
+      it = next;
+    }
+  } else if (any) {
+    // ================= row warps =================
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    // the held operands of item k, which have been fetched, to where the MMAs read them
+    auto put_held = [&](const Item& it, int k) {
+      Check check;
+      if constexpr (L::kHeldT) {
+        copy_async_wait();
+        __syncwarp();
+        place_held<HD>(lanes + L::kHeldCol + group * (OW / 2), raw0, check);
+        place_held<HD>(lanes + L::kHeldCol + 3 * HD / 2 + group * (OW / 2), raw1, check);
+        tmem_st_wait();
+        tc_fence_before_sync();
+      } else {
+        Held stage0, stage1;
+        stage0.load(held0(it), it.first, owned, g.hd);
+        stage1.load(held1(it), it.first, owned, g.hd_v);
+        stage0.store(base + L::kHeld0, check);
+        stage1.store(base + L::kHeld1, check);
+        fence_async_shared();
+      }
+      warp_arrives(bar(kHeldThere));
+      if (check.bad()) again |= 1u << k;
+    };
+    put_held(it, 0);
+    int t = 0;
+    for (int k = 0;; ++k) {
+      const int mine = it.first + row;  // this thread's row
+      float my_hi = 0.f, my_lo = 0.f, my_delta = 0.f;  // dQ: of this thread's row
+      bool live = mine < owned;
+      if constexpr (kKV) {
+        if (live && g.mask) live = g.mask[it.b * g.t_k + mine] != 0.f;
+      } else if (live) {
+        to_log2(g.lse_in[it.b * g.t_q + mine], my_hi, my_lo);
+        my_delta = g.delta[it.b * g.t_q + mine];
+      }
+      uint64_t acc0[OW / 2], acc1[OW / 2];  // dQ, or dK and dV
+#pragma unroll
+      for (int c = 0; c < OW / 2; ++c) acc0[c] = acc1[c] = 0;
+      auto gather = [&](uint32_t from, uint64_t(&acc)[OW / 2]) {
+        uint32_t o[OW];
+        tmem_ld<OW>(lanes + from + group * OW, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < OW / 2; ++c) acc[c] = f2_add(acc[c], f2_pack_bits(o[2 * c], o[2 * c + 1]));
+      };
+      auto gather_products = [&](int t) {  // of tile t
+        ok = ok && warp_waits(bar(kWeighed), t & 1, g.status, 0x0b22u);
+        if (!ok) return;
+        tc_fence_after_sync();
+        if (kKV) gather(L::kOut1, acc1);
+        gather(L::kOut0, acc0);
+      };
+      Item next = it;
+      bool more = false;
+      for (int j = 0; j < it.tiles; ++j, ++t) {
+        const int x0 = it.begin + j * kStream;
+        if (kKV || g.mask) ok = ok && warp_waits(bar(kStaged0 + place(t, L::kPlaces0)), round(t, L::kPlaces0), g.status, 0x0b20u);
+        ok = ok && warp_waits(bar(kScored), t & 1, g.status, 0x0b21u);
+        if (!ok) break;
+        tc_fence_after_sync();
+        uint32_t s[CW], dp[CW];
+        tmem_ld<CW>(lanes + L::kS + group * CW, s);
+        tmem_ld<CW>(lanes + L::kDp + group * CW, dp);
+        if (j == 0) {  // (every warp has put its held operands in place: the tile has been scored)
+          more = item(k + 1, next);
+          if (more && L::kHeldT) fetch(next);
+          else if (more) prefetch_held(next);
+        }
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        warp_arrives(bar(kFree));
+        int from = 0, to = streamed - x0 - group * CW;
+        if (g.causal) {
+          if (kKV) from = mine - x0 - group * CW;
+          else to = min(to, mine - x0 - group * CW + 1);
+        }
+        uint32_t unseen = outside<CW>(from, live ? to : 0);
+        if (!kKV && g.mask) unseen |= my_hidden<CW>(hidden[place(t, L::kPlaces0)], group);
+        uint64_t p[CW / 2], ds[CW / 2];
+        weigh_scores<CW>(g, s, dp, unseen, [&](int c, uint64_t& hi, uint64_t& lo, uint64_t& delta) {
+          if (kKV) {
+            hi = *reinterpret_cast<const uint64_t*>(&lse_hi[place(t, L::kPlaces0)][group * CW + c]);
+            lo = *reinterpret_cast<const uint64_t*>(&lse_lo[place(t, L::kPlaces0)][group * CW + c]);
+            delta = *reinterpret_cast<const uint64_t*>(&deltas[place(t, L::kPlaces0)][group * CW + c]);
+          } else {
+            hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
+          }
+        }, p, ds);
+        if (j > 0) gather_products(t - 1);
+        if (!ok) break;
+        // (the products of the tile before have been gathered, so its P and dS have been read)
+        Check none;
+        hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, none);
+        if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, none);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        warp_arrives(bar(kHanded));
+      }
+      if (!ok) break;
+      if (more) put_held(next, k + 1);
+      gather_products(t - 1);
+      if (!ok) break;
+      tc_fence_before_sync();
+      Check check;
+      settle(acc0, check);
+      if (check.bad()) again |= 1u << k;
+      const int top = it.first + quarter * 32;
+      if (kKV) {
+        store_rows<OW>(g.dk + it.b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
+        store_rows<OW>(g.dv + it.b * owned * g.hd_v, acc1, top, owned, group * OW, g.hd_v, g.wide_out);
+      } else {
+        store_rows<OW>(g.dq + it.b * owned * g.hd, acc0, top, owned, group * OW, g.hd, g.wide_out);
+      }
+      if (!more) break;
+      it = next;
+    }
+    copy_async_wait();
+  }
+  __syncwarp();
+  if (again != 0) atomicOr(&again_all, again);
+  tc_fence_before_sync();
+  ok = __syncthreads_and(ok);
+  if (ok && again_all != 0 && !abort_flag && warp < kRowWarps) {
+    for (uint32_t left = again_all; left != 0; left &= left - 1)
+      if (item(__ffs(static_cast<int>(left)) - 1, it))
+        rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+  }
+  tear_down<L::kCols, kIssuer>(g, tmem);
 }
 
 // ---- backward at head dims above 64 ----
@@ -1121,16 +1307,19 @@ int launch_sized(Op op, const Problem& p) {
   using F = Fwd<HD, kWide>;
   void (*kernel)(const Params) = f32_fwd_kernel<HD, kWide>;
   uint32_t shared = F::kBytes, threads = F::kThreads;
+  long long grid = blocks;
   if (op != Op::Fwd) {
     if constexpr (HD > 64) {
       using B = BwdWide<HD, kWide>;
       kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
       shared = B::kBytes, threads = B::kThreads;
     } else {
-      using Q = Pipe<HD, false, kWide>;
-      using KV = Pipe<HD, true, kWide>;
       kernel = op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide> : f32_bwd_kernel<HD, true, kWide>;
-      shared = op == Op::BwdQ ? Q::kBytes : KV::kBytes, threads = Q::kThreads;
+      shared = op == Op::BwdQ ? Pipe<HD, false>::kBytes : Pipe<HD, true>::kBytes, threads = kRoleThreads;
+      // every SM has its block, and they are done together: as many blocks to an SM one after the other as the limit on a
+      // block's items asks for
+      const long long turn = static_cast<long long>(sms) * kMostItems;
+      grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
     }
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
@@ -1142,7 +1331,7 @@ int launch_sized(Op op, const Problem& p) {
               "sizing shared memory for a float32 sdpa kernel");
     if (device >= 0 && device < 64) sized[device][static_cast<int>(op)] = true;
   }
-  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks)), dim3(threads), shared, p.stream, g),
+  LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(grid)), dim3(threads), shared, p.stream, g),
             "launching a float32 sdpa kernel");
   note_launches(1);
   return LIMN_B200_OK;

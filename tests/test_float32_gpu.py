@@ -200,3 +200,22 @@ def test_truncated_scores_do_not_show_in_l(t_q, t_k, hd):
     causal = t_q == t_k
     got, want = (f(q, k, v, do, None, causal, hd**-0.5)[1] for f in (_step, _step64))
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 3.2e-8
+
+
+@pytest.mark.parametrize(("bh", "t_q", "t_k", "hd", "hd_v", "causal"), [(4800, 70, 70, 32, 32, True), (4800, 66, 130, 64, 40, False), (300, 200, 200, 37, 33, True),
+                                                                        (100, 257, 257, 64, 64, True), (37, 1000, 65, 24, 24, False)])
+def test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
+    """A block of the kernels that work in roles goes through several work items (one round, several, and more than a block may
+    take): a problem has the same bits wherever it comes, also where the item before or after it leaves the tensor cores (hidden rows of V
+    that do not split) and where the operands are not whole 16-byte pieces."""
+    q, k, v, do = _problem(bh + t_q, bh, t_q, t_k, hd, hd_v)
+    mask = np.ones((bh, t_k), np.float32)
+    mask[:, -1] = 0
+    v[[1, bh // 2, bh - 1], -1] = np.finfo(np.float32).max
+    picks = sorted({0, 1, 2, 147 % bh, 148 % bh, 295 % bh, bh // 2 - 1, bh // 2, bh // 2 + 1, bh - 2, bh - 1})
+    scale = hd**-0.5
+    got = _step(q, k, v, do, mask, causal, scale)
+    alone = _step(q[picks], k[picks], v[picks], do[picks], mask[picks], causal, scale)
+    for g, a, what in zip(got, alone, ("O", "L", "dQ", "dK", "dV")):
+        assert np.isfinite(g[:, :-1]).all(), what
+        assert np.array_equal(g[picks], a), what
