@@ -374,23 +374,21 @@ __device__ __forceinline__ uint32_t my_hidden(const uint32_t* words, int group) 
 
 __device__ __forceinline__ uint32_t align_1024(uint32_t addr) { return (addr + 1023u) & ~1023u; }
 
-// ---- forward ----
+// ---- forward at head dims above 64 ----
 template <int HD, bool kWide>
-struct Fwd {
-  static constexpr int kGroups = HD > 64 ? 4 : 2;  // threads to a row
+struct FwdWide {
+  static constexpr int kGroups = 4;  // threads to a row
   static constexpr int kThreads = kRows * kGroups;
-  static constexpr int kBlocks = HD > 64 ? 1 : 2;  // per SM
   using Held = Stage<HD, kRows, kThreads, kWide>;
   using Tile = Stage<HD, kStream, kThreads, kWide>;
   static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
   static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kS2 = kO + HD;
-  static constexpr bool kTwo = HD > 64;
-  static constexpr int kCols = HD > 64 ? 512 : 256;
+  static constexpr int kCols = 512;
 };
 
 template <int HD, bool kWide>
-__global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlocks) f32_fwd_kernel(const __grid_constant__ Params g) {
-  using L = Fwd<HD, kWide>;
+__global__ void __launch_bounds__(FwdWide<HD, kWide>::kThreads, 1) f32_fwd_wide_kernel(const __grid_constant__ Params g) {
+  using L = FwdWide<HD, kWide>;
   constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, hidden[2][2];
@@ -429,7 +427,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
   fence_async_shared();
   __syncthreads();
   if (issues && elect_one()) {
-    issue_scores<HD, false, L::kTwo>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
+    issue_scores<HD, false, true>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
     mma_commit(scored);
   }
   stage_v.load(v, 0, g.t_k, g.hd_v);
@@ -448,15 +446,11 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
     tc_fence_after_sync();
     uint32_t s[CW];
     tmem_ld<CW>(lanes + L::kS + group * CW, s);
-    if constexpr (L::kTwo) {
-      uint32_t more_s[CW];
-      tmem_ld<CW>(lanes + L::kS2 + group * CW, more_s);
-      tmem_ld_wait();
+    uint32_t more_s[CW];
+    tmem_ld<CW>(lanes + L::kS2 + group * CW, more_s);
+    tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < CW; ++c) s[c] = __float_as_uint(__uint_as_float(s[c]) + __uint_as_float(more_s[c]));
-    } else {
-      tmem_ld_wait();
-    }
+    for (int c = 0; c < CW; ++c) s[c] = __float_as_uint(__uint_as_float(s[c]) + __uint_as_float(more_s[c]));
     int limit = g.t_k - j0;
     if (g.causal) limit = min(limit, i - j0 + 1);
     limit -= group * CW;
@@ -513,7 +507,7 @@ __global__ void __launch_bounds__(Fwd<HD, kWide>::kThreads, Fwd<HD, kWide>::kBlo
       __syncthreads();
       if (issues && elect_one()) {
         tc_fence_after_sync();
-        issue_scores<HD, false, L::kTwo>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
+        issue_scores<HD, false, true>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
         mma_commit(scored);
       }
       stage_v.load(v, j0 + kStream, g.t_k, g.hd_v);
@@ -733,11 +727,324 @@ __device__ __forceinline__ void place_held(uint32_t to, uint32_t at, Check& chec
   }
 }
 
+// A work item: `tiles` tiles of the streamed rows from `begin` on for the own rows from `first` on of problem b.
+struct Item {
+  long long b;
+  int first, begin, tiles;
+};
+
+// The splitting warps' way through a block's items: tile after tile of the two streamed operands into the places of their rings
+// (consecutive ones, HD-wide pieces; ring r's barriers `done` and `staged` lie 8 bytes apart from done_r and staged_r on). `carry` holds the
+// first half already. load_rows(item, row) fetches what goes with a tile's rows, post_rows(place) leaves it in shared memory beside
+// the tile of the first or (kRowsSecond) the second operand: the one whose place is free only when the row warps are done with
+// the tile. Returns the items in which something does not split.
+template <int HD, bool kWide, int kPlaces0, int kPlaces1, bool kRowsSecond, typename Items, typename Source0, typename Source1, typename LoadRows, typename PostRows>
+__device__ __forceinline__ uint32_t split_streams(Carry<HD, kWide>& carry, Item it, bool more, Items item, Source0 stream0, Source1 stream1, int streamed, int width0,
+                                                  int width1, uint32_t done0, uint32_t done1, uint32_t staged0, uint32_t staged1, uint32_t ring0,
+                                                  uint32_t ring1, unsigned* status, bool& ok, LoadRows load_rows, PostRows post_rows) {
+  constexpr uint32_t kTile = 3 * kStream * 128;
+  uint32_t again = 0;
+  int t = 0;
+  if (more) load_rows(it, it.begin);
+  for (int k = 0; ok && more; ++k) {
+    Check check;
+    Item next = it;
+    more = item(k + 1, next);
+    for (int j = 0; j < it.tiles; ++j, ++t) {
+      const int x0 = it.begin + j * kStream, place0 = t % kPlaces0, place1 = t % kPlaces1;
+      if (t >= kPlaces0) ok = ok && warp_waits(done0 + 8 * place0, ((t / kPlaces0) & 1) ^ 1, status, 0x0b30u);
+      if (!ok) break;
+      if (!kRowsSecond) post_rows(place0);
+#pragma unroll
+      for (int n = 0; n < carry.kTurns; ++n) {
+        carry.store(n, ring0 + place0 * kTile, check);
+        carry.load(n, stream1(it), x0, streamed, width1);
+      }
+      fence_async_shared();
+      warp_arrives(staged0 + 8 * place0);
+      if (t >= kPlaces1) ok = ok && warp_waits(done1 + 8 * place1, ((t / kPlaces1) & 1) ^ 1, status, 0x0b31u);
+      if (!ok) break;
+      if (kRowsSecond) post_rows(place1);
+      const bool last = j + 1 == it.tiles;
+      const Item& then = last ? next : it;
+      const int x1 = last ? next.begin : x0 + kStream, rows = last && !more ? 0 : streamed;  // 0: nothing left to load
+      if (rows > 0) load_rows(then, x1);
+      const float* from = stream0(then);
+#pragma unroll
+      for (int n = 0; n < carry.kTurns; ++n) {
+        carry.store(n, ring1 + place1 * kTile, check);
+        carry.load(n, from, x1, rows, width0);
+      }
+      fence_async_shared();
+      warp_arrives(staged1 + 8 * place1);
+    }
+    if (check.bad()) again |= 1u << k;
+    it = next;
+  }
+  return again;
+}
+
+// ---- forward at head dims up to 64 ----
+template <int HD>
+struct Fwd {
+  // tensor memory: scores, the pieces of P, a tile's product, the pieces of Q
+  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kHeldCol = kO + HD;
+  static constexpr int kCols = 512;
+  static_assert(kHeldCol + 3 * HD / 2 <= kCols, "tensor memory");
+  static constexpr int kPlaces0 = 3, kPlaces1 = 3;  // of K and of V
+  static constexpr uint32_t kTile = 3 * kStream * 128;
+  static constexpr uint32_t kTile0 = 0, kTile1 = kPlaces0 * kTile, kHeld = kTile1 + kPlaces1 * kTile, kBytes = kHeld + kRows * HD * 4 + 1024;
+};
+
+template <int HD, bool kWide>
+__global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_constant__ Params g) {
+  using L = Fwd<HD>;
+  constexpr int G = kRowGroups, CW = kStream / G, OW = HD / G;
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ uint32_t slot, abort_flag, again_all, hidden[L::kPlaces1][2];
+  // by the tensor cores: scored, weighed, and a place's tile no longer needed (done0, done1); by the row warps: Q there,
+  // scores read (free), P there (handed); by the splitting warps: a tile there (staged0, staged1)
+  enum { kScored, kWeighed, kHeldThere, kFree, kHanded, kDone0, kDone1 = kDone0 + L::kPlaces0, kStaged0 = kDone1 + L::kPlaces1, kStaged1 = kStaged0 + L::kPlaces0, kBars = kStaged1 + L::kPlaces1 };
+  __shared__ __align__(8) uint64_t bars[kBars];
+  __shared__ float exchange[2][G][kRows];
+  const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < kBars; ++i)
+      mbar_init(smem_addr(bars + i), i >= kStaged0 ? kSplitWarps : i == kHeldThere || i == kFree || i == kHanded ? kRowWarps : 1);
+    mbar_init_fence();
+    again_all = 0;
+  }
+  auto bar = [&](int i) { return smem_addr(bars + i); };
+  auto place = [](int t, int places) { return t % places; };
+  auto round = [](int t, int places) { return static_cast<uint32_t>(t / places) & 1u; };
+  const uint32_t base = align_1024(smem_addr(raw));
+  auto tile0_at = [&](int t) { return base + L::kTile0 + place(t, L::kPlaces0) * L::kTile; };
+  auto tile1_at = [&](int t) { return base + L::kTile1 + place(t, L::kPlaces1) * L::kTile; };
+  auto item = [&](int k, Item& it) {
+    int problem = 0, at = 0;
+    if (!work_item(g, k, problem, at)) return false;
+    it.b = problem;
+    it.first = (g.slots - 1 - at) * kRows;  // long causal rows first
+    it.begin = 0;
+    it.tiles = ((g.causal ? min(g.t_k, it.first + kRows) : g.t_k) + kStream - 1) / kStream;
+    return true;
+  };
+  const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+  const uint32_t raw_q = base + L::kHeld + warp * (32 * OW * 4);
+  auto fetch = [&](const Item& it) { fetch_held<HD, kWide>(raw_q, g.q + it.b * g.t_q * g.hd, it.first + quarter * 32, g.t_q, group * OW, g.hd); };
+  auto keys = [&](const Item& it) { return g.k + it.b * g.t_k * g.hd; };
+  auto values = [&](const Item& it) { return g.v + it.b * g.t_k * g.hd_v; };
+
+  Item it;
+  const bool any = item(0, it);
+  grid_dependency_wait();
+  if (warp == kIssuer) {
+    tmem_alloc(smem_addr(&slot), L::kCols);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk;
+  // the first operands set out before the block is set up
+  Carry<HD, kWide> carry(threadIdx.x - kRowThreads);
+  if (any && warp < kRowWarps) {
+    fetch(it);
+  } else if (any && warp < kIssuer) {
+#pragma unroll
+    for (int n = 0; n < carry.kTurns; ++n) carry.load(n, keys(it), 0, g.t_k, g.hd);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(kFull, slot, 0);
+  bool ok = true;
+  uint32_t again = 0;  // items in which this thread met something that does not split
+  if (abort_flag) {
+    // an earlier kernel on this device gave up on a wait: take no work
+    copy_async_wait();
+  } else if (warp == kIssuer) {
+    // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
+    grid_launch_dependents();
+    int t = 0;  // tiles so far
+    auto weigh = [&](int t) {
+      ok = ok && warp_waits(bar(kStaged1 + place(t, L::kPlaces1)), round(t, L::kPlaces1), g.status, 0x0a14u);
+      ok = ok && warp_waits(bar(kHanded), t & 1, g.status, 0x0a12u);
+      if (!ok) return;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        issue_weigh<HD>(tmem + L::kO, tmem + L::kP, tile1_at(t));
+        mma_commit(bar(kWeighed));
+        mma_commit(bar(kDone1 + place(t, L::kPlaces1)));
+      }
+      __syncwarp();
+    };
+    for (int k = 0; ok && item(k, it); ++k) {
+      ok = warp_waits(bar(kHeldThere), k & 1, g.status, 0x0a13u);
+      for (int j = 0; ok && j < it.tiles; ++j, ++t) {
+        ok = warp_waits(bar(kStaged0 + place(t, L::kPlaces0)), round(t, L::kPlaces0), g.status, 0x0a10u);
+        if (t > 0) ok = ok && warp_waits(bar(kFree), (t - 1) & 1, g.status, 0x0a11u);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_scores<HD, true>(tmem + L::kS, tmem + L::kHeldCol, tile0_at(t));
+          mma_commit(bar(kScored));
+          mma_commit(bar(kDone0 + place(t, L::kPlaces0)));
+        }
+        __syncwarp();
+        if (j > 0) weigh(t - 1);
+      }
+      if (ok) weigh(t - 1);
+    }
+  } else if (warp >= kRowWarps) {
+    // ================= splitting warps =================
+    const int thread = threadIdx.x - kRowThreads;
+    float flag = 0.f;
+    again = split_streams<HD, kWide, L::kPlaces0, L::kPlaces1, true>(
+        carry, it, any, item, keys, values, g.t_k, g.hd, g.hd_v, bar(kDone0), bar(kDone1), bar(kStaged0), bar(kStaged1), base + L::kTile0, base + L::kTile1, g.status, ok,
+        [&](const Item& it, int x0) {
+          if (g.mask) flag = row_value(g.mask + it.b * g.t_k, x0, g.t_k, thread);
+        },
+        [&](int place) {
+          if (g.mask) post_hidden(hidden[place], flag, thread);
+        });
+  } else if (any) {
+    // ================= row warps =================
+    // A warp that gave up on a wait waits for nothing any more but goes through its tiles like the others: the four warps that share
+    // rows meet at a barrier in each.
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    auto meet = [&] { named_barrier_sync(1 + quarter, 32 * G); };
+    auto put_held = [&](int k) {  // Q of item k, which has been fetched
+      Check check;
+      copy_async_wait();
+      __syncwarp();
+      place_held<HD>(lanes + L::kHeldCol + group * (OW / 2), raw_q, check);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      warp_arrives(bar(kHeldThere));
+      if (check.bad()) again |= 1u << k;
+    };
+    put_held(0);
+    const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo);
+    int t = 0;
+    for (int k = 0;; ++k) {
+      const int i = it.first + row;
+      float top = -INFINITY, shift = 0.f, denom = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
+      float shrink = 0.f;                               // what the sums so far are multiplied with when the last tile's product comes
+      uint64_t acc[OW / 2];
+#pragma unroll
+      for (int c = 0; c < OW / 2; ++c) acc[c] = 0;
+      auto gather_product = [&](int t) {  // of tile t
+        ok = ok && warp_waits(bar(kWeighed), t & 1, g.status, 0x0a22u);
+        tc_fence_after_sync();
+        uint32_t o[OW];
+        tmem_ld<OW>(lanes + L::kO + group * OW, o);
+        tmem_ld_wait();
+        const uint64_t shrink2 = f2_pack(shrink, shrink);
+#pragma unroll
+        for (int c = 0; c < OW / 2; ++c) acc[c] = f2_fma(acc[c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
+      };
+      Item next = it;
+      bool more = false;
+      for (int j = 0; j < it.tiles; ++j, ++t) {
+        const int j0 = j * kStream;
+        if (g.mask) ok = ok && warp_waits(bar(kStaged1 + place(t, L::kPlaces1)), round(t, L::kPlaces1), g.status, 0x0a20u);
+        ok = ok && warp_waits(bar(kScored), t & 1, g.status, 0x0a21u);
+        tc_fence_after_sync();
+        uint32_t s[CW];
+        tmem_ld<CW>(lanes + L::kS + group * CW, s);
+        if (j == 0) {
+          more = item(k + 1, next);
+          if (more) fetch(next);
+        }
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        warp_arrives(bar(kFree));
+        int limit = g.t_k - j0;
+        if (g.causal) limit = min(limit, i - j0 + 1);
+        limit -= group * CW;
+        uint32_t unseen = limit >= CW ? 0u : limit <= 0 ? kFull : ~((1u << limit) - 1u);
+        if (g.mask) unseen |= my_hidden<CW>(hidden[place(t, L::kPlaces1)], group);
+        if (unseen != 0u) {
+#pragma unroll
+          for (int c = 0; c < CW; ++c)
+            if ((unseen >> c) & 1u) s[c] = 0xff800000u;
+        }
+        float tile_top = -INFINITY;
+#pragma unroll
+        for (int c = 0; c < CW; c += 2) tile_top = max3(tile_top, __uint_as_float(s[c]), __uint_as_float(s[c + 1]));
+        exchange[t & 1][group][row] = tile_top;
+        meet();
+        float raised = top;
+#pragma unroll
+        for (int c = 0; c < G; ++c) raised = fmaxf(raised, exchange[t & 1][c][row]);
+        const float moved = raised == -INFINITY ? 0.f : raised * g.c_hi;
+        const float less = top == -INFINITY ? 0.f : exp2_approx(shift - moved);  // nothing gathered yet: nothing to rescale
+        top = raised, shift = moved;
+        const uint64_t minus_shift = f2_pack(-shift, -shift);
+        uint64_t w[CW / 2];
+        uint64_t sum = 0;
+#pragma unroll
+        for (int c = 0; c < CW / 2; ++c) {
+          const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
+          float x0, x1;
+          f2_unpack(f2_fma(s2, c_lo, f2_fma(s2, c_hi, minus_shift)), x0, x1);
+          w[c] = f2_pack(exp2_approx(x0), exp2_approx(x1));
+          sum = f2_add(sum, w[c]);
+        }
+        float sum0, sum1;
+        f2_unpack(sum, sum0, sum1);
+        denom = fmaf(denom, less, sum0 + sum1);  // this thread's share; the shares meet after the last tile
+        if (j > 0) gather_product(t - 1);
+        shrink = less;
+        // (the product of the tile before has been gathered, so its P has been read)
+        Check none;
+        hand_over<CW>(lanes + L::kP + group * (CW / 2), w, none);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        warp_arrives(bar(kHanded));
+      }
+      if (more) put_held(k + 1);
+      gather_product(t - 1);
+      tc_fence_before_sync();
+      if (!(denom < INFINITY)) again |= 1u << k;
+      exchange[t & 1][group][row] = denom;
+      meet();
+      float total = 0.f;
+#pragma unroll
+      for (int c = 0; c < G; ++c) total += exchange[t & 1][c][row];
+      meet();  // (the next item's first maxima may go there)
+      if (ok) {
+#pragma unroll
+        for (int c = 0; c < OW / 2; ++c) {
+          float x0, x1;
+          f2_unpack(acc[c], x0, x1);
+          acc[c] = f2_pack(x0 / total, x1 / total);  // 0/0 = NaN for a row with no key, as the oracle has it
+        }
+        store_rows<OW>(g.out + it.b * g.t_q * g.hd_v, acc, it.first + quarter * 32, g.t_q, group * OW, g.hd_v, g.wide_out);
+        // once per row, so in double: L is then as good as its sum
+        if (group == 0 && i < g.t_q)
+          g.lse_out[it.b * g.t_q + i] =
+              top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
+      }
+      if (!more) break;
+      it = next;
+    }
+  }
+  __syncwarp();
+  if (again != 0) atomicOr(&again_all, again);
+  tc_fence_before_sync();
+  ok = __syncthreads_and(ok);
+  if (ok && again_all != 0 && !abort_flag && warp < kRowWarps) {
+    for (uint32_t left = again_all; left != 0; left &= left - 1)
+      if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+  }
+  tear_down<L::kCols, kIssuer>(g, tmem);
+}
+
 // ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
 // A tile's scores are computed while the row warps are at the tile before it, and its products are gathered while the next tile's
 // are: a row warp comes to each of its waits with the answer there, as long as the tensor cores keep up.
 template <int HD, bool kKV>
-struct Pipe {
+struct Bwd {
   // tensor memory: scores, dP, the pieces of dS and (dK/dV) of P, a tile's products, and the held operands if they fit:
   // they are the A side of the scores, an MMA then only reads the streamed tile from shared memory (whose bandwidth
   // bounds it at 48 clocks with both there, for 32)
@@ -756,7 +1063,7 @@ struct Pipe {
 
 template <int HD, bool kKV, bool kWide>
 __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
-  using L = Pipe<HD, kKV>;
+  using L = Bwd<HD, kKV>;
   using Held = Stage<HD, kRows, kRowThreads, kWide>;
   constexpr int CW = kStream / kRowGroups, OW = HD / kRowGroups;
   extern __shared__ __align__(16) unsigned char raw[];
@@ -783,10 +1090,6 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
 
   // the held pair (against which the tiles are scored) and the streamed pair
   const int owned = kKV ? g.t_k : g.t_q, streamed = kKV ? g.t_q : g.t_k;
-  struct Item {
-    long long b;
-    int first, begin, tiles;  // first own row; first streamed row, tiles of them
-  };
   auto item = [&](int k, Item& it) {
     int problem = 0, at = 0;
     if (!work_item(g, k, problem, at)) return false;
@@ -889,64 +1192,30 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   } else if (warp >= kRowWarps) {
     // ================= splitting warps =================
     const int thread = threadIdx.x - kRowThreads;
-    const float* mask = g.mask;
     float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
-    auto load_rows = [&](const Item& it, int x0) {
-      if (kKV) {
-        row_a = row_value(g.lse_in + it.b * g.t_q, x0, streamed, thread);
-        row_b = row_value(g.delta + it.b * g.t_q, x0, streamed, thread);
-      } else if (mask) {
-        row_a = row_value(mask + it.b * g.t_k, x0, streamed, thread);
-      }
-    };
-    if (any) load_rows(it, it.begin);
-    int t = 0;
-    bool more = any;
-    for (int k = 0; ok && more; ++k) {
-      Check check;
-      Item next = it;
-      more = item(k + 1, next);
-      for (int j = 0; j < it.tiles; ++j, ++t) {
-        const int x0 = it.begin + j * kStream;
-        if (t >= L::kPlaces0) ok = ok && warp_waits(bar(kDone0 + place(t, L::kPlaces0)), round(t, L::kPlaces0) ^ 1u, g.status, 0x0b30u);
-        if (!ok) break;
-        if (kKV) {
-          if (thread < kStream) {
-            float hi, lo;
-            to_log2(row_a, hi, lo);
-            lse_hi[place(t, L::kPlaces0)][thread] = hi;
-            lse_lo[place(t, L::kPlaces0)][thread] = lo;
-            deltas[place(t, L::kPlaces0)][thread] = row_b;
+    again = split_streams<HD, kWide, L::kPlaces0, L::kPlaces1, false>(
+        carry, it, any, item, stream0, stream1, streamed, g.hd, g.hd_v, bar(kDone0), bar(kDone1), bar(kStaged0), bar(kStaged1), base + L::kTile0, base + L::kTile1, g.status, ok,
+        [&](const Item& it, int x0) {
+          if (kKV) {
+            row_a = row_value(g.lse_in + it.b * g.t_q, x0, streamed, thread);
+            row_b = row_value(g.delta + it.b * g.t_q, x0, streamed, thread);
+          } else if (g.mask) {
+            row_a = row_value(g.mask + it.b * g.t_k, x0, streamed, thread);
           }
-        } else if (mask) {
-          post_hidden(hidden[place(t, L::kPlaces0)], row_a, thread);
-        }
-#pragma unroll
-        for (int n = 0; n < carry.kTurns; ++n) {
-          carry.store(n, tile0_at(t), check);
-          carry.load(n, stream1(it), x0, streamed, g.hd_v);
-        }
-        fence_async_shared();
-        warp_arrives(bar(kStaged0 + place(t, L::kPlaces0)));
-        if (t >= L::kPlaces1) ok = ok && warp_waits(bar(kDone1 + place(t, L::kPlaces1)), round(t, L::kPlaces1) ^ 1u, g.status, 0x0b31u);
-        if (!ok) break;
-        const bool last = j + 1 == it.tiles;
-        const Item& then = last ? next : it;
-        const int x1 = last ? next.begin : x0 + kStream;
-        const float* from = stream0(then);
-        const int rows = last && !more ? 0 : streamed;  // nothing left to load
-        if (rows > 0) load_rows(then, x1);
-#pragma unroll
-        for (int n = 0; n < carry.kTurns; ++n) {
-          carry.store(n, tile1_at(t), check);
-          carry.load(n, from, x1, rows, g.hd);
-        }
-        fence_async_shared();
-        warp_arrives(bar(kStaged1 + place(t, L::kPlaces1)));
-      }
-      if (check.bad()) again |= 1u << k;
-      it = next;
-    }
+        },
+        [&](int place) {
+          if (kKV) {
+            if (thread < kStream) {
+              float hi, lo;
+              to_log2(row_a, hi, lo);
+              lse_hi[place][thread] = hi;
+              lse_lo[place][thread] = lo;
+              deltas[place][thread] = row_b;
+            }
+          } else if (g.mask) {
+            post_hidden(hidden[place], row_a, thread);
+          }
+        });
   } else if (any) {
     // ================= row warps =================
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -1304,23 +1573,21 @@ int launch_sized(Op op, const Problem& p) {
   int sms = 0;
   if (int rc = sm_count(&sms)) return rc;
   g.group = work_group(p, blocks, sms);
-  using F = Fwd<HD, kWide>;
-  void (*kernel)(const Params) = f32_fwd_kernel<HD, kWide>;
-  uint32_t shared = F::kBytes, threads = F::kThreads;
+  void (*kernel)(const Params) = nullptr;
+  uint32_t shared = 0, threads = 0;
   long long grid = blocks;
-  if (op != Op::Fwd) {
-    if constexpr (HD > 64) {
-      using B = BwdWide<HD, kWide>;
-      kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
-      shared = B::kBytes, threads = B::kThreads;
-    } else {
-      kernel = op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide> : f32_bwd_kernel<HD, true, kWide>;
-      shared = op == Op::BwdQ ? Pipe<HD, false>::kBytes : Pipe<HD, true>::kBytes, threads = kRoleThreads;
-      // every SM has its block, and they are done together: as many blocks to an SM one after the other as the limit on a
-      // block's items asks for
-      const long long turn = static_cast<long long>(sms) * kMostItems;
-      grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
-    }
+  if constexpr (HD > 64) {
+    using F = FwdWide<HD, kWide>;
+    using B = BwdWide<HD, kWide>;
+    kernel = op == Op::Fwd ? f32_fwd_wide_kernel<HD, kWide> : op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
+    shared = op == Op::Fwd ? F::kBytes : B::kBytes, threads = B::kThreads;
+  } else {
+    kernel = op == Op::Fwd ? f32_fwd_kernel<HD, kWide> : op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide> : f32_bwd_kernel<HD, true, kWide>;
+    shared = op == Op::Fwd ? Fwd<HD>::kBytes : op == Op::BwdQ ? Bwd<HD, false>::kBytes : Bwd<HD, true>::kBytes, threads = kRoleThreads;
+    // every SM has its block, and they are done together: as many blocks to an SM one after the other as the limit on a
+    // block's items asks for
+    const long long turn = static_cast<long long>(sms) * kMostItems;
+    grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64][3] = {};
