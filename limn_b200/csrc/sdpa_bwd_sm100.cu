@@ -68,6 +68,15 @@ constexpr float kLog2e = 1.4426950408889634f;
 #endif
 constexpr int kPolyPairsOf8 = LIMN_BWD_POLY_PAIRS;
 
+// How results that are not tile-stored leave. Measured, us, every thread its own row / pieces of neighbouring rows exchanged first / staged
+// by the warp: dQ of 192 padded problems of 500 x 64 41.8 / 39.7 / 40.1; causal at head dim 64, 256 of 256 18.5 / 19.0 / 18.7 and 64 of 1024
+// 26.5 / - / 27.0 (but 256 of 128 11.5 / 11.1 / 11.1); head dim 128, where shared memory has no room, 160 causal of 3000 and 128 of 1024
+// dQ 531 / 517 and 105 / 101, dK and dV 684 / 658 and 133 / 125.
+template <int D, bool kCausal>
+constexpr RowStore row_store() {
+  return D == 128 ? RowStore::kExchanged : kCausal ? RowStore::kOwn : RowStore::kStaged;
+}
+
 template <int D, bool kKV, bool kMask>
 struct BwdLayout {
   static constexpr int kTileBytes = kTile * D * 2;
@@ -86,7 +95,9 @@ struct BwdLayout {
   // cost as much as they save (+2 % at S = 2048), so it keeps storing from registers.
   static constexpr bool kTileStore = D == 64 && kKV;
   static constexpr int kStoreOff = kStreamBOff + kStagesB * kTileBytes;
-  static constexpr int kStatOff = kStoreOff + (kTileStore ? (kKV ? 2 : 1) * kAtomBytes : 0);
+  // The others: see row_store.
+  static constexpr int kWarpStage = D == 64 && !kKV ? 2048 : 0;  // of each elementwise warp, for 32 columns of its rows
+  static constexpr int kStatOff = kStoreOff + (kTileStore ? (kKV ? 2 : 1) * kAtomBytes : 8 * kWarpStage);
   static constexpr int kBarOff = kStatOff + (kKV ? 8 * 2 * 2 * 64 * 4 : 0);  // dK/dV pass, per warp [2 buffers][128 floats]: statistics of the streamed queries
   static constexpr int kBytes = kBarOff + 512 + 1024;
   static_assert(kBytes <= 227 * 1024, "shared memory per CTA");
@@ -161,24 +172,6 @@ struct BwdParams {
   int q_tiles, kv_tiles;
   float scale;
 };
-
-// One accumulator row slice (32 fp32 columns) scaled, rounded and written as 64 bytes, or as many 16-byte pieces
-// of them as the row has columns left.
-template <bool kFp16>
-__device__ __forceinline__ void store_row32(void* base, long long elem_offset, const uint32_t (&acc)[32], float mul, int cols_left) {
-  uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(base) + elem_offset * 2);
-#pragma unroll
-  for (int v4 = 0; v4 < 4; ++v4) {
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float a = __uint_as_float(acc[v4 * 8 + 2 * i]) * mul;
-      const float b = __uint_as_float(acc[v4 * 8 + 2 * i + 1]) * mul;
-      w[i] = kFp16 ? pack_f16(a, b) : pack_bf16(a, b);
-    }
-    if (8 * v4 < cols_left) dst[v4] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
 
 // sum_d a[d] * b[d] over one row of `pieces` * 8 <= D 16-bit elements each, in fp32 (four partial sums): the delta
 // of one query row from its O and dO rows (limn/tensor.py:705-706).
@@ -966,33 +959,37 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
     } else if (ok) {
       tc_fence_after_sync();
-      const int row = own0 + r;
+      const int top = own0 + (warp & 3) * 32;  // the warp's first row
       if (kKV) {
-        // group 0 writes this key's dV row, group 1 its dK row
-        const bool in = row < prm.t_k;
+        // group 0 writes its keys' dV rows, group 1 their dK rows
         const Strides& mine = group == 0 ? prm.out1_strides : prm.out_strides;
-        const long long out_at = item.batch * mine.batch + item.head * mine.head + row * mine.row;
+        unsigned char* to = static_cast<unsigned char*>(group == 0 ? prm.out1 : prm.out0) + 2 * (item.batch * mine.batch + item.head * mine.head + top * mine.row);
         const uint32_t t_acc = tmem + lane_base + (group == 0 ? L::kAcc0 : L::kAcc1);
-        void* dst = group == 0 ? prm.out1 : prm.out0;
         const float mul = group == 0 ? 1.f : prm.scale;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t acc[32];
           tmem_ld32(t_acc + 32 * c, acc);
           tmem_ld_wait();
-          if (in) store_row32<kFp16>(dst, out_at + 32 * c, acc, mul, (group == 0 ? prm.width_v : prm.width) - 32 * c);
+          store_rows32<kFp16, RowStore::kExchanged>(to + 64 * c, 2 * mine.row, top, prm.t_k, acc, mul, (group == 0 ? prm.width_v : prm.width) - 32 * c);
         }
       } else {
-        // each group writes half of this query's dQ row
+        // each group writes half of its queries' dQ rows
+        const int row = own0 + r;
         const bool in = row < prm.t_q;
         const long long out_at = item.batch * prm.out_strides.batch + item.head * prm.out_strides.head + row * prm.out_strides.row;
+        unsigned char* to = static_cast<unsigned char*>(prm.out0) + 2 * (item.batch * prm.out_strides.batch + item.head * prm.out_strides.head + top * prm.out_strides.row);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
           const int col = group * (D / 2) + 32 * c;
           uint32_t acc[32];
           tmem_ld32(tmem + lane_base + L::kAcc0 + col, acc);
           tmem_ld_wait();
-          if (in) store_row32<kFp16>(prm.out0, out_at + col, acc, prm.scale, prm.width - col);
+          if constexpr (row_store<D, kCausal>() == RowStore::kOwn) {
+            if (in) store_row32<kFp16>(static_cast<unsigned char*>(prm.out0) + 2 * (out_at + col), acc, prm.scale, prm.width - col);
+          } else {
+            store_rows32<kFp16, row_store<D, kCausal>()>(to + 2 * col, 2 * prm.out_strides.row, top, prm.t_q, acc, prm.scale, prm.width - col, base + L::kStoreOff + warp * L::kWarpStage);
+          }
         }
       }
       // the accumulators are in registers or stored: the next item's first products may overwrite them

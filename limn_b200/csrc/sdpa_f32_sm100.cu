@@ -225,31 +225,8 @@ __device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2
   tmem_st<N / 2>(at + 2 * kPieceCols, l);
 }
 
-// B lanes of a warp (B = 2 or 4) hold B pieces of 16 bytes each of a row of their own; afterwards x[r] is piece (lane % B) of the
-// row of lane r of the B.
-template <int B>
-__device__ __forceinline__ void swap_rows_for_pieces(float (&x)[B][4]) {
-  const uint32_t lane = lane_id();
-#pragma unroll
-  for (int d = 1; d < B; d *= 2) {
-    const bool upper = (lane & d) != 0;
-#pragma unroll
-    for (int i = 0; i < B; ++i) {
-      if (i & d) continue;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float got = __shfl_xor_sync(kFull, upper ? x[i][c] : x[i | d][c], d);
-        if (upper) x[i][c] = got;
-        else x[i | d][c] = got;
-      }
-    }
-  }
-}
-
-// The N columns from `col` on of a warp's 32 rows from `first` on, a row to a thread, into a matrix of (rows, width). A row's
-// own 16-byte pieces, stored one after the other, are 32 lines of memory an instruction, and the load/store unit takes a clock for
-// each (a block's 128 x 64 results 2 000 to 6 000 clocks); with the pieces of B neighbouring rows exchanged first, an instruction
-// writes 64 bytes (N = 8: 32) of each row it touches.
+// The N columns from `col` on of a warp's 32 rows from `first` on, a row to a thread, into a matrix of (rows, width), rows exchanged
+// for pieces (a block's 128 x 64 results took 2 000 to 6 000 clocks without).
 template <int N>
 __device__ __forceinline__ void store_rows(float* dst, const uint64_t (&acc)[N / 2], int first, int rows, int col, int width, bool wide) {
   const int lane = static_cast<int>(lane_id());
@@ -258,17 +235,20 @@ __device__ __forceinline__ void store_rows(float* dst, const uint64_t (&acc)[N /
     const int top = first + (lane & ~(B - 1)), at = col + 4 * (lane & (B - 1));
 #pragma unroll
     for (int set = 0; set < N / 4; set += B) {
-      float x[B][4];
+      uint32_t x[B][4];
 #pragma unroll
-      for (int i = 0; i < B; ++i) {
-        f2_unpack(acc[2 * (set + i)], x[i][0], x[i][1]);
-        f2_unpack(acc[2 * (set + i) + 1], x[i][2], x[i][3]);
-      }
+      for (int i = 0; i < B; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float a, b;
+          f2_unpack(acc[2 * (set + i) + c], a, b);
+          x[i][2 * c] = __float_as_uint(a), x[i][2 * c + 1] = __float_as_uint(b);
+        }
       swap_rows_for_pieces<B>(x);
 #pragma unroll
       for (int r = 0; r < B; ++r)
         if (top + r < rows && at + 4 * set < width)
-          *reinterpret_cast<float4*>(dst + static_cast<long long>(top + r) * width + at + 4 * set) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
+          *reinterpret_cast<uint4*>(dst + static_cast<long long>(top + r) * width + at + 4 * set) = make_uint4(x[r][0], x[r][1], x[r][2], x[r][3]);
     }
   } else if (first + lane < rows) {
     float* row = dst + static_cast<long long>(first + lane) * width;

@@ -342,6 +342,29 @@ __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
   return r;
 }
 
+// B lanes of a warp (B = 2 or 4) hold B pieces of 16 bytes each of a row of their own; afterwards x[r] is piece (lane % B) of the
+// row of lane r of the B. For results a thread has a row (or part) of: a row's own pieces, stored one after the other, are 32 lines of
+// memory an instruction, and the load/store unit takes a clock for each of them; with the pieces of B neighbouring rows exchanged
+// first, an instruction writes 16 B bytes of each row it touches.
+template <int B>
+__device__ __forceinline__ void swap_rows_for_pieces(uint32_t (&x)[B][4]) {
+  const uint32_t lane = lane_id();
+#pragma unroll
+  for (int d = 1; d < B; d *= 2) {
+    const bool upper = (lane & d) != 0;
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      if (i & d) continue;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? x[i][c] : x[i | d][c], d);
+        if (upper) x[i][c] = got;
+        else x[i | d][c] = got;
+      }
+    }
+  }
+}
+
 // h - x, h being the bfloat16 in the low or high half of `pair`: the mixed-precision subtraction reads the half-word as it lies.
 __device__ __forceinline__ float sub_bf16_lo(uint32_t pair, float x) {
   float r;
@@ -429,6 +452,62 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float& lo, float& hi) {
   f2_unpack(t2, t0, t1);
   const uint32_t two = 0x40000000u;
   f2_unpack(f2_mul_ftz(p2, f2_pack_bits((__float_as_uint(t0) << 23) + two, (__float_as_uint(t1) << 23) + two)), lo, hi);
+}
+
+// How a warp writes 32 columns of its 32 rows, a row to a thread: every thread its own row's pieces, neighbouring rows' pieces exchanged
+// first, or by way of 2 KB of shared memory of the warp's own.
+enum class RowStore { kOwn, kExchanged, kStaged };
+// Own: 32 fp32 columns of a row times `mul`, rounded and written as 64 bytes, or as many 16-byte pieces of them as the row has columns
+// left (a multiple of 8).
+template <bool kFp16>
+__device__ __forceinline__ void store_row32(void* to, const uint32_t (&o)[32], float mul, int cols_left) {
+  uint4* at = static_cast<uint4*>(to);
+#pragma unroll
+  for (int v4 = 0; v4 < 4; ++v4) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = __uint_as_float(o[v4 * 8 + 2 * i]) * mul, b = __uint_as_float(o[v4 * 8 + 2 * i + 1]) * mul;
+      w[i] = kFp16 ? pack_f16(a, b) : pack_bf16(a, b);
+    }
+    if (8 * v4 < cols_left) at[v4] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+// The others: to rows [first, first + 32) of a 16-bit matrix of `rows` rows: `to` is where row `first` has them, `row_bytes`
+// the distance between rows, `cols_left` how many of the columns there are (a multiple of 8). Every lane takes part.
+template <bool kFp16, RowStore kHow>
+__device__ __forceinline__ void store_rows32(unsigned char* to, long long row_bytes, int first, int rows, const uint32_t (&o)[32], float mul, int cols_left, uint32_t stage = 0) {
+  uint32_t w[4][4];
+#pragma unroll
+  for (int v4 = 0; v4 < 4; ++v4)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = __uint_as_float(o[v4 * 8 + 2 * i]) * mul, b = __uint_as_float(o[v4 * 8 + 2 * i + 1]) * mul;
+      w[v4][i] = kFp16 ? pack_f16(a, b) : pack_bf16(a, b);
+    }
+  const int lane = static_cast<int>(lane_id());
+  static_assert(kHow != RowStore::kOwn);
+  if constexpr (kHow == RowStore::kExchanged) {
+    swap_rows_for_pieces<4>(w);
+    const int top = lane & ~3, piece = lane & 3;
+    unsigned char* at = to + top * row_bytes + 16 * piece;
+#pragma unroll
+    for (int r = 0; r < 4; ++r, at += row_bytes)
+      if (first + top + r < rows && 8 * piece < cols_left) *reinterpret_cast<uint4*>(at) = make_uint4(w[r][0], w[r][1], w[r][2], w[r][3]);
+  } else {
+    auto place = [&](int row, int piece) { return stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)); };  // 8 rows' pieces on distinct banks
+#pragma unroll
+    for (int v4 = 0; v4 < 4; ++v4) st_shared_v4(place(lane, v4), w[v4][0], w[v4][1], w[v4][2], w[v4][3]);
+    __syncwarp();
+    const int top = lane >> 2, piece = lane & 3;
+    unsigned char* at = to + top * row_bytes + 16 * piece;
+#pragma unroll
+    for (int r = 0; r < 32; r += 8, at += 8 * row_bytes) {
+      uint4 x;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(place(r + top, piece)) : "memory");
+      if (first + r + top < rows && 8 * piece < cols_left) *reinterpret_cast<uint4*>(at) = x;
+    }
+  }
 }
 
 // Which (problem, slot) work item `index` is. Items are fetched in index order, so the order is the schedule:
