@@ -597,15 +597,17 @@ __device__ __forceinline__ uint32_t outside(int from, int to) {
   return unseen;
 }
 
-// ---- the kernels that work in roles: sixteen row warps, three splitting warps, one issuing warp ----
-// Four row threads to a row take scores out of tensor memory, turn them into weights, split those and sum a tile's products; the
+// ---- the kernels that work in roles: row warps, splitting warps, one issuing warp ----
+// Two or four row threads to a row take scores out of tensor memory, turn them into weights, split those and sum a tile's products; the
 // splitting warps bring the streamed operands into shared memory in pieces, a few tiles ahead; the issuing warp issues every MMA.
 // The roles meet at mbarriers whose waits are bounded; no barrier of the block stands inside their loops, so a warp that gave up on a
 // wait cannot hang the others. A block goes through several work items: the splitting warps run ahead into the next item while the
 // row warps end this one.
-constexpr int kRowWarps = 16, kSplitWarps = 3, kIssuer = kRowWarps + kSplitWarps;
-constexpr int kRowThreads = 32 * kRowWarps, kSplitThreads = 32 * kSplitWarps, kRoleThreads = 32 * (kIssuer + 1);
-constexpr int kRowGroups = kRowThreads / kRows;  // threads to a row
+template <int kGroups>
+struct Roles {  // kGroups threads to a row, the other warps by what registers are left
+  static constexpr int kRowWarps = 4 * kGroups, kSplitWarps = kGroups == 4 ? 3 : 7, kIssuer = kRowWarps + kSplitWarps;
+  static constexpr int kRowThreads = 32 * kRowWarps, kSplitThreads = 32 * kSplitWarps, kThreads = 32 * (kIssuer + 1);
+};
 constexpr int kMostItems = 32;                   // work items of a block: each has a bit of a word
 
 // Work item `k` of this block. Blocks take turns, there and back: items are in the order of their length under a causal mask, and a
@@ -619,13 +621,13 @@ __device__ __forceinline__ bool work_item(const Params& g, int k, int& problem, 
 
 // What the splitting warps carry from global memory to pieces in shared memory, half a streamed tile (one operand) at a time, and in
 // registers meanwhile: a thread that has split one of its eighths of a row loads the next half's in its place.
-template <int HD, bool kWide>
+template <int HD, int kThreads, bool kWide>
 struct Carry {
-  static constexpr int kChunks = HD / 8, kStep = kSplitThreads / kChunks;  // rows from one turn to the next
+  static constexpr int kChunks = HD / 8, kStep = kThreads / kChunks;  // rows from one turn to the next
   static constexpr int kTurns = (kStream + kStep - 1) / kStep;
-  static constexpr int kHalves = HD > 32 ? 1 : 2;  // that a thread's registers hold: with two, each operand's next tile is under way
+  static constexpr int kHalves = kTurns > 3 ? 1 : 2;  // that a thread's registers hold: with two, each operand's next tile is under way
   static constexpr uint32_t kPiece = kStream * 128;
-  static_assert(HD <= 64 && kSplitThreads % kChunks == 0 && kStep % 4 == 0, "a thread keeps its columns");
+  static_assert(HD <= 64 && kThreads % kChunks == 0 && kStep % 4 == 0, "a thread keeps its columns");
   float x[kTurns][8];
   int row, column;    // of the first turn
   uint32_t where[2];  // of the first turn's pieces in a tile; of the second's, less the rows between them
@@ -710,45 +712,48 @@ __device__ __forceinline__ void copy_async16(uint32_t dst, const float* src, int
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Where a row warp's part of a held operand (its 32 rows, its group's HD / 4 columns) waits, as float32, for its turn in tensor
+// Where a row warp's part of a held operand (its 32 rows, its group's OW columns) waits, as float32, for its turn in tensor
 // memory: only that warp touches it. 16-byte piece p of row r; eight rows' pieces lie on distinct banks.
-template <int HD>
+template <int OW>
 __device__ __forceinline__ uint32_t held_piece(uint32_t at, int r, int p) {
-  constexpr int kPieces = HD / 16;  // of a row
-  static_assert(kPieces == 4 || kPieces == 2, "head dims 64 and 32");
-  const int where = kPieces == 4 ? p ^ ((r >> 1) & 3) : p ^ ((r >> 2) & 1);
+  constexpr int kPieces = OW / 4;  // of a row
+  static_assert(kPieces == 8 || kPieces == 4 || kPieces == 2, "a row's part is 32 to 128 bytes");
+  const int where = kPieces == 8 ? p ^ (r & 7) : kPieces == 4 ? p ^ ((r >> 1) & 3) : p ^ ((r >> 2) & 1);
   return at + static_cast<uint32_t>(r * kPieces + where) * 16u;
 }
-template <int HD, bool kWide>
+template <int OW, bool kWide>
 __device__ __forceinline__ void fetch_held(uint32_t at, const float* src, int first, int rows, int col, int width) {
-  constexpr int kPieces = HD / 16;
+  constexpr int kPieces = OW / 4;
   const int lane = static_cast<int>(lane_id());
 #pragma unroll
   for (int n = 0; n < kPieces; ++n) {
     const int e = lane + 32 * n, r = e / kPieces, p = e % kPieces;
     const bool there = first + r < rows;
     const int c = col + 4 * p;
-    copy_async16<kWide>(held_piece<HD>(at, r, p), there && c < width ? src + static_cast<long long>(first + r) * width + c : src, there ? width - c : 0);
+    copy_async16<kWide>(held_piece<OW>(at, r, p), there && c < width ? src + static_cast<long long>(first + r) * width + c : src, there ? width - c : 0);
   }
 }
 // ... and from there, split, to this thread's lane of tensor memory at column `to` (pieces HD / 2 columns apart).
-template <int HD>
+template <int HD, int OW>
 __device__ __forceinline__ void place_held(uint32_t to, uint32_t at, Check& check) {
-  constexpr int kPieces = HD / 16;
   const int lane = static_cast<int>(lane_id());
-  float x[4 * kPieces];
 #pragma unroll
-  for (int p = 0; p < kPieces; ++p)
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(x[4 * p]), "=f"(x[4 * p + 1]), "=f"(x[4 * p + 2]), "=f"(x[4 * p + 3])
-                 : "r"(held_piece<HD>(at, lane, p)) : "memory");
-  uint32_t h[2 * kPieces], m[2 * kPieces], l[2 * kPieces];
+  for (int c = 0; c < OW; c += OW < 16 ? OW : 16) {  // (16 columns at a time)
+    constexpr int N = OW < 16 ? OW : 16;
+    float x[N];
 #pragma unroll
-  for (int e = 0; e < 2 * kPieces; ++e) split_pair<true>(f2_pack(x[2 * e], x[2 * e + 1]), h[e], m[e], l[e], check);
-  if constexpr (kPieces == 4) {
-    tmem_st8(to, h), tmem_st8(to + HD / 2, m), tmem_st8(to + HD, l);
-  } else {
-    tmem_st4(to, h), tmem_st4(to + HD / 2, m), tmem_st4(to + HD, l);
+    for (int p = 0; p < N / 4; ++p)
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(x[4 * p]), "=f"(x[4 * p + 1]), "=f"(x[4 * p + 2]), "=f"(x[4 * p + 3])
+                   : "r"(held_piece<OW>(at, lane, c / 4 + p)) : "memory");
+    uint32_t h[N / 2], m[N / 2], l[N / 2];
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) split_pair<true>(f2_pack(x[2 * e], x[2 * e + 1]), h[e], m[e], l[e], check);
+    if constexpr (N == 16) {
+      tmem_st8(to + c / 2, h), tmem_st8(to + c / 2 + HD / 2, m), tmem_st8(to + c / 2 + HD, l);
+    } else {
+      tmem_st4(to + c / 2, h), tmem_st4(to + c / 2 + HD / 2, m), tmem_st4(to + c / 2 + HD, l);
+    }
   }
 }
 
@@ -770,13 +775,13 @@ __device__ __forceinline__ uint32_t ring_parity(int t) { return static_cast<uint
 // tile there is an arrival at the ring there_r. `carry` holds the first half already. load_rows(item, row) fetches what goes with a
 // tile's rows, post_rows(tile) leaves it in shared memory before the first operand is there. Returns the items in which something does not
 // split.
-template <int HD, bool kWide, int kPlaces0, int kPlaces1, bool kCall, typename Items, typename Source0, typename Source1, typename LoadRows, typename PostRows>
-__device__ __forceinline__ uint32_t split_streams(Carry<HD, kWide> (&carry)[Carry<HD, kWide>::kHalves], Item it, bool more, Items item, Source0 stream0, Source1 stream1, int streamed, int width0,
+template <int HD, int kThreads, bool kWide, int kPlaces0, int kPlaces1, bool kCall, typename Items, typename Source0, typename Source1, typename LoadRows, typename PostRows>
+__device__ __forceinline__ uint32_t split_streams(Carry<HD, kThreads, kWide> (&carry)[Carry<HD, kThreads, kWide>::kHalves], Item it, bool more, Items item, Source0 stream0, Source1 stream1, int streamed, int width0,
                                                   int width1, uint32_t free0, uint32_t free1, uint32_t there0, uint32_t there1, uint32_t tiles0,
                                                   uint32_t tiles1, unsigned* status, bool& ok, LoadRows load_rows, PostRows post_rows) {
   static_assert(kPlaces0 <= kRing && kPlaces1 <= kRing, "a barrier for each");
   constexpr uint32_t kTile = 3 * kStream * 128;
-  constexpr bool kDeep = Carry<HD, kWide>::kHalves == 2;
+  constexpr bool kDeep = Carry<HD, kThreads, kWide>::kHalves == 2;
   uint32_t again = 0;
   int t = 0;
   if (more) load_rows(it, it.begin);
@@ -817,15 +822,19 @@ struct Fwd {
   static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kHeldCol = kO + HD;
   static constexpr int kCols = 512;
   static_assert(kHeldCol + 3 * HD / 2 <= kCols, "tensor memory");
+  // Threads to a row: eight row warps and seven splitting ones. With sixteen and three, 256 x 512 x 64 takes 125 us for 105, 6 x 8192 x 32
+  // causal 237 for 225: what a warp spends on a tile whatever its width, and on the row maxima, is spent half as often.
+  static constexpr int kGroups = 2;
   static constexpr int kPlaces0 = 3, kPlaces1 = 3;  // of K and of V
   static constexpr uint32_t kTile = 3 * kStream * 128;
   static constexpr uint32_t kTile0 = 0, kTile1 = kPlaces0 * kTile, kHeld = kTile1 + kPlaces1 * kTile, kBytes = kHeld + kRows * HD * 4 + 1024;
 };
 
 template <int HD, bool kWide>
-__global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_constant__ Params g) {
+__global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_kernel(const __grid_constant__ Params g) {
   using L = Fwd<HD>;
-  constexpr int G = kRowGroups, CW = kStream / G, OW = HD / G;
+  using W = Roles<L::kGroups>;
+  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
   extern __shared__ __align__(16) unsigned char raw[];
   // A tile's hidden keys come with K, whose place is free again when the tile has been scored, before the row warps are done with it:
   // they have twice as many places (five would do: the row warps are in the tile after next by then).
@@ -840,7 +849,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 0; i < kBars; ++i)
-      mbar_init(smem_addr(bars + i), i < kScored ? kRowWarps + kSplitWarps : 1);
+      mbar_init(smem_addr(bars + i), i < kScored ? W::kRowWarps + W::kSplitWarps : 1);
     mbar_init_fence();
     again_all = 0;
   }
@@ -860,26 +869,26 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
   };
   const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
   const uint32_t raw_q = base + L::kHeld + warp * (32 * OW * 4);
-  auto fetch = [&](const Item& it) { fetch_held<HD, kWide>(raw_q, g.q + it.b * g.t_q * g.hd, it.first + quarter * 32, g.t_q, group * OW, g.hd); };
+  auto fetch = [&](const Item& it) { fetch_held<OW, kWide>(raw_q, g.q + it.b * g.t_q * g.hd, it.first + quarter * 32, g.t_q, group * OW, g.hd); };
   auto keys = [&](const Item& it) { return g.k + it.b * g.t_k * g.hd; };
   auto values = [&](const Item& it) { return g.v + it.b * g.t_k * g.hd_v; };
 
   Item it;
   const bool any = item(0, it);
   grid_dependency_wait();
-  if (warp == kIssuer) {
+  if (warp == W::kIssuer) {
     tmem_alloc(smem_addr(&slot), L::kCols);
     tmem_relinquish();
   }
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk;
   // the first operands set out before the block is set up
-  using Carried = Carry<HD, kWide>;
+  using Carried = Carry<HD, W::kSplitThreads, kWide>;
   Carried carry[Carried::kHalves];
 #pragma unroll
-  for (int h = 0; h < Carried::kHalves; ++h) carry[h].set_up(threadIdx.x - kRowThreads);
-  if (any && warp < kRowWarps) {
+  for (int h = 0; h < Carried::kHalves; ++h) carry[h].set_up(threadIdx.x - W::kRowThreads);
+  if (any && warp < W::kRowWarps) {
     fetch(it);
-  } else if (any && warp < kIssuer) {
+  } else if (any && warp < W::kIssuer) {
     carry[0].load_all(carry[0].source(keys(it), 0, g.t_k, g.hd));
     if (Carried::kHalves > 1) carry[Carried::kHalves - 1].load_all(carry[0].source(values(it), 0, g.t_k, g.hd_v));
   }
@@ -892,7 +901,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
   if (abort_flag) {
     // an earlier kernel on this device gave up on a wait: take no work
     copy_async_wait();
-  } else if (warp == kIssuer) {
+  } else if (warp == W::kIssuer) {
     // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
     grid_launch_dependents();
     int t = 0;  // tiles so far
@@ -920,11 +929,11 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
       }
       if (ok) weigh(t - 1);
     }
-  } else if (warp >= kRowWarps) {
+  } else if (warp >= W::kRowWarps) {
     // ================= splitting warps =================
-    const int thread = threadIdx.x - kRowThreads;
+    const int thread = threadIdx.x - W::kRowThreads;
     float flag = 0.f;
-    again = split_streams<HD, kWide, L::kPlaces0, L::kPlaces1, false>(
+    again = split_streams<HD, W::kSplitThreads, kWide, L::kPlaces0, L::kPlaces1, false>(
         carry, it, any, item, keys, values, g.t_k, g.hd, g.hd_v, ring(kScored, 0), ring(kWeighed, 0), ring(kGo, 0), ring(kReady, 0), base + L::kTile0, base + L::kTile1, g.status, ok,
         [&](const Item& it, int x0) {
           if (g.mask) flag = row_value(g.mask + it.b * g.t_k, x0, g.t_k, thread);
@@ -942,7 +951,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
       Check check;
       copy_async_wait();
       __syncwarp();
-      place_held<HD>(lanes + L::kHeldCol + group * (OW / 2), raw_q, check);
+      place_held<HD, OW>(lanes + L::kHeldCol + group * (OW / 2), raw_q, check);
       tmem_st_wait();
       tc_fence_before_sync();
       if (check.bad()) again |= 1u << k;
@@ -1062,11 +1071,11 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_fwd_kernel(const __grid_c
   if (again != 0) atomicOr(&again_all, again);
   tc_fence_before_sync();
   ok = __syncthreads_and(ok);
-  if (ok && again_all != 0 && !abort_flag && warp < kRowWarps) {
+  if (ok && again_all != 0 && !abort_flag && warp < W::kRowWarps) {
     for (uint32_t left = again_all; left != 0; left &= left - 1)
-      if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+      if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, W::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
   }
-  tear_down<L::kCols, kIssuer>(g, tmem);
+  tear_down<L::kCols, W::kIssuer>(g, tmem);
 }
 
 // ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
@@ -1094,11 +1103,15 @@ struct Bwd {
   static constexpr uint32_t kBytes = kHeld1 + (kHeldT ? kHeldRaw : kHeldPieces) + 1024;
 };
 
-template <int HD, bool kKV, bool kWide>
-__global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
+// kGroups threads to a row (and the split of the warps that goes with it): the same bits either way. Two are faster where a block has
+// one item (2 x 128 x 32 7.8 us for 8.4), as the splitting warps have it ready sooner, four in the long run (6 x 8192 x 32 causal 233 for 239,
+// 256 x 512 x 64 143 for 150; two spill).
+template <int HD, bool kKV, bool kWide, int kGroups>
+__global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
   using L = Bwd<HD, kKV>;
-  using Held = Stage<HD, kRows, kRowThreads, kWide>;
-  constexpr int CW = kStream / kRowGroups, OW = HD / kRowGroups;
+  using W = Roles<kGroups>;
+  using Held = Stage<HD, kRows, W::kRowThreads, kWide>;
+  constexpr int CW = kStream / kGroups, OW = HD / kGroups;
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ uint32_t slot, abort_flag, again_all, hidden[kRing][2];
   // kGo: a tile can be scored (both its operands are there, the scores before it have been read, the held operands are there).
@@ -1111,7 +1124,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 0; i < kBars; ++i)
-      mbar_init(smem_addr(bars + i), i < kReady ? kRowWarps + (L::kLate1 ? 1 : 2) * kSplitWarps : i < kScored ? kRowWarps : i < kGoOn ? 1 : kSplitWarps);
+      mbar_init(smem_addr(bars + i), i < kReady ? W::kRowWarps + (L::kLate1 ? 1 : 2) * W::kSplitWarps : i < kScored ? W::kRowWarps : i < kGoOn ? 1 : W::kSplitWarps);
     mbar_init_fence();
     again_all = 0;
   }
@@ -1142,8 +1155,8 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
   const uint32_t raw0 = base + L::kHeld0 + warp * (32 * OW * 4), raw1 = base + L::kHeld1 + warp * (32 * OW * 4);
   auto fetch = [&](const Item& it) {
-    fetch_held<HD, kWide>(raw0, held0(it), it.first + quarter * 32, owned, group * OW, g.hd);
-    fetch_held<HD, kWide>(raw1, held1(it), it.first + quarter * 32, owned, group * OW, g.hd_v);
+    fetch_held<OW, kWide>(raw0, held0(it), it.first + quarter * 32, owned, group * OW, g.hd);
+    fetch_held<OW, kWide>(raw1, held1(it), it.first + quarter * 32, owned, group * OW, g.hd_v);
   };
 
   // the held operands of an item into L2, a 128-byte line to a thread
@@ -1159,19 +1172,19 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   Item it;
   const bool any = item(0, it);
   grid_dependency_wait();
-  if (warp == kIssuer) {
+  if (warp == W::kIssuer) {
     tmem_alloc(smem_addr(&slot), L::kCols);
     tmem_relinquish();
   }
   if (threadIdx.x == 0) abort_flag = *reinterpret_cast<volatile unsigned*>(g.status) != kStatusOk;
   // the first operands set out before the block is set up
-  using Carried = Carry<HD, kWide>;
+  using Carried = Carry<HD, W::kSplitThreads, kWide>;
   Carried carry[Carried::kHalves];
 #pragma unroll
-  for (int h = 0; h < Carried::kHalves; ++h) carry[h].set_up(threadIdx.x - kRowThreads);
-  if (any && warp < kRowWarps) {
+  for (int h = 0; h < Carried::kHalves; ++h) carry[h].set_up(threadIdx.x - W::kRowThreads);
+  if (any && warp < W::kRowWarps) {
     if (L::kHeldT) fetch(it);
-  } else if (any && warp < kIssuer) {
+  } else if (any && warp < W::kIssuer) {
     carry[0].load_all(carry[0].source(stream0(it), it.begin, streamed, g.hd));
     if (Carried::kHalves > 1) carry[Carried::kHalves - 1].load_all(carry[0].source(stream1(it), it.begin, streamed, g.hd_v));
   }
@@ -1184,7 +1197,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   if (abort_flag) {
     // an earlier kernel on this device gave up on a wait: take no work
     copy_async_wait();
-  } else if (warp == kIssuer) {
+  } else if (warp == W::kIssuer) {
     // ================= issuing warp: it stays together and elects a lane for each bunch of MMAs =================
     grid_launch_dependents();
     int t = 0;  // tiles so far
@@ -1224,11 +1237,11 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
       }
       if (ok) weigh(t - 1);
     }
-  } else if (warp >= kRowWarps) {
+  } else if (warp >= W::kRowWarps) {
     // ================= splitting warps =================
-    const int thread = threadIdx.x - kRowThreads;
+    const int thread = threadIdx.x - W::kRowThreads;
     float row_a = 0.f, row_b = 0.f;  // dK/dV: L and delta of a query row; dQ: a key's flag
-    again = split_streams<HD, kWide, L::kPlaces0, L::kPlaces1, true>(
+    again = split_streams<HD, W::kSplitThreads, kWide, L::kPlaces0, L::kPlaces1, true>(
         carry, it, any, item, stream0, stream1, streamed, g.hd, g.hd_v, ring(kWeighed, 0), ring(kKV ? kHalfWeighed : kScored, 0), ring(kGo, 0), ring(L::kLate1 ? kGoOn : kGo, 0), base + L::kTile0, base + L::kTile1, g.status, ok,
         [&](const Item& it, int x0) {
           if (kKV) {
@@ -1261,8 +1274,8 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
       if constexpr (L::kHeldT) {
         copy_async_wait();
         __syncwarp();
-        place_held<HD>(lanes + L::kHeldCol + group * (OW / 2), raw0, check);
-        place_held<HD>(lanes + L::kHeldCol + 3 * HD / 2 + group * (OW / 2), raw1, check);
+        place_held<HD, OW>(lanes + L::kHeldCol + group * (OW / 2), raw0, check);
+        place_held<HD, OW>(lanes + L::kHeldCol + 3 * HD / 2 + group * (OW / 2), raw1, check);
         tmem_st_wait();
         tc_fence_before_sync();
       } else {
@@ -1378,12 +1391,12 @@ __global__ void __launch_bounds__(kRoleThreads, 1) f32_bwd_kernel(const __grid_c
   if (again != 0) atomicOr(&again_all, again);
   tc_fence_before_sync();
   ok = __syncthreads_and(ok);
-  if (ok && again_all != 0 && !abort_flag && warp < kRowWarps) {
+  if (ok && again_all != 0 && !abort_flag && warp < W::kRowWarps) {
     for (uint32_t left = again_all; left != 0; left &= left - 1)
       if (item(__ffs(static_cast<int>(left)) - 1, it))
-        rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+        rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, W::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
   }
-  tear_down<L::kCols, kIssuer>(g, tmem);
+  tear_down<L::kCols, W::kIssuer>(g, tmem);
 }
 
 // ---- backward at head dims above 64 ----
@@ -1621,21 +1634,29 @@ int launch_sized(Op op, const Problem& p) {
     kernel = op == Op::Fwd ? f32_fwd_wide_kernel<HD, kWide> : op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
     shared = op == Op::Fwd ? F::kBytes : B::kBytes, threads = B::kThreads;
   } else {
-    kernel = op == Op::Fwd ? f32_fwd_kernel<HD, kWide> : op == Op::BwdQ ? f32_bwd_kernel<HD, false, kWide> : f32_bwd_kernel<HD, true, kWide>;
-    shared = op == Op::Fwd ? Fwd<HD>::kBytes : op == Op::BwdQ ? Bwd<HD, false>::kBytes : Bwd<HD, true>::kBytes, threads = kRoleThreads;
+    const bool one_each = blocks <= sms;
+    if (op == Op::Fwd) {
+      kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
+    } else if (op == Op::BwdQ) {
+      kernel = one_each ? f32_bwd_kernel<HD, false, kWide, 2> : f32_bwd_kernel<HD, false, kWide, 4>;
+      shared = Bwd<HD, false>::kBytes, threads = one_each ? Roles<2>::kThreads : Roles<4>::kThreads;
+    } else {
+      kernel = f32_bwd_kernel<HD, true, kWide, 4>, shared = Bwd<HD, true>::kBytes, threads = Roles<4>::kThreads;
+    }
     // every SM has its block, and they are done together: as many blocks to an SM one after the other as the limit on a
     // block's items asks for
     const long long turn = static_cast<long long>(sms) * kMostItems;
     grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
-  static bool sized[64][3] = {};
+  const int which = op == Op::BwdQ && HD <= 64 && blocks <= sms ? 3 : static_cast<int>(op);
+  static bool sized[64][4] = {};
   int device = 0;
   LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");
-  if (device < 0 || device >= 64 || !sized[device][static_cast<int>(op)]) {
+  if (device < 0 || device >= 64 || !sized[device][which]) {
     LIMN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared)),
               "sizing shared memory for a float32 sdpa kernel");
-    if (device >= 0 && device < 64) sized[device][static_cast<int>(op)] = true;
+    if (device >= 0 && device < 64) sized[device][which] = true;
   }
   LIMN_CUDA(launch_overlapped(kernel, dim3(static_cast<unsigned>(grid)), dim3(threads), shared, p.stream, g),
             "launching a float32 sdpa kernel");
