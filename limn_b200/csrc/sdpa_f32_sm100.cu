@@ -608,6 +608,7 @@ struct Roles {  // kGroups threads to a row, the other warps by what registers a
   static constexpr int kRowWarps = 4 * kGroups, kSplitWarps = kGroups == 4 ? 3 : 7, kIssuer = kRowWarps + kSplitWarps;
   static constexpr int kRowThreads = 32 * kRowWarps, kSplitThreads = 32 * kSplitWarps, kThreads = 32 * (kIssuer + 1);
 };
+constexpr int kAgainGroups = 2;                  // of tiled::kThreads of a block's threads, whatever their roles, for items done again on the CUDA cores
 constexpr int kMostItems = 32;                   // work items of a block: each has a bit of a word
 
 // Work item `k` of this block. Blocks take turns, there and back: items are in the order of their length under a causal mask, and a
@@ -1071,9 +1072,9 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
   if (again != 0) atomicOr(&again_all, again);
   tc_fence_before_sync();
   ok = __syncthreads_and(ok);
-  if (ok && again_all != 0 && !abort_flag && warp < W::kRowWarps) {
+  if (ok && again_all != 0 && !abort_flag && threadIdx.x < kAgainGroups * tiled::kThreads) {
     for (uint32_t left = again_all; left != 0; left &= left - 1)
-      if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, W::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+      if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, kAgainGroups, L::kBytes, kWide>(g, it.b, it.first, raw);
   }
   tear_down<L::kCols, W::kIssuer>(g, tmem);
 }
@@ -1391,10 +1392,10 @@ __global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(co
   if (again != 0) atomicOr(&again_all, again);
   tc_fence_before_sync();
   ok = __syncthreads_and(ok);
-  if (ok && again_all != 0 && !abort_flag && warp < W::kRowWarps) {
+  if (ok && again_all != 0 && !abort_flag && threadIdx.x < kAgainGroups * tiled::kThreads) {
     for (uint32_t left = again_all; left != 0; left &= left - 1)
       if (item(__ffs(static_cast<int>(left)) - 1, it))
-        rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, W::kRowThreads / tiled::kThreads, L::kBytes, kWide>(g, it.b, it.first, raw);
+        rows_again<HD, kKV ? Op::BwdKV : Op::BwdQ, kAgainGroups, L::kBytes, kWide>(g, it.b, it.first, raw);
   }
   tear_down<L::kCols, W::kIssuer>(g, tmem);
 }
