@@ -357,184 +357,6 @@ __device__ __forceinline__ uint32_t my_hidden(const uint32_t* words, int group) 
 
 __device__ __forceinline__ uint32_t align_1024(uint32_t addr) { return (addr + 1023u) & ~1023u; }
 
-// ---- forward at head dims above 64 ----
-template <int HD, bool kWide>
-struct FwdWide {
-  static constexpr int kGroups = 4;  // threads to a row
-  static constexpr int kThreads = kRows * kGroups;
-  using Held = Stage<HD, kRows, kThreads, kWide>;
-  using Tile = Stage<HD, kStream, kThreads, kWide>;
-  static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
-  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kS2 = kO + HD;
-  static constexpr int kCols = 512;
-};
-
-template <int HD, bool kWide>
-__global__ void __launch_bounds__(FwdWide<HD, kWide>::kThreads, 1) f32_fwd_wide_kernel(const __grid_constant__ Params g) {
-  using L = FwdWide<HD, kWide>;
-  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
-  extern __shared__ __align__(16) unsigned char raw[];
-  __shared__ uint32_t slot, abort_flag, hidden[2][2];
-  __shared__ __align__(8) uint64_t bars[2];
-  __shared__ float exchange[G][kRows];
-  uint32_t tmem;
-  if (!set_up<L::kCols, 2>(g, &slot, &abort_flag, bars, tmem)) return;
-  const uint32_t base = align_1024(smem_addr(raw));
-  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1);
-  const int warp = threadIdx.x >> 5, group = warp >> 2;
-  const int row = (warp & 3) * 32 + (threadIdx.x & 31);
-  const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  const bool issues = __shfl_sync(kFull, warp, 0) == 0;  // the warp that issues, one lane of it elected per bunch
-
-  int problem, at;
-  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
-  const int i0 = (g.slots - 1 - at) * kRows;  // long causal rows first
-  const long long b = problem;
-  const float* k = g.k + b * g.t_k * g.hd;
-  const float* v = g.v + b * g.t_k * g.hd_v;
-  const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
-  const int keys_end = g.causal ? min(g.t_k, i0 + kRows) : g.t_k;
-  const int n = (keys_end + kStream - 1) / kStream;
-  const int i = i0 + row;
-
-  Check check;
-  typename L::Tile stage_k, stage_v;
-  stage_k.load(k, 0, g.t_k, g.hd);
-  {
-    typename L::Held stage_q;
-    stage_q.load(g.q + b * g.t_q * g.hd, i0, g.t_q, g.hd);
-    stage_q.store(base + L::kQ, check);
-  }
-  stage_k.store(base + L::kK, check);
-  if (mask) post_hidden(hidden[0], row_value(mask, 0, g.t_k));
-  fence_async_shared();
-  __syncthreads();
-  if (issues && elect_one()) {
-    issue_scores<HD, false, true>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
-    mma_commit(scored);
-  }
-  stage_v.load(v, 0, g.t_k, g.hd_v);
-  stage_v.store(base + L::kV, check);
-  fence_async_shared();
-
-  float top = -INFINITY, shift = 0.f, denom = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
-  uint64_t acc[OW / 2];
-#pragma unroll
-  for (int c = 0; c < OW / 2; ++c) acc[c] = 0;
-  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo);
-  bool ok = true;
-  for (int j = 0; j < n; ++j) {
-    const int j0 = j * kStream;
-    ok &= mbar_wait(scored, j & 1, g.status, 0x0a00u);
-    tc_fence_after_sync();
-    uint32_t s[CW];
-    tmem_ld<CW>(lanes + L::kS + group * CW, s);
-    uint32_t more_s[CW];
-    tmem_ld<CW>(lanes + L::kS2 + group * CW, more_s);
-    tmem_ld_wait();
-#pragma unroll
-    for (int c = 0; c < CW; ++c) s[c] = __float_as_uint(__uint_as_float(s[c]) + __uint_as_float(more_s[c]));
-    int limit = g.t_k - j0;
-    if (g.causal) limit = min(limit, i - j0 + 1);
-    limit -= group * CW;
-    uint32_t unseen = limit >= CW ? 0u : limit <= 0 ? kFull : ~((1u << limit) - 1u);
-    if (mask) unseen |= my_hidden<CW>(hidden[j & 1], group);
-    if (unseen != 0u) {
-#pragma unroll
-      for (int c = 0; c < CW; ++c)
-        if ((unseen >> c) & 1u) s[c] = 0xff800000u;
-    }
-    float tile_top = -INFINITY;
-#pragma unroll
-    for (int c = 0; c < CW; c += 2) tile_top = max3(tile_top, __uint_as_float(s[c]), __uint_as_float(s[c + 1]));
-    exchange[group][row] = tile_top;
-    __syncthreads();
-    float raised = top;
-#pragma unroll
-    for (int c = 0; c < G; ++c) raised = fmaxf(raised, exchange[c][row]);
-    const float moved = raised == -INFINITY ? 0.f : raised * g.c_hi;
-    const float shrink = top == -INFINITY ? 0.f : exp2_approx(shift - moved);  // nothing gathered yet: nothing to rescale
-    top = raised, shift = moved;
-    const uint64_t minus_shift = f2_pack(-shift, -shift);
-    uint64_t w[CW / 2];
-    uint64_t sum = 0;
-#pragma unroll
-    for (int c = 0; c < CW / 2; ++c) {
-      const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
-      float x0, x1;
-      f2_unpack(f2_fma(s2, c_lo, f2_fma(s2, c_hi, minus_shift)), x0, x1);
-      w[c] = f2_pack(exp2_approx(x0), exp2_approx(x1));
-      sum = f2_add(sum, w[c]);
-    }
-    float sum0, sum1;
-    f2_unpack(sum, sum0, sum1);
-    denom = fmaf(denom, shrink, sum0 + sum1);  // this thread's share; the shares meet after the last tile
-    check.sums |= !(denom < INFINITY);
-    hand_over<CW>(lanes + L::kP + group * (CW / 2), w, check);
-    tmem_st_wait();
-    tc_fence_before_sync();
-    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
-    if (issues && elect_one()) {
-      tc_fence_after_sync();
-      issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
-      mma_commit(weighed);
-    }
-    const bool more = j + 1 < n;
-    if (more) {
-      // K's buffer has been read (the scores are there) and so have the scores themselves
-      stage_k.load(k, j0 + kStream, g.t_k, g.hd);
-      const float flag = mask ? row_value(mask, j0 + kStream, g.t_k) : 0.f;
-      stage_k.store(base + L::kK, check);
-      if (mask) post_hidden(hidden[(j + 1) & 1], flag);
-      fence_async_shared();
-      __syncthreads();
-      if (issues && elect_one()) {
-        tc_fence_after_sync();
-        issue_scores<HD, false, true>(tmem + L::kS, base + L::kQ, base + L::kK, tmem + L::kS2);
-        mma_commit(scored);
-      }
-      stage_v.load(v, j0 + kStream, g.t_k, g.hd_v);
-    }
-    ok &= mbar_wait(weighed, j & 1, g.status, 0x0a01u);
-    tc_fence_after_sync();
-    uint32_t o[OW];
-    tmem_ld<OW>(lanes + L::kO + group * OW, o);
-    tmem_ld_wait();
-    tc_fence_before_sync();
-    const uint64_t shrink2 = f2_pack(shrink, shrink);
-#pragma unroll
-    for (int c = 0; c < OW / 2; ++c) acc[c] = f2_fma(acc[c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
-    if (more) {
-      stage_v.store(base + L::kV, check);  // the weighing has read the tile before this one
-      fence_async_shared();
-    }
-  }
-  ok = __syncthreads_and(ok);
-  if (ok) {
-    if (__syncthreads_or(check.bad())) {
-      rows_again<HD, Op::Fwd, L::kThreads / tiled::kThreads, L::kBytes, kWide>(g, b, i0, raw);
-    } else {
-      exchange[group][row] = denom;
-      __syncthreads();
-      float total = 0.f;
-#pragma unroll
-      for (int c = 0; c < G; ++c) total += exchange[c][row];
-#pragma unroll
-      for (int c = 0; c < OW / 2; ++c) {
-        float x0, x1;
-        f2_unpack(acc[c], x0, x1);
-        acc[c] = f2_pack(x0 / total, x1 / total);  // 0/0 = NaN for a row with no key, as the oracle has it
-      }
-      store_rows<OW>(g.out + b * g.t_q * g.hd_v, acc, i0 + (warp & 3) * 32, g.t_q, group * OW, g.hd_v, g.wide_out);
-      // once per row, so in double: L is then as good as its sum
-      if (group == 0 && i < g.t_q)
-        g.lse_out[b * g.t_q + i] =
-            top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
-    }
-  }
-  tear_down<L::kCols>(g, tmem);
-}
-
 // log2(e) in two parts: minus a log-sum-exp in log2 units, as hi + lo
 __device__ __forceinline__ void to_minus_log2(const float lse, float& hi, float& lo) {
   constexpr float kHi = 1.44269502f, kLo = 1.92596303e-8f;
@@ -627,16 +449,17 @@ struct Carry {
   static constexpr int kChunks = HD / 8, kStep = kThreads / kChunks;  // rows from one turn to the next
   static constexpr int kTurns = (kStream + kStep - 1) / kStep;
   static constexpr int kHalves = kTurns > 3 ? 1 : 2;  // that a thread's registers hold: with two, each operand's next tile is under way
-  static constexpr uint32_t kPiece = kStream * 128;
-  static_assert(HD <= 64 && kThreads % kChunks == 0 && kStep % 4 == 0, "a thread keeps its columns");
+  static constexpr uint32_t kPiece = (HD > 64 ? 2 : 1) * kStream * 128, kTile = 3 * kPiece;
+  static constexpr int kPeriod = kStep % 4 == 0 ? 2 : 4;  // turns after which the swizzle is the same again
+  static_assert(kThreads % kChunks == 0 && kStep % 2 == 0, "a thread keeps its columns");
   float x[kTurns][8];
   int row, column;    // of the first turn
-  uint32_t where[2];  // of the first turn's pieces in a tile; of the second's, less the rows between them
+  uint32_t where[kPeriod];  // of the turns' pieces in a tile, less the rows between them
 
   __device__ __forceinline__ void set_up(int thread) {
     row = thread / kChunks, column = thread % kChunks * 8;
-    where[0] = swizzled_piece(0, row, thread % kChunks);
-    where[1] = swizzled_piece(0, row + kStep, thread % kChunks) - kStep * 128;
+#pragma unroll
+    for (int n = 0; n < kPeriod; ++n) where[n] = swizzled_piece(column / 64 * (kStream * 128), row + n * kStep, column / 8 % 8) - n * kStep * 128;
   }
   __device__ __forceinline__ bool has(int n) const { return n * kStep + kStep <= kStream || n * kStep + row < kStream; }
   // The rows of a half that starts with row `first` of a (rows, width) matrix.
@@ -656,14 +479,13 @@ struct Carry {
   }
   // This half to the tile at dst, the next one's rows to registers.
   __device__ __forceinline__ void store_and_load(uint32_t dst, Check& check, const Source& next) {
-    const uint32_t at[2] = {dst + where[0], dst + where[1]};
 #pragma unroll
     for (int n = 0; n < kTurns; ++n) {
       if (has(n)) {  // (whole warps have it or not)
         uint32_t h[4], m[4], l[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) split_pair<true>(f2_pack(x[n][2 * i], x[n][2 * i + 1]), h[i], m[i], l[i], check);
-        const uint32_t to = at[n & 1] + n * kStep * 128;
+        const uint32_t to = dst + where[n % kPeriod] + n * kStep * 128;
         st_shared_v4(to, h[0], h[1], h[2], h[3]);
         st_shared_v4(to + kPiece, m[0], m[1], m[2], m[3]);
         st_shared_v4(to + 2 * kPiece, l[0], l[1], l[2], l[3]);
@@ -781,7 +603,7 @@ __device__ __forceinline__ uint32_t split_streams(Carry<HD, kThreads, kWide> (&c
                                                   int width1, uint32_t free0, uint32_t free1, uint32_t there0, uint32_t there1, uint32_t tiles0,
                                                   uint32_t tiles1, unsigned* status, bool& ok, LoadRows load_rows, PostRows post_rows) {
   static_assert(kPlaces0 <= kRing && kPlaces1 <= kRing, "a barrier for each");
-  constexpr uint32_t kTile = 3 * kStream * 128;
+  constexpr uint32_t kTile = Carry<HD, kThreads, kWide>::kTile;
   constexpr bool kDeep = Carry<HD, kThreads, kWide>::kHalves == 2;
   uint32_t again = 0;
   int t = 0;
@@ -816,19 +638,75 @@ __device__ __forceinline__ uint32_t split_streams(Carry<HD, kThreads, kWide> (&c
   return again;
 }
 
-// ---- forward at head dims up to 64 ----
+// The same with one place for each operand, the next tile's first operand before this tile's second: its place is free as soon as the
+// tile has been scored, the other's only when the tile before it has been weighed. (The order of the other function would leave the
+// tensor cores waiting for both.)
+template <int HD, int kThreads, bool kWide, bool kCall, typename Items, typename Source0, typename Source1, typename LoadRows, typename PostRows>
+__device__ __forceinline__ uint32_t split_streams_one(Carry<HD, kThreads, kWide>& carry, const Item& start, bool any, Items item, Source0 stream0, Source1 stream1, int streamed,
+                                                      int width0, int width1, uint32_t free0, uint32_t free1, uint32_t there0, uint32_t there1, uint32_t tile0,
+                                                      uint32_t tile1, unsigned* status, bool& ok, LoadRows load_rows, PostRows post_rows) {
+  struct Cursor {
+    Item it;
+    int k, j;
+    bool there;
+  };
+  auto advance = [&](Cursor& c) {
+    if (++c.j < c.it.tiles) return;
+    c.j = 0;
+    c.there = item(++c.k, c.it);
+  };
+  auto first_row = [](const Cursor& c) { return c.it.begin + c.j * kStream; };
+  uint32_t again = 0;
+  Cursor a = {start, 0, 0, any}, b = a;  // the tile whose first operand is due, and the one before it
+  if (any) load_rows(a.it, first_row(a));
+  for (int t = 0; ok && (a.there || t > 0); ++t) {
+    Cursor next = a;
+    if (a.there) {
+      advance(next);
+      if (t > 0) ok = warp_waits<kCall>(ring_bar(free0, t - 1), ring_parity(t - 1), status, 0x0b30u);
+      if (!ok) break;
+      post_rows(t);
+      if (next.there) load_rows(next.it, first_row(next));
+      Check check;
+      if (t > 0) carry.store_and_load(tile0, check, carry.source(stream1(b.it), first_row(b), streamed, width1));
+      else carry.store_and_load(tile0, check, next.there ? carry.source(stream0(next.it), first_row(next), streamed, width0) : carry.source(stream1(a.it), first_row(a), streamed, width1));
+      fence_async_shared();
+      warp_arrives(ring_bar(there0, t));
+      if (check.bad()) again |= 1u << a.k;
+    }
+    if (t > 0) {
+      if (t > 1) ok = warp_waits<kCall>(ring_bar(free1, t - 2), ring_parity(t - 2), status, 0x0b31u);
+      if (!ok) break;
+      Check check;
+      carry.store_and_load(tile1, check, next.there ? carry.source(stream0(next.it), first_row(next), streamed, width0) : carry.source(stream1(a.it), first_row(a), a.there ? streamed : 0, width1));
+      fence_async_shared();
+      warp_arrives(ring_bar(there1, t - 1));
+      if (check.bad()) again |= 1u << b.k;
+    }
+    if (!a.there) break;
+    b = a, a = next;
+  }
+  return again;
+}
+
+// ---- forward ----
 template <int HD>
 struct Fwd {
-  // tensor memory: scores, the pieces of P, a tile's product, the pieces of Q
-  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols, kHeldCol = kO + HD;
+  // tensor memory: scores (above head dim 64 in two parts, see issue_scores), the pieces of P, a tile's product, and the pieces of Q
+  // where there is room
+  static constexpr bool kTwo = HD > 64, kHeldT = HD <= 64;
+  static constexpr uint32_t kS = 0, kS2 = kStream, kP = kTwo ? 2 * kStream : kStream, kO = kP + 3 * kPieceCols, kHeldCol = kO + HD;
   static constexpr int kCols = 512;
-  static_assert(kHeldCol + 3 * HD / 2 <= kCols, "tensor memory");
+  static_assert(kHeldCol + (kHeldT ? 3 * HD / 2 : 0) <= kCols, "tensor memory");
   // Threads to a row: eight row warps and seven splitting ones. With sixteen and three, 256 x 512 x 64 takes 125 us for 105, 6 x 8192 x 32
   // causal 237 for 225: what a warp spends on a tile whatever its width, and on the row maxima, is spent half as often.
   static constexpr int kGroups = 2;
-  static constexpr int kPlaces0 = 3, kPlaces1 = 3;  // of K and of V
-  static constexpr uint32_t kTile = 3 * kStream * 128;
-  static constexpr uint32_t kTile0 = 0, kTile1 = kPlaces0 * kTile, kHeld = kTile1 + kPlaces1 * kTile, kBytes = kHeld + kRows * HD * 4 + 1024;
+  static constexpr int kShares = HD > 64 ? 2 : 1;  // of a thread in its row's denominator: sums of 16 columns above head dim 64 (0.6 % nearer to float64), of 32 below
+  static constexpr int kPlaces0 = HD > 64 ? 1 : 3, kPlaces1 = HD > 64 ? 1 : 3;  // of K and of V
+  static constexpr uint32_t kTile = 3 * (HD > 64 ? 2 : 1) * kStream * 128;
+  static constexpr uint32_t kHeldPiece = (HD > 64 ? 2 : 1) * kRows * 128;
+  static constexpr uint32_t kTile0 = 0, kTile1 = kPlaces0 * kTile, kHeld = kTile1 + kPlaces1 * kTile;
+  static constexpr uint32_t kBytes = kHeld + (kHeldT ? kRows * HD * 4 : 3 * kHeldPiece) + 1024;
 };
 
 template <int HD, bool kWide>
@@ -845,7 +723,7 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
   // V is there). kScored, kWeighed: the tensor cores have done it.
   enum { kGo = 0, kReady = kRing, kScored = 2 * kRing, kWeighed = 3 * kRing, kBars = 4 * kRing };
   __shared__ __align__(8) uint64_t bars[kBars];
-  __shared__ float exchange[2][G][kRows];
+  __shared__ float exchange[2][G * L::kShares][kRows];
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -870,7 +748,9 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
   };
   const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
   const uint32_t raw_q = base + L::kHeld + warp * (32 * OW * 4);
-  auto fetch = [&](const Item& it) { fetch_held<OW, kWide>(raw_q, g.q + it.b * g.t_q * g.hd, it.first + quarter * 32, g.t_q, group * OW, g.hd); };
+  auto fetch = [&](const Item& it) {
+    if constexpr (L::kHeldT) fetch_held<OW, kWide>(raw_q, g.q + it.b * g.t_q * g.hd, it.first + quarter * 32, g.t_q, group * OW, g.hd);
+  };
   auto keys = [&](const Item& it) { return g.k + it.b * g.t_k * g.hd; };
   auto values = [&](const Item& it) { return g.v + it.b * g.t_k * g.hd_v; };
 
@@ -922,7 +802,7 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
         if (!ok) break;
         tc_fence_after_sync();
         if (elect_one()) {
-          issue_scores<HD, true>(tmem + L::kS, tmem + L::kHeldCol, tile0_at(t));
+          issue_scores<HD, L::kHeldT, L::kTwo>(tmem + L::kS, L::kHeldT ? tmem + L::kHeldCol : base + L::kHeld, tile0_at(t), tmem + L::kS2);
           mma_commit(ring(kScored, t));
         }
         __syncwarp();
@@ -934,36 +814,65 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
     // ================= splitting warps =================
     const int thread = threadIdx.x - W::kRowThreads;
     float flag = 0.f;
-    again = split_streams<HD, W::kSplitThreads, kWide, L::kPlaces0, L::kPlaces1, false>(
-        carry, it, any, item, keys, values, g.t_k, g.hd, g.hd_v, ring(kScored, 0), ring(kWeighed, 0), ring(kGo, 0), ring(kReady, 0), base + L::kTile0, base + L::kTile1, g.status, ok,
-        [&](const Item& it, int x0) {
-          if (g.mask) flag = row_value(g.mask + it.b * g.t_k, x0, g.t_k, thread);
-        },
-        [&](int t) {
-          if (g.mask) post_hidden(hidden[t % kHiddenPlaces], flag, thread);
-        });
+    auto load_rows = [&](const Item& it, int x0) {
+      if (g.mask) flag = row_value(g.mask + it.b * g.t_k, x0, g.t_k, thread);
+    };
+    auto post_rows = [&](int t) {
+      if (g.mask) post_hidden(hidden[t % kHiddenPlaces], flag, thread);
+    };
+    if constexpr (L::kPlaces0 > 1)
+      again = split_streams<HD, W::kSplitThreads, kWide, L::kPlaces0, L::kPlaces1, false>(
+          carry, it, any, item, keys, values, g.t_k, g.hd, g.hd_v, ring(kScored, 0), ring(kWeighed, 0), ring(kGo, 0), ring(kReady, 0), base + L::kTile0, base + L::kTile1,
+          g.status, ok, load_rows, post_rows);
+    else
+      again = split_streams_one<HD, W::kSplitThreads, kWide, false>(carry[0], it, any, item, keys, values, g.t_k, g.hd, g.hd_v, ring(kScored, 0), ring(kWeighed, 0),
+                                                                    ring(kGo, 0), ring(kReady, 0), base + L::kTile0, base + L::kTile1, g.status, ok, load_rows, post_rows);
   } else if (any) {
     // ================= row warps =================
     // A warp that gave up on a wait waits for nothing any more but goes through its tiles like the others: the four warps that share
     // rows meet at a barrier in each.
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     auto meet = [&] { named_barrier_sync(1 + quarter, 32 * G); };
-    auto put_held = [&](int k) {  // Q of item k, which has been fetched
+    auto put_held = [&](const Item& it, int k) {  // Q of item k, to where the MMAs read it
       Check check;
-      copy_async_wait();
-      __syncwarp();
-      place_held<HD, OW>(lanes + L::kHeldCol + group * (OW / 2), raw_q, check);
-      tmem_st_wait();
-      tc_fence_before_sync();
+      if constexpr (L::kHeldT) {  // (it has been fetched)
+        copy_async_wait();
+        __syncwarp();
+        place_held<HD, OW>(lanes + L::kHeldCol + group * (OW / 2), raw_q, check);
+        tmem_st_wait();
+        tc_fence_before_sync();
+      } else {
+        constexpr int kChunks = HD / 8, kStep = W::kRowThreads / kChunks, kAtOnce = 4;
+        const int r = threadIdx.x / kChunks, chunk = threadIdx.x % kChunks;
+        const float* q = g.q + it.b * g.t_q * g.hd;
+#pragma unroll
+        for (int n = 0; n < kRows / kStep; n += kAtOnce) {
+          float x[kAtOnce][8];
+#pragma unroll
+          for (int u = 0; u < kAtOnce; ++u) load8<kWide>(x[u], q, it.first + r + (n + u) * kStep, g.t_q, 8 * chunk, g.hd);
+#pragma unroll
+          for (int u = 0; u < kAtOnce; ++u) {
+            uint32_t h[4], m[4], l[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split_pair<true>(f2_pack(x[u][2 * i], x[u][2 * i + 1]), h[i], m[i], l[i], check);
+            const uint32_t to = swizzled_piece(base + L::kHeld + chunk / 8 * (kRows * 128), r + (n + u) * kStep, chunk % 8);
+            st_shared_v4(to, h[0], h[1], h[2], h[3]);
+            st_shared_v4(to + L::kHeldPiece, m[0], m[1], m[2], m[3]);
+            st_shared_v4(to + 2 * L::kHeldPiece, l[0], l[1], l[2], l[3]);
+          }
+        }
+        fence_async_shared();
+      }
       if (check.bad()) again |= 1u << k;
     };
-    put_held(0);
+    put_held(it, 0);
     warp_arrives(ring(kGo, 0));
     const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo);
     int t = 0;
     for (int k = 0;; ++k) {
       const int i = it.first + row;
-      float top = -INFINITY, shift = 0.f, denom = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
+      float denom[L::kShares] = {};
+      float top = -INFINITY, shift = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
       float shrink = 0.f;                               // what the sums so far are multiplied with when the last tile's product comes
       uint64_t acc[OW / 2];
 #pragma unroll
@@ -971,12 +880,16 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
       auto gather_product = [&](int t) {  // of tile t
         ok = ok && warp_waits<false>(ring(kWeighed, t), ring_parity(t), g.status, 0x0a22u);
         tc_fence_after_sync();
-        uint32_t o[OW];
-        tmem_ld<OW>(lanes + L::kO + group * OW, o);
-        tmem_ld_wait();
         const uint64_t shrink2 = f2_pack(shrink, shrink);
+        constexpr int N = OW > 32 ? 16 : OW;  // columns at a time
 #pragma unroll
-        for (int c = 0; c < OW / 2; ++c) acc[c] = f2_fma(acc[c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
+        for (int part = 0; part < OW; part += N) {
+          uint32_t o[N];
+          tmem_ld<N>(lanes + L::kO + group * OW + part, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < N / 2; ++c) acc[part / 2 + c] = f2_fma(acc[part / 2 + c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
+        }
       };
       Item next = it;
       bool more = false;
@@ -987,6 +900,16 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
         tc_fence_after_sync();
         uint32_t s[CW];
         tmem_ld<CW>(lanes + L::kS + group * CW, s);
+        if constexpr (L::kTwo) {
+#pragma unroll
+          for (int part = 0; part < CW; part += 16) {
+            uint32_t more_s[16];
+            tmem_ld<16>(lanes + L::kS2 + group * CW + part, more_s);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 16; ++c) s[part + c] = __float_as_uint(__uint_as_float(s[part + c]) + __uint_as_float(more_s[c]));
+          }
+        }
         if (j == 0) {
           more = item(k + 1, next);
           if (more) fetch(next);
@@ -1017,18 +940,21 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
         top = raised, shift = moved;
         const uint64_t minus_shift = f2_pack(-shift, -shift);
         uint64_t w[CW / 2];
-        uint64_t sum = 0;
+        uint64_t sum[L::kShares] = {};
 #pragma unroll
         for (int c = 0; c < CW / 2; ++c) {
           const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
           float x0, x1;
           f2_unpack(f2_fma(s2, c_lo, f2_fma(s2, c_hi, minus_shift)), x0, x1);
           w[c] = f2_pack(exp2_approx(x0), exp2_approx(x1));
-          sum = f2_add(sum, w[c]);
+          sum[c * L::kShares / (CW / 2)] = f2_add(sum[c * L::kShares / (CW / 2)], w[c]);
         }
-        float sum0, sum1;
-        f2_unpack(sum, sum0, sum1);
-        denom = fmaf(denom, less, sum0 + sum1);  // this thread's share; the shares meet after the last tile
+#pragma unroll
+        for (int c = 0; c < L::kShares; ++c) {
+          float sum0, sum1;
+          f2_unpack(sum[c], sum0, sum1);
+          denom[c] = fmaf(denom[c], less, sum0 + sum1);  // this thread's shares; they meet after the last tile
+        }
         if (j > 0) gather_product(t - 1);
         shrink = less;
         // (the product of the tile before has been gathered, so its P has been read)
@@ -1039,17 +965,20 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
         warp_arrives(ring(kReady, t));
       }
       if (more) {
-        put_held(k + 1);
+        put_held(next, k + 1);
         warp_arrives(ring(kGo, t));
       }
       gather_product(t - 1);
       tc_fence_before_sync();
-      if (!(denom < INFINITY)) again |= 1u << k;
-      exchange[t & 1][group][row] = denom;
+#pragma unroll
+      for (int c = 0; c < L::kShares; ++c) {
+        if (!(denom[c] < INFINITY)) again |= 1u << k;
+        exchange[t & 1][group * L::kShares + c][row] = denom[c];
+      }
       meet();
       float total = 0.f;
 #pragma unroll
-      for (int c = 0; c < G; ++c) total += exchange[t & 1][c][row];
+      for (int c = 0; c < G * L::kShares; ++c) total += exchange[t & 1][c][row];
       meet();  // (the next item's first maxima may go there)
       if (ok) {
 #pragma unroll
@@ -1629,28 +1558,29 @@ int launch_sized(Op op, const Problem& p) {
   void (*kernel)(const Params) = nullptr;
   uint32_t shared = 0, threads = 0;
   long long grid = blocks;
-  if constexpr (HD > 64) {
-    using F = FwdWide<HD, kWide>;
+  const bool one_each = blocks <= sms;
+  bool roles = true;
+  if (op == Op::Fwd) {
+    kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
+  } else if constexpr (HD > 64) {
     using B = BwdWide<HD, kWide>;
-    kernel = op == Op::Fwd ? f32_fwd_wide_kernel<HD, kWide> : op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
-    shared = op == Op::Fwd ? F::kBytes : B::kBytes, threads = B::kThreads;
+    kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
+    shared = B::kBytes, threads = B::kThreads;
+    roles = false;
+  } else if (op == Op::BwdQ) {
+    kernel = one_each ? f32_bwd_kernel<HD, false, kWide, 2> : f32_bwd_kernel<HD, false, kWide, 4>;
+    shared = Bwd<HD, false>::kBytes, threads = one_each ? Roles<2>::kThreads : Roles<4>::kThreads;
   } else {
-    const bool one_each = blocks <= sms;
-    if (op == Op::Fwd) {
-      kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
-    } else if (op == Op::BwdQ) {
-      kernel = one_each ? f32_bwd_kernel<HD, false, kWide, 2> : f32_bwd_kernel<HD, false, kWide, 4>;
-      shared = Bwd<HD, false>::kBytes, threads = one_each ? Roles<2>::kThreads : Roles<4>::kThreads;
-    } else {
-      kernel = f32_bwd_kernel<HD, true, kWide, 4>, shared = Bwd<HD, true>::kBytes, threads = Roles<4>::kThreads;
-    }
+    kernel = f32_bwd_kernel<HD, true, kWide, 4>, shared = Bwd<HD, true>::kBytes, threads = Roles<4>::kThreads;
+  }
+  if (roles) {
     // every SM has its block, and they are done together: as many blocks to an SM one after the other as the limit on a
     // block's items asks for
     const long long turn = static_cast<long long>(sms) * kMostItems;
     grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
-  const int which = op == Op::BwdQ && HD <= 64 && blocks <= sms ? 3 : static_cast<int>(op);
+  const int which = op == Op::BwdQ && one_each ? 3 : static_cast<int>(op);
   static bool sized[64][4] = {};
   int device = 0;
   LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");

@@ -203,7 +203,8 @@ def test_truncated_scores_do_not_show_in_l(t_q, t_k, hd):
 
 
 @pytest.mark.parametrize(("bh", "t_q", "t_k", "hd", "hd_v", "causal"), [(4800, 70, 70, 32, 32, True), (4800, 66, 130, 64, 40, False), (300, 200, 200, 37, 33, True),
-                                                                        (100, 257, 257, 64, 64, True), (37, 1000, 65, 24, 24, False)])
+                                                                        (100, 257, 257, 64, 64, True), (37, 1000, 65, 24, 24, False), (320, 130, 130, 100, 128, True),
+                                                                        (200, 129, 257, 128, 70, False), (4740, 33, 65, 80, 80, False)])
 def test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
     """A block of the kernels that work in roles goes through several work items (one round, several, and more than a block may
     take): a problem has the same bits wherever it comes, also where the item before or after it leaves the tensor cores (hidden rows of V
