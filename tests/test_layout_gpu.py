@@ -185,6 +185,63 @@ def test_cross_attention_out_of_a_key_value_projection_gives_the_dense_bits(t_q,
     np.testing.assert_array_equal(runtime.download(lse, np.uint32, (batch, heads, t_q)), want["lse"].view(np.uint32))
 
 
+@pytest.mark.parametrize("t_q,t_k,hd,causal", [(131, 131, 72, True), (100, 129, 120, False), (130, 70, 64, False), (33, 33, 8, True), (257, 250, 128, False), (96, 513, 40, False)])
+def test_results_leave_what_lies_between_their_rows_alone(t_q, t_k, hd, causal):
+    """Results whose rows, heads and batches have room between them: the epilogues exchange and stage pieces of neighbouring rows, and
+    write the rows and columns there are, bit for bit, and nothing else."""
+    import ctypes
+
+    from limn_b200 import runtime
+    from limn_b200._lib import check, lib
+
+    L = lib()
+    batch, heads = 2, 3
+    dense = _inputs(41, batch, heads, t_q, t_k, hd, BF16)
+    want = _run("bhtd", dense, None, batch, heads, t_q, t_k, hd, causal, BF16)
+    q, k, v, do = (runtime.upload(a) for a in dense)
+
+    def packed(t):
+        return heads * t * hd, t * hd, hd
+
+    def roomy(t):  # (batch, heads, t + 1, hd + 8)
+        return heads * (t + 1) * (hd + 8), (t + 1) * (hd + 8), hd + 8
+
+    def result(t):
+        return runtime.empty(2 * batch * heads * (t + 1) * (hd + 8))
+
+    out, dq, dk, dv = result(t_q), result(t_q), result(t_k), result(t_k)
+    lse, delta = runtime.empty(batch * heads * t_q * 4), runtime.empty(batch * heads * t_q * 4)
+    arr = lambda *triples: (ctypes.c_longlong * (3 * len(triples)))(*[x for tr in triples for x in tr])
+    tail = (2, batch, heads, t_q, t_k, hd, hd, int(causal), hd**-0.5, None)
+    a, b = packed(t_q), packed(t_k)
+    check(L.limn_b200_sdpa_fwd_strided(q.ptr, k.ptr, v.ptr, None, out.ptr, lse.ptr, arr(a, b, b, roomy(t_q)), *tail), "sdpa")
+    check(L.limn_b200_sdpa_bwd_q_fused_strided(q.ptr, k.ptr, v.ptr, out.ptr, do.ptr, lse.ptr, None, dq.ptr, delta.ptr, arr(a, b, b, roomy(t_q), a, roomy(t_q)), *tail), "dq")
+    check(L.limn_b200_sdpa_bwd_kv_strided(q.ptr, k.ptr, v.ptr, do.ptr, lse.ptr, delta.ptr, None, dk.ptr, dv.ptr, arr(a, b, b, a, roomy(t_k), roomy(t_k)), *tail), "dk, dv")
+    runtime.synchronize()
+    assert runtime.device_status() == 0
+    for buf, t, name in ((out, t_q, "out"), (dq, t_q, "dq"), (dk, t_k, "dk"), (dv, t_k, "dv")):
+        got = runtime.download(buf, np.uint16, (batch, heads, t + 1, hd + 8))
+        assert (got[:, :, t:] == 0xFFFF).all() and (got[..., hd:] == 0xFFFF).all(), name
+        inner = np.ascontiguousarray(got[:, :, :t, :hd])
+        if name == "out":
+            np.testing.assert_array_equal(inner, want[name].view(np.uint16))
+        else:  # the fused row dot sums in another order than the reduce kernel
+            np.testing.assert_allclose(widen(inner.view(BF16)), widen(want[name]), rtol=2**-7, atol=2e-3, err_msg=name)
+
+
+@pytest.mark.parametrize("t_q,t_k,hd", [(513, 200, 64), (700, 129, 40), (1100, 65, 64)])
+def test_key_blocks_one_after_the_other_give_the_bits_of_one_alone(t_q, t_k, hd):
+    """The dK/dV pass without masks from five query tiles on: a block's results are taken out while it is at its next item. More items
+    than SMs, against launches of three problems."""
+    batch, heads = 57, 3
+    arrays = _inputs(43, batch, heads, t_q, t_k, hd, BF16)
+    got = _run("bhtd", arrays, None, batch, heads, t_q, t_k, hd, False, BF16)
+    for at in (0, 28, 49, 56):
+        want = _run("bhtd", [x[at : at + 1] for x in arrays], None, 1, heads, t_q, t_k, hd, False, BF16)
+        for name in ("dk", "dv", "dq", "out"):
+            np.testing.assert_array_equal(got[name][at].view(np.uint16), want[name][0].view(np.uint16), err_msg=f"{name} of batch {at}")
+
+
 def test_dense_layout_code_is_the_dense_entry_point():
     from limn_b200 import runtime
     from limn_b200._lib import check, lib
