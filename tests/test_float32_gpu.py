@@ -222,10 +222,12 @@ def test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
         assert np.array_equal(g[picks], a), what
 
 
-@pytest.mark.parametrize(("t_q", "t_k", "hd_v", "causal"), [(130, 130, 64, True), (70, 200, 40, False), (200, 65, 100, False), (129, 129, 128, True), (33, 70, 17, False)])
+@pytest.mark.parametrize(("t_q", "t_k", "hd_v", "causal"), [(130, 130, 64, True), (70, 200, 40, False), (200, 65, 100, False), (129, 129, 128, True), (33, 70, 17, False),
+                                                            (70, 70, 200, False), (100, 33, 130, True)])
 def test_rows_are_divided_to_the_nearest(t_q, t_k, hd_v, causal):
-    """The forward's quotients come from one reciprocal a row where the row's columns are of an ordinary size, from divisions where they are
-    not. Powers of two go through everything else as they are: the same bits either way, so the former are rounded like the latter."""
+    """The forward's quotients (on the tensor cores, and in the tiled kernels above 128 columns) come from one reciprocal a row where the
+    row's columns are of an ordinary size, from divisions where they are not. Powers of two go through everything else as they are: the same
+    bits either way, so the former are rounded like the latter."""
     q, k, v, do = _problem(t_q + hd_v, 20, t_q, t_k, 32, hd_v)
     mask = np.ones((20, t_k), np.float32)
     ordinary = _step(q, k, v, do, mask, causal, 32**-0.5)[0]
