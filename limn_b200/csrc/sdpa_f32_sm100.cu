@@ -1628,25 +1628,27 @@ int launch_sized(Op op, const Problem& p) {
 
 // Many short problems are better off in the tiled CUDA-core kernels: with both sides inside one 64-row tile half of a block's
 // 128 rows are empty, a head dim below the kernel's width is padding, and a block's fixed cost is all there is, while several
-// of their 256-thread blocks share an SM. Measured on B200 as time here over time there, 16 x 16 to 64 x 64 rows:
-//   forward  head dims 8 and 16: 0.9-1.1 at 256 problems, 1.2-1.5 at 384 and more; 24: 1.07-1.2 from 384 on; 32: 0.65-0.8;
-//            72 to 128 with up to 32 keys: 1.1-1.8 from 256 problems on (beyond 32 keys 1.1 at 72, 0.7 at 128)
-//   dQ       8 and 16: 1.0-1.3 at 256 and 384 problems, 1.1-1.7 beyond; 32: 0.95-1.05 at 512, 1.0-1.2 beyond; 72 and 100 with
-//            up to 32 keys 1.04-1.4; 128 with up to 16 keys 0.9-1.1
-//   dK, dV   8: 1.0-1.1 at 384; 8 and 16: 1.0-1.2 at 512, 1.1-1.4 beyond; 32 with up to 32 queries 0.9-1.05 at 512, 1.04-1.13
-//            beyond; 72 to 128: 0.5-0.9
-// At head dim 64 all three gain here (0.5-1.0), at 40 all but dQ of thousands of problems of 16 rows (1.1); so does everything at
-// 128 problems, one block to an SM (0.5-0.9, the forward at 72 with up to 32 keys 1.1), and nearly everything from 65 rows on.
+// of their 256-thread blocks share an SM. Measured on B200 as time here over time there, 16 x 16 / 32 x 32 / 64 x 64 rows:
+//   forward  8: 1.23-1.35 / 1.20-1.29 / 1.09-1.19; 16: 1.14-1.23 / 1.11-1.18 / 1.03-1.10; 24: 1.08-1.14 / 1.05-1.10 / 0.97-0.99;
+//            32: 1.03-1.05 / 0.99-1.02 / 0.86-0.94; 40: 0.7-0.95; 72: 1.1-1.36 / 1.0-1.3 / 0.63-0.77; 100: 1.04-1.26 / 0.97-1.2 /
+//            0.55-0.72; 128: 0.98-1.18 / 0.88-1.13 / 0.51-0.68
+//   dQ       8: 0.88-1.25; 16: 0.67-1.13; 24: 0.58-1.0; 32: 0.56-0.93; 72: 1.31-1.46 / 1.09-1.34 / 0.6-0.8; 100: 1.16-1.27 / 1.02-1.18 /
+//            0.56-0.7; 128: 1.05-1.13 / 0.89-1.08 / 0.53-0.66
+//   dK, dV   8, up to 256 problems 0.94-1.07 and beyond 0.85-0.97 / 0.85-0.94 / 0.76-0.85; 16: 0.8-0.98 / 0.77-0.95 / 0.59-0.88; 24 and 32:
+//            0.48-0.9; 72: 0.83-1.01; more: 0.35-0.9
+// At head dim 64 all three gain here (0.4-0.96), and so does everything at 128 problems, one block to an SM, and from 65 rows on. What
+// is nearer to float64 on one side stays there: the forward at up to 24 with at most two problems to an SM here, dQ and dK below 24 there
+// (2-norm, here over there: dQ 0.94-1.09, dK 0.94-1.12; from 24 on 0.75-0.98, dK at 16 with 32 queries or more 0.92-0.98).
 bool short_rows(Op op, const Problem& p) {
   if (p.t_q > 64 || p.t_k > 64) return false;
   int sms = 0;
   if (sm_count(&sms) != LIMN_B200_OK || p.bh <= sms) return false;
   const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
   if (widest > 64) return op == Op::Fwd ? p.t_k <= 32 : op == Op::BwdQ && p.t_k <= (widest <= 100 ? 32 : 16);
-  if (widest > 32) return false;
-  if (widest <= 16) return op == Op::BwdQ || p.bh > (op == Op::Fwd ? 2LL : 3LL) * sms;
   if (op == Op::Fwd) return widest <= 24 && p.bh > 2LL * sms;
-  return p.bh > 4LL * sms && (op == Op::BwdQ || p.t_q <= 32);
+  if (widest >= 24) return false;
+  if (widest > 16) return p.bh > 4LL * sms && (op == Op::BwdQ || p.t_q <= 32);
+  return op == Op::BwdQ || (p.bh > 3LL * sms && (widest < 16 || p.t_q < 32));
 }
 
 }  // namespace
