@@ -11,23 +11,28 @@
 //
 // What bounds it: six bfloat16 products at 4096 multiply-adds a clock and SM are 683 float32 multiply-adds a clock,
 // against 128 on the CUDA cores; the split, the softmax and the running totals stay there and take about as long as the
-// MMAs (dQ at head dim 64: 2 300 and 2 500 clocks of a tile's 3 700). Measured on B200 (forward / dQ / dK and dV, us, causal;
-// the CUDA-core kernels in brackets): 256 x 256 keys x 64: 38 / 55 / 71 (121 / 166 / 219); 6 x 8192 x 32: 282 / 286 / 399
-// (1333 / 1777 / 2402); 64 x 1024 x 128: 170 / 224 / 289 (813 / 1117 / 1714); 64 x 32 x 64: 7.3 / 7.6 / 9.2 (10.8 / 12.4 /
-// 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.4e-7 for 6.1e-7, dQ 3.2e-7 for 7.6e-7
-// in the 2-norm), and so is L (256 x 256 x 64: 2.9e-8 for 3.5e-8; rounding it once is 2.6e-8).
+// MMAs (dQ at head dim 64, clocks a tile: row warps 2 500, MMAs 2 300, splitting warps 3 800 with the loads). Up to head dim 64, and above
+// in the forward, a block's warps have roles: row warps (a row to two or four threads: softmax or dS, the split of their operand, the
+// totals), splitting warps (the streamed tiles, from global memory to three pieces in shared memory) and one that issues the MMAs;
+// they meet at barriers only, a block takes up to 32 items one after the other, and a tile's scores, the products of the one before
+// and the split of the ones behind go on at the same time. Measured on B200 (forward / dQ / dK and dV, us, causal; before the roles; in
+// brackets the CUDA-core kernels): 256 x 256 keys x 64: 31 / 45 / 50, 39 / 61 / 73 (121 / 166 / 219); 6 x 8192 x 32: 225 / 231 / 290, 291 / 290 /
+// 389 (1333 / 1777 / 2402); 64 x 1024 x 128: 121 / 225 / 275, 178 / 227 / 293 (813 / 1117 / 1714); 64 x 32 x 64: 6.9 / 8.8 / 8.5, 7.3 / 8.4 /
+// 9.2 (10.8 / 12.4 / 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.4e-7 for 6.1e-7, dQ 3.2e-7
+// for 7.6e-7 in the 2-norm), and so is L (256 x 256 x 64: 2.9e-8 for 3.5e-8; rounding it once is 2.6e-8).
 //
-// A block owns 128 rows (query rows in the forward and the dQ pass, key rows in the dK/dV pass), one row to each
+// A block owns 128 rows at a time (query rows in the forward and the dQ pass, key rows in the dK/dV pass), one row to each
 // tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
 // with ordinary loads (the split has to pass through registers anyway), split and left in shared memory in the
-// 128-byte-swizzled layout; probabilities and dS are split in registers and go to tensor memory as the A operand.
+// 128-byte-swizzled layout, or in tensor memory where they are held; probabilities and dS are split in registers and go to tensor
+// memory as the A operand.
 //
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
 // number (inf - inf in the split, inf * 0 between pieces), and one below about 2^-110 would lose its last bits. The split
 // notices both, and a block that met one computes its rows again on the CUDA cores, with the code of the tiled kernels
-// there (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 213 / 1 984 / 2 548, the tiled
-// kernels alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500). The forward and the backward above
-// head dim 64 leave their loop when they meet one; the backward up to 64, whose warps run apart, goes on to its end first.
+// there. The backward above head dim 64 leaves its loop when it meets one; the others, whose warps run apart, go on to their end first and
+// then do the items again (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 470 / 1 980 / 2 570, the tiled kernels
+// alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -1064,9 +1069,10 @@ struct Bwd {
   static constexpr uint32_t kBytes = kHeld1 + (kHeldT ? kHeldRaw : kHeldPieces) + 1024;
 };
 
-// kGroups threads to a row (and the split of the warps that goes with it): the same bits either way. Two are faster where a block has
-// one item (2 x 128 x 32 7.8 us for 8.4), as the splitting warps have it ready sooner, four in the long run (6 x 8192 x 32 causal 233 for 239,
-// 256 x 512 x 64 143 for 150; two spill).
+// kGroups threads to a row (and the split of the warps that goes with it): the same bits either way. Two are faster in dQ up to head dim 32
+// where a block has one item (2 x 128 x 32 7.7 us for 8.3, 64 x 128 8.6 for 8.9, 2 x 8192 152 for 156), as the splitting warps have it ready
+// sooner; four in the long run (6 x 8192 x 32 causal 233 for 239) and at head dim 64 (64 x 128 x 64 11.5 for 12.1, 16 x 600 x 64 23.4 for
+// 26.8, 256 x 512 x 64 143 for 150; two spill).
 template <int HD, bool kKV, bool kWide, int kGroups>
 __global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
   using L = Bwd<HD, kKV>;
@@ -1589,7 +1595,7 @@ int launch_sized(Op op, const Problem& p) {
   void (*kernel)(const Params) = nullptr;
   uint32_t shared = 0, threads = 0;
   long long grid = blocks;
-  const bool one_each = blocks <= sms;
+  const bool two = HD <= 32 && op == Op::BwdQ && blocks <= sms;  // threads to a row (see f32_bwd_kernel)
   bool roles = true;
   if (op == Op::Fwd) {
     kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
@@ -1599,8 +1605,9 @@ int launch_sized(Op op, const Problem& p) {
     shared = B::kBytes, threads = B::kThreads;
     roles = false;
   } else if (op == Op::BwdQ) {
-    kernel = one_each ? f32_bwd_kernel<HD, false, kWide, 2> : f32_bwd_kernel<HD, false, kWide, 4>;
-    shared = Bwd<HD, false>::kBytes, threads = one_each ? Roles<2>::kThreads : Roles<4>::kThreads;
+    kernel = f32_bwd_kernel<HD, false, kWide, 4>, shared = Bwd<HD, false>::kBytes, threads = Roles<4>::kThreads;
+    if constexpr (HD <= 32)
+      if (two) kernel = f32_bwd_kernel<HD, false, kWide, 2>, threads = Roles<2>::kThreads;
   } else {
     kernel = f32_bwd_kernel<HD, true, kWide, 4>, shared = Bwd<HD, true>::kBytes, threads = Roles<4>::kThreads;
   }
@@ -1611,7 +1618,7 @@ int launch_sized(Op op, const Problem& p) {
     grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
-  const int which = op == Op::BwdQ && one_each ? 3 : static_cast<int>(op);
+  const int which = two ? 3 : static_cast<int>(op);
   static bool sized[64][4] = {};
   int device = 0;
   LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");
