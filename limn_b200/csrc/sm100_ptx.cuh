@@ -496,6 +496,7 @@ __device__ __forceinline__ void store_rows32(unsigned char* to, long long row_by
       if (first + top + r < rows && 8 * piece < cols_left) *reinterpret_cast<uint4*>(at) = make_uint4(w[r][0], w[r][1], w[r][2], w[r][3]);
   } else {
     auto place = [&](int row, int piece) { return stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)); };  // 8 rows' pieces on distinct banks
+    __syncwarp();  // the other lanes have read what lay there before
 #pragma unroll
     for (int v4 = 0; v4 < 4; ++v4) st_shared_v4(place(lane, v4), w[v4][0], w[v4][1], w[v4][2], w[v4][3]);
     __syncwarp();

@@ -242,6 +242,20 @@ def test_key_blocks_one_after_the_other_give_the_bits_of_one_alone(t_q, t_k, hd)
             np.testing.assert_array_equal(got[name][at].view(np.uint16), want[name][0].view(np.uint16), err_msg=f"{name} of batch {at}")
 
 
+@pytest.mark.parametrize("dtype", [BF16, np.dtype(np.float16)], ids=["bf16", "f16"])
+@pytest.mark.parametrize("t_q,hd", [(250, 64), (384, 56)])
+def test_rows_staged_item_after_item_are_the_rows_of_one_item(t_q, hd, dtype):
+    """A warp whose rows go by way of shared memory uses the same bytes for the next item's rows: more items than SMs, against one problem
+    alone."""
+    batch, heads = 80, 5
+    arrays = _inputs(44, batch, heads, t_q, 100, hd, dtype)
+    got = _run("bhtd", arrays, None, batch, heads, t_q, 100, hd, False, dtype)
+    for at in (0, 41, 79):
+        want = _run("bhtd", [x[at : at + 1, 4:] for x in arrays], None, 1, 1, t_q, 100, hd, False, dtype)
+        for name in ("out", "dq"):
+            np.testing.assert_array_equal(got[name][at, 4].view(np.uint16), want[name][0, 0].view(np.uint16), err_msg=f"{name} of batch {at}")
+
+
 def test_dense_layout_code_is_the_dense_entry_point():
     from limn_b200 import runtime
     from limn_b200._lib import check, lib
