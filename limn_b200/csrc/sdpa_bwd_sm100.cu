@@ -70,16 +70,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 #endif
 constexpr int kPolyPairsOf8 = LIMN_BWD_POLY_PAIRS;
 
-// How results that are not tile-stored leave. Measured, us, every thread its own row / pieces of neighbouring rows exchanged first / staged
-// by the warp: dQ of 192 padded problems of 500 x 64 41.8 / 39.7 / 40.1; causal at head dim 64, 256 of 256 18.5 / 19.0 / 18.7 and 64 of 1024
-// 26.5 / - / 27.0 (but 256 of 128 11.5 / 11.1 / 11.1); head dim 128, where shared memory has no room, 160 causal of 3000 and 128 of 1024
-// dQ 531 / 517 and 105 / 101, dK and dV 684 / 658 and 133 / 125.
-template <int D, bool kCausal>
-constexpr RowStore row_store() {
-  return D == 128 ? RowStore::kExchanged : kCausal ? RowStore::kOwn : RowStore::kStaged;
-}
-
-template <int D, bool kKV, bool kMask>
+template <int D, bool kKV, RowStore kStore>
 struct BwdLayout {
   static constexpr int kTileBytes = kTile * D * 2;
   static constexpr int kAtomBytes = kTile * 128;
@@ -94,11 +85,10 @@ struct BwdLayout {
   // 128 rows x 128 B in the swizzled layout and TMA stores them, instead of every thread storing its own row in
   // 16-byte pieces (32 transactions per instruction for the load/store unit: 2 000 clocks per work item). Measured:
   // 13 % off the pass at S = 256, 2 % at S = 2048. In the dQ pass, where a thread stores half a row, the hand-overs
-  // cost as much as they save (+2 % at S = 2048), so it keeps storing from registers.
+  // cost as much as they save (+2 % at S = 2048): its rows, and all rows at head dim 128, leave as kStore says (see rows_leave).
   static constexpr bool kTileStore = D == 64 && kKV;
   static constexpr int kStoreOff = kStreamBOff + kStagesB * kTileBytes;
-  // The others: see row_store.
-  static constexpr int kWarpStage = D == 64 && !kKV ? 2048 : 0;  // of each elementwise warp, for 32 columns of its rows
+  static constexpr int kWarpStage = kStore == RowStore::kStaged ? 2048 : 0;  // of each elementwise warp, for 32 columns of its rows
   static constexpr int kStatOff = kStoreOff + (kTileStore ? (kKV ? 2 : 1) * kAtomBytes : 8 * kWarpStage);
   static constexpr int kBarOff = kStatOff + (kKV ? 8 * 2 * 2 * 64 * 4 : 0);  // dK/dV pass, per warp [2 buffers][128 floats]: statistics of the streamed queries
   static constexpr int kBytes = kBarOff + 512 + 1024;
@@ -116,7 +106,7 @@ struct BwdLayout {
 
 template <int D, bool kKV, bool kMask>
 struct BwdBars {
-  static constexpr int kSA = BwdLayout<D, kKV, kMask>::kStagesA, kSB = BwdLayout<D, kKV, kMask>::kStagesB;
+  static constexpr int kSA = BwdLayout<D, kKV, RowStore::kOwn>::kStagesA, kSB = BwdLayout<D, kKV, RowStore::kOwn>::kStagesB;
   static constexpr int held_full = 0;
   static constexpr int a_full = 1;                // + slot
   static constexpr int a_empty = a_full + kSA;
@@ -221,12 +211,12 @@ __device__ __forceinline__ float row_dot(const void* a_row, const void* b_row, i
 // S^T and dP^T take turns in one 128-column region, S^T first, dP^T as soon as S^T is in registers, so that
 // 128 columns are left for the operands and every MMA is full width.
 // kDefer: an item's results are taken out after the elementwise stage of the next item's first tile (see launch_bwd).
-template <int D, bool kCausal, bool kFp16, bool kKV, bool kEarly, bool kSeq, bool kMask, bool kDefer>
+template <int D, bool kCausal, bool kFp16, bool kKV, bool kEarly, bool kSeq, bool kMask, bool kDefer, RowStore kStore>
 __global__ void __launch_bounds__((bwd_threads<D, kCausal, kKV, kMask>()), 1)
 sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                 const __grid_constant__ CUtensorMap map_out0, const __grid_constant__ CUtensorMap map_out1, const BwdParams prm) {
-  using L = BwdLayout<D, kKV, kMask>;
+  using L = BwdLayout<D, kKV, kStore>;
   using B = BwdBars<D, kKV, kMask>;
   extern __shared__ unsigned char smem_unaligned[];
   __shared__ uint32_t tmem_slot;
@@ -566,9 +556,10 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           if (got) got = waits(b_full(it), b_wrap(it), 0x1211u);
           return got;
         };
-        // Two ways round the items. The first can have an item's first scores issued ahead (kDefer), and the dQ pass without a causal mask is 1 to
-        // 2 % faster with it all the same; 256 causal problems of 256 x 64 take 18.5 us with the second and 19.0 with the first.
-        if constexpr (kDefer || (!kKV && !kCausal)) {
+        // Two ways round the items, in the same order. The first can have an item's first scores issued ahead (kDefer), and a dQ pass whose rows are
+        // staged is faster with it all the same (256 problems of 2048 x 64 462 us, 473 with the second); the others are not (148 of 32 x 64 6.8 and 6.6
+        // us, 700 of 160 x 80 57.3 and 56.8, 256 causal ones of 256 x 64 19.0 and 18.5).
+        if constexpr (kDefer || (!kKV && kStore == RowStore::kStaged)) {
           auto take = [&](unsigned n_item, unsigned& index, int& count) {
             if constexpr (kKV) {
               Item taken;
@@ -826,13 +817,12 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           uint32_t acc[32];
           tmem_ld32(t_acc + 32 * c, acc);
           tmem_ld_wait();
-          store_rows32<kFp16, RowStore::kExchanged>(to + 64 * c, 2 * mine.row, top, prm.t_k, acc, mul, (group == 0 ? prm.width_v : prm.width) - 32 * c);
+          const int left = (group == 0 ? prm.width_v : prm.width) - 32 * c;
+          if constexpr (kStore != RowStore::kOwn) store_rows32<kFp16, kStore>(to + 64 * c, 2 * mine.row, top, prm.t_k, acc, mul, left);
+          else if (top + lane < prm.t_k) store_row32<kFp16>(to + 2 * lane * mine.row + 64 * c, acc, mul, left);
         }
       } else {
         // each group writes half of its queries' dQ rows
-        const int row = of.own0 + r;
-        const bool in = row < prm.t_q;
-        const long long out_at = of.batch * prm.out_strides.batch + of.head * prm.out_strides.head + row * prm.out_strides.row;
         unsigned char* to = static_cast<unsigned char*>(prm.out0) + 2 * (of.batch * prm.out_strides.batch + of.head * prm.out_strides.head + top * prm.out_strides.row);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
@@ -841,10 +831,10 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           uint32_t acc[32];
           tmem_ld32(tmem + lane_base + L::kAcc0 + col, acc);
           tmem_ld_wait();
-          if constexpr (row_store<D, kCausal>() == RowStore::kOwn) {
-            if (in) store_row32<kFp16>(static_cast<unsigned char*>(prm.out0) + 2 * (out_at + col), acc, prm.scale, prm.width - col);
+          if constexpr (kStore == RowStore::kOwn) {
+            if (top + lane < prm.t_q) store_row32<kFp16>(to + 2 * (lane * prm.out_strides.row + col), acc, prm.scale, prm.width - col);
           } else {
-            store_rows32<kFp16, row_store<D, kCausal>()>(to + 2 * col, 2 * prm.out_strides.row, top, prm.t_q, acc, prm.scale, prm.width - col, base + L::kStoreOff + warp * L::kWarpStage);
+            store_rows32<kFp16, kStore>(to + 2 * col, 2 * prm.out_strides.row, top, prm.t_q, acc, prm.scale, prm.width - col, base + L::kStoreOff + warp * L::kWarpStage);
           }
         }
       }
@@ -1163,11 +1153,11 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 }
 
-template <int D, bool kCausal, bool kFp16, bool kKV, bool kMask, bool kDefer = false>
-int launch_bwd(const Problem& p) {
+template <int D, bool kCausal, bool kFp16, bool kKV, bool kMask, bool kDefer, RowStore kStore>
+int launch_bwd_s(const Problem& p) {
   constexpr bool kEarly = !kKV || D == 64;  // the dK/dV pass at head dim 128 has no spare tensor-memory columns ...
   constexpr bool kSeq = !kEarly;            // ... so there S^T and dP^T share one region, one after the other
-  using L = BwdLayout<D, kKV, kMask>;
+  using L = BwdLayout<D, kKV, kStore>;
   CUtensorMap map_q, map_k, map_v, map_do;
   const int heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh), batch = static_cast<int>(p.bh / heads);
   if (int rc = make_tile_map(&map_q, p.q, kFp16, batch, heads, p.t_q, p.hd, kTile, operand_strides(p, kOpQ, heads, p.t_q, p.hd))) return rc;
@@ -1229,7 +1219,7 @@ int launch_bwd(const Problem& p) {
   if (int rc = sm_count(&sms)) return rc;
   prm.group = work_group(p, items, sms);
   const long long ctas = items < sms ? items : sms;  // one CTA per SM, each fetching items until none is left
-  auto kernel = sdpa_bwd_kernel<D, kCausal, kFp16, kKV, kEarly, kSeq, kMask, kDefer>;
+  auto kernel = sdpa_bwd_kernel<D, kCausal, kFp16, kKV, kEarly, kSeq, kMask, kDefer, kStore>;
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64] = {};
   int device = 0;
@@ -1243,6 +1233,39 @@ int launch_bwd(const Problem& p) {
             "launching an sdpa backward kernel");
   note_launches(1);
   return LIMN_B200_OK;
+}
+
+// How the rows of dQ leave, and at head dim 128 those of dK and dV (at 64 they are tile-stored): each thread its own, exchanged (head dim
+// 128, where shared memory has no room), or staged (dQ at 64 without a causal mask). As in the forward, the latter two take a warp the same time however few
+// rows it has. Measured on B200, us, own / exchanged or staged, dense rows:
+//   dK and dV, 128 columns: 2000 problems of 32 42.7 / 48.2, of 48 47.7 / 48.4, of 64 52.9 / 48.9, of 128 79.7 / 62.7; 148 of 32 6.6 / 6.9, of 48 7.1 / 7.0;
+//     112 columns: 2000 of 48 45.1 / 48.7; 80 columns: 2000 causal of 64 47.8 / 50.0, of 80 51.1 / 50.9, 148 of 48 6.8 / 6.9, of 64 7.1 / 7.0
+//   dQ, 128 columns: 2000 of 32 61.9 / 65.6, of 48 64.8 / 67.5, of 64 75.7 / 71.9, of 128 122 / 112; 148 of 48 8.9 / 9.0; 80 columns: 2000 of 64
+//     63.5 / 67.1, of 80 68.6 / 70.0, of 112 79.5 / 76.9; 64 columns: 700 of 48 18.0 / 18.5, of 80 18.4 / 19.2, 2000 of 112 53.2 / 51.3, of 128 57.1 / 52.9;
+//     56 columns: 700 of 160 37.0 / 38.2, 200 of 384 24.6 / 23.1; 48 columns: 700 of 128 16.5 / 17.3, 148 of 512 23.5 / 23.7
+//   causal dQ at head dim 64: 256 of 256 18.5 / 18.7, 64 of 1024 26.5 / 27.0
+// and token-major with 12 heads (scattered_rows): dK and dV, 128 columns 204 of 32 9.9 / 9.8, of 64 12.2 / 9.9; dQ 204 of 32 11.7 / 11.7, of 64 14.2 / 13.4; 64 columns 204 of 64
+//   9.1 / 9.2, of 128 11.2 / 10.1.
+template <int D, bool kCausal, bool kKV>
+RowStore rows_leave(const Problem& p) {
+  const int rows = kKV ? p.t_k : p.t_q, widest = kKV && p.hd_v > p.hd ? p.hd_v : p.hd, heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh);
+  const long long size = 1LL * rows * widest;
+  constexpr RowStore kLong = D == 128 ? RowStore::kExchanged : kKV || kCausal ? RowStore::kOwn : RowStore::kStaged;
+  int sms = 0;
+  const bool one_item = sm_count(&sms) == LIMN_B200_OK && p.bh <= sms;  // to a block
+  bool pays;
+  if (scattered_rows(operand_strides(p, kKV ? kOpDk : kOpDq, heads, rows, p.hd).row, p.hd)) pays = size > 4096;
+  else if (D == 64) pays = p.hd > 48 && (p.hd < 64 ? rows > 2 * kTile : size > 5120);
+  else pays = rows >= kTile || size > (!kKV ? 6144 : one_item ? 4096 : 5632);
+  return pays ? kLong : RowStore::kOwn;
+}
+
+template <int D, bool kCausal, bool kFp16, bool kKV, bool kMask, bool kDefer = false>
+int launch_bwd(const Problem& p) {
+  constexpr RowStore kLong = D == 128 ? RowStore::kExchanged : kKV || kCausal ? RowStore::kOwn : RowStore::kStaged;
+  if constexpr (kLong != RowStore::kOwn)
+    if (rows_leave<D, kCausal, kKV>(p) == kLong) return launch_bwd_s<D, kCausal, kFp16, kKV, kMask, kDefer, kLong>(p);
+  return launch_bwd_s<D, kCausal, kFp16, kKV, kMask, kDefer, RowStore::kOwn>(p);
 }
 
 template <int D, bool kKV, bool kMask>

@@ -69,7 +69,7 @@ constexpr int poly_pairs_of_8() {
 #endif
 }
 
-template <int D, bool kCausal, bool kMask>
+template <int D, bool kCausal, RowStore kStore>
 struct FwdLayout {
   static constexpr int kTileBytes = kTileRows * D * 2;
   static constexpr int kAtomBytes = kTileRows * 128;        // one 64-element-wide column block of a tile
@@ -86,11 +86,8 @@ struct FwdLayout {
   // at head dim 128, -6 % at 64, measured).
   static constexpr bool kTileStore = D == 128 && kCausal;
   static constexpr int kStageOff = kVOff + kStages * kTileBytes;
-  // Without the tile store. A thread's own row, piece by piece, is 32 lines an instruction; measured on B200, us, own / exchanged / staged:
-  // 192 padded problems of 500 x 64 33.3 / 32.4 / 32.1, 128 of 1024 x 128 72.3 / 70.1 / 71.7, 64 of 100 x 1500 x 64 14.1 / 14.0 / 14.1;
-  // under a causal mask at head dim 64, where the last tiles' chain is all there is, 256 of 256 13.7 / 14.6 / 14.0, 256 of 128 9.0 / 9.4 / 9.1.
-  static constexpr RowStore kRowStore = D == 128 ? RowStore::kExchanged : kCausal ? RowStore::kOwn : RowStore::kStaged;
-  static constexpr int kWarpStage = kRowStore == RowStore::kStaged ? 4096 : 0;  // of each softmax warp, for two 32-column pieces of its rows
+  // Without it rows leave as kStore says (see rows_leave).
+  static constexpr int kWarpStage = kStore == RowStore::kStaged ? 4096 : 0;  // of each softmax warp, for two 32-column pieces of its rows
   static constexpr int kBarOff = kStageOff + (kTileStore ? kQTiles * kAtomBytes : 8 * kWarpStage);
   static constexpr int kBytes = kBarOff + 512 + 1024;       // room for 64 barriers + slack to align the base to 1024
   // tensor-memory columns
@@ -101,7 +98,7 @@ struct FwdLayout {
 // barrier indices inside the barrier block
 template <int D>
 struct FwdBars {
-  static constexpr int kS = FwdLayout<D, false, false>::kStages;
+  static constexpr int kS = FwdLayout<D, false, RowStore::kOwn>::kStages;
   static constexpr int q_full = 0;               // + t
   static constexpr int k_full = 2;               // + stage
   static constexpr int k_empty = k_full + kS;
@@ -150,11 +147,11 @@ struct FwdParams {
   float scale;
 };
 
-template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared>
+template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared, RowStore kStore>
 __global__ void __launch_bounds__((fwd_threads<D, kMask>()), 1)
 sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const FwdParams prm) {
-  using L = FwdLayout<D, kCausal, kMask>;
+  using L = FwdLayout<D, kCausal, kStore>;
   using B = FwdBars<D>;
   extern __shared__ unsigned char smem_unaligned[];
   __shared__ uint32_t tmem_slot;
@@ -708,18 +705,24 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         if (row < prm.t_q) prm.lse[out_row] = m * prm.scale + logf(l);
       } else {
-      const int top = item.q0[t] + (warp & 3) * 32;  // the warp's first row
-      const long long row_bytes = 2 * prm.out_strides.row;
-      unsigned char* to = static_cast<unsigned char*>(prm.out) + 2 * (item.batch * prm.out_strides.batch + item.head * prm.out_strides.head) + top * row_bytes;
+      if constexpr (kStore == RowStore::kOwn) {
+        const long long out_at = item.batch * prm.out_strides.batch + item.head * prm.out_strides.head + row * prm.out_strides.row;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        take(32 * c, o);
-        if constexpr (L::kRowStore == RowStore::kOwn) {
-          if (row < prm.t_q) store_row32<kFp16>(to + lane * row_bytes + 64 * c, o, inv, prm.width - 32 * c);
-        } else if (32 * c < prm.width && top < prm.t_q) {  // (256 x 2048 x 64 341 us without the second, 335 with it)
-          store_rows32<kFp16, L::kRowStore>(to + 64 * c, row_bytes, top, prm.t_q, o, inv, prm.width - 32 * c,
-                                            base + L::kStageOff + warp * L::kWarpStage + (c & 1) * (L::kWarpStage / 2));
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          take(32 * c, o);
+          if (row < prm.t_q) store_row32<kFp16>(static_cast<unsigned char*>(prm.out) + 2 * (out_at + 32 * c), o, inv, prm.width - 32 * c);
+        }
+      } else {
+        const int top = item.q0[t] + (warp & 3) * 32;  // the warp's first row
+        const long long row_bytes = 2 * prm.out_strides.row;
+        unsigned char* to = static_cast<unsigned char*>(prm.out) + 2 * (item.batch * prm.out_strides.batch + item.head * prm.out_strides.head) + top * row_bytes;
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          take(32 * c, o);
+          if (32 * c < prm.width && top < prm.t_q)  // (256 x 2048 x 64 341 us without the second, 335 with it)
+            store_rows32<kFp16, kStore>(to + 64 * c, row_bytes, top, prm.t_q, o, inv, prm.width - 32 * c, base + L::kStageOff + warp * L::kWarpStage + (c & 1) * (L::kWarpStage / 2));
         }
       }
       if (row < prm.t_q) prm.lse[out_row] = m * prm.scale + logf(l);
@@ -753,9 +756,9 @@ sdpa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 }
 
-template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared>
+template <int D, bool kCausal, bool kFp16, bool kMask, bool kShared, RowStore kStore>
 int launch_fwd_s(const Problem& p) {
-  using L = FwdLayout<D, kCausal, kMask>;
+  using L = FwdLayout<D, kCausal, kStore>;
   CUtensorMap map_q, map_k, map_v, map_o;
   const int heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh), batch = static_cast<int>(p.bh / heads);
   if (int rc = make_tile_map(&map_q, p.q, kFp16, batch, heads, p.t_q, p.hd, kTileRows, operand_strides(p, kOpQ, heads, p.t_q, p.hd))) return rc;
@@ -793,7 +796,7 @@ int launch_fwd_s(const Problem& p) {
   if (int rc = sm_count(&sms)) return rc;
   prm.group = work_group(p, items, sms);
   const long long ctas = items < sms ? items : sms;  // one CTA per SM (shared and tensor memory allow no more), each fetching items until none is left
-  auto kernel = sdpa_fwd_kernel<D, kCausal, kFp16, kMask, kShared>;
+  auto kernel = sdpa_fwd_kernel<D, kCausal, kFp16, kMask, kShared, kStore>;
   // the attribute is per device and per kernel instantiation; set it on first use there
   static bool sized[64] = {};
   int device = 0;
@@ -807,6 +810,39 @@ int launch_fwd_s(const Problem& p) {
             "launching the sdpa kernel");
   note_launches(1);
   return LIMN_B200_OK;
+}
+
+// How the rows of O leave without a causal mask. A thread's own row, piece by piece, is up to 32 lines of memory an instruction, but an
+// instruction touches only the rows there are; exchanging pieces (head dim 128) or going by way of shared memory (64) takes a warp the
+// same time whatever number of rows it has, in a chain of its own. So it is a matter of how full the tiles of rows are, of what a row
+// has of its kernel's width, and of how far apart rows lie (scattered_rows). Measured on B200, us, own / exchanged or staged, dense rows:
+//   128 columns: 700 problems of 32 17.7 / 21.8, of 96 19.0 / 22.2, of 128 19.6 / 20.3; 148 of 160 9.8 / 10.1, of 192 10.2 / 10.2, of 224 10.7 / 10.3, of
+//     256 10.8 / 9.9, of 272 18.0 / 18.6, of 384 (64 of them) 11.2 / 10.8
+//   80 columns: 700 of 128 17.0 / 18.3, 148 of 160 9.4 / 10.0, of 224 9.8 / 10.2, of 256 9.8 / 9.6, of 320 17.0 / 18.0; 200 of 256 15.3 / 14.8
+//   64 columns: 2000 of 64 39.8 / 43.4, of 128 37.2 / 36.3, 148 of 160 8.2 / 8.5, of 224 8.5 / 8.5, of 256 8.2 / 8.1, of 320 15.1 / 15.6, of 512 18.7 / 18.1;
+//     under a key mask 192 of 128 10.0 / 10.4, of 500 36.9 / 37.1, 400 of 2000 820 / 843
+//   48 columns: 2000 of 64 39.7 / 43.3, 148 of 256 8.1 / 8.2, of 320 14.7 / 15.4, of 512 18.4 / 18.3
+// Token-major with 12 heads: 128 columns 204 of 64 9.6 / 10.2, of 128 11.1 / 9.9, of 160 17.1 / 15.6; 64 columns 204 of 64 8.2 / 8.4, of 128 8.7 / 8.0, of 200
+//   13.8 / 13.2; under a key mask 192 of 256 14.4 / 12.9. With 5 heads 700 of 100 under a mask 21.7 / 22.9, at 128 columns 24.6 / 26.3.
+// Two groups that share the keys, dense: 128 columns 148 of 128 x 512 10.4 / 10.7; 64 columns 200 of 64 x 600 15.4 / 15.5, of 128 x 600 15.8 / 15.7, 700 of 100 x 1500
+//   71.8 / 70.4. Under a causal mask at head dim 64 own rows (256 of 256 13.7 / 14.0).
+template <int D, bool kMask, bool kShared>
+RowStore rows_leave(const Problem& p) {
+  constexpr RowStore kLong = D == 128 ? RowStore::kExchanged : RowStore::kStaged;
+  const int heads = p.heads > 0 ? p.heads : static_cast<int>(p.bh);
+  const long long missing = (kTileRows - p.t_q % kTileRows) % kTileRows, size = 1LL * p.t_q * p.hd_v;  // rows of the last tile; elements
+  bool pays;
+  if (scattered_rows(operand_strides(p, kOpOut, heads, p.t_q, p.hd_v).row, p.hd_v)) pays = size >= 112 * D;
+  else if (D == 128) pays = !kShared && p.t_q > kTileRows && (p.hd_v > 80 ? 3 : 8) * missing < p.t_q;
+  else if (kShared) pays = !kMask && p.hd_v > 48 && p.t_q >= 96;
+  else pays = !kMask && p.hd_v > 48 && size >= 64 * kTileRows && 8 * missing < p.t_q;
+  return pays ? kLong : RowStore::kOwn;
+}
+
+template <int D, bool kFp16, bool kMask, bool kShared>
+int launch_fwd_rows(const Problem& p) {
+  if (rows_leave<D, kMask, kShared>(p) == RowStore::kOwn) return launch_fwd_s<D, false, kFp16, kMask, kShared, RowStore::kOwn>(p);
+  return launch_fwd_s<D, false, kFp16, kMask, kShared, D == 128 ? RowStore::kExchanged : RowStore::kStaged>(p);
 }
 
 // A problem with one Q tile: its tile goes into both places, the even key tiles to the first and the odd ones to the second,
@@ -823,11 +859,13 @@ int launch_fwd_s(const Problem& p) {
 // tried too: a gain of 3 % at head dim 64, a loss of up to 24 % at 128, where the kernel then spills.)
 template <int D, bool kCausal, bool kFp16, bool kMask>
 int launch_fwd(const Problem& p) {
-  if constexpr (!kCausal) {  // (a causal problem of one Q tile has one key tile)
+  if constexpr (kCausal) {  // (a problem of one Q tile has one key tile)
+    return launch_fwd_s<D, kCausal, kFp16, kMask, false, RowStore::kOwn>(p);
+  } else {
     constexpr int kAlone = (D == 128 && !kMask) ? 2 * kTileRows : kTileRows;  // keys up to which one group takes them all
-    if (p.t_q <= kTileRows && p.t_k > kAlone) return launch_fwd_s<D, kCausal, kFp16, kMask, true>(p);
+    if (p.t_q <= kTileRows && p.t_k > kAlone) return launch_fwd_rows<D, kFp16, kMask, true>(p);
+    return launch_fwd_rows<D, kFp16, kMask, false>(p);
   }
-  return launch_fwd_s<D, kCausal, kFp16, kMask, false>(p);
 }
 
 template <int D, bool kMask>

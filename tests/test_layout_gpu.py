@@ -243,6 +243,52 @@ def test_key_blocks_one_after_the_other_give_the_bits_of_one_alone(t_q, t_k, hd)
 
 
 @pytest.mark.parametrize("dtype", [BF16, np.dtype(np.float16)], ids=["bf16", "f16"])
+@pytest.mark.parametrize("rows,all_rows,hd,causal", [(31, 127, 64, False), (79, 81, 64, False), (127, 128, 64, False), (200, 256, 64, False), (48, 49, 128, False), (32, 64, 128, True),
+                                                     (127, 128, 128, False), (50, 70, 96, True), (77, 78, 80, False), (128, 130, 80, False), (40, 256, 48, False), (19, 255, 72, False)])
+@pytest.mark.parametrize("batch", [1, 40])
+def test_a_row_leaves_with_the_same_bits_in_every_way(rows, all_rows, hd, causal, dtype, batch):
+    """Which way a kernel's rows leave depends on how many there are, of how many columns, and on how many problems: the first rows of a
+    problem, on either side of those lines, are the rows of the shorter problem. A row of dK and dV does not see the other keys either,
+    where it is given the row's own L and delta."""
+    from limn_b200 import runtime
+    from limn_b200._lib import DTYPE_CODES, check, lib
+
+    L = lib()
+    other, heads = (all_rows if causal else 100), 5
+    bh, code = batch * heads, DTYPE_CODES["bfloat16" if dtype == BF16 else "float16"]
+    q, k, v, do = (x.reshape(bh, -1, hd) for x in _inputs(45, batch, heads, all_rows, other, hd, dtype))
+    up = lambda x: runtime.upload(np.ascontiguousarray(x))
+
+    def forward_and_dq(n):
+        t_k = n if causal else other
+        ops = [up(x) for x in (q[:, :n], k[:, :t_k], v[:, :t_k], do[:, :n])]
+        out, dq, lse, delta = (runtime.empty(size) for size in (2 * bh * n * hd, 2 * bh * n * hd, 4 * bh * n, 4 * bh * n))
+        tail = (code, bh, n, t_k, hd, hd, int(causal), hd**-0.5, None)
+        check(L.limn_b200_sdpa_fwd(ops[0].ptr, ops[1].ptr, ops[2].ptr, None, out.ptr, lse.ptr, *tail), "sdpa")
+        check(L.limn_b200_sdpa_delta(out.ptr, ops[3].ptr, delta.ptr, code, bh * n, hd, None), "row dot")
+        check(L.limn_b200_sdpa_bwd_q(ops[0].ptr, ops[1].ptr, ops[2].ptr, ops[3].ptr, lse.ptr, delta.ptr, None, dq.ptr, *tail), "dq")
+        got = [runtime.download(out, np.uint16, (bh, n, hd)), runtime.download(dq, np.uint16, (bh, n, hd)), runtime.download(lse, np.uint32, (bh, n))]
+        return got, lse, delta
+
+    short, _, _ = forward_and_dq(rows)
+    full, lse, delta = forward_and_dq(all_rows)
+    for a, b, name in zip(short, full, ("out", "dq", "lse")):
+        np.testing.assert_array_equal(a, b[:, :rows], err_msg=name)
+    if causal:  # (its queries would be others)
+        return
+
+    def dkv(n):  # dK and dV of the first n rows of dO's problem taken as keys; the other side are the rows above
+        ops = [up(x) for x in (q, do[:, :n], do[:, :n], q)]
+        dk, dv = (runtime.empty(2 * bh * n * hd) for _ in range(2))
+        check(L.limn_b200_sdpa_bwd_kv(ops[0].ptr, ops[1].ptr, ops[2].ptr, ops[3].ptr, lse.ptr, delta.ptr, None, dk.ptr, dv.ptr, code, bh, all_rows, n, hd, hd, 0, hd**-0.5, None), "dk, dv")
+        return [runtime.download(x, np.uint16, (bh, n, hd)) for x in (dk, dv)]
+
+    for a, b, name in zip(dkv(rows), dkv(all_rows), ("dk", "dv")):
+        np.testing.assert_array_equal(a, b[:, :rows], err_msg=name)
+    assert runtime.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, np.dtype(np.float16)], ids=["bf16", "f16"])
 @pytest.mark.parametrize("t_q,hd", [(250, 64), (384, 56)])
 def test_rows_staged_item_after_item_are_the_rows_of_one_item(t_q, hd, dtype):
     """A warp whose rows go by way of shared memory uses the same bytes for the next item's rows: more items than SMs, against one problem
