@@ -1644,8 +1644,9 @@ int launch_sized(Op op, const Problem& p) {
 //   dK, dV   8, up to 256 problems 0.94-1.07 and beyond 0.85-0.97 / 0.85-0.94 / 0.76-0.85; 16: 0.8-0.98 / 0.77-0.95 / 0.59-0.88; 24 and 32:
 //            0.48-0.9; 72: 0.83-1.01; more: 0.35-0.9
 // At head dim 64 all three gain here (0.4-0.96), and so does everything at 128 problems, one block to an SM, and from 65 rows on. What
-// is nearer to float64 on one side stays there: the forward at up to 24 with at most two problems to an SM here, dQ and dK below 24 there
-// (2-norm, here over there: dQ 0.94-1.09, dK 0.94-1.12; from 24 on 0.75-0.98, dK at 16 with 32 queries or more 0.92-0.98).
+// is nearer to float64 on one side stays there: the forward at up to 24 with at most two problems to an SM here, the backward at up to 24
+// there (2-norm, here over there, the worst of 13 to 19 shapes: widths 24 and 24 dV 1.05; 24 and 8 dQ 1.09, dK 1.05; 8 and 24 dQ 1.06; 16 and 8 dK 1.05; from 25 on 0.55
+// to 0.88, whatever the other width) but for dK and dV at 16 and 16 with 32 queries or more (0.82-0.99).
 bool short_rows(Op op, const Problem& p) {
   if (p.t_q > 64 || p.t_k > 64) return false;
   int sms = 0;
@@ -1653,9 +1654,9 @@ bool short_rows(Op op, const Problem& p) {
   const int widest = p.hd > p.hd_v ? p.hd : p.hd_v;
   if (widest > 64) return op == Op::Fwd ? p.t_k <= 32 : op == Op::BwdQ && p.t_k <= (widest <= 100 ? 32 : 16);
   if (op == Op::Fwd) return widest <= 24 && p.bh > 2LL * sms;
-  if (widest >= 24) return false;
+  if (widest > 24) return false;
   if (widest > 16) return p.bh > 4LL * sms && (op == Op::BwdQ || p.t_q <= 32);
-  return op == Op::BwdQ || (p.bh > 3LL * sms && (widest < 16 || p.t_q < 32));
+  return op == Op::BwdQ || (p.bh > 3LL * sms && (p.hd < 16 || p.hd_v < 16 || p.t_q < 32));
 }
 
 }  // namespace
