@@ -694,13 +694,10 @@ __device__ __forceinline__ uint32_t split_streams_one(Carry<HD, kThreads, kWide>
   return again;
 }
 
-// A row's share of its columns by the row's total, every quotient rounded to nearest: one reciprocal and two corrections. (Markstein 1990:
-// with the correctly rounded reciprocal, a quotient within an ulp and its exact remainder, the corrected quotient is the correctly
-// rounded one; the first correction gives the quotient within an ulp.) The remainder is exact for totals from 1/2 and quotients from
-// 2^-102, so a warp with anything but totals of that kind and rows whose largest column is from 2^-40 divides. A division by itself is a
-// chain with a branch for each column, and a column of zeros, as a width below the kernel's has them, takes its slow side. Measured, a
-// division a column -> so: 256 x 256 x 64 causal 33.9 -> 31.4 us, 64 x 1024 x 128 127 -> 121, 2048 x 128 x 40 123.8 -> 78.2, 2048 x 192 x 100
-// 512 -> 398, 6 x 8192 x 32 225 either way.
+// A row's share of its columns by the row's total (tiled_rows.cuh says how, and when that is exact): a warp with a row of another kind
+// divides. A division by itself is a chain with a branch for each column, and a column of zeros, as a width below the kernel's has
+// them, takes its slow side. Measured, a division a column -> so: 256 x 256 x 64 causal 33.9 -> 31.4 us, 64 x 1024 x 128 127 -> 121, 2048 x 128 x 40
+// 123.8 -> 78.2, 2048 x 192 x 100 512 -> 398, 6 x 8192 x 32 225 either way.
 template <int N>
 __device__ __forceinline__ void divide_row(uint64_t (&x)[N], float total) {
   float largest = 0.f;
@@ -708,17 +705,18 @@ __device__ __forceinline__ void divide_row(uint64_t (&x)[N], float total) {
   for (int c = 0; c < N; ++c) {
     float x0, x1;
     f2_unpack(x[c], x0, x1);
-    largest = fmaxf(largest, fmaxf(fabsf(x0), fabsf(x1)));
+    largest = max3(largest, fabsf(x0), fabsf(x1));
   }
-  const bool ordinary = total >= 0.5f && total < 0x1p40f && (largest == 0.f || (largest >= 0x1p-40f && largest < INFINITY));
-  if (__all_sync(kFull, ordinary)) {
+  if (__all_sync(kFull, tiled::by_reciprocal(largest, total))) {
+    constexpr float kUp = tiled::kQuotientUp;
     const float r = __frcp_rn(total);
-    const uint64_t r2 = f2_pack(r, r), less = f2_pack(-total, -total);
+    const uint64_t first = f2_pack(r * kUp, r * kUp), less = f2_pack(-r, -r), total2 = f2_pack(total, total), up = f2_pack(-kUp, -kUp), down = f2_pack(1.f / kUp, 1.f / kUp);
 #pragma unroll
     for (int c = 0; c < N; ++c) {
-      uint64_t q = f2_mul(x[c], r2);
-      q = f2_fma(f2_fma(q, less, x[c]), r2, q);
-      x[c] = f2_fma(f2_fma(q, less, x[c]), r2, q);
+      const uint64_t minus_x = f2_mul(x[c], up);
+      uint64_t q = f2_mul(x[c], first);
+      q = f2_fma(f2_fma(q, total2, minus_x), less, q);
+      x[c] = f2_mul(f2_fma(f2_fma(q, total2, minus_x), less, q), down);
     }
   } else {
 #pragma unroll

@@ -163,6 +163,14 @@ __device__ __forceinline__ float group_sum(float x) {
   return x;
 }
 
+// A row's columns by its total, every quotient rounded to nearest from one reciprocal and two corrections. (Markstein 1990: with the correctly
+// rounded reciprocal, a quotient within an ulp and its exact remainder, the corrected quotient is the correctly rounded one; the first
+// correction gives the quotient within an ulp.) The remainder q total - x is a multiple of ulp(q) ulp(total), which is a float32 for totals from 1/2 if
+// q is from 2^-102: so columns go up by 2^64 first and quotients down again, and a row of columns too large for that, or of another total,
+// divides. (A quotient below 2^-126 is rounded twice, to 24 bits and to those that it has.) With that sign of the remainder a zero keeps its own.
+constexpr float kQuotientUp = 0x1p64f;
+__device__ __forceinline__ bool by_reciprocal(float largest, float total) { return total >= 0.5f && total < 0x1p40f && largest < 0x1p60f; }
+
 struct Args {
   const void *q, *k, *v, *mask, *dout;
   const float *lse_in, *delta;
@@ -248,19 +256,18 @@ __device__ __forceinline__ void fwd_rows(const Args& g, long long b, int i0, flo
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     const float total = group_sum(denom[a]);
-    // Every quotient rounded to nearest, from one reciprocal and two corrections where totals and columns are of an ordinary size (Markstein
-    // 1990; divide_row of sdpa_f32_sm100.cu has the bounds): head dims above 32 take 0.88 to 0.97 of the time, up to 32 (two columns a
-    // thread) 0.99 to 1.04.
+    // (head dims above 32 take 0.88 to 0.97 of the time that divisions do, up to 32, two columns a thread, 0.99 to 1.04)
     float largest = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) largest = fmaxf(largest, fabsf(acc[a][i]));
-    if (NV > 2 && total >= 0.5f && total < 0x1p40f && (largest == 0.f || (largest >= 0x1p-40f && largest < INFINITY))) {
+    if (NV > 2 && by_reciprocal(largest, total)) {
       const float r = __frcp_rn(total);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        float q = acc[a][i] * r;
-        q = fmaf(fmaf(q, -total, acc[a][i]), r, q);
-        acc[a][i] = fmaf(fmaf(q, -total, acc[a][i]), r, q);
+        const float x = acc[a][i] * kQuotientUp;
+        float q = x * r;
+        q = fmaf(fmaf(q, total, -x), -r, q);
+        acc[a][i] = fmaf(fmaf(q, total, -x), -r, q) * (1.f / kQuotientUp);
       }
     } else {
 #pragma unroll

@@ -243,3 +243,33 @@ def test_rows_are_divided_to_the_nearest(t_q, t_k, hd_v, causal):
     for power in (-45, 45, 100):
         scaled = _step(q, k, np.ldexp(v, power), np.zeros_like(do), mask, causal, 32**-0.5)[0]
         assert np.array_equal(np.ldexp(ordinary, power), scaled), power
+
+
+@pytest.mark.parametrize(("t", "hd", "hd_v", "causal"), [(130, 32, 200, True), (130, 64, 64, True), (130, 32, 128, False), (70, 40, 130, True)])
+def test_columns_far_smaller_than_their_neighbours_are_divided_to_the_nearest(t, hd, hd_v, causal):
+    """Two columns of V are 2^-116 of the others (in the second run one of them is of their size): the quotients are those of the column at
+    that size, bit for bit, in the tiled kernels and where the tensor cores hand items to them. V lies between 1 and 2 and scores are small, so the
+    sums scale exactly."""
+    q, k, v, do = _problem(t + hd_v, 64, t, t, hd, hd_v)
+    v = 1 + np.abs(v) % 1
+    small = np.float32(2.0**-116)
+    v[..., [2, hd_v - 1]] *= small
+    mixed = _step(0.5 * q, k, v, do, None, causal, hd**-0.5)[0]
+    v[..., 2] /= small
+    other = _step(0.5 * q, k, v, do, None, causal, hd**-0.5)[0]
+    other[..., 2] *= small
+    assert np.array_equal(mixed, other)
+
+
+@pytest.mark.parametrize(("hd", "hd_v"), [(32, 200), (192, 96)])
+def test_a_zero_keeps_its_sign(hd, hd_v):
+    """Columns that the first keys take below zero and later ones, of far larger scores, scale to a zero of that sign, and of a quotient of that
+    sign."""
+    t_q, t_k = 70, 144  # (whole tiles of keys: a padding key would add a positive zero)
+    q, k = np.ones((2, t_q, hd), np.float32), np.zeros((2, t_k, hd), np.float32)
+    k[:, 128:] = 300.0
+    v = np.full((2, t_k, hd_v), -1.0, np.float32)
+    v[:, 128:] = -0.0
+    v[:, 128:, ::2] = 1.5
+    out = _step(q, k, v, np.zeros((2, t_q, hd_v), np.float32), None, False, 1.0)[0]
+    assert (out[..., ::2] == 1.5).all() and (out[..., 1::2] == 0).all() and np.signbit(out[..., 1::2]).all()
