@@ -221,10 +221,11 @@ __device__ __forceinline__ void issue_weigh(uint32_t d, uint32_t w0, uint32_t x0
 
 // N numbers of one row, split, to tensor memory at `at` (pieces kPieceCols columns apart).
 template <int N>
-__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2], Check& check) {
+__device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2]) {
   uint32_t h[N / 2], m[N / 2], l[N / 2];
+  Check none;
 #pragma unroll
-  for (int i = 0; i < N / 2; ++i) split_pair<false>(w[i], h[i], m[i], l[i], check);
+  for (int i = 0; i < N / 2; ++i) split_pair<false>(w[i], h[i], m[i], l[i], none);
   tmem_st<N / 2>(at, h);
   tmem_st<N / 2>(at + kPieceCols, m);
   tmem_st<N / 2>(at + 2 * kPieceCols, l);
@@ -997,8 +998,7 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
         if (j > 0) gather_product(t - 1);
         shrink = less;
         // (the product of the tile before has been gathered, so its P has been read)
-        Check none;
-        hand_over<CW>(lanes + L::kP + group * (CW / 2), w, none);
+        hand_over<CW>(lanes + L::kP + group * (CW / 2), w);
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrives(ring(kReady, t));
@@ -1040,6 +1040,173 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
       if (item(__ffs(static_cast<int>(left)) - 1, it)) rows_again<HD, Op::Fwd, kAgainGroups, L::kBytes, kWide>(g, it.b, it.first, raw);
   }
   tear_down<L::kCols, W::kIssuer>(g, tmem);
+}
+
+// ---- forward of short problems: two blocks of 256 threads to an SM, no roles ----
+// The same sums in the same order, everything by all of a block's threads, one thing after the other. An item of one key tile is a chain of
+// latencies whichever way the work is shared out; here an SM has two of them at once, and a block is ready sooner.
+template <int HD, bool kWide>
+struct FwdPair {
+  static constexpr int kGroups = 2, kThreads = kRows * kGroups;
+  using Held = Stage<HD, kRows, kThreads, kWide>;
+  using Tile = Stage<HD, kStream, kThreads, kWide>;
+  static constexpr uint32_t kQ = 0, kK = Held::kBytes, kV = kK + Tile::kBytes, kBytes = kV + Tile::kBytes + 1024;
+  static constexpr uint32_t kS = 0, kP = kStream, kO = kP + 3 * kPieceCols;
+  static constexpr int kCols = 256;
+  static_assert(kO + HD <= kCols, "tensor memory");
+};
+
+template <int HD, bool kWide>
+__global__ void __launch_bounds__(FwdPair<HD, kWide>::kThreads, 2) f32_fwd_pair_kernel(const __grid_constant__ Params g) {
+  using L = FwdPair<HD, kWide>;
+  constexpr int G = L::kGroups, CW = kStream / G, OW = HD / G;
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ uint32_t slot, abort_flag, hidden[2][2];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ float exchange[G][kRows];
+  uint32_t tmem;
+  if (!set_up<L::kCols, 2>(g, &slot, &abort_flag, bars, tmem)) return;
+  const uint32_t base = align_1024(smem_addr(raw));
+  const uint32_t scored = smem_addr(bars), weighed = smem_addr(bars + 1);
+  const int warp = threadIdx.x >> 5, group = warp >> 2;
+  const int row = (warp & 3) * 32 + (threadIdx.x & 31);
+  const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const bool issues = __shfl_sync(kFull, warp, 0) == 0;  // the warp that issues, one lane of it elected per bunch
+
+  int problem, at;
+  cta_work(blockIdx.x, g.slots, g.bh, g.group, problem, at);
+  const int first = (g.slots - 1 - at) * kRows;  // long causal rows first
+  const long long b = problem;
+  const float* k = g.k + b * g.t_k * g.hd;
+  const float* v = g.v + b * g.t_k * g.hd_v;
+  const float* mask = g.mask ? g.mask + b * g.t_k : nullptr;
+  const int tiles = ((g.causal ? min(g.t_k, first + kRows) : g.t_k) + kStream - 1) / kStream;
+  const int i = first + row;
+  auto score = [&] {
+    if (issues && elect_one()) {
+      tc_fence_after_sync();
+      issue_scores<HD, false>(tmem + L::kS, base + L::kQ, base + L::kK);
+      mma_commit(scored);
+    }
+  };
+
+  Check check;
+  typename L::Tile stage_k, stage_v;
+  stage_k.load(k, 0, g.t_k, g.hd);
+  {
+    typename L::Held stage_q;
+    stage_q.load(g.q + b * g.t_q * g.hd, first, g.t_q, g.hd);
+    stage_q.store(base + L::kQ, check);
+  }
+  stage_k.store(base + L::kK, check);
+  if (mask) post_hidden(hidden[0], row_value(mask, 0, g.t_k));
+  fence_async_shared();
+  __syncthreads();
+  score();
+  stage_v.load(v, 0, g.t_k, g.hd_v);
+  stage_v.store(base + L::kV, check);
+  fence_async_shared();
+
+  float top = -INFINITY, shift = 0.f, denom = 0.f;  // row maximum (raw scores); shift = top * c, in log2 units
+  uint64_t acc[OW / 2];
+#pragma unroll
+  for (int c = 0; c < OW / 2; ++c) acc[c] = 0;
+  const uint64_t c_hi = f2_pack(g.c_hi, g.c_hi), c_lo = f2_pack(g.c_lo, g.c_lo);
+  bool ok = true;
+  for (int j = 0; j < tiles; ++j) {
+    const int j0 = j * kStream;
+    const bool more = j + 1 < tiles;
+    ok &= mbar_wait(scored, j & 1, g.status, 0x0a00u);
+    tc_fence_after_sync();
+    uint32_t s[CW];
+    tmem_ld<CW>(lanes + L::kS + group * CW, s);
+    tmem_ld_wait();
+    int limit = g.t_k - j0;
+    if (g.causal) limit = min(limit, i - j0 + 1);
+    limit -= group * CW;
+    uint32_t unseen = limit >= CW ? 0u : limit <= 0 ? kFull : ~((1u << limit) - 1u);
+    if (mask) unseen |= my_hidden<CW>(hidden[j & 1], group);
+    if (unseen != 0u) {
+#pragma unroll
+      for (int c = 0; c < CW; ++c)
+        if ((unseen >> c) & 1u) s[c] = 0xff800000u;
+    }
+    float tile_top = -INFINITY;
+#pragma unroll
+    for (int c = 0; c < CW; c += 2) tile_top = max3(tile_top, __uint_as_float(s[c]), __uint_as_float(s[c + 1]));
+    exchange[group][row] = tile_top;
+    __syncthreads();
+    float raised = top;
+#pragma unroll
+    for (int c = 0; c < G; ++c) raised = fmaxf(raised, exchange[c][row]);
+    const float moved = raised == -INFINITY ? 0.f : raised * g.c_hi;
+    const float shrink = top == -INFINITY ? 0.f : exp2_approx(shift - moved);  // nothing gathered yet: nothing to rescale
+    top = raised, shift = moved;
+    const uint64_t minus_shift = f2_pack(-shift, -shift);
+    uint64_t w[CW / 2];
+    uint64_t sum = 0;
+#pragma unroll
+    for (int c = 0; c < CW / 2; ++c) {
+      const uint64_t s2 = f2_pack_bits(s[2 * c], s[2 * c + 1]);
+      float x0, x1;
+      f2_unpack(f2_fma(s2, c_lo, f2_fma(s2, c_hi, minus_shift)), x0, x1);
+      w[c] = f2_pack(exp2_approx(x0), exp2_approx(x1));
+      sum = f2_add(sum, w[c]);
+    }
+    float sum0, sum1;
+    f2_unpack(sum, sum0, sum1);
+    denom = fmaf(denom, shrink, sum0 + sum1);  // this thread's share; the shares meet after the last tile
+    check.sums |= !(denom < INFINITY);
+    hand_over<CW>(lanes + L::kP + group * (CW / 2), w);
+    tmem_st_wait();
+    tc_fence_before_sync();
+    if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
+    if (issues && elect_one()) {
+      tc_fence_after_sync();
+      issue_weigh<HD>(tmem + L::kO, tmem + L::kP, base + L::kV);
+      mma_commit(weighed);
+    }
+    if (more) {
+      // K's place has been read (the scores are there) and so have the scores themselves
+      stage_k.load(k, j0 + kStream, g.t_k, g.hd);
+      const float flag = mask ? row_value(mask, j0 + kStream, g.t_k) : 0.f;
+      stage_k.store(base + L::kK, check);
+      if (mask) post_hidden(hidden[(j + 1) & 1], flag);
+      fence_async_shared();
+      __syncthreads();
+      score();
+      stage_v.load(v, j0 + kStream, g.t_k, g.hd_v);
+    }
+    ok &= mbar_wait(weighed, j & 1, g.status, 0x0a01u);
+    tc_fence_after_sync();
+    uint32_t o[OW];
+    tmem_ld<OW>(lanes + L::kO + group * OW, o);
+    tmem_ld_wait();
+    tc_fence_before_sync();
+    const uint64_t shrink2 = f2_pack(shrink, shrink);
+#pragma unroll
+    for (int c = 0; c < OW / 2; ++c) acc[c] = f2_fma(acc[c], shrink2, f2_pack_bits(o[2 * c], o[2 * c + 1]));
+    if (more) {
+      stage_v.store(base + L::kV, check);  // the weighing has read the tile before this one
+      fence_async_shared();
+    }
+  }
+  exchange[group][row] = denom;  // (every read of the maxima lies before a barrier of the block)
+  ok = __syncthreads_and(ok);
+  const bool bad = __syncthreads_or(check.bad());
+  if (ok && bad) {
+    rows_again<HD, Op::Fwd, 1, L::kBytes, kWide>(g, b, first, raw);
+  } else if (ok) {
+    float total = 0.f;
+#pragma unroll
+    for (int c = 0; c < G; ++c) total += exchange[c][row];
+    divide_row(acc, total);  // 0/0 = NaN for a row with no key, as the oracle has it
+    store_rows<OW>(g.out + b * g.t_q * g.hd_v, acc, first + (warp & 3) * 32, g.t_q, group * OW, g.hd_v, g.wide_out);
+    // once per row, so in double: L is then as good as its sum
+    if (group == 0 && i < g.t_q)
+      g.lse_out[b * g.t_q + i] = top == -INFINITY ? -INFINITY : static_cast<float>(shift * 0.69314718055994530942 + log(static_cast<double>(total)));
+  }
+  tear_down<L::kCols>(g, tmem);
 }
 
 // ---- backward at head dims up to 64: dQ for 128 query rows, or dK and dV for 128 key rows ----
@@ -1322,9 +1489,8 @@ __global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(co
         if (j > 0) gather_products(t - 1);
         if (!ok) break;
         // (the products of the tile before have been gathered, so its P and dS have been read)
-        Check none;
-        hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, none);
-        if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, none);
+        hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds);
+        if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p);
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrives(ring(kReady, t));
@@ -1512,8 +1678,8 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
         hi = f2_pack(my_hi, my_hi), lo = f2_pack(my_lo, my_lo), delta = f2_pack(my_delta, my_delta);
       }
     }, p, ds);
-    hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds, check);
-    if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p, check);
+    hand_over<CW>(lanes + L::kDs + group * (CW / 2), ds);
+    if (kKV) hand_over<CW>(lanes + L::kP + group * (CW / 2), p);
     tmem_st_wait();
     tc_fence_before_sync();
     if (!__syncthreads_and(ok && !check.bad())) break;  // (nothing is in flight here)
@@ -1560,6 +1726,19 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
 
 bool aligned(const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; }  // (null is)
 
+// Forwards up to head dim 64 in f32_fwd_pair_kernel: those of one key tile that have a block for two SMs out of three and up to four for each,
+// and those of up to five tiles that have one to two blocks to an SM, which it holds all at once where the other kernel takes two rounds.
+// Measured on B200, us, here / in roles:
+//   16 x 16 x 32: 16 problems 5.0 / 5.1, 100 5.1 / 5.7, 148 5.1 / 6.0, 149 6.4 / 8.3, 296 6.8 / 8.8, 400 10.7 / 11.4, 592 12.8 / 14.4, 5000 97 / 105
+//   64 x 64 x 32: 16 5.1 / 5.0, 100 5.2 / 5.7, 148 5.2 / 6.0, 149 6.5 / 8.1, 296 7.1 / 8.6, 400 11.0 / 11.2, 592 13.0 / 14.1, 700 16.8 / 16.8, 5000 109 / 103
+//   64 x 64 x 64: 16 6.2 / 6.3, 100 6.3 / 7.0, 149 7.9 / 10.5, 296 8.7 / 11.1, 592 16.1 / 18.5, 5000 146 / 143; 1000 of 300 x 64 94 / 89
+//   128 x 128 x 32: 148 7.3 / 7.1, 149 9.0 / 10.6, 296 9.7 / 11.1, 297 14.6 / 14.1; 64 x 320 x 32: 149 15.7 / 17.5, 296 16.5 / 17.9
+//   64 x 100 x 64: 148 8.9 / 8.6, 149 11.3 / 13.4, 296 11.9 / 13.9, 297 18.3 / 17.8; 64 x 320 x 64: 149 20.6 / 21.8, 222 22.0 / 22.1; 100 x 448 x 64: 222 29.0 / 28.2
+bool two_to_an_sm(const Problem& p, long long blocks, int sms) {
+  if (p.t_k <= kStream) return 3 * blocks > 2LL * sms && blocks <= 4LL * sms;
+  return p.t_k <= 5 * kStream && blocks > sms && blocks <= 2LL * sms;
+}
+
 template <int HD, bool kWide>
 int launch_sized(Op op, const Problem& p) {
   Params g = {};
@@ -1595,7 +1774,11 @@ int launch_sized(Op op, const Problem& p) {
   long long grid = blocks;
   const bool two = HD <= 32 && op == Op::BwdQ && blocks <= sms;  // threads to a row (see f32_bwd_kernel)
   bool roles = true;
-  if (op == Op::Fwd) {
+  const bool pair = HD <= 64 && op == Op::Fwd && two_to_an_sm(p, blocks, sms);
+  if (pair) {
+    if constexpr (HD <= 64) kernel = f32_fwd_pair_kernel<HD, kWide>, shared = FwdPair<HD, kWide>::kBytes, threads = FwdPair<HD, kWide>::kThreads;
+    roles = false;
+  } else if (op == Op::Fwd) {
     kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
   } else if constexpr (HD > 64) {
     using B = BwdWide<HD, kWide>;
@@ -1616,8 +1799,8 @@ int launch_sized(Op op, const Problem& p) {
     grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
-  const int which = two ? 3 : static_cast<int>(op);
-  static bool sized[64][4] = {};
+  const int which = pair ? 4 : two ? 3 : static_cast<int>(op);
+  static bool sized[64][5] = {};
   int device = 0;
   LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");
   if (device < 0 || device >= 64 || !sized[device][which]) {

@@ -231,6 +231,13 @@ def test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
         assert np.array_equal(g[picks], a), what
 
 
+@pytest.mark.parametrize(("bh", "t_q", "t_k", "hd", "hd_v", "causal"), [(100, 17, 64, 32, 30, False), (149, 64, 64, 64, 64, True), (296, 16, 16, 32, 32, True), (592, 33, 40, 64, 37, False),
+                                                                        (150, 70, 130, 28, 32, False), (75, 200, 200, 64, 40, True), (296, 128, 320, 64, 64, False), (98, 300, 65, 32, 25, False)])
+def test_a_short_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
+    """The same on both sides of the rule that gives short problems two blocks to an SM and no roles."""
+    test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal)
+
+
 @pytest.mark.parametrize(("t_q", "t_k", "hd_v", "causal"), [(130, 130, 64, True), (70, 200, 40, False), (200, 65, 100, False), (129, 129, 128, True), (33, 70, 17, False),
                                                             (70, 70, 200, False), (100, 100, 130, True)])
 def test_rows_are_divided_to_the_nearest(t_q, t_k, hd_v, causal):
