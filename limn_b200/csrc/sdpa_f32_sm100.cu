@@ -99,7 +99,8 @@ __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[N]) {
 template <int N>
 __device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&r)[N]) {
   if constexpr (N == 16) tmem_st16(addr, r);
-  else tmem_st8(addr, r);
+  else if constexpr (N == 8) tmem_st8(addr, r);
+  else tmem_st4(addr, r);
 }
 
 // Eight consecutive floats, those from `left` on zero (they are not there). kWide: the width is a multiple of 4 and the base 16-byte
@@ -235,6 +236,7 @@ __device__ __forceinline__ void hand_over(uint32_t at, const uint64_t (&w)[N / 2
 // for pieces (a block's 128 x 64 results took 2 000 to 6 000 clocks without).
 template <int N>
 __device__ __forceinline__ void store_rows(float* dst, const uint64_t (&acc)[N / 2], int first, int rows, int col, int width, bool wide) {
+  if (first >= rows) return;  // (the whole warp; dK and dV of 700 problems of 16 x 72 59.4 us without, 58.1 with it)
   const int lane = static_cast<int>(lane_id());
   if (wide) {
     constexpr int B = N / 4 < 4 ? N / 4 : 4;
@@ -1530,10 +1532,10 @@ __global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(co
   tear_down<L::kCols, W::kIssuer>(g, tmem);
 }
 
-// ---- backward at head dims above 64 ----
-// Two held operands and two streamed tiles do not fit in shared memory: the first held operand lies in tensor memory, the
+// ---- backward at head dims above 64, and of items of one tile (one_tile) ----
+// Above 64 two held operands and two streamed tiles do not fit in shared memory: the first held operand lies in tensor memory, the
 // streamed tiles have one buffer, and a tile's products are written over the scores they came from. What is left to run
-// side by side is little, so the row warps also issue.
+// side by side is little, so the row warps also issue. An item of one tile has nothing to run side by side.
 template <int HD, bool kWide>
 struct BwdWide {
   static constexpr int kGroups = 4;
@@ -1541,7 +1543,9 @@ struct BwdWide {
   using Held = Stage<HD, kRows, kThreads, kWide>;
   using Tile = Stage<HD, kStream, kThreads, kWide>;
   static constexpr uint32_t kHeld1 = 0, kTile0 = Held::kBytes, kTile1 = kTile0 + Tile::kBytes;
-  static constexpr uint32_t kBytes = kTile1 + Tile::kBytes + 1024;
+  // (up to head dim 64 as much as the kernel with roles has, so that items done again on the CUDA cores stream the same tiles)
+  static constexpr uint32_t kBytes = HD <= 64 ? std::min(Bwd<HD, false>::kBytes, Bwd<HD, true>::kBytes) : kTile1 + Tile::kBytes + 1024;
+  static_assert(kTile1 + Tile::kBytes + 1024 <= kBytes, "shared memory");
   static constexpr uint32_t kS = 0, kDp = kStream, kDs = 2 * kStream, kP = kDs + 3 * kPieceCols, kHeldT = kP + 3 * kPieceCols;
   static constexpr uint32_t kOut = 0;
   static constexpr int kCols = 512;
@@ -1739,6 +1743,31 @@ bool two_to_an_sm(const Problem& p, long long blocks, int sms) {
   return p.t_k <= 5 * kStream && blocks > sms && blocks <= 2LL * sms;
 }
 
+// Backward passes up to head dim 64 in the kernel without roles: one tile of streamed rows, one block to a problem and at most one to an SM.
+// Measured on B200, us, here / in roles, by own x streamed rows x width:
+//   dQ: 16 x 16 x 64 1 problem 7.7 / 8.5, 148 8.4 / 8.7; 64 x 64 x 64 1 8.5 / 8.5, 148 9.2 / 9.3; 100 x 64 x 64 100 10.0 / 9.4; 100 x 64 x 40 1 8.4 / 8.5, 148 9.2 / 9.7;
+//     16 x 16 x 32 1 6.3 / 6.6, 148 6.8 / 6.9; 32 x 32 x 32 1 6.3 / 6.5, 100 6.7 / 7.0; 64 x 64 x 32 1 6.5 / 6.5, 148 7.3 / 7.1; 64 x 64 x 16 100 6.6 / 6.9, 148 6.9 / 6.9
+//   dK and dV: 16 x 16 x 32 64 6.4 / 6.4, 100 6.4 / 6.6, 148 6.4 / 7.0; 64 x 64 x 32 64 6.7 / 6.7, 148 6.8 / 7.2; 100 x 64 x 32 148 7.3 / 7.6; 64 x 64 x 64 64 8.9 / 8.6,
+//     100 9.0 / 9.0, 148 9.0 / 9.3
+//   rows that are not whole 16-byte pieces: dQ 16 x 16 x 25 1 7.1 / 8.0, 148 7.4 / 8.6; 128 x 64 x 50 64 15.3 / 16.5; dK and dV 16 x 16 x 25 1 6.3 / 7.0, 100 x 64 x 30 148 11.9 / 12.6
+bool one_tile(Op op, const Problem& p, bool wide, int sms) {
+  const int widest = p.hd > p.hd_v ? p.hd : p.hd_v, owned = op == Op::BwdQ ? p.t_q : p.t_k, streamed = op == Op::BwdQ ? p.t_k : p.t_q;
+  if (streamed > kStream || owned > kRows || p.bh > sms) return false;
+  if (!wide) return true;
+  if (op == Op::BwdKV) return 3 * p.bh > 2LL * sms;
+  if (widest > 32) return owned <= 64 || widest <= 40;
+  return owned <= 64 && (widest <= 24 || (owned <= 32 && streamed <= 32));
+}
+
+// A problem's bits do not depend on which kernel it comes to, on the CUDA cores either.
+template <int HD, bool kWide>
+constexpr bool same_tiles_again() {
+  return again_tile<HD, Op::Fwd, 1, FwdPair<HD, kWide>::kBytes>() == again_tile<HD, Op::Fwd, kAgainGroups, Fwd<HD>::kBytes>() &&
+         again_tile<HD, Op::BwdQ, kAgainGroups, BwdWide<HD, kWide>::kBytes>() == again_tile<HD, Op::BwdQ, kAgainGroups, Bwd<HD, false>::kBytes>() &&
+         again_tile<HD, Op::BwdKV, kAgainGroups, BwdWide<HD, kWide>::kBytes>() == again_tile<HD, Op::BwdKV, kAgainGroups, Bwd<HD, true>::kBytes>();
+}
+static_assert(same_tiles_again<32, true>() && same_tiles_again<32, false>() && same_tiles_again<64, true>() && same_tiles_again<64, false>());
+
 template <int HD, bool kWide>
 int launch_sized(Op op, const Problem& p) {
   Params g = {};
@@ -1775,12 +1804,18 @@ int launch_sized(Op op, const Problem& p) {
   const bool two = HD <= 32 && op == Op::BwdQ && blocks <= sms;  // threads to a row (see f32_bwd_kernel)
   bool roles = true;
   const bool pair = HD <= 64 && op == Op::Fwd && two_to_an_sm(p, blocks, sms);
+  const bool alone = HD <= 64 && op != Op::Fwd && one_tile(op, p, kWide, sms);
   if (pair) {
     if constexpr (HD <= 64) kernel = f32_fwd_pair_kernel<HD, kWide>, shared = FwdPair<HD, kWide>::kBytes, threads = FwdPair<HD, kWide>::kThreads;
     roles = false;
   } else if (op == Op::Fwd) {
     kernel = f32_fwd_kernel<HD, kWide>, shared = Fwd<HD>::kBytes, threads = Roles<Fwd<HD>::kGroups>::kThreads;
   } else if constexpr (HD > 64) {
+    using B = BwdWide<HD, kWide>;
+    kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
+    shared = B::kBytes, threads = B::kThreads;
+    roles = false;
+  } else if (alone) {
     using B = BwdWide<HD, kWide>;
     kernel = op == Op::BwdQ ? f32_bwd_wide_kernel<HD, false, kWide> : f32_bwd_wide_kernel<HD, true, kWide>;
     shared = B::kBytes, threads = B::kThreads;
@@ -1799,8 +1834,8 @@ int launch_sized(Op op, const Problem& p) {
     grid = std::min(blocks, sms * ((blocks + turn - 1) / turn));
   }
   // the attribute is per device and per kernel instantiation; set it on first use there
-  const int which = pair ? 4 : two ? 3 : static_cast<int>(op);
-  static bool sized[64][5] = {};
+  const int which = alone ? 4 + static_cast<int>(op) : pair ? 4 : two ? 3 : static_cast<int>(op);
+  static bool sized[64][7] = {};
   int device = 0;
   LIMN_CUDA(cudaGetDevice(&device), "asking for the current device");
   if (device < 0 || device >= 64 || !sized[device][which]) {

@@ -232,9 +232,10 @@ def test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
 
 
 @pytest.mark.parametrize(("bh", "t_q", "t_k", "hd", "hd_v", "causal"), [(100, 17, 64, 32, 30, False), (149, 64, 64, 64, 64, True), (296, 16, 16, 32, 32, True), (592, 33, 40, 64, 37, False),
-                                                                        (150, 70, 130, 28, 32, False), (75, 200, 200, 64, 40, True), (296, 128, 320, 64, 64, False), (98, 300, 65, 32, 25, False)])
+                                                                        (150, 70, 130, 28, 32, False), (75, 200, 200, 64, 40, True), (296, 128, 320, 64, 64, False), (98, 300, 65, 32, 25, False),
+                                                                        (148, 64, 64, 64, 64, True), (300, 40, 64, 64, 50, False), (148, 16, 30, 32, 20, False), (120, 64, 33, 64, 64, False)])
 def test_a_short_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal):
-    """The same on both sides of the rule that gives short problems two blocks to an SM and no roles."""
+    """The same on both sides of the rules that give short problems kernels without roles."""
     test_a_problem_alone_and_among_many(bh, t_q, t_k, hd, hd_v, causal)
 
 
