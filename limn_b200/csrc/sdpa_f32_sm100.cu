@@ -1600,6 +1600,7 @@ __global__ void __launch_bounds__(BwdWide<HD, kWide>::kThreads, 1) f32_bwd_wide_
         lse_hi[threadIdx.x] = hi;
         lse_lo[threadIdx.x] = lo;
         deltas[threadIdx.x] = -delta;
+        check.sums |= !(lse < INFINITY);  // (its weights are not finite, which would only be seen in the sums)
       }
     } else if (mask) {
       post_hidden(hidden, row_value(mask, x0, streamed));

@@ -139,6 +139,24 @@ def test_a_row_whose_only_key_is_nan(hd, dtype, dev):
     assert np.isfinite(out[1].astype(np.float32)).all() and np.isfinite(lse[1]).all()
 
 
+@pytest.mark.parametrize("hd", [32, 64, 100])
+def test_a_query_whose_l_is_nan(hd):
+    """Its weights are NaN for the keys it sees (0 to 3); the other keys, and the queries before it, are what they are without it. A problem with
+    no key at all (L is -inf throughout) beside it."""
+    q, k, v, do = _problem(47 + hd, 2, 150, 150, hd, hd)
+    mask = np.stack([np.ones(150, np.float32), np.zeros(150, np.float32)])
+    q[0, 3, 1] = np.nan
+    out, lse, dq, dk, dv = _step(q, k, v, do, mask, True, hd**-0.5)
+    assert np.isnan(lse[0, 3]) and np.isneginf(lse[1]).all() and np.isnan(dk[0, :4]).all() and np.isnan(dv[0, :4]).all()
+    assert (dk[1] == 0).all() and (dv[1] == 0).all()
+    q[0, 3] = 0
+    do[0, 3] = 0  # (query 3 then adds nothing to any key)
+    want = _step64(q[:1], k[:1], v[:1], do[:1], None, True, hd**-0.5)
+    others = np.arange(150) != 3
+    _compare([out[:1, others], lse[:1, others], dq[:1, others], dk[:1, 4:], dv[:1, 4:]],
+             [want[0][:, others], want[1][:, others], want[2][:, others], want[3][:, 4:], want[4][:, 4:]], 8 * 150**0.5 * 2.0**-24)
+
+
 @pytest.mark.parametrize("hd", [32, 64, 128])
 @pytest.mark.parametrize(("which", "power"), [("q", -118), ("v", -118), ("do", -118)])
 def test_small_operands_keep_their_bits(which, power, hd):
