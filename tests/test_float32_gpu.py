@@ -141,20 +141,24 @@ def test_a_row_whose_only_key_is_nan(hd, dtype, dev):
 
 @pytest.mark.parametrize("hd", [32, 64, 100])
 def test_a_query_whose_l_is_nan(hd):
-    """Its weights are NaN for the keys it sees (0 to 3); the other keys, and the queries before it, are what they are without it. A problem with
-    no key at all (L is -inf throughout) beside it."""
+    """dK and dV from operands that are finite and an L that is not: NaN for the keys that query sees (0 to 3), for the others what they are
+    without it. A problem with no key at all (L is -inf throughout) beside it."""
+    from limn_b200 import runtime
+    from limn_b200._lib import check, lib
+
     q, k, v, do = _problem(47 + hd, 2, 150, 150, hd, hd)
+    do[0, 3] = 0  # (query 3 adds nothing to any key when its weights are finite)
     mask = np.stack([np.ones(150, np.float32), np.zeros(150, np.float32)])
-    q[0, 3, 1] = np.nan
-    out, lse, dq, dk, dv = _step(q, k, v, do, mask, True, hd**-0.5)
-    assert np.isnan(lse[0, 3]) and np.isneginf(lse[1]).all() and np.isnan(dk[0, :4]).all() and np.isnan(dv[0, :4]).all()
-    assert (dk[1] == 0).all() and (dv[1] == 0).all()
-    q[0, 3] = 0
-    do[0, 3] = 0  # (query 3 then adds nothing to any key)
     want = _step64(q[:1], k[:1], v[:1], do[:1], None, True, hd**-0.5)
-    others = np.arange(150) != 3
-    _compare([out[:1, others], lse[:1, others], dq[:1, others], dk[:1, 4:], dv[:1, 4:]],
-             [want[0][:, others], want[1][:, others], want[2][:, others], want[3][:, 4:], want[4][:, 4:]], 8 * 150**0.5 * 2.0**-24)
+    lse, delta = (np.stack([x, np.full(150, fill)]).astype(np.float32) for x, fill in ((want[1][0], -np.inf), ((do[0] * want[0][0]).sum(-1), np.nan)))
+    lse[0, 3] = np.nan
+    ops = [runtime.upload(x) for x in (q, k, v, do, lse, delta, mask)]
+    dk, dv = runtime.empty(k.nbytes), runtime.empty(v.nbytes)
+    check(lib().limn_b200_sdpa_bwd_kv(*(x.ptr for x in ops), dk.ptr, dv.ptr, 0, 2, 150, 150, hd, hd, 1, hd**-0.5, None), "dk, dv")
+    for got, w in ((runtime.download(dk, np.float32, k.shape), want[3]), (runtime.download(dv, np.float32, v.shape), want[4])):
+        assert np.isnan(got[0, :4]).all() and (got[1] == 0).all()
+        error = np.linalg.norm(got[0, 4:] - w[0, 4:]) / np.linalg.norm(w[0, 4:])
+        assert error <= 8 * 150**0.5 * 2.0**-24, error
 
 
 @pytest.mark.parametrize("hd", [32, 64, 128])
