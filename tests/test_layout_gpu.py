@@ -302,6 +302,18 @@ def test_rows_staged_item_after_item_are_the_rows_of_one_item(t_q, hd, dtype):
             np.testing.assert_array_equal(got[name][at, 4].view(np.uint16), want[name][0, 0].view(np.uint16), err_msg=f"{name} of batch {at}")
 
 
+@pytest.mark.parametrize("t_q,t_k,hd", [(513, 200, 64), (1100, 65, 40)])
+def test_key_blocks_one_after_the_other_in_half_precision(t_q, t_k, hd):
+    """The deferred dK and dV as above, float16."""
+    batch, heads, dtype = 57, 3, np.dtype(np.float16)
+    arrays = _inputs(46, batch, heads, t_q, t_k, hd, dtype)
+    got = _run("bhtd", arrays, None, batch, heads, t_q, t_k, hd, False, dtype)
+    for at in (0, 28, 49, 56):
+        want = _run("bhtd", [x[at : at + 1] for x in arrays], None, 1, heads, t_q, t_k, hd, False, dtype)
+        for name in ("dk", "dv"):
+            np.testing.assert_array_equal(got[name][at].view(np.uint16), want[name][0].view(np.uint16), err_msg=f"{name} of batch {at}")
+
+
 def test_dense_layout_code_is_the_dense_entry_point():
     from limn_b200 import runtime
     from limn_b200._lib import check, lib

@@ -113,6 +113,64 @@ def test_every_kernel_stands_down_and_leaves_nothing_behind(shape):
     assert runtime.device_status() == 0
 
 
+# dK and dV deferred (more items than SMs, and fewer); rows staged and exchanged; own rows of few
+@pytest.mark.parametrize("shape", [(100, 600, 200, 64, 0), (20, 700, 100, 40, 0), (300, 250, 100, 64, 0), (160, 250, 130, 80, 0), (300, 40, 40, 128, 1)], ids=str)
+def test_deferred_results_and_row_stores_stand_down(shape):
+    test_every_kernel_stands_down_and_leaves_nothing_behind(shape)
+
+
+# bh, t_q, t_k, hd, causal: in roles with one item to a block, several, and operands fetched ahead; two blocks to an SM; one-tile items; above head dim
+# 64; rows that are not whole 16-byte pieces
+FLOAT32_STANDING_DOWN = [(20, 300, 300, 64, 1), (100, 500, 500, 32, 0), (400, 129, 257, 64, 0), (200, 64, 200, 64, 0), (120, 64, 64, 64, 1), (148, 20, 30, 32, 0),
+                         (160, 200, 200, 128, 1), (200, 150, 150, 30, 0)]
+
+
+@pytest.mark.parametrize("shape", FLOAT32_STANDING_DOWN, ids=str)
+def test_every_float32_kernel_stands_down_and_leaves_nothing_behind(shape):
+    from limn_b200 import runtime
+    from limn_b200._lib import DEVICE_TIMEOUT, check, lib
+
+    L = lib()
+    runtime.set_device(0)
+    assert runtime.device_status() == 0
+    bh, t_q, t_k, hd, causal = shape
+    rng = np.random.default_rng(sum(shape))
+    mask_host = (rng.random((bh, t_k)) > 0.1).astype(np.float32)
+    mask_host[:, 0] = 1
+    q, k, v, do, mask = (runtime.upload(x) for x in (*(rng.standard_normal((bh, t, hd)).astype(np.float32) for t in (t_q, t_k, t_k, t_q)), mask_host))
+    tail = (0, bh, t_q, t_k, hd, hd, causal, hd**-0.5, None)
+    rows, keys = 4 * bh * t_q, 4 * bh * t_k
+    sizes = {"out": rows * hd, "lse": rows, "delta": rows, "dq": rows * hd, "dk": keys * hd, "dv": keys * hd}
+    known = {}
+
+    def launch(poison):
+        """The three kernels and, the first time, the row dot, which waits for nothing; the backward ones on the first launch's L and delta."""
+        to = {name: runtime.empty(size, poison=poison) for name, size in sizes.items()}
+        given = known or to
+        check(L.limn_b200_sdpa_fwd(q.ptr, k.ptr, v.ptr, mask.ptr, to["out"].ptr, to["lse"].ptr, *tail), "sdpa")
+        if not known:
+            check(L.limn_b200_sdpa_delta(to["out"].ptr, do.ptr, to["delta"].ptr, 0, bh * t_q, hd, None), "row dot")
+        check(L.limn_b200_sdpa_bwd_q(q.ptr, k.ptr, v.ptr, do.ptr, given["lse"].ptr, given["delta"].ptr, mask.ptr, to["dq"].ptr, *tail), "dq")
+        check(L.limn_b200_sdpa_bwd_kv(q.ptr, k.ptr, v.ptr, do.ptr, given["lse"].ptr, given["delta"].ptr, mask.ptr, to["dk"].ptr, to["dv"].ptr, *tail), "dk, dv")
+        runtime.synchronize()
+        return to
+
+    def bytes_of(buffers):
+        return {name: runtime.download(buffers[name], np.uint8, (size,)) for name, size in sizes.items() if name != "delta"}
+
+    known.update(launch(0xFF))
+    good = bytes_of(known)
+    check(L.limn_b200_wait_probe(20000, None, None), "wait probe")
+    for name, seen in bytes_of(launch(0xAB)).items():
+        assert (seen == 0xAB).all(), f"{name} was written although an earlier kernel had given up"
+    word = ctypes.c_uint(0)
+    assert L.limn_b200_device_status(ctypes.byref(word)) == DEVICE_TIMEOUT and word.value == 0x57417E57
+    for _ in range(2):
+        for name, seen in bytes_of(launch(0xAB)).items():
+            np.testing.assert_array_equal(seen, good[name], err_msg=name)
+    assert runtime.device_status() == 0
+
+
 def test_finish_raises_like_a_failed_kernel_of_the_reference():
     """limn_b200.install() wraps the device's finish(): after a batch in which one of our Runners ran, a set
     status word surfaces as RuntimeError("cuda: ..."), where limn raises for a failed kernel of its own."""
