@@ -89,7 +89,7 @@ struct BwdLayout {
   static constexpr bool kTileStore = D == 64 && kKV;
   static constexpr int kStoreOff = kStreamBOff + kStagesB * kTileBytes;
   static constexpr int kWarpStage = kStore == RowStore::kStaged ? 2048 : 0;  // of each elementwise warp, for 32 columns of its rows
-  static constexpr int kStatOff = kStoreOff + (kTileStore ? (kKV ? 2 : 1) * kAtomBytes : 8 * kWarpStage);
+  static constexpr int kStatOff = kStoreOff + (kTileStore ? 2 * kAtomBytes : 8 * kWarpStage);
   static constexpr int kBarOff = kStatOff + (kKV ? 8 * 2 * 2 * 64 * 4 : 0);  // dK/dV pass, per warp [2 buffers][128 floats]: statistics of the streamed queries
   static constexpr int kBytes = kBarOff + 512 + 1024;
   static_assert(kBytes <= 227 * 1024, "shared memory per CTA");
@@ -769,15 +769,14 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
       ok = __all_sync(0xffffffffu, mbar_wait(bar(B::store_free), n_of & 1u, prm.status, 0x1350u));
       if (ok) {
-        // dK/dV pass: group 0 stages this key's dV row, group 1 its dK row, a block each; dQ pass: each group half
-        // of this query's dQ row, in the one block
-        const uint32_t block = base + L::kStoreOff + (kKV ? group * L::kAtomBytes : 0);
-        const float mul = (kKV && group == 0) ? 1.f : prm.scale;
+        // (the dK/dV pass) group 0 stages this key's dV row, group 1 its dK row, a block each
+        const uint32_t block = base + L::kStoreOff + group * L::kAtomBytes;
+        const float mul = group == 0 ? 1.f : prm.scale;
 #pragma unroll
-        for (int c = 0; c < (kKV ? 2 : 1); ++c) {
-          const int col = kKV ? 32 * c : group * 32;
+        for (int c = 0; c < 2; ++c) {
+          const int col = 32 * c;
           uint32_t acc[32];
-          tmem_ld32(tmem + lane_base + ((kKV && group == 1) ? L::kAcc1 : L::kAcc0) + col, acc);
+          tmem_ld32(tmem + lane_base + (group == 1 ? L::kAcc1 : L::kAcc0) + col, acc);
           tmem_ld_wait();
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
@@ -797,8 +796,8 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         fence_async_shared();
         mbar_arrive(bar(B::store_full));
         if (leader && mbar_wait(bar(B::store_full), n_of & 1u, prm.status, 0x1360u)) {
-          tma_store_4d(&map_out0, base + L::kStoreOff + (kKV ? L::kAtomBytes : 0), 0, of.own0, of.head, of.batch);  // dQ, or dK
-          if (kKV) tma_store_4d(&map_out1, base + L::kStoreOff, 0, of.own0, of.head, of.batch);                      // dV
+          tma_store_4d(&map_out0, base + L::kStoreOff + L::kAtomBytes, 0, of.own0, of.head, of.batch);  // dK
+          tma_store_4d(&map_out1, base + L::kStoreOff, 0, of.own0, of.head, of.batch);                  // dV
           tma_store_commit();
         }
       }
@@ -823,6 +822,9 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       } else {
         // each group writes half of its queries' dQ rows
+        const int row = of.own0 + r;
+        const bool in = row < prm.t_q;
+        const long long out_at = of.batch * prm.out_strides.batch + of.head * prm.out_strides.head + row * prm.out_strides.row;
         unsigned char* to = static_cast<unsigned char*>(prm.out0) + 2 * (of.batch * prm.out_strides.batch + of.head * prm.out_strides.head + top * prm.out_strides.row);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
@@ -832,7 +834,7 @@ sdpa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           tmem_ld32(tmem + lane_base + L::kAcc0 + col, acc);
           tmem_ld_wait();
           if constexpr (kStore == RowStore::kOwn) {
-            if (top + lane < prm.t_q) store_row32<kFp16>(to + 2 * (lane * prm.out_strides.row + col), acc, prm.scale, prm.width - col);
+            if (in) store_row32<kFp16>(static_cast<unsigned char*>(prm.out0) + 2 * (out_at + col), acc, prm.scale, prm.width - col);
           } else {
             store_rows32<kFp16, kStore>(to + 2 * col, 2 * prm.out_strides.row, top, prm.t_q, acc, prm.scale, prm.width - col, base + L::kStoreOff + warp * L::kWarpStage);
           }
@@ -1166,12 +1168,8 @@ int launch_bwd_s(const Problem& p) {
   if (int rc = make_tile_map(&map_do, p.dout, kFp16, batch, heads, p.t_q, p.hd_v, kTile, operand_strides(p, kOpDout, heads, p.t_q, p.hd_v))) return rc;
   CUtensorMap map_out0 = map_q, map_out1 = map_q;  // only read by the kernels that store tiles
   if (L::kTileStore) {
-    if (kKV) {
-      if (int rc = make_tile_map(&map_out0, p.dk, kFp16, batch, heads, p.t_k, p.hd, kTile, operand_strides(p, kOpDk, heads, p.t_k, p.hd))) return rc;
-      if (int rc = make_tile_map(&map_out1, p.dv, kFp16, batch, heads, p.t_k, p.hd_v, kTile, operand_strides(p, kOpDv, heads, p.t_k, p.hd_v))) return rc;
-    } else {
-      if (int rc = make_tile_map(&map_out0, p.dq, kFp16, batch, heads, p.t_q, p.hd, kTile, operand_strides(p, kOpDq, heads, p.t_q, p.hd))) return rc;
-    }
+    if (int rc = make_tile_map(&map_out0, p.dk, kFp16, batch, heads, p.t_k, p.hd, kTile, operand_strides(p, kOpDk, heads, p.t_k, p.hd))) return rc;
+    if (int rc = make_tile_map(&map_out1, p.dv, kFp16, batch, heads, p.t_k, p.hd_v, kTile, operand_strides(p, kOpDv, heads, p.t_k, p.hd_v))) return rc;
   }
   BwdParams prm;
   prm.mask = static_cast<const unsigned short*>(p.mask);
@@ -1274,7 +1272,8 @@ int launch_bwd_m(const Problem& p) {
   if (p.causal) return fp16 ? launch_bwd<D, true, true, kKV, kMask>(p) : launch_bwd<D, true, false, kKV, kMask>(p);
   // The dK/dV pass at head dim 64 without masks, from five query tiles on: results deferred (the tensor cores have the next item's first
   // scores done meanwhile, and the warps do not wait for an item's last products). Measured, time deferred / not: 256 problems of 512 1.00,
-  // 640 0.98, 768 0.97, 1024 0.96, 2048 0.94; 16 of 1024 0.95; 64 of 100 x 1500 1.03. Not under a mask (1.06, it spills), nor a causal one (1.03
+  // 640 0.98, 768 0.97, 1024 0.96, 2048 0.94; 16 of 1024 0.95; 64 of 100 x 1500 1.03. (They all spill, the deferred one 132 bytes stored and 120
+  // loaded again, the plain one 164 and 64, the masked one 132 and 48.) Not under a mask (1.06), nor a causal one (1.03
   // to 1.05), nor in the dQ pass (1.02 to 1.05).
   if constexpr (D == 64 && kKV && !kMask) {
     if (p.t_q > 4 * kTile) return fp16 ? launch_bwd<D, false, true, kKV, kMask, true>(p) : launch_bwd<D, false, false, kKV, kMask, true>(p);

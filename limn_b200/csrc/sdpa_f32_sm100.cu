@@ -15,11 +15,12 @@
 // in the forward, a block's warps have roles: row warps (a row to two or four threads: softmax or dS, the split of their operand, the
 // totals), splitting warps (the streamed tiles, from global memory to three pieces in shared memory) and one that issues the MMAs;
 // they meet at barriers only, a block takes up to 32 items one after the other, and a tile's scores, the products of the one before
-// and the split of the ones behind go on at the same time. Measured on B200 (forward / dQ / dK and dV, us, causal; before the roles; in
-// brackets the CUDA-core kernels): 256 x 256 keys x 64: 31 / 45 / 50, 39 / 61 / 73 (121 / 166 / 219); 6 x 8192 x 32: 225 / 231 / 290, 291 / 290 /
-// 389 (1333 / 1777 / 2402); 64 x 1024 x 128: 121 / 225 / 275, 178 / 227 / 293 (813 / 1117 / 1714); 64 x 32 x 64: 6.9 / 8.8 / 8.5, 7.3 / 8.4 /
-// 9.2 (10.8 / 12.4 / 14.4). Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.4e-7 for 6.1e-7, dQ 3.2e-7
-// for 7.6e-7 in the 2-norm), and so is L (256 x 256 x 64: 2.9e-8 for 3.5e-8; rounding it once is 2.6e-8).
+// and the split of the ones behind go on at the same time. Items of few tiles, where that has nothing to work on, go to kernels without
+// roles (f32_fwd_pair_kernel, f32_bwd_wide_kernel). Measured on B200 (forward / dQ without the row dot / dK and dV, us, causal; before the
+// roles; in brackets the CUDA-core kernels): 256 x 256 keys x 64: 31 / 36 / 49, 39 / 54 / 73 (120 / 170 / 217); 6 x 8192 x 32: 225 / 232 / 293, 291 /
+// 288 / 388 (1 456 / 1 743 / 2 345); 64 x 1024 x 128: 120 / 214 / 269, 175 / 227 / 293 (796 / 1 105 / 1 805); 64 x 32 x 64: 6.3 / 7.0 / 8.4, 7.4 / 7.0 / 9.1
+// (8.7 / 10.4 / 13.0); the row dot beside dQ 8, 5, 20 and 1.1. Against float64, O, dQ, dK and dV are closer than theirs (8192 keys x 32: O 1.4e-7 for 6.1e-7, dQ
+// 3.2e-7 for 7.6e-7 in the 2-norm), and so is L (256 x 256 x 64: 2.9e-8 for 3.5e-8; rounding it once is 2.6e-8).
 //
 // A block owns 128 rows at a time (query rows in the forward and the dQ pass, key rows in the dK/dV pass), one row to each
 // tensor-memory lane, and streams the other side in tiles of 64 rows. Operands are loaded
@@ -30,9 +31,10 @@
 // A non-finite operand would turn up as NaN in places where float32 arithmetic gives an infinity or even a finite
 // number (inf - inf in the split, inf * 0 between pieces), and one below about 2^-110 would lose its last bits. The split
 // notices both, and a block that met one computes its rows again on the CUDA cores, with the code of the tiled kernels
-// there. The backward above head dim 64 leaves its loop when it meets one; the others, whose warps run apart, go on to their end first and
-// then do the items again (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 470 / 1 980 / 2 570, the tiled kernels
-// alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500).
+// there. The kernels without roles leave their loops when they meet one; the others, whose warps run apart, go on to their end first and
+// then do the items again (a step whose every block does, forward / dQ / dK and dV, us: 6 x 8192 x 32 1 446 / 1 970 / 2 560, the tiled kernels
+// alone 1 340 / 1 790 / 2 410; one row to a warp took 57 900 / 52 000 / 59 500). Going through an item's barriers without its work, once it is
+// known to be done again, took 1 341 us in the forward, and 3 to 10 % more in calls with ordinary operands: more code in the loops.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -300,15 +302,13 @@ __device__ __noinline__ void rows_again(const Params& g, long long b, int first,
   }
 }
 
-// ---- block set-up and teardown shared by the kernels ----
-// False: an earlier kernel on this device gave up on a wait, take no work.
-// Barriers whose bit is set in `by_warps` expect `warps` arrivals, the others one.
+// ---- block set-up (of the kernels without roles) and teardown ----
+// False: an earlier kernel on this device gave up on a wait, take no work. Every barrier expects one arrival.
 template <int kCols, int kBars>
-__device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t* abort_flag, uint64_t* bars, uint32_t& tmem,
-                                       uint32_t by_warps = 0u, uint32_t warps = 1u) {
+__device__ __forceinline__ bool set_up(const Params& g, uint32_t* slot, uint32_t* abort_flag, uint64_t* bars, uint32_t& tmem) {
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < kBars; ++i) mbar_init(smem_addr(bars + i), (by_warps >> i) & 1u ? warps : 1u);
+    for (int i = 0; i < kBars; ++i) mbar_init(smem_addr(bars + i), 1);
     mbar_init_fence();
   }
   grid_dependency_wait();
@@ -871,7 +871,7 @@ __global__ void __launch_bounds__(Roles<Fwd<HD>::kGroups>::kThreads, 1) f32_fwd_
                                                                     ring(kGo, 0), ring(kReady, 0), base + L::kTile0, base + L::kTile1, g.status, ok, load_rows, post_rows);
   } else if (any) {
     // ================= row warps =================
-    // A warp that gave up on a wait waits for nothing any more but goes through its tiles like the others: the four warps that share
+    // A warp that gave up on a wait waits for nothing any more but goes through its tiles like the others: the two warps that share
     // rows meet at a barrier in each.
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     auto meet = [&] { named_barrier_sync(1 + quarter, 32 * G); };
@@ -1237,9 +1237,11 @@ struct Bwd {
 };
 
 // kGroups threads to a row (and the split of the warps that goes with it): the same bits either way. Two are faster in dQ up to head dim 32
-// where a block has one item (2 x 128 x 32 7.7 us for 8.3, 64 x 128 8.6 for 8.9, 2 x 8192 152 for 156), as the splitting warps have it ready
+// where a block has one item of several tiles (2 x 128 x 32 7.7 us for 8.3, 64 x 128 8.6 for 8.9, 2 x 8192 152 for 156), as the splitting warps have it ready
 // sooner; four in the long run (6 x 8192 x 32 causal 233 for 239) and at head dim 64 (64 x 128 x 64 11.5 for 12.1, 16 x 600 x 64 23.4 for
-// 26.8, 256 x 512 x 64 143 for 150; two spill).
+// 26.8, 256 x 512 x 64 143 for 150). All of them spill: with four threads to a row and 96 registers 76 to 152 bytes are stored and 56 to 140
+// loaded again a thread, with two and 128 up to 36; of the forwards those above head dim 64, 184 and 216. That is not in the tile loops: 16
+// causal problems of 2048 x 64 execute 25 000 local loads and 13 000 stores in dQ (of 31.8 M instructions), 9 600 and 12 800 in dK and dV (43.9 M).
 template <int HD, bool kKV, bool kWide, int kGroups>
 __global__ void __launch_bounds__(Roles<kGroups>::kThreads, 1) f32_bwd_kernel(const __grid_constant__ Params g) {
   using L = Bwd<HD, kKV>;

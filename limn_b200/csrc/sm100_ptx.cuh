@@ -184,7 +184,7 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lead
 }
 
 // Instruction descriptor for tcgen05.mma.kind::f16: fp32 accumulate, A and B both bf16 or
-
+// both fp16. a_mn / b_mn say the operand is MN-major (0 = K-major), a_minus that A is taken with its sign turned round.
 __host__ __device__ constexpr uint32_t mma_idesc(int m, int n, bool fp16, bool a_mn, bool b_mn, bool a_minus = false) {
   return (1u << 4)                      // D format: f32
          | ((fp16 ? 0u : 1u) << 7)      // A format: f16 = 0, bf16 = 1
