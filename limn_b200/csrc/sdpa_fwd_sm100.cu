@@ -828,7 +828,7 @@ int launch_fwd_s(const Problem& p) {
 // Token-major with 12 heads: 128 columns 204 of 64 9.6 / 10.2, of 128 11.1 / 9.9, of 160 17.1 / 15.6; 64 columns 204 of 64 8.2 / 8.4, of 128 8.7 / 8.0, of 200
 //   13.8 / 13.2; under a key mask 192 of 256 14.4 / 12.9. With 5 heads 700 of 100 under a mask 21.7 / 22.9, at 128 columns 24.6 / 26.3.
 // Two groups that share the keys, dense: 128 columns 148 of 128 x 512 10.4 / 10.7; 64 columns 200 of 64 x 600 15.4 / 15.5, of 128 x 600 15.8 / 15.7, 700 of 100 x 1500
-//   71.8 / 70.4. Under a causal mask at head dim 64 own rows (256 of 256 13.7 / 14.0).
+//   71.8 / 70.4, 16 of 40 x 2463 19.3 / 19.0, masked of 100 x 300 9.0 / 8.8. Under a causal mask at head dim 64 own rows (256 of 256 13.7 / 14.0).
 template <int D, bool kMask, bool kShared>
 RowStore rows_leave(const Problem& p) {
   constexpr RowStore kLong = D == 128 ? RowStore::kExchanged : RowStore::kStaged;
@@ -837,7 +837,7 @@ RowStore rows_leave(const Problem& p) {
   bool pays;
   if (scattered_rows(operand_strides(p, kOpOut, heads, p.t_q, p.hd_v).row, p.hd_v)) pays = size >= 112 * D;
   else if (D == 128) pays = !kShared && p.t_q > kTileRows && (p.hd_v > 80 ? 3 : 8) * missing < p.t_q;
-  else if (kShared) pays = !kMask && p.hd_v > 48 && p.t_q >= 96;
+  else if (kShared) pays = p.hd_v > 48 && (p.t_q >= 96 || p.t_k >= 1024);
   else pays = !kMask && p.hd_v > 48 && size >= 64 * kTileRows && 8 * missing < p.t_q;
   return pays ? kLong : RowStore::kOwn;
 }
